@@ -24,6 +24,7 @@
 #include <string>
 #include <vector>
 
+#include "links.cuh"
 #include "pipeline.cuh"
 
 using namespace ph;
@@ -346,14 +347,15 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   for (int c = 0; c <= K; ++c) res->off[0][c] = c < K ? segs[c].vbase : N;
 
   // per-cloud host arrays read back in bulk: [0, K] edge offsets, then K counts
-  PinnedLease hb(sizeof(int64_t) * (6 * (size_t)K + 8) + 256);
+  PinnedLease hb(sizeof(int64_t) * (7 * (size_t)K + 8) + 256);
   if (!hb.p.host) return give_up(fail(PH_ERR_CUDA, "ph_rips_persistence_batch: pinned host buffer unavailable"));
   int64_t* hcnt = hb.as<int64_t>();            // 16 words of cnt
   int64_t* hoff = hcnt + 16;                  // K + 1 offsets
   int64_t* hper = hoff + (K + 1);             // K per-cloud counts
   int64_t* hoff2 = hper + K;                  // K + 1 more offsets
   int64_t* htot = hoff2 + (K + 1);            // K exact totals of the clouds that may be over the limit
-  uint8_t* hwant = reinterpret_cast<uint8_t*>(htot + K);  // K flags: which clouds those are
+  int64_t* hrows = htot + K;                  // K counts of H1 rows
+  uint8_t* hwant = reinterpret_cast<uint8_t*>(hrows + K);  // K flags: the clouds counted exactly
 
   if (dim_all == 0) {
     Part parts[2] = {{cnt, hcnt, 16 * sizeof(int64_t)}, {e_off, hoff, sizeof(int64_t) * (K + 1)}};
@@ -367,13 +369,33 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   }
 
   // ---- 4. triangles: per-cloud counts, the limit per cloud ----------------------------------------
+  // counted an edge, with those that can be pivots (links.cu), which are the
+  // rows of the H1 reduction; all of them are stored only for H2
+  LinkGraph graph{adj_ptr, adj_idx, adj_rank, N, nullptr, nullptr, vcloud, dsegs};
+  LinkCounts links{};
+  links.tri_cnt = A.take<i32>(E);
+  links.row_cnt = A.take<i32>(E);
+  links.len_cnt = A.take<i32>(E);
+  links.cursor = A.take<i32>(E);
   int64_t* tri_off = A.take<int64_t>(E + 1);
-  int64_t* tcof_off = A.take<int64_t>(E + 1);
+  links.tri_off = tri_off;
+  links.row_off = A.take<int64_t>(E + 1);
+  links.off = A.take<i32>(E + 1);
+  links.stash.cap = link_stash_cap(E, N, 2 * E);  // 1.0 to 1.6 rows an edge are usual
+  links.stash.totals = reinterpret_cast<LinkTotals*>(cnt + 8);
+  // rank tables of the dense clouds, as far as 2 GiB go
+  i64 table_cap = 0;
+  for (int c = 0; c < K; ++c)
+    if (max_dim[c] >= 1 && n[c] <= LINK_TABLE_MAX_N) table_cap += n[c] * n[c];
+  table_cap = std::min<i64>(table_cap, i64(1) << 29);
+  i32* table = table_cap ? A.take<i32>(table_cap) : nullptr;
+  int64_t* table_off = table ? A.take<int64_t>(K) : nullptr;
   int64_t* per = A.take<int64_t>(K);
+  int64_t* per_rows = A.take<int64_t>(K);
   uint8_t* cflag = A.take<uint8_t>(2 * K);  // per-cloud flags: [0, K) H1 kept, [K, 2K) H2 kept
   uint8_t* eflag = A.take<uint8_t>(E);
-  const size_t tc_b = ph_triangles_count_workspace_bytes(E);
-  void* tc_ws = A.bytes(tc_b);
+  const size_t lk_b = link_count_workspace_bytes(E);
+  void* lk_ws = A.bytes(lk_b);
   // clouds that may be over max_triangles are counted exactly first (the
   // bitmap total: far cheaper than the per-edge pass on a dense cloud), and
   // the per-edge pass skips those over it
@@ -393,48 +415,76 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
     ph::launch_pdl(k_tri_keep, dim3(grid_for(K)), dim3(256), 0, s, (const uint8_t*)want,
                    (const unsigned long long*)ttot, K, (i64)max_triangles, tkeep);
   }
-  PH_TRY(triangles_count_masked(si, sj, E, adj_ptr, adj_idx, adj_rank, tri_off, tcof_off, tc_ws, tc_b,
-                                pre ? tkeep : nullptr, pre ? vcloud : nullptr, s));
-  PH_TRY(ph_max_count(tcof_off, E, cnt + 8, s));  // the longest cofacet row (before any clearing: a bound)
-  count_launch();
-  ph::launch_pdl(k_seg_diff, dim3(grid_for(K)), dim3(256), 0, s, (const int64_t*)tri_off, (const int64_t*)e_off, K,
-                 per);
   {
-    Part parts[5] = {{cnt, hcnt, 16 * sizeof(int64_t)},
+    int rc = PH_OK;
+    if (table) {
+      rc = link_table_offsets(dsegs, e_off, K, table_cap, table_off, s);
+      graph.table = table;
+      graph.table_off = table_off;
+      if (rc == PH_OK) rc = link_table(graph, table, s);
+    }
+    if (rc != PH_OK) return give_up(rc);
+  }
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    links.stash.rows = A.take<LinkRow>(links.stash.cap);
+    if (A.failed) return alloc_fail();
+    if (E) {
+      const int rc = link_count(si, sj, E, graph, pre ? tkeep : nullptr, mask, links, lk_ws, lk_b, s);
+      if (rc != PH_OK) return give_up(rc);
+    } else {
+      ph::zero_async(tri_off, sizeof(int64_t), s, links.row_off, sizeof(int64_t));
+    }
+    count_launch();
+    ph::launch_pdl(k_seg_diff, dim3(grid_for(K)), dim3(256), 0, s, (const int64_t*)tri_off, (const int64_t*)e_off, K,
+                   per);
+    count_launch();
+    ph::launch_pdl(k_seg_diff, dim3(grid_for(K)), dim3(256), 0, s, (const int64_t*)links.row_off,
+                   (const int64_t*)e_off, K, per_rows);
+    Part parts[6] = {{cnt, hcnt, 16 * sizeof(int64_t)},
                      {e_off, hoff, sizeof(int64_t) * (K + 1)},
                      {per, hper, sizeof(int64_t) * K},
+                     {per_rows, hrows, sizeof(int64_t) * K},
                      {ttot, htot, sizeof(int64_t) * K},
                      {want, hwant, (size_t)K}};
-    if (readback_parts(parts, pre ? 5 : 3, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
+    if (readback_parts(parts, pre ? 6 : 4, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
+    if (hcnt[10] <= links.stash.cap) break;
+    links.stash.cap = link_stash_cap(E, N, hcnt[9]);
+    ph::zero_async(cnt + 8, sizeof(LinkTotals), s);
   }
+  if (hcnt[10] > links.stash.cap)
+    return give_up(fail(PH_ERR_CUDA, "ph_rips_persistence_batch: the triangle rows outgrew their buffer twice"));
   // a cloud counted exactly and over the limit counted nothing in the per-edge pass
   if (pre)
     for (int c = 0; c < K; ++c)
       if (hwant[c] && htot[c] > max_triangles) hper[c] = htot[c];
   if ((int)(hcnt[1] >> 32) != 0) return give_up(fail((int)(hcnt[1] >> 32), "ph_boruvka_mst failed"));
   std::vector<uint8_t> keep1(K, 0), keep2(K, 0);
-  i64 T = 0, span1 = 0;
+  // T: triangles of the clouds within the limit; T2: of those stored for H2;
+  // R1: H1 rows (those of every cloud counted: the columns of the clouds left
+  // out are skipped, not their rows)
+  i64 T = 0, T2 = 0, R1 = 0, span1 = 0;
   bool any_cleared = false, any_h2 = false;
   for (int c = 0; c < K; ++c) {
     res->stat[0][c] = hoff[c + 1] - hoff[c];
     res->stat[1][c] = hper[c];
-    if (max_dim[c] < 1) {
-      any_cleared = any_cleared || hper[c] > 0;
-      continue;
-    }
+    R1 += hrows[c];
+    if (max_dim[c] < 1) continue;
     if (hper[c] > max_triangles) {
       res->status[c] = PH_ERR_LIMIT;
       res->message[c] = tri_limit_msg(hper[c], max_triangles);
-      any_cleared = any_cleared || hper[c] > 0;
       continue;
     }
     keep1[c] = 1;
     keep2[c] = max_dim[c] == 2;
     any_h2 = any_h2 || keep2[c];
     T += hper[c];
-    span1 = std::max<i64>(span1, hper[c]);
+    if (keep2[c]) T2 += hper[c];
+    span1 = std::max<i64>(span1, hrows[c]);
   }
-  if (E + 3 * T >= (int64_t(1) << 31) || (K > 1 && max_batch_simplices > 0 && T > max_batch_simplices)) {
+  for (int c = 0; c < K; ++c) any_cleared = any_cleared || (any_h2 && !keep2[c] && hper[c] > 0);
+  if (E + 3 * R1 >= (int64_t(1) << 31) || (K == 1 && E + 3 * T >= (int64_t(1) << 31)) ||
+      E + 3 * T2 >= (int64_t(1) << 31) ||
+      (K > 1 && max_batch_simplices > 0 && R1 + T2 > max_batch_simplices)) {
     // the union's ranks do not fit int32: the caller splits the batch (the
     // per-cloud counts in the result tell it how)
     A.release_to(res->scratch);
@@ -447,45 +497,36 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
     record_error(cudaGetLastError());
     return give_up(PH_ERR_CUDA);
   }
-  if (any_cleared && E) {  // no triangles for clouds over the limit or asking for H0 only
+  if (any_cleared && E) {  // triangles are stored for the clouds kept for H2 only
     count_launch();
     ph::launch_pdl(k_edge_flags, dim3(grid_for(E)), dim3(256), 0, s, (const i32*)si, E, (const i32*)vcloud,
-                   (const uint8_t*)cflag, 0, (const uint8_t*)nullptr, eflag);
+                   (const uint8_t*)(cflag + K), 0, (const uint8_t*)nullptr, eflag);
     PH_TRY(mask_offsets(A, s, tri_off, E, eflag));
-    PH_TRY(mask_offsets(A, s, tcof_off, E, eflag));  // their cofacet rows go too
   }
-  i32* tri_m = A.take<i32>(T);
-  i32* tri_w = A.take<i32>(T);
-  i32* tri_fa = A.take<i32>(T);
-  i32* tri_fb = A.take<i32>(T);
-  i32* off1 = A.take<i32>(E + 1);
-  i32* data1 = A.take<i32>(3 * T);
-  i32* cmf1 = A.take<i32>(T);
+  i32 *tri_m = nullptr, *tri_w = nullptr, *tri_fa = nullptr, *tri_fb = nullptr, *row_tri = nullptr;
+  if (any_h2) {
+    tri_m = A.take<i32>(T2);
+    tri_w = A.take<i32>(T2);
+    tri_fa = A.take<i32>(T2);
+    tri_fb = A.take<i32>(T2);
+    row_tri = A.take<i32>(R1);
+  }
+  i32* row_m = A.take<i32>(R1);
+  i32* data1 = A.take<i32>(3 * R1);
+  i32* cmf1 = A.take<i32>(R1);
   uint8_t* skip1 = A.take<uint8_t>(E);
   int64_t* row_off1 = A.take<int64_t>(K + 1);
   int64_t* nrows1 = A.take<int64_t>(1);
-  const size_t cc_b = ph_cofacet_csr_workspace_bytes(T, 3), r1_b = ph_batch_persistence_rows_workspace_bytes(E);
-  void* cc_ws = A.bytes(cc_b);
+  const size_t r1_b = ph_batch_persistence_rows_workspace_bytes(E);
   void* r1_ws = A.bytes(r1_b);
   if (A.failed || cudaMallocAsync((void**)&res->rows[1], sizeof(float) * 2 * std::max<i64>(E, 1), s) != cudaSuccess)
     return alloc_fail();
-  const i64 max_row = hcnt[8];
-  if (T) {
-    int rc = ph_triangles_emit(si, sj, E, adj_ptr, adj_idx, adj_rank, tri_off, tri_m, tri_w, tri_fa, tri_fb, s);
-    // rows scattered and sorted in shared memory when every row fits, else the radix form
-    if (rc == PH_OK && max_row <= ph_cofacet_rows3_max_row()) {
-      const size_t r3_b = ph_cofacet_rows3_workspace_bytes(E);
-      void* r3_ws = A.bytes(r3_b);
-      if (A.failed) return alloc_fail();
-      rc = ph_cofacet_rows3(tri_m, tri_fa, tri_fb, T, E, (i32)E, tcof_off, (int32_t)max_row, off1, data1, st + 5,
-                            r3_ws, r3_b, s);
-    } else if (rc == PH_OK) {
-      rc = ph_cofacet_csr(nullptr, tri_m, tri_fa, tri_fb, 3, T, E, (i32)E, off1, data1, cc_ws, cc_b, s);
-    }
-    if (rc == PH_OK) rc = ph_cof_max_face(nullptr, tri_m, tri_fa, tri_fb, 3, T, 0, mask, cmf1, s);
+  if (E) {
+    int rc = PH_OK;
+    if (T2)
+      rc = ph_triangles_emit(si, sj, E, adj_ptr, adj_idx, adj_rank, tri_off, tri_m, tri_w, tri_fa, tri_fb, s);
+    if (rc == PH_OK) rc = link_rows(R1, mask, links, (i32)E, row_m, row_tri, cmf1, data1, st + 5, s);
     if (rc != PH_OK) return give_up(rc);
-  } else {
-    ph::zero_async(off1, sizeof(i32) * (E + 1), s);
   }
   // H1 columns: the non-forest edges of the clouds kept for H1
   if (E) {
@@ -495,7 +536,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   }
 
   // ---- 5. H1 reduction and rows per cloud --------------------------------------------------------
-  i64 pool1 = pool_capacity(3 * T, E);
+  i64 pool1 = pool_capacity(3 * R1, E);
   RedOut r1{};
   int64_t* tet_off = nullptr;
   uint8_t* en2 = nullptr;
@@ -509,9 +550,9 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
     if (A.failed) return alloc_fail();
   }
   for (int attempt = 0;; ++attempt) {
-    int rc = reduce_only(A, s, off1, data1, E, 0, T, (i32)E, span1, skip1, cmf1, pool1, st + 2, r1);
+    int rc = reduce_only(A, s, links.off, data1, E, 0, R1, (i32)E, span1, skip1, cmf1, pool1, st + 2, r1);
     if (rc == PH_OK)
-      rc = ph_batch_persistence_rows(r1.state, r1.piv, E, (i32)E, filt, nullptr, tri_m, e_off, K, res->rows[1],
+      rc = ph_batch_persistence_rows(r1.state, r1.piv, E, (i32)E, filt, nullptr, row_m, e_off, K, res->rows[1],
                                      row_off1, nrows1, r1_ws, r1_b, s);
     if (rc != PH_OK) return give_up(rc);
     if (any_h2 && attempt == 0) {
@@ -532,7 +573,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
                      {per, hper, any_h2 ? sizeof(int64_t) * K : 0}};
     if (readback_parts(parts, 3, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
     const int st_red = (int)(hcnt[2] & 0xffffffff);
-    if ((int)(hcnt[3] >> 32) != 0) return give_up(fail((int)(hcnt[3] >> 32), "ph_cofacet_rows3 failed"));
+    if ((int)(hcnt[3] >> 32) != 0) return give_up(fail((int)(hcnt[3] >> 32), "the triangle rows of the two passes differ"));
     if (st_red == PH_OK) break;
     if (st_red != PH_ERR_POOL || attempt >= 3 || pool1 >= POOL_MAX)
       return give_up(fail(st_red, "ph_reduce (H1) failed"));
@@ -562,8 +603,8 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
     Q += hper[c];
     span2 = std::max<i64>(span2, hper[c]);
   }
-  if (E + T + Q >= (int64_t(1) << 31) || 4 * Q >= (int64_t(1) << 31) ||
-      (K > 1 && max_batch_simplices > 0 && T + Q > max_batch_simplices)) {
+  if (E + T2 + Q >= (int64_t(1) << 31) || 4 * Q >= (int64_t(1) << 31) ||
+      (K > 1 && max_batch_simplices > 0 && T2 + Q > max_batch_simplices)) {
     A.release_to(res->scratch);
     *out = res;
     return fail(PH_ERR_CAPACITY, "ph_rips_persistence_batch: the batch's simplices exceed the rank range or the batch budget; split it");
@@ -581,49 +622,42 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   }
   i32* tet_m = A.take<i32>(Q);
   i32* tet_faces = A.take<i32>(4 * Q);
-  uint8_t* skip2 = A.take<uint8_t>(T);
+  uint8_t* skip2 = A.take<uint8_t>(T2);
   i32* cmf2 = A.take<i32>(Q);
-  i32* off2 = A.take<i32>(T + 1);
+  i32* off2 = A.take<i32>(T2 + 1);
   i32* data2 = A.take<i32>(4 * Q);
   int64_t* t_off = A.take<int64_t>(K + 1);
   int64_t* row_off2 = A.take<int64_t>(K + 1);
   int64_t* nrows2 = A.take<int64_t>(1);
-  // the H2 cofacet rows without a global sort when every row fits the per-row
-  // sorts: a triangle's tetrahedra number at most its cloud's points less 3
-  i64 max_n = 0;
-  for (int c = 0; c < K; ++c) max_n = std::max<i64>(max_n, segs[c].n);
-  const bool rows4 = max_n - 3 <= COF_ROWS_MAX;
-  const size_t c2_b = rows4 ? cofacet_rows_aos_workspace_bytes(T) : ph_cofacet_csr_workspace_bytes(Q, 4),
-               r2_b = ph_batch_persistence_rows_workspace_bytes(T);
+  const size_t c2_b = cofacet_lists_workspace_bytes(T2),
+               r2_b = ph_batch_persistence_rows_workspace_bytes(T2);
   void* c2_ws = A.bytes(c2_b);
   void* r2_ws = A.bytes(r2_b);
-  if (A.failed || cudaMallocAsync((void**)&res->rows[2], sizeof(float) * 2 * std::max<i64>(T, 1), s) != cudaSuccess)
+  if (A.failed || cudaMallocAsync((void**)&res->rows[2], sizeof(float) * 2 * std::max<i64>(T2, 1), s) != cudaSuccess)
     return alloc_fail();
   {
     int rc = PH_OK;
     if (Q)
       rc = ph_tets_emit(si, sj, E, tri_off, tri_w, tri_fa, tri_fb, adj_ptr, adj_idx, adj_rank, en2, tet_off, tet_m,
                         tet_faces, st + 3, s);
-    if (rc == PH_OK) rc = ph_mark_pivots(r1.state, r1.piv, E, (i32)E, skip2, T, s);
+    if (rc == PH_OK) rc = mark_pivots_mapped(r1.state, r1.piv, E, (i32)E, row_tri, skip2, T2, s);
     // triangles of the clouds without H2 are not columns
-    if (rc == PH_OK && T) rc = ph_or_gather_mask(skip2, en2, tri_m, T, 1, s);
+    if (rc == PH_OK && T2) rc = ph_or_gather_mask(skip2, en2, tri_m, T2, 1, s);
     if (rc == PH_OK && Q) rc = ph_cof_max_face(tet_faces, nullptr, nullptr, nullptr, 4, Q, (i32)E, skip2, cmf2, s);
     if (rc == PH_OK && Q)
-      rc = rows4 ? cofacet_rows_aos(tet_faces, 4, Q, T, (i32)(E + T), off2, data2, st + 3, c2_ws, c2_b, s)
-                 : ph_cofacet_csr(tet_faces, nullptr, nullptr, nullptr, 4, Q, T, (i32)(E + T), off2, data2, c2_ws,
-                                  c2_b, s);
+      rc = cofacet_lists(tet_faces, 4, Q, T2, (i32)(E + T2), off2, data2, st + 3, c2_ws, c2_b, s);
     if (rc != PH_OK) return give_up(rc);
-    if (!Q) ph::zero_async(off2, sizeof(i32) * (T + 1), s);
+    if (!Q) ph::zero_async(off2, sizeof(i32) * (T2 + 1), s);
     count_launch();
     ph::launch_pdl(k_gather_off, dim3(grid_for(K + 1)), dim3(256), 0, s, (const int64_t*)tri_off,
                    (const int64_t*)e_off, K, t_off);
   }
-  i64 pool2 = pool_capacity(4 * Q, T);
+  i64 pool2 = pool_capacity(4 * Q, T2);
   RedOut r2{};
   for (int attempt = 0;; ++attempt) {
-    int rc = reduce_only(A, s, off2, data2, T, (i32)E, Q, (i32)(E + T), span2, skip2, cmf2, pool2, st + 4, r2);
+    int rc = reduce_only(A, s, off2, data2, T2, (i32)E, Q, (i32)(E + T2), span2, skip2, cmf2, pool2, st + 4, r2);
     if (rc == PH_OK)
-      rc = ph_batch_persistence_rows(r2.state, r2.piv, T, (i32)(E + T), filt, tri_m, tet_m, t_off, K, res->rows[2],
+      rc = ph_batch_persistence_rows(r2.state, r2.piv, T2, (i32)(E + T2), filt, tri_m, tet_m, t_off, K, res->rows[2],
                                      row_off2, nrows2, r2_ws, r2_b, s);
     if (rc != PH_OK) return give_up(rc);
     Part parts[2] = {{cnt, hcnt, 16 * sizeof(int64_t)}, {row_off2, hoff2, sizeof(int64_t) * (K + 1)}};

@@ -41,16 +41,19 @@ void count_launch();
 // The reducer's step cap per column (ph_set_reduce_limits; 2^24 by default)
 // and the cap on a native call's first reduction pool (0: none).
 long long reduce_max_steps();
-// the cofacet CSR of simplices given as k faces each, without a global sort (simplices.cu)
-constexpr int COF_ROWS_MAX = 8192;  // longest row the per-row sorts take
-size_t cofacet_rows_aos_workspace_bytes(int64_t n_faces);
-int cofacet_rows_aos(const int32_t* faos, int32_t k, int64_t S, int64_t n_faces, int32_t row_base, int32_t* cof_off,
-                     int32_t* cof_data, int* d_status, void* workspace, size_t workspace_bytes, cudaStream_t s);
-// the triangle count pass with an optional per-cloud mask (simplices.cu)
-int triangles_count_masked(const int32_t* edge_i, const int32_t* edge_j, int64_t E, const int32_t* adj_ptr,
-                           const int32_t* adj_idx, const int32_t* adj_rank, int64_t* tri_off, int64_t* cof_off,
-                           void* workspace, size_t workspace_bytes, const uint8_t* keep, const int32_t* vcloud,
-                           cudaStream_t s);
+// the cofacet lists, in any order, of simplices given as k faces each (simplices.cu)
+size_t cofacet_lists_workspace_bytes(int64_t n_faces);
+int cofacet_lists(const int32_t* faos, int32_t k, int64_t S, int64_t n_faces, int32_t row_base, int32_t* cof_off,
+                  int32_t* cof_data, int* d_status, void* workspace, size_t workspace_bytes, cudaStream_t s);
+// ph_reduce of cofacet lists in any order (reduce.cu)
+int reduce_lists(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32_t col_base, int64_t R,
+                 int32_t row_base, int64_t span, const uint8_t* skip, const int32_t* row_cmf, int32_t* col_state,
+                 int32_t* col_piv, int32_t* pool, int64_t pool_cap, int64_t* d_info, int* d_status, void* workspace,
+                 size_t workspace_bytes, cudaStream_t s);
+// flag[row] = 1 for the pivots of the paired columns; map (may be null) takes
+// a reduction's row to the index flagged, negative for none (reduce.cu)
+int mark_pivots_mapped(const int32_t* col_state, const int32_t* col_piv, int64_t K, int32_t row_base,
+                       const int32_t* map, uint8_t* row_flag, int64_t R, cudaStream_t s);
 long long reduce_first_pool_limit();
 
 // Raises a kernel's dynamic shared memory limit to the device's opt-in

@@ -25,6 +25,7 @@
 #include <string>
 #include <vector>
 
+#include "links.cuh"
 #include "pipeline.cuh"
 
 using namespace ph;
@@ -229,7 +230,7 @@ int reduce_only(Arena& A, cudaStream_t s, const i32* off, const i32* data, i64 K
   const size_t rb = ph_reduce_workspace_bytes(K, R, span);
   void* rws = A.bytes(rb);
   if (A.failed) return fail(PH_ERR_CUDA, "rips_persistence: device allocation failed");
-  return ph_reduce(off, data, K, col_base, R, row_base, span, skip, cmf, o.state, o.piv, pool, pool_cap, o.info,
+  return reduce_lists(off, data, K, col_base, R, row_base, span, skip, cmf, o.state, o.piv, pool, pool_cap, o.info,
                    status, rws, rb, s);
 }
 
@@ -245,7 +246,7 @@ __global__ void k_single_seg(ph_cloud_seg* seg, int64_t* blk_off, int64_t n, int
                              int64_t nblocks, int64_t* cnt) {
   ph::pdl_wait();
   ph::pdl_trigger();
-  for (int k = 0; k < 8; ++k) cnt[k] = 0;
+  for (int k = 0; k < 16; ++k) cnt[k] = 0;
   ph_cloud_seg s;
   s.pt_off = 0;
   s.vbase = 0;
@@ -311,8 +312,8 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   int64_t* blk = A.take<int64_t>(2);
   // cnt[0]: edge count; statuses as int32 words from cnt + 1: st[0] edges,
   // st[1] forest, st[2] H1 reduction, st[3] tetrahedra, st[4] H2 reduction;
-  // cnt[5] triangle total, cnt[6] its work counter
-  int64_t* cnt = A.take<int64_t>(8);
+  // cnt[5] triangle total, cnt[6] its work counter, cnt[8..10] LinkTotals
+  int64_t* cnt = A.take<int64_t>(16);
   if (A.failed) return alloc_fail();
   int* st = reinterpret_cast<int*>(cnt + 1);
   count_launch();
@@ -441,21 +442,46 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   }
 
   // ---- 4. triangles (triangle_kernel.py:288; reduce_h1_gpu.py:65-100) -------------------------
-  int64_t* tri_off = A.take<int64_t>(E + 1);
-  int64_t* tcof_off = A.take<int64_t>(E + 1);
-  const size_t tc_b = ph_triangles_count_workspace_bytes(E);
-  void* tc_ws = A.bytes(tc_b);
+  // Counted an edge, with those that can be pivots (links.cu), which are the
+  // rows of the H1 reduction; all of them are stored only for H2.
+  LinkGraph graph{adj_ptr, adj_idx, adj_rank, n, nullptr, nullptr, nullptr, nullptr};
+  LinkCounts links{};
+  links.tri_cnt = A.take<i32>(E);
+  links.row_cnt = A.take<i32>(E);
+  links.len_cnt = A.take<i32>(E);
+  links.cursor = A.take<i32>(E);
+  links.tri_off = max_dim == 2 ? A.take<int64_t>(E + 1) : nullptr;
+  links.row_off = A.take<int64_t>(E + 1);
+  links.off = A.take<i32>(E + 1);
+  links.stash.cap = link_stash_cap(E, n, 2 * E);  // 1.0 to 1.6 rows an edge are usual
+  links.stash.totals = reinterpret_cast<LinkTotals*>(cnt + 8);
+  const size_t lk_b = link_count_workspace_bytes(E);
+  void* lk_ws = A.bytes(lk_b);
+  i32* table = link_table_pays(n, E) ? A.take<i32>(n * n) : nullptr;
   if (A.failed) return alloc_fail();
   {
-    int rc = ph_triangles_count(si, sj, E, adj_ptr, adj_idx, adj_rank, tri_off, tcof_off, tc_ws, tc_b, s);
-    if (rc == PH_OK) rc = ph_max_count(tcof_off, E, cnt + 7, s);  // the longest cofacet row
-    if (rc != PH_OK) return give_up(rc);
-    const int64_t* src[3] = {tri_off + E, cnt + 1, cnt + 7};
-    if (readback(src, 3, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
+    int rc = PH_OK;
+    if (table) {
+      graph.table = table;
+      rc = link_table(graph, table, s);
+    }
+    for (int attempt = 0; attempt < 2; ++attempt) {
+      links.stash.rows = A.take<LinkRow>(links.stash.cap);
+      if (A.failed) return alloc_fail();
+      if (rc == PH_OK && E) rc = link_count(si, sj, E, graph, nullptr, mask, links, lk_ws, lk_b, s);
+      if (rc != PH_OK) return give_up(rc);
+      const int64_t* src[4] = {cnt + 8, cnt + 1, cnt + 9, cnt + 10};
+      if (readback(src, 4, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
+      if (H[3] <= links.stash.cap || H[0] > max_triangles) break;
+      links.stash.cap = link_stash_cap(E, n, H[2]);
+      ph::zero_async(cnt + 8, sizeof(LinkTotals), s);
+    }
   }
   const i64 T = H[0];
-  const i64 max_row = H[2];
+  const i64 R1 = H[2];  // rows of the H1 reduction
   if ((int)(H[1] >> 32) != 0) return give_up(fail((int)(H[1] >> 32), "ph_boruvka_mst failed"));
+  if (H[3] > links.stash.cap && T <= max_triangles)
+    return give_up(fail(PH_ERR_CAPACITY, "ph_rips_persistence: the triangle rows outgrew their buffer twice"));
   if (T_total >= 0 && T != T_total) {
     char m[160];
     snprintf(m, sizeof m, "triangle counts disagree: %lld per edge, %lld in total", (long long)T,
@@ -475,18 +501,21 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
     return give_up(fail(PH_ERR_LIMIT, m));
   }
   res->stats[1] = T;
-  i32* tri_m = A.take<i32>(T);
-  i32* tri_w = A.take<i32>(T);
-  i32* tri_fa = A.take<i32>(T);
-  i32* tri_fb = A.take<i32>(T);
-  i32* off1 = A.take<i32>(E + 1);
-  i32* data1 = A.take<i32>(3 * T);
-  i32* cmf1 = A.take<i32>(T);
-  const size_t cc_b = ph_cofacet_csr_workspace_bytes(T, 3);
-  void* cc_ws = A.bytes(cc_b);
+  const int64_t* tri_off = links.tri_off;
+  i32 *tri_m = nullptr, *tri_w = nullptr, *tri_fa = nullptr, *tri_fb = nullptr, *row_tri = nullptr;
+  if (max_dim == 2) {
+    tri_m = A.take<i32>(T);
+    tri_w = A.take<i32>(T);
+    tri_fa = A.take<i32>(T);
+    tri_fb = A.take<i32>(T);
+    row_tri = A.take<i32>(R1);
+  }
+  i32* row_m = A.take<i32>(R1);
+  i32* data1 = A.take<i32>(3 * R1);
+  i32* cmf1 = A.take<i32>(R1);
   if (A.failed || cudaMallocAsync((void**)&res->rows[1], sizeof(float) * 2 * std::max<i64>(E, 1), s) != cudaSuccess)
     return alloc_fail();
-  if (T) {
+  if (T && max_dim == 2) {
     const int rc = ph_triangles_emit(si, sj, E, adj_ptr, adj_idx, adj_rank, tri_off, tri_m, tri_w, tri_fa, tri_fb, s);
     if (rc != PH_OK) return give_up(rc);
   }
@@ -520,37 +549,23 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
     const int rc = tets_limit();
     if (rc != PH_OK) return give_up(rc);
   }
-  if (T) {
-    // the rows' lengths are the cofacet counts: scattered and sorted per row
-    // when every row fits the shared-memory sort, else the radix form
-    int rc;
-    if (max_row <= ph_cofacet_rows3_max_row()) {
-      const size_t r3_b = ph_cofacet_rows3_workspace_bytes(E);
-      void* r3_ws = A.bytes(r3_b);
-      if (A.failed) return alloc_fail();
-      rc = ph_cofacet_rows3(tri_m, tri_fa, tri_fb, T, E, (i32)E, tcof_off, (int32_t)max_row, off1, data1, st + 3,
-                            r3_ws, r3_b, s);
-    } else {
-      rc = ph_cofacet_csr(nullptr, tri_m, tri_fa, tri_fb, 3, T, E, (i32)E, off1, data1, cc_ws, cc_b, s);
-    }
-    if (rc == PH_OK) rc = ph_cof_max_face(nullptr, tri_m, tri_fa, tri_fb, 3, T, 0, mask, cmf1, s);
+  if (E) {
+    const int rc = link_rows(R1, mask, links, (i32)E, row_m, row_tri, cmf1, data1, st + 3, s);
     if (rc != PH_OK) return give_up(rc);
-  } else {
-    ph::zero_async(off1, sizeof(i32) * (E + 1), s);
   }
 
   // ---- 5. H1 reduction and rows (reduce_h1_gpu.py:159-223, 574-604) --------------------------
-  i64 pool1 = pool_capacity(3 * T, E);
+  i64 pool1 = pool_capacity(3 * R1, E);
   RedOut r1{};
   for (int attempt = 0;; ++attempt) {
-    int rc = reduce_rows(A, s, off1, data1, E, 0, T, (i32)E, mask, cmf1, filt, nullptr, tri_m, pool1, st + 2,
+    int rc = reduce_rows(A, s, links.off, data1, E, 0, R1, (i32)E, mask, cmf1, filt, nullptr, row_m, pool1, st + 2,
                          res->rows[1], r1);
     if (rc != PH_OK) return give_up(rc);
     const int64_t* src[4] = {cnt + 2, r1.nrows, r1.info + 1, max_dim == 2 ? tet_off + E : r1.nrows};
     if (readback(src, 4, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
     const int st_red = (int)(H[0] & 0xffffffff);
     // the word beside it: the cofacet rows' status (the tetrahedra's only later)
-    if ((int)(H[0] >> 32) != 0) return give_up(fail((int)(H[0] >> 32), "ph_cofacet_rows3 failed"));
+    if ((int)(H[0] >> 32) != 0) return give_up(fail((int)(H[0] >> 32), "the triangle rows of the two passes differ"));
     if (st_red == PH_OK) break;
     if (st_red != PH_ERR_POOL || attempt >= 3 || pool1 >= POOL_MAX)
       return give_up(fail(st_red, "ph_reduce (H1) failed"));
@@ -583,10 +598,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   i32* cmf2 = A.take<i32>(Q);
   i32* off2 = A.take<i32>(T + 1);
   i32* data2 = A.take<i32>(4 * Q);
-  // the H2 cofacet rows without a global sort when every row fits the per-row
-  // sorts: a triangle's tetrahedra number at most n - 3
-  const bool rows4 = n - 3 <= COF_ROWS_MAX;
-  const size_t c2_b = rows4 ? cofacet_rows_aos_workspace_bytes(T) : ph_cofacet_csr_workspace_bytes(Q, 4);
+  const size_t c2_b = cofacet_lists_workspace_bytes(T);
   void* c2_ws = A.bytes(c2_b);
   if (A.failed || cudaMallocAsync((void**)&res->rows[2], sizeof(float) * 2 * std::max<i64>(T, 1), s) != cudaSuccess)
     return alloc_fail();
@@ -595,12 +607,10 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
     if (Q)
       rc = ph_tets_emit(si, sj, E, tri_off, tri_w, tri_fa, tri_fb, adj_ptr, adj_idx, adj_rank, nullptr, tet_off,
                         tet_m, tet_faces, st + 3, s);
-    if (rc == PH_OK) rc = ph_mark_pivots(r1.state, r1.piv, E, (i32)E, skip2, T, s);
+    if (rc == PH_OK) rc = mark_pivots_mapped(r1.state, r1.piv, E, (i32)E, row_tri, skip2, T, s);
     if (rc == PH_OK && Q) rc = ph_cof_max_face(tet_faces, nullptr, nullptr, nullptr, 4, Q, (i32)E, skip2, cmf2, s);
     if (rc == PH_OK && Q)
-      rc = rows4 ? cofacet_rows_aos(tet_faces, 4, Q, T, (i32)(E + T), off2, data2, st + 3, c2_ws, c2_b, s)
-                 : ph_cofacet_csr(tet_faces, nullptr, nullptr, nullptr, 4, Q, T, (i32)(E + T), off2, data2, c2_ws,
-                                  c2_b, s);
+      rc = cofacet_lists(tet_faces, 4, Q, T, (i32)(E + T), off2, data2, st + 3, c2_ws, c2_b, s);
     if (rc != PH_OK) return give_up(rc);
     if (!Q) ph::zero_async(off2, sizeof(i32) * (T + 1), s);
   }

@@ -145,6 +145,178 @@ __global__ void k_classify(const i32* __restrict__ off, const i32* __restrict__ 
   }
 }
 
+// ---- cofacet lists in any order ------------------------------------------------------
+// k_ready does k_classify's work on lists that are not sorted yet, so that
+// they need no pass of their own: column c's record lies at off[c] + c of the
+// pool (no allocation). A lane sorts a list of up to 8 entries in registers
+// (most lists: the rows number 1-1.6 an edge), a warp one of up to 32 across
+// its lanes and of up to RY_LIST in its shared memory, the block longer ones
+// in all of it, and where they are (in the pool) beyond that.
+constexpr int RY_NT = 256;
+constexpr int RY_WARPS = RY_NT / 32;
+constexpr int RY_LIST = 1024;
+
+__device__ __forceinline__ void order(i32& x, i32& y) {
+  const i32 lo = min(x, y);
+  y = max(x, y);
+  x = lo;
+}
+
+// Batcher's network for eight values
+__device__ __forceinline__ void sort8(i32 (&v)[8]) {
+  order(v[0], v[1]), order(v[2], v[3]), order(v[4], v[5]), order(v[6], v[7]);
+  order(v[0], v[2]), order(v[1], v[3]), order(v[4], v[6]), order(v[5], v[7]);
+  order(v[1], v[2]), order(v[5], v[6]);
+  order(v[0], v[4]), order(v[1], v[5]), order(v[2], v[6]), order(v[3], v[7]);
+  order(v[2], v[4]), order(v[3], v[5]);
+  order(v[1], v[2]), order(v[3], v[4]), order(v[5], v[6]);
+}
+
+// ascending bitonic sort of n values by a group of threads: every comparison
+// ascending (each merge starts with a mirrored step), so that the missing
+// values past n, larger than all others, never move
+template <typename Sync>
+__device__ __forceinline__ void bitonic_group(i32* v, int n, int tid, int nthreads, Sync sync) {
+  int len2 = 2;
+  while (len2 < n) len2 <<= 1;
+  for (int size = 2; size <= len2; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      const bool mirror = stride == (size >> 1);
+      for (int i = tid; i < (len2 >> 1); i += nthreads) {
+        const int lo = 2 * i - (i & (stride - 1));
+        const int hi = mirror ? (lo & ~(size - 1)) + size - 1 - (lo & (size - 1)) : lo + stride;
+        if (hi >= n) continue;
+        const i32 x = v[lo], y = v[hi];
+        if (x > y) {
+          v[lo] = y;
+          v[hi] = x;
+        }
+      }
+      sync();
+    }
+  }
+}
+
+__global__ void __launch_bounds__(RY_NT) k_ready(const i32* __restrict__ off, const i32* __restrict__ cof, i64 K,
+                                                i32 col_base, i32 row_base, const uint8_t* __restrict__ skip,
+                                                const i32* __restrict__ cmf, i32* __restrict__ state,
+                                                i32* __restrict__ piv, u64* __restrict__ owner,
+                                                u64* __restrict__ rec, i32* __restrict__ pool, i64 pool_cap,
+                                                RedCtl* ctl, int* status) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  __shared__ i32 buf[RY_WARPS * RY_LIST];
+  __shared__ i32 longs[RY_NT];
+  __shared__ int nlong;
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const i64 top = (i64)off[K] + K;  // records of all columns
+  const bool fits = top <= pool_cap;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctl->pool_top = (unsigned long long)top;
+    if (!fits) {
+      set_status(status, PH_ERR_POOL);
+      ctl->abort = 1;
+    }
+  }
+  // the column is classified once its first entry is known
+  auto settle = [&](i64 c, i32 t, u64 at) {
+    if (cmf[t - row_base] == col_base + (i32)c) {
+      state[c] = 1;
+      piv[c] = t;
+      owner[t - row_base] = owner_word((i32)c, at);
+      return false;
+    }
+    state[c] = 2;
+    rec[c] = at;
+    return true;
+  };
+  const i64 stride = (i64)gridDim.x * RY_NT;
+  int nres = 0;
+  for (i64 b0 = (i64)blockIdx.x * RY_NT; b0 < K; b0 += stride) {
+    if (threadIdx.x == 0) nlong = 0;
+    __syncthreads();
+    const i64 c0 = b0 + (threadIdx.x & ~31), c = c0 + lane;
+    i32 o = 0;
+    int len = 0;
+    if (c < K) {
+      o = off[c];
+      len = off[c + 1] - o;
+      const bool skipped = skip && skip[c];
+      if (skipped || len == 0 || !fits) {
+        state[c] = skipped ? 0 : 3;
+        piv[c] = -1;
+        len = 0;
+      }
+    }
+    if (len > 0 && len <= 8) {
+      i32 v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = k < len ? cof[o + k] : INT_MAX;
+      sort8(v);
+      i32* r = pool + (i64)o + c;
+      r[0] = len;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k < len) r[1 + k] = v[k];
+      nres += settle(c, v[0], (u64)((i64)o + c));
+    }
+    if (len > RY_LIST) longs[atomicAdd(&nlong, 1)] = (i32)threadIdx.x;
+    u32 todo = __ballot_sync(FULL, len > 8 && len <= RY_LIST);
+    while (todo) {
+      const int l = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const i64 cc = c0 + l;
+      const i32 oo = __shfl_sync(FULL, o, l);
+      const int n = __shfl_sync(FULL, len, l);
+      i32* r = pool + (i64)oo + cc;
+      i32 first;
+      if (n <= 32) {
+        i32 x = lane < n ? cof[oo + lane] : INT_MAX;
+        for (int size = 2; size <= 32; size <<= 1)
+          for (int st = size >> 1; st > 0; st >>= 1) {
+            const i32 y = __shfl_xor_sync(FULL, x, st);
+            x = ((lane & st) == 0) == ((lane & size) == 0) ? min(x, y) : max(x, y);
+          }
+        if (lane < n) r[1 + lane] = x;
+        first = x;
+      } else {
+        i32* w = buf + wl * RY_LIST;
+        for (int i = lane; i < n; i += 32) w[i] = cof[oo + i];
+        __syncwarp();
+        bitonic_group(w, n, lane, 32, []() { __syncwarp(); });
+        for (int i = lane; i < n; i += 32) r[1 + i] = w[i];
+        first = w[0];
+        __syncwarp();
+      }
+      if (lane == 0) {
+        r[0] = n;
+        nres += settle(cc, first, (u64)((i64)oo + cc));
+      }
+    }
+    __syncthreads();  // the list of long columns is complete, and the warps are done with their buffers
+    const int nl = nlong;
+    for (int q = 0; q < nl; ++q) {
+      const i64 cc = b0 + longs[q];
+      const i32 oo = off[cc];
+      const int n = off[cc + 1] - oo;
+      i32* r = pool + (i64)oo + cc;
+      i32* w = n <= RY_WARPS * RY_LIST ? buf : r + 1;
+      for (int i = threadIdx.x; i < n; i += RY_NT) w[i] = cof[oo + i];
+      __syncthreads();
+      bitonic_group(w, n, threadIdx.x, RY_NT, []() { __syncthreads(); });
+      if (w == buf)
+        for (int i = threadIdx.x; i < n; i += RY_NT) r[1 + i] = w[i];
+      if (threadIdx.x == 0) {
+        r[0] = n;
+        nres += settle(cc, w[0], (u64)((i64)oo + cc));
+      }
+      __syncthreads();
+    }
+  }
+  nres = __reduce_add_sync(FULL, nres);
+  if (lane == 0 && nres) atomicAdd(&ctl->nres, nres);
+}
+
 // Loads that must see data written by other SMs during this kernel go to L2.
 template <bool G>
 __device__ __forceinline__ i32 ld(const i32* p) {
@@ -1115,11 +1287,14 @@ __global__ void k_finish_rows(const u64* __restrict__ owner, i64 R, i32 row_base
 }
 
 __global__ void k_mark_pivots(const i32* __restrict__ state, const i32* __restrict__ piv, i64 K, i32 row_base,
-                              uint8_t* __restrict__ flag) {
+                              const i32* __restrict__ map, uint8_t* __restrict__ flag) {
   ph::pdl_wait();
   ph::pdl_trigger();
   for (i64 c = (i64)blockIdx.x * blockDim.x + threadIdx.x; c < K; c += (i64)gridDim.x * blockDim.x)
-    if (state[c] == 1 || state[c] == 2) flag[piv[c] - row_base] = 1;
+    if (state[c] == 1 || state[c] == 2) {
+      const i32 r = map ? map[piv[c] - row_base] : piv[c] - row_base;
+      if (r >= 0) flag[r] = 1;
+    }
 }
 
 inline int grid_for(i64 n, int nt = 256) {
@@ -1172,12 +1347,13 @@ extern "C" size_t ph_reduce_workspace_bytes(int64_t K, int64_t R, int64_t span) 
          (dw ? Carve::need((size_t)dw * 4 * reduce_blocks(K) * RD_WARPS) : 0);
 }
 
-extern "C" int ph_reduce(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32_t col_base,
-                         int64_t R, int32_t row_base, int64_t span, const uint8_t* skip, const int32_t* row_cmf,
-                         int32_t* col_state, int32_t* col_piv, int32_t* pool, int64_t pool_cap,
-                         int64_t* d_info, int* d_status, void* workspace, size_t workspace_bytes,
-                         void* stream) {
-  cudaStream_t s = (cudaStream_t)stream;
+namespace {
+// SORTED: the cofacet rows are ascending (ph_reduce), else lists in any order
+template <bool SORTED>
+int reduce_run(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32_t col_base, int64_t R,
+               int32_t row_base, int64_t span, const uint8_t* skip, const int32_t* row_cmf, int32_t* col_state,
+               int32_t* col_piv, int32_t* pool, int64_t pool_cap, int64_t* d_info, int* d_status, void* workspace,
+               size_t workspace_bytes, cudaStream_t s) {
   if (K < 0 || R < 0 || pool_cap < 0) return PH_ERR_ARG;
   if (K >= (int64_t(1) << 31) || R >= (int64_t(1) << 31) || pool_cap >= (int64_t(1) << OW_SHIFT))
     return PH_ERR_OVERFLOW;
@@ -1193,8 +1369,12 @@ extern "C" int ph_reduce(const int32_t* cof_off, const int32_t* cof_data, int64_
   if (!owner || !rec || !ctl) return PH_ERR_ARG;
   ph::zero_async(owner, sizeof(u64) * std::max<i64>(R, 1), s, ctl, sizeof(RedCtl));
   ph::count_launch();
-  ph::launch_pdl(k_classify, dim3(grid_for(K)), dim3(256), 0, s, cof_off, cof_data, K, col_base, row_base, skip, row_cmf, col_state,
-                                         col_piv, owner, rec, pool, pool_cap, ctl, d_status);
+  if (SORTED)
+    ph::launch_pdl(k_classify, dim3(grid_for(K)), dim3(256), 0, s, cof_off, cof_data, K, col_base, row_base, skip,
+                   row_cmf, col_state, col_piv, owner, rec, pool, pool_cap, ctl, d_status);
+  else
+    ph::launch_pdl(k_ready, dim3(grid_for(K, RY_NT)), dim3(RY_NT), 0, s, cof_off, cof_data, K, col_base, row_base,
+                   skip, row_cmf, col_state, col_piv, owner, rec, pool, pool_cap, ctl, d_status);
   if (ph::allow_dynamic_smem((const void*)k_reduce) != cudaSuccess) {
     PH_CHECK_LAUNCH();
     return PH_ERR_CUDA;
@@ -1220,17 +1400,40 @@ extern "C" int ph_reduce(const int32_t* cof_off, const int32_t* cof_data, int64_
   return PH_OK;
 }
 
-extern "C" int ph_mark_pivots(const int32_t* col_state, const int32_t* col_piv, int64_t K, int32_t row_base,
-                              uint8_t* row_flag, int64_t R, void* stream) {
-  cudaStream_t s = (cudaStream_t)stream;
+}  // namespace
+
+extern "C" int ph_reduce(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32_t col_base,
+                         int64_t R, int32_t row_base, int64_t span, const uint8_t* skip, const int32_t* row_cmf,
+                         int32_t* col_state, int32_t* col_piv, int32_t* pool, int64_t pool_cap,
+                         int64_t* d_info, int* d_status, void* workspace, size_t workspace_bytes,
+                         void* stream) {
+  return reduce_run<true>(cof_off, cof_data, K, col_base, R, row_base, span, skip, row_cmf, col_state, col_piv, pool,
+                          pool_cap, d_info, d_status, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
+int ph::reduce_lists(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32_t col_base, int64_t R,
+                     int32_t row_base, int64_t span, const uint8_t* skip, const int32_t* row_cmf, int32_t* col_state,
+                     int32_t* col_piv, int32_t* pool, int64_t pool_cap, int64_t* d_info, int* d_status,
+                     void* workspace, size_t workspace_bytes, cudaStream_t s) {
+  return reduce_run<false>(cof_off, cof_data, K, col_base, R, row_base, span, skip, row_cmf, col_state, col_piv, pool,
+                           pool_cap, d_info, d_status, workspace, workspace_bytes, s);
+}
+
+int ph::mark_pivots_mapped(const int32_t* col_state, const int32_t* col_piv, int64_t K, int32_t row_base,
+                           const int32_t* map, uint8_t* row_flag, int64_t R, cudaStream_t s) {
   if (K < 0 || R < 0) return PH_ERR_ARG;
   if (R > 0) ph::zero_async(row_flag, (size_t)R, s);
   if (K > 0) {
     ph::count_launch();
-    ph::launch_pdl(k_mark_pivots, dim3(grid_for(K)), dim3(256), 0, s, col_state, col_piv, K, row_base, row_flag);
+    ph::launch_pdl(k_mark_pivots, dim3(grid_for(K)), dim3(256), 0, s, col_state, col_piv, K, row_base, map, row_flag);
   }
   PH_CHECK_LAUNCH();
   return PH_OK;
+}
+
+extern "C" int ph_mark_pivots(const int32_t* col_state, const int32_t* col_piv, int64_t K, int32_t row_base,
+                              uint8_t* row_flag, int64_t R, void* stream) {
+  return mark_pivots_mapped(col_state, col_piv, K, row_base, nullptr, row_flag, R, (cudaStream_t)stream);
 }
 
 extern "C" size_t ph_persistence_rows_workspace_bytes(int64_t K) { return rows_nosort_workspace_bytes(K); }

@@ -53,8 +53,7 @@ __global__ void __launch_bounds__(SX_NT) k_triangles(const i32* __restrict__ ei,
                                                     i32* __restrict__ tri_cnt, i32* __restrict__ cof_cnt,
                                                     const i64* __restrict__ tri_off, i32* __restrict__ tm,
                                                     i32* __restrict__ tw, i32* __restrict__ tfa,
-                                                    i32* __restrict__ tfb, const uint8_t* __restrict__ keep,
-                                                    const i32* __restrict__ vcloud) {
+                                                    i32* __restrict__ tfb) {
   ph::pdl_wait();
   ph::pdl_trigger();
   __shared__ i32 st_idx[SX_WARPS][SX_STAGE];
@@ -66,14 +65,6 @@ __global__ void __launch_bounds__(SX_NT) k_triangles(const i32* __restrict__ ei,
   for (i64 m = warp; m < E; m += nwarps) {
     __syncwarp();  // the previous edge's searches of the staged row are done
     const i32 a = ei[m], b = ej[m];
-    // a batch's count pass: the edges of a cloud already over its limit count nothing
-    if (keep && !keep[vcloud[a]]) {
-      if (!EMIT && lane == 0) {
-        tri_cnt[m] = 0;
-        cof_cnt[m] = 0;
-      }
-      continue;
-    }
     int sa = aptr[a], ea = aptr[a + 1], sb = aptr[b], eb = aptr[b + 1];
     // walk the shorter row, search the longer
     const bool a_short = (ea - sa) <= (eb - sb);
@@ -383,7 +374,6 @@ __global__ void k_cmf(const i32* __restrict__ faos, const i32* __restrict__ f0, 
 // radix sort of all 3T entries by face, whose passes dominate dense batches.
 constexpr int RS_WARP_MAX = 1024;        // entries a warp sorts in shared memory
 constexpr int RS_BIG = 8192;             // entries a block sorts in shared memory
-static_assert(RS_BIG == ph::COF_ROWS_MAX, "the callers' row bound is the block sort's size");
 constexpr int RS_NT = 256;
 
 __global__ void k_off_i64_to_i32(const i64* __restrict__ in, i64 n, i32* __restrict__ out) {
@@ -546,16 +536,7 @@ extern "C" int ph_triangles_count(const int32_t* edge_i, const int32_t* edge_j, 
                                   const int32_t* adj_ptr, const int32_t* adj_idx, const int32_t* adj_rank,
                                   int64_t* tri_off, int64_t* cof_off, void* workspace,
                                   size_t workspace_bytes, void* stream) {
-  return ph::triangles_count_masked(edge_i, edge_j, E, adj_ptr, adj_idx, adj_rank, tri_off, cof_off, workspace,
-                                    workspace_bytes, nullptr, nullptr, (cudaStream_t)stream);
-}
-
-// The count pass with an optional per-cloud mask (keep[vcloud[i]] == 0: the
-// edge counts nothing), for a batch whose over-limit clouds are known first.
-int ph::triangles_count_masked(const int32_t* edge_i, const int32_t* edge_j, int64_t E, const int32_t* adj_ptr,
-                               const int32_t* adj_idx, const int32_t* adj_rank, int64_t* tri_off, int64_t* cof_off,
-                               void* workspace, size_t workspace_bytes, const uint8_t* keep, const int32_t* vcloud,
-                               cudaStream_t s) {
+  cudaStream_t s = (cudaStream_t)stream;
   if (E < 0) return PH_ERR_ARG;
   Carve c(workspace, workspace_bytes);
   i32* tc = c.take<i32>(E + 1);
@@ -565,7 +546,7 @@ int ph::triangles_count_masked(const int32_t* edge_i, const int32_t* edge_j, int
   if (E > 0) {
     ph::count_launch();
     ph::launch_pdl(k_triangles<false>, dim3(warp_grid(E)), dim3(SX_NT), 0, s, edge_i, edge_j, E, adj_ptr, adj_idx, adj_rank, tc, cc,
-                                                      nullptr, nullptr, nullptr, nullptr, nullptr, keep, vcloud);
+                                                      nullptr, nullptr, nullptr, nullptr, nullptr);
   }
   PH_TRY(scan_exclusive_i32_i64(tc, tri_off, E, sws, scan_workspace_bytes(E), s));
   PH_TRY(scan_exclusive_i32_i64(cc, cof_off, E, sws, scan_workspace_bytes(E), s));
@@ -687,8 +668,7 @@ extern "C" int ph_triangles_emit(const int32_t* edge_i, const int32_t* edge_j, i
   if (E <= 0) return E < 0 ? PH_ERR_ARG : PH_OK;
   ph::count_launch();
   ph::launch_pdl(k_triangles<true>, dim3(warp_grid(E)), dim3(SX_NT), 0, (cudaStream_t)stream, 
-      edge_i, edge_j, E, adj_ptr, adj_idx, adj_rank, nullptr, nullptr, tri_off, tri_m, tri_w, tri_fa, tri_fb,
-      (const uint8_t*)nullptr, (const i32*)nullptr);
+      edge_i, edge_j, E, adj_ptr, adj_idx, adj_rank, nullptr, nullptr, tri_off, tri_m, tri_w, tri_fa, tri_fb);
   PH_CHECK_LAUNCH();
   return PH_OK;
 }
@@ -846,55 +826,41 @@ extern "C" int ph_cof_max_face(const int32_t* faces_aos, const int32_t* f0, cons
 }
 
 namespace ph {
-size_t cofacet_rows_aos_workspace_bytes(int64_t n_faces) {
+size_t cofacet_lists_workspace_bytes(int64_t n_faces) {
   const i64 nf = std::max<i64>(n_faces, 1);
-  return Carve::need(sizeof(i32) * (size_t)(nf + 1)) + 2 * Carve::need(sizeof(i32) * (size_t)nf) +
-         Carve::need(sizeof(int)) + Carve::need(scan_workspace_bytes(nf));
+  return Carve::need(sizeof(i32) * (size_t)(nf + 1)) + Carve::need(sizeof(i32) * (size_t)nf) +
+         Carve::need(scan_workspace_bytes(nf));
 }
 
-// The cofacet CSR of S simplices with k faces each (AoS, the tetrahedra's four
-// triangles) without a sort of the S k entries: rows counted, offsets scanned,
-// ranks scattered into their rows, each row sorted in shared memory. Rows must
-// hold at most RS_BIG entries (a triangle's tetrahedra number at most the
-// cloud's points less three: the caller checks that bound). The rows equal
-// ph_cofacet_csr's.
-int cofacet_rows_aos(const int32_t* faos, int32_t k, int64_t S, int64_t n_faces, int32_t row_base, int32_t* cof_off,
-                     int32_t* cof_data, int* d_status, void* workspace, size_t workspace_bytes, cudaStream_t s) {
+// The cofacet lists of S simplices with k faces each (AoS, the tetrahedra's
+// four triangles): lengths counted, offsets scanned, ranks scattered into
+// their lists in any order (reduce_lists orders them).
+int cofacet_lists(const int32_t* faos, int32_t k, int64_t S, int64_t n_faces, int32_t row_base, int32_t* cof_off,
+                  int32_t* cof_data, int* d_status, void* workspace, size_t workspace_bytes, cudaStream_t s) {
   const i64 H = S * k;
   if (k < 1 || S < 0 || n_faces < 0 || H >= (int64_t(1) << 31)) return PH_ERR_ARG;
   Carve c(workspace, workspace_bytes);
   const i64 nf = std::max<i64>(n_faces, 1);
   i32* cnt = c.take<i32>(nf + 1);
   i32* cursor = c.take<i32>(nf);
-  i32* big = c.take<i32>(nf);
-  int* nbig = c.take<int>(1);
   void* sws = c.take<char>((i64)scan_workspace_bytes(nf));
-  if (!cnt || !cursor || !big || !nbig || !sws) return PH_ERR_ARG;
+  if (!cnt || !cursor || !sws) return PH_ERR_ARG;
   if (n_faces == 0) {
     ph::zero_async(cof_off, sizeof(i32), s);
     PH_CHECK_LAUNCH();
     return PH_OK;
   }
   ph::zero_async(cnt, sizeof(i32) * (size_t)n_faces, s, cursor, sizeof(i32) * (size_t)n_faces);
-  ph::zero_async(nbig, sizeof(int), s);
   if (H > 0) {
     ph::count_launch();
     ph::launch_pdl(k_cof_count_aos, dim3(grid_for(H)), dim3(256), 0, s, faos, H, cnt);
   }
   PH_TRY(scan_exclusive_i32_i32(cnt, cof_off, n_faces, sws, scan_workspace_bytes(nf), s));
-  if (H == 0) {
-    PH_CHECK_LAUNCH();
-    return PH_OK;
+  if (H > 0) {
+    ph::count_launch();
+    ph::launch_pdl(k_cof_scatter_aos, dim3(grid_for(H)), dim3(256), 0, s, faos, H, (int)k, row_base,
+                   (const i32*)cof_off, cursor, cof_data, d_status);
   }
-  ph::count_launch();
-  ph::launch_pdl(k_cof_scatter_aos, dim3(grid_for(H)), dim3(256), 0, s, faos, H, (int)k, row_base,
-                 (const i32*)cof_off, cursor, cof_data, d_status);
-  const int gw = (int)std::max<i64>(1, std::min<i64>((n_faces + RS_NT / 32 - 1) / (RS_NT / 32), 148 * 16));
-  ph::count_launch();
-  ph::launch_pdl(k_cof_sort_rows, dim3(gw), dim3(RS_NT), 0, s, (const i32*)cof_off, n_faces, cof_data, big, nbig);
-  ph::count_launch();
-  ph::launch_pdl(k_cof_sort_big, dim3(148 * 2), dim3(RS_NT), 0, s, (const i32*)cof_off, cof_data, (const i32*)big,
-                 (const int*)nbig, d_status);
   PH_CHECK_LAUNCH();
   return PH_OK;
 }
