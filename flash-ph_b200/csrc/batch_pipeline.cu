@@ -538,40 +538,57 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   // ---- 5. H1 reduction and rows per cloud --------------------------------------------------------
   i64 pool1 = pool_capacity(3 * R1, E);
   RedOut r1{};
-  int64_t* tet_off = nullptr;
   uint8_t* en2 = nullptr;
+  const bool tets = any_h2 && T2 > 0;
+  const TetInput tin{tri_m, tri_w, tri_fa, tri_fb, tri_off, T2};
+  TetCounts tc{};
+  int64_t* t_off = nullptr;
   void* tq_ws = nullptr;
-  size_t tq_b = 0;
+  const size_t tq_b = link_count_workspace_bytes(T2);
   if (any_h2) {
-    tet_off = A.take<int64_t>(E + 1);
     en2 = A.take<uint8_t>(E);
-    tq_b = ph_tets_count_workspace_bytes(E);
+    t_off = A.take<int64_t>(K + 1);
+    tc.tet_cnt = A.take<i32>(T2);
+    tc.row_cnt = A.take<i32>(T2);
+    tc.tet_off = A.take<int64_t>(T2 + 1);
+    tc.row_off = A.take<int64_t>(T2 + 1);
+    tc.stash.cap = tet_stash_cap(T2, 2 * T2);
+    tc.stash.totals = reinterpret_cast<LinkTotals*>(cnt + 11);
     tq_ws = A.bytes(tq_b);
     if (A.failed) return alloc_fail();
+    count_launch();
+    ph::launch_pdl(k_gather_off, dim3(grid_for(K + 1)), dim3(256), 0, s, (const int64_t*)tri_off,
+                   (const int64_t*)e_off, K, t_off);
   }
+  // tetrahedra of the clouds kept (all of them at first), and their rows, per cloud
+  auto count_tets = [&](const uint8_t* keep) {
+    tc.stash.rows = A.take<TetRow>(tc.stash.cap);
+    if (A.failed) return fail(PH_ERR_CUDA, "ph_rips_persistence_batch: device allocation failed");
+    const int rc = tet_count(graph, tin, keep, tc, tq_ws, tq_b, s);
+    if (rc != PH_OK) return rc;
+    count_launch();
+    ph::launch_pdl(k_seg_diff, dim3(grid_for(K)), dim3(256), 0, s, (const int64_t*)tc.tet_off, (const int64_t*)t_off,
+                   K, per);
+    count_launch();
+    ph::launch_pdl(k_seg_diff, dim3(grid_for(K)), dim3(256), 0, s, (const int64_t*)tc.row_off, (const int64_t*)t_off,
+                   K, per_rows);
+    return (int)PH_OK;
+  };
   for (int attempt = 0;; ++attempt) {
     int rc = reduce_only(A, s, links.off, data1, E, 0, R1, (i32)E, span1, skip1, cmf1, pool1, st + 2, r1);
     if (rc == PH_OK)
       rc = ph_batch_persistence_rows(r1.state, r1.piv, E, (i32)E, filt, nullptr, row_m, e_off, K, res->rows[1],
                                      row_off1, nrows1, r1_ws, r1_b, s);
     if (rc != PH_OK) return give_up(rc);
-    if (any_h2 && attempt == 0) {
-      // tetrahedra of the clouds kept for H2, counted before waiting
-      count_launch();
-      ph::launch_pdl(k_edge_flags, dim3(grid_for(E)), dim3(256), 0, s, (const i32*)si, E, (const i32*)vcloud,
-                     (const uint8_t*)(cflag + K), 0, (const uint8_t*)nullptr, en2);
-      rc = ph_tets_count(tri_off, tri_w, E, adj_ptr, adj_idx, adj_rank, en2, tet_off, tq_ws, tq_b, s);
-      if (rc == PH_OK) {
-        count_launch();
-        ph::launch_pdl(k_seg_diff, dim3(grid_for(K)), dim3(256), 0, s, (const int64_t*)tet_off, (const int64_t*)e_off,
-                       K, per);
-      }
+    if (tets && attempt == 0) {  // counted before waiting
+      rc = count_tets(nullptr);
       if (rc != PH_OK) return give_up(rc);
     }
-    Part parts[3] = {{cnt, hcnt, 16 * sizeof(int64_t)},
+    Part parts[4] = {{cnt, hcnt, 16 * sizeof(int64_t)},
                      {row_off1, hoff2, sizeof(int64_t) * (K + 1)},
-                     {per, hper, any_h2 ? sizeof(int64_t) * K : 0}};
-    if (readback_parts(parts, 3, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
+                     {per, hper, tets ? sizeof(int64_t) * K : 0},
+                     {per_rows, hrows, tets ? sizeof(int64_t) * K : 0}};
+    if (readback_parts(parts, 4, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
     const int st_red = (int)(hcnt[2] & 0xffffffff);
     if ((int)(hcnt[3] >> 32) != 0) return give_up(fail((int)(hcnt[3] >> 32), "the triangle rows of the two passes differ"));
     if (st_red == PH_OK) break;
@@ -588,7 +605,9 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   }
 
   // ---- 6. H2 for the clouds that ask for it -------------------------------------------------------
-  i64 Q = 0, span2 = 0;
+  if (!tets)
+    for (int c = 0; c < K; ++c) hper[c] = hrows[c] = 0;
+  i64 Q = 0;
   bool any_cleared2 = false;
   for (int c = 0; c < K; ++c) {
     if (!keep2[c]) continue;
@@ -601,7 +620,6 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
       continue;
     }
     Q += hper[c];
-    span2 = std::max<i64>(span2, hper[c]);
   }
   if (E + T2 + Q >= (int64_t(1) << 31) || 4 * Q >= (int64_t(1) << 31) ||
       (K > 1 && max_batch_simplices > 0 && T2 + Q > max_batch_simplices)) {
@@ -615,47 +633,57 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
       record_error(cudaGetLastError());
       return give_up(PH_ERR_CUDA);
     }
-    count_launch();
-    ph::launch_pdl(k_edge_flags, dim3(grid_for(E)), dim3(256), 0, s, (const i32*)si, E, (const i32*)vcloud,
-                   (const uint8_t*)(cflag + K), 0, (const uint8_t*)nullptr, en2);
-    PH_TRY(mask_offsets(A, s, tet_off, E, en2));
   }
-  i32* tet_m = A.take<i32>(Q);
-  i32* tet_faces = A.take<i32>(4 * Q);
+  // once more where a cloud dropped out (its rows are not wanted) or the stash
+  // was too small
+  if (tets && (any_cleared2 || hcnt[13] > tc.stash.cap)) {
+    i64 rows = 0;
+    for (int c = 0; c < K; ++c) rows += keep2[c] ? hrows[c] : 0;
+    tc.stash.cap = tet_stash_cap(T2, rows);
+    ph::zero_async(cnt + 11, sizeof(LinkTotals), s);
+    const int rc = count_tets(any_cleared2 ? cflag + K : nullptr);
+    if (rc != PH_OK) return give_up(rc);
+    Part parts[2] = {{cnt, hcnt, 16 * sizeof(int64_t)}, {per_rows, hrows, sizeof(int64_t) * K}};
+    if (readback_parts(parts, 2, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
+    if (hcnt[13] > tc.stash.cap)
+      return give_up(fail(PH_ERR_CUDA, "ph_rips_persistence_batch: the tetrahedron rows outgrew their buffer twice"));
+  }
+  const i64 R2 = tets ? hcnt[12] : 0;  // tetrahedra that can be pivots: the rows of the H2 reduction
+  i64 span2 = 0;
+  for (int c = 0; c < K; ++c) span2 = std::max<i64>(span2, hrows[c]);
+  i32* tet_m = A.take<i32>(R2);
+  i32* tet_faces = A.take<i32>(4 * R2);
   uint8_t* skip2 = A.take<uint8_t>(T2);
-  i32* cmf2 = A.take<i32>(Q);
+  i32* cmf2 = A.take<i32>(R2);
   i32* off2 = A.take<i32>(T2 + 1);
-  i32* data2 = A.take<i32>(4 * Q);
-  int64_t* t_off = A.take<int64_t>(K + 1);
+  i32* len2 = A.take<i32>(T2);
+  i32* cursor2 = A.take<i32>(T2);
+  i32* data2 = A.take<i32>(4 * R2);
   int64_t* row_off2 = A.take<int64_t>(K + 1);
   int64_t* nrows2 = A.take<int64_t>(1);
-  const size_t c2_b = cofacet_lists_workspace_bytes(T2),
-               r2_b = ph_batch_persistence_rows_workspace_bytes(T2);
-  void* c2_ws = A.bytes(c2_b);
+  const size_t r2_b = ph_batch_persistence_rows_workspace_bytes(T2);
   void* r2_ws = A.bytes(r2_b);
   if (A.failed || cudaMallocAsync((void**)&res->rows[2], sizeof(float) * 2 * std::max<i64>(T2, 1), s) != cudaSuccess)
     return alloc_fail();
   {
-    int rc = PH_OK;
-    if (Q)
-      rc = ph_tets_emit(si, sj, E, tri_off, tri_w, tri_fa, tri_fb, adj_ptr, adj_idx, adj_rank, en2, tet_off, tet_m,
-                        tet_faces, st + 3, s);
-    if (rc == PH_OK) rc = mark_pivots_mapped(r1.state, r1.piv, E, (i32)E, row_tri, skip2, T2, s);
+    int rc = mark_pivots_mapped(r1.state, r1.piv, E, (i32)E, row_tri, skip2, T2, s);
+    if (rc == PH_OK && E) {
+      count_launch();
+      ph::launch_pdl(k_edge_flags, dim3(grid_for(E)), dim3(256), 0, s, (const i32*)si, E, (const i32*)vcloud,
+                     (const uint8_t*)(cflag + K), 0, (const uint8_t*)nullptr, en2);
+    }
     // triangles of the clouds without H2 are not columns
     if (rc == PH_OK && T2) rc = ph_or_gather_mask(skip2, en2, tri_m, T2, 1, s);
-    if (rc == PH_OK && Q) rc = ph_cof_max_face(tet_faces, nullptr, nullptr, nullptr, 4, Q, (i32)E, skip2, cmf2, s);
-    if (rc == PH_OK && Q)
-      rc = cofacet_lists(tet_faces, 4, Q, T2, (i32)(E + T2), off2, data2, st + 3, c2_ws, c2_b, s);
+    if (rc == PH_OK && tets)
+      rc = tet_rows(si, sj, tin, skip2, tc, (i32)E, (i32)(E + T2), R2, tet_m, tet_faces, cmf2, len2, cursor2, off2,
+                    data2, tq_ws, tq_b, st + 3, s);
     if (rc != PH_OK) return give_up(rc);
-    if (!Q) ph::zero_async(off2, sizeof(i32) * (T2 + 1), s);
-    count_launch();
-    ph::launch_pdl(k_gather_off, dim3(grid_for(K + 1)), dim3(256), 0, s, (const int64_t*)tri_off,
-                   (const int64_t*)e_off, K, t_off);
+    if (!tets) ph::zero_async(off2, sizeof(i32) * (T2 + 1), s);
   }
-  i64 pool2 = pool_capacity(4 * Q, T2);
+  i64 pool2 = pool_capacity(4 * R2, T2);
   RedOut r2{};
   for (int attempt = 0;; ++attempt) {
-    int rc = reduce_only(A, s, off2, data2, T2, (i32)E, Q, (i32)(E + T2), span2, skip2, cmf2, pool2, st + 4, r2);
+    int rc = reduce_only(A, s, off2, data2, T2, (i32)E, R2, (i32)(E + T2), span2, skip2, cmf2, pool2, st + 4, r2);
     if (rc == PH_OK)
       rc = ph_batch_persistence_rows(r2.state, r2.piv, T2, (i32)(E + T2), filt, tri_m, tet_m, t_off, K, res->rows[2],
                                      row_off2, nrows2, r2_ws, r2_b, s);
@@ -663,7 +691,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
     Part parts[2] = {{cnt, hcnt, 16 * sizeof(int64_t)}, {row_off2, hoff2, sizeof(int64_t) * (K + 1)}};
     if (readback_parts(parts, 2, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
     const int st_emit = (int)(hcnt[2] >> 32), st_red = (int)(hcnt[3] & 0xffffffff);
-    if (st_emit) return give_up(fail(st_emit, "ph_tets_emit failed"));
+    if (st_emit) return give_up(fail(st_emit, "the tetrahedron rows of the two passes differ"));
     if (st_red == PH_OK) break;
     if (st_red != PH_ERR_POOL || attempt >= 3 || pool2 >= POOL_MAX)
       return give_up(fail(st_red, "ph_reduce (H2) failed"));

@@ -41,10 +41,6 @@ void count_launch();
 // The reducer's step cap per column (ph_set_reduce_limits; 2^24 by default)
 // and the cap on a native call's first reduction pool (0: none).
 long long reduce_max_steps();
-// the cofacet lists, in any order, of simplices given as k faces each (simplices.cu)
-size_t cofacet_lists_workspace_bytes(int64_t n_faces);
-int cofacet_lists(const int32_t* faos, int32_t k, int64_t S, int64_t n_faces, int32_t row_base, int32_t* cof_off,
-                  int32_t* cof_data, int* d_status, void* workspace, size_t workspace_bytes, cudaStream_t s);
 // ph_reduce of cofacet lists in any order (reduce.cu)
 int reduce_lists(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32_t col_base, int64_t R,
                  int32_t row_base, int64_t span, const uint8_t* skip, const int32_t* row_cmf, int32_t* col_state,

@@ -1,4 +1,4 @@
-// The rows of the H1 reduction: the triangles that can be pivots.
+// The rows of the H1 and H2 reductions: the simplices that can be pivots.
 //
 // The H1 coboundary matrix has a row per triangle, but most triangles can
 // never be the pivot of a reduced column. Write a triangle as (m, w): its
@@ -23,6 +23,11 @@
 // 90K) 3.8 -> 1.0 ms; a union of 192 clouds of 64-4096 points 119 -> 27 ms;
 // 20,000 x 10 at 1.4 (17.6K, 13.4K) unchanged, 0.88 ms.
 //
+// H2 likewise: a tetrahedron (m, p, q), p < q in m's link, comes after every
+// (m, y, .) with y < p, so it is no pivot when the link holds a y < p joined to
+// both p and q below m (the five-vertex clique's boundary). 6-13% of the
+// tetrahedra of dense clouds remain (331 x 50: 0.44M of 4.9M).
+//
 // k_links: a group of G lanes an edge. The lanes intersect the ends' adjacency
 // rows into the link (its length is the edge's triangle count). Then each lane
 // takes a third vertex and all test the link's first vertices together: in a
@@ -37,6 +42,11 @@
 // rows (over 64 entries: 155 us for 10^6 edges against 180 at 32 and 210 at
 // 16) together. The rows found go to a stash in no order, from which
 // k_link_rows places them once the counts are scanned.
+//
+// k_tet_links: a warp a triangle (m, p). The earlier link vertices joined to p
+// go to shared memory; the later ones, q, a lane each, are tetrahedra where
+// they are joined to p, and each is tested against the former, by all lanes
+// together first and one after another then, as above.
 #include <algorithm>
 #include <climits>
 
@@ -53,6 +63,15 @@ constexpr int LK_BLOCKS = 4;   // resident blocks an SM
 constexpr int LK_CHUNK = 8;    // stash rows a group takes at a time
 constexpr u32 FULL = 0xffffffffu;
 constexpr i32 NO_RANK = INT_MAX;
+
+__device__ __forceinline__ int lower_bound_i32(const i32* __restrict__ a, int lo, int hi, i32 x) {
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (a[mid] < x) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
 
 // the graph as one warp sees it for an edge: adjacency rows, and the rank
 // table of the edge's cloud where there is one
@@ -379,8 +398,9 @@ struct StashChunk {
 
   // where the n <= G rows of one call go: the first `room` of them from pos on,
   // the others from the new chunk on
-  __device__ __forceinline__ void put(const Group<G>& gr, const LinkStash& st, int n, bool mine, int z,
-                                      const LinkRow& row) {
+  template <typename Row>
+  __device__ __forceinline__ void put(const Group<G>& gr, const Stash<Row>& st, int n, bool mine, int z,
+                                      const Row& row) {
     const int room = (int)min((i64)n, end - pos);
     const int take = max(n - room, LK_CHUNK);
     i64 next = 0;
@@ -400,7 +420,8 @@ struct StashChunk {
     }
   }
 
-  __device__ __forceinline__ void finish(const Group<G>& gr, const LinkStash& st) {
+  template <typename Row>
+  __device__ __forceinline__ void finish(const Group<G>& gr, const Stash<Row>& st) {
     for (i64 at = pos + gr.lane; at < min(end, st.cap); at += G) st.rows[at].m = -1;
   }
 };
@@ -523,6 +544,183 @@ __global__ void __launch_bounds__(LK_NT) k_link_rows(LinkStash stash, const uint
   }
 }
 
+// ---- tetrahedra -------------------------------------------------------------------------
+struct TetArgs {
+  const i32* tri_m;
+  const i32* tri_w;
+  const i64* tri_off;
+  i64 T;
+  const uint8_t* keep;  // per cloud, may be null: the others' tetrahedra are neither counted nor kept
+};
+
+__global__ void __launch_bounds__(LK_NT) k_tet_links(LinkGraph lg, TetArgs ta,
+                                                     i32* __restrict__ tet_cnt, i32* __restrict__ row_cnt,
+                                                     TetStash stash) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  constexpr int U = 4;  // lookups a lane has in flight
+  __shared__ i32 lists[LK_WARPS][LK_LIST];
+  __shared__ unsigned long long sum[2];
+  const Group<32> gr;
+  const int lane = gr.lane;
+  const u32 lt = gr.below();
+  i32* list = lists[threadIdx.x >> 5];
+  const i64 warp = ((i64)blockIdx.x * LK_NT + threadIdx.x) >> 5;
+  const i64 nwarps = ((i64)gridDim.x * LK_NT) >> 5;
+  if (threadIdx.x < 2) sum[threadIdx.x] = 0;
+  __syncthreads();
+  StashChunk<32> chunk;
+  i64 ntet = 0, nrow = 0;
+  for (i64 t = warp; t < ta.T; t += nwarps) {
+    const i32 m = ta.tri_m[t], p = ta.tri_w[t];
+    const i64 t0 = ta.tri_off[m], t1 = ta.tri_off[m + 1];
+    int tets = 0, rows = 0;
+    if (t + 1 < t1 && (!ta.keep || ta.keep[lg.vcloud[p]])) {
+      const Graph g = graph_of(lg, p);
+      // the earlier vertices of the link joined to p
+      int held = 0;
+      i64 stop = t;  // link position after the last of those in the list
+      for (i64 base = t0; base < t; base += 32) {
+        const i32 y = base + lane < t ? ta.tri_w[base + lane] : -1;
+        const bool in = y >= 0 && g.rank(p, y) < m;
+        const u32 b = gr.ballot(in);
+        if (held + __popc(b) > LK_LIST) {
+          stop = base;  // the rest is walked below
+          break;
+        }
+        if (in) list[held + __popc(b & lt)] = y;
+        held += __popc(b);
+      }
+      gr.sync();
+      for (i64 base = t + 1; base < t1; base += 32) {
+        const i64 k = base + lane;
+        const i32 q = k < t1 ? ta.tri_w[k] : -1;
+        const i32 rpq = q >= 0 ? g.rank(p, q) : NO_RANK;
+        const bool tet = rpq < m;
+        bool open = tet;
+        u32 left = gr.ballot(tet);
+        tets += __popc(left);
+        int tested = 0;
+        while (tested < held && __popc(left) * ((held - tested + 31) / 32) > (tested ? (held - tested) / U : 0)) {
+          i32 r[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) r[u] = open && tested + u < held ? g.rank(list[tested + u], q) : NO_RANK;
+#pragma unroll
+          for (int u = 0; u < U; ++u) open &= r[u] >= m;
+          tested += U;
+          left = gr.ballot(open);
+        }
+        if (tested < held) {
+          while (left) {
+            const int l = __ffs(left) - 1;
+            left &= left - 1;
+            const i32 ql = gr.from(q, l);
+            for (int j = tested; j < held; j += 32) {
+              const i32 y = list[min(j + lane, held - 1)];
+              if (gr.ballot(g.rank(ql, y) < m)) {
+                if (lane == l) open = false;
+                break;
+              }
+            }
+          }
+        }
+        for (i64 x = stop; open && x < t; ++x) {  // a list that did not hold them all
+          const i32 y = ta.tri_w[x];
+          if (g.rank(p, y) < m && g.rank(y, q) < m) open = false;
+        }
+        gr.sync();
+        const u32 lanes = gr.ballot(open);
+        if (lanes) {
+          const int n = __popc(lanes), z = __popc(lanes & lt);
+          chunk.put(gr, stash, n, open, z, TetRow{(i32)t, rows + z, (i32)k, rpq});
+          rows += n;
+        }
+      }
+      gr.sync();  // the list is free for the next triangle
+    }
+    if (lane == 0) {
+      if (tet_cnt) tet_cnt[t] = tets;
+      row_cnt[t] = rows;
+    }
+    ntet += tets;
+    nrow += rows;
+  }
+  chunk.finish(gr, stash);
+  if (lane == 0) {
+    if (ntet) atomicAdd(&sum[0], (unsigned long long)ntet);
+    if (nrow) atomicAdd(&sum[1], (unsigned long long)nrow);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (sum[0]) atomicAdd(&stash.totals->triangles, sum[0]);
+    if (sum[1]) atomicAdd(&stash.totals->rows, sum[1]);
+  }
+}
+
+// The kept tetrahedra in their order: row r = row_off[t] + z is the z-th of
+// triangle t = (m, p). Each gets its largest edge, its four faces, its largest
+// face that is a column, and counts in the cofacet lists of its faces.
+__global__ void __launch_bounds__(LK_NT) k_tet_rows(TetStash stash, const i32* __restrict__ ei,
+                                                    const i32* __restrict__ ej, TetArgs ta,
+                                                    const i32* __restrict__ tfa, const i32* __restrict__ tfb,
+                                                    const uint8_t* __restrict__ skip, const i64* __restrict__ row_off,
+                                                    i32 face_base, i64 nrows, i32* __restrict__ row_m,
+                                                    i32* __restrict__ faces, i32* __restrict__ cmf,
+                                                    i32* __restrict__ len_cnt, int* status) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  const i64 n = min((i64)stash.totals->stash, stash.cap);
+  for (i64 x = (i64)blockIdx.x * LK_NT + threadIdx.x; x < n; x += (i64)gridDim.x * LK_NT) {
+    const TetRow row = stash.rows[x];
+    if (row.m < 0) continue;
+    const i64 t = row.m, k = row.k, r = row_off[t] + row.z;
+    if (r >= nrows) {  // the counts and the rows disagree: never write past the buffers
+      set_status(status, PH_ERR_ARG);
+      continue;
+    }
+    const i32 m = ta.tri_m[t], p = ta.tri_w[t], q = ta.tri_w[k], rpq = row.r;
+    i32 f[4] = {(i32)t, (i32)k, 0, 0};
+    // {a, p, q} and {b, p, q}: their largest edge and third vertex
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      const i32 v = side ? ej[m] : ei[m];
+      const i32 rp = side ? tfb[t] : tfa[t], rq = side ? tfb[k] : tfa[k];
+      const i32 big = max(max(rp, rq), rpq), third = big == rp ? q : (big == rq ? p : v);
+      const int lo = (int)ta.tri_off[big], hi = (int)ta.tri_off[big + 1];
+      f[2 + side] = lower_bound_i32(ta.tri_w, lo, hi, third);
+      if (f[2 + side] >= hi || ta.tri_w[f[2 + side]] != third) {  // cannot happen for a consistent adjacency
+        set_status(status, PH_ERR_ARG);
+        f[2 + side] = (i32)t;
+      }
+    }
+    row_m[r] = m;
+    reinterpret_cast<int4*>(faces)[r] = make_int4(f[0], f[1], f[2], f[3]);
+    i32 best = -1;
+#pragma unroll
+    for (int z = 0; z < 4; ++z)
+      if (!skip[f[z]]) {
+        best = max(best, face_base + f[z]);
+        atomicAdd(&len_cnt[f[z]], 1);
+      }
+    cmf[r] = best;
+  }
+}
+
+// the rows' ranks into the cofacet lists of their faces that are columns
+__global__ void k_tet_scatter(const i32* __restrict__ faces, i64 entries, const uint8_t* __restrict__ skip,
+                              i32 row_base, const i32* __restrict__ off, i32* __restrict__ cursor,
+                              i32* __restrict__ data, int* status) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  for (i64 x = (i64)blockIdx.x * blockDim.x + threadIdx.x; x < entries; x += (i64)gridDim.x * blockDim.x) {
+    const i32 f = faces[x];
+    if (skip[f]) continue;
+    const i32 pos = off[f] + atomicAdd(&cursor[f], 1);
+    if (pos < off[f + 1]) data[pos] = row_base + (i32)(x >> 2);
+    else set_status(status, PH_ERR_ARG);
+  }
+}
+
 inline int grid_for(i64 n, int nt = 256) {
   return (int)std::max<i64>(1, std::min<i64>((n + nt - 1) / nt, 148 * 16));
 }
@@ -581,6 +779,46 @@ int link_rows(i64 nrows, const uint8_t* skip, const LinkCounts& o, i32 row_base,
   ph::launch_pdl(k_link_rows, dim3(grid_for(o.stash.cap, LK_NT)), dim3(LK_NT), 0,
                  s, o.stash, skip, (const i64*)o.row_off, (const i64*)o.tri_off, (const i32*)o.off, o.cursor, row_base,
                  nrows, row_m, row_tri, cmf, data, status);
+  PH_CHECK_LAUNCH();
+  return PH_OK;
+}
+
+// ---- tetrahedra ---------------------------------------------------------------------------
+namespace {
+inline int tets_grid(i64 T) {
+  return (int)std::max<i64>(1, std::min<i64>((T + LK_WARPS - 1) / LK_WARPS, (i64)ph::device_sms() * 8));
+}
+}  // namespace
+
+i64 tet_stash_cap(i64 T, i64 rows) { return rows + (i64)tets_grid(T) * LK_WARPS * LK_CHUNK; }
+
+int tet_count(const LinkGraph& g, const TetInput& in, const uint8_t* keep, const TetCounts& o, void* ws,
+              size_t ws_bytes, cudaStream_t s) {
+  if (in.T < 1) return PH_ERR_ARG;
+  const TetArgs ta{in.tri_m, in.tri_w, in.tri_off, in.T, keep};
+  ph::count_launch();
+  ph::launch_pdl(k_tet_links, dim3(tets_grid(in.T)), dim3(LK_NT), 0, s, g, ta, o.tet_cnt, o.row_cnt, o.stash);
+  if (o.tet_off) PH_TRY(scan_exclusive_i32_i64(o.tet_cnt, o.tet_off, in.T, ws, ws_bytes, s));
+  PH_TRY(scan_exclusive_i32_i64(o.row_cnt, o.row_off, in.T, ws, ws_bytes, s));
+  PH_CHECK_LAUNCH();
+  return PH_OK;
+}
+
+int tet_rows(const i32* ei, const i32* ej, const TetInput& in, const uint8_t* skip, const TetCounts& o, i32 face_base,
+             i32 row_base, i64 nrows, i32* row_m, i32* faces, i32* cmf, i32* len_cnt, i32* cursor, i32* off, i32* data,
+             void* ws, size_t ws_bytes, int* status, cudaStream_t s) {
+  if (in.T < 1) return PH_ERR_ARG;
+  const TetArgs ta{in.tri_m, in.tri_w, in.tri_off, in.T, nullptr};
+  ph::zero_async(len_cnt, sizeof(i32) * in.T, s, cursor, sizeof(i32) * in.T);
+  ph::count_launch();
+  ph::launch_pdl(k_tet_rows, dim3(grid_for(o.stash.cap, LK_NT)), dim3(LK_NT), 0, s, o.stash, ei, ej, ta, in.tri_fa,
+                 in.tri_fb, skip, (const i64*)o.row_off, face_base, nrows, row_m, faces, cmf, len_cnt, status);
+  PH_TRY(scan_exclusive_i32_i32(len_cnt, off, in.T, ws, ws_bytes, s));
+  if (nrows > 0) {
+    ph::count_launch();
+    ph::launch_pdl(k_tet_scatter, dim3(grid_for(4 * nrows, LK_NT)), dim3(LK_NT), 0, s, (const i32*)faces, 4 * nrows,
+                   skip, row_base, (const i32*)off, cursor, data, status);
+  }
   PH_CHECK_LAUNCH();
   return PH_OK;
 }

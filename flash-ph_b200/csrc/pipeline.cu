@@ -51,13 +51,14 @@ std::vector<Slots> g_slots_free;
 std::mutex g_pinned_mu;
 std::vector<Pinned> g_pinned_free;
 
-// copies up to four device int64 values into the mapped host slots
-__global__ void k_report(const int64_t* a, const int64_t* b, const int64_t* c, const int64_t* d, int count,
-                         volatile int64_t* out, int64_t seq) {
+// copies device int64 values into the mapped host slots
+struct Report {
+  const int64_t* src[kSeqSlot];
+};
+__global__ void k_report(const Report r, int count, volatile int64_t* out, int64_t seq) {
   ph::pdl_wait();
   ph::pdl_trigger();
-  const int64_t* src[4] = {a, b, c, d};
-  if (threadIdx.x < count && threadIdx.x < 4) out[threadIdx.x] = *src[threadIdx.x];
+  if (threadIdx.x < count) out[threadIdx.x] = *r.src[threadIdx.x];
   __threadfence_system();
   __syncwarp();
   // the sequence word last: the host reads the values once it sees it
@@ -179,11 +180,12 @@ int fail(int code, const std::string& msg) {
 }
 
 int readback(const int64_t* const* src, int count, const Slots& dst, cudaStream_t s) {
+  if (count > kSeqSlot) return PH_ERR_ARG;
   const int64_t seq = ++*dst.seq;
   count_launch();
-  if (ph::launch_pdl(k_report, dim3(1), dim3(32), 0, s, src[0], count > 1 ? src[1] : src[0],
-                     count > 2 ? src[2] : src[0], count > 3 ? src[3] : src[0], count, dst.dev,
-                     seq) != cudaSuccess) {
+  Report r{};
+  for (int k = 0; k < count; ++k) r.src[k] = src[k];
+  if (ph::launch_pdl(k_report, dim3(1), dim3(32), 0, s, r, count, dst.dev, seq) != cudaSuccess) {
     record_error(cudaGetLastError());
     return PH_ERR_CUDA;
   }
@@ -203,8 +205,7 @@ int readback_parts(const Part* parts, int nparts, const Slots& slots, cudaStream
   // word arrives, every part is in host memory
   const int64_t seq = ++*slots.seq;
   count_launch();
-  if (ph::launch_pdl(k_report, dim3(1), dim3(32), 0, s, (const int64_t*)nullptr, (const int64_t*)nullptr,
-                     (const int64_t*)nullptr, (const int64_t*)nullptr, 0, slots.dev, seq) != cudaSuccess) {
+  if (ph::launch_pdl(k_report, dim3(1), dim3(32), 0, s, Report{}, 0, slots.dev, seq) != cudaSuccess) {
     record_error(cudaGetLastError());
     return PH_ERR_CUDA;
   }
@@ -312,7 +313,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   int64_t* blk = A.take<int64_t>(2);
   // cnt[0]: edge count; statuses as int32 words from cnt + 1: st[0] edges,
   // st[1] forest, st[2] H1 reduction, st[3] tetrahedra, st[4] H2 reduction;
-  // cnt[5] triangle total, cnt[6] its work counter, cnt[8..10] LinkTotals
+  // cnt[5] triangle total, cnt[6] its work counter, cnt[8..10] LinkTotals of the triangles, cnt[11..13] of the tetrahedra
   int64_t* cnt = A.take<int64_t>(16);
   if (A.failed) return alloc_fail();
   int* st = reinterpret_cast<int*>(cnt + 1);
@@ -523,15 +524,25 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   // (T >= 16 E) it is read back here, so that a call over the tetrahedron
   // limit fails before the H1 columns are built and reduced; otherwise it is
   // launched here and read back with the H1 status (one host wait fewer)
-  int64_t* tet_off = nullptr;
-  i64 Q = 0;
-  const bool tets_first = max_dim == 2 && T >= 16 * E;
-  if (max_dim == 2) {
-    tet_off = A.take<int64_t>(E + 1);
-    const size_t tq_b = ph_tets_count_workspace_bytes(E);
-    void* tq_ws = A.bytes(tq_b);
+  i64 Q = 0, R2 = 0;  // tetrahedra, and those that can be pivots: the rows of the H2 reduction
+  const bool tets = max_dim == 2 && T > 0, tets_first = tets && T >= 16 * E;
+  const TetInput tin{tri_m, tri_w, tri_fa, tri_fb, tri_off, T};
+  TetCounts tc{};
+  void* tq_ws = nullptr;
+  const size_t tq_b = link_count_workspace_bytes(T);
+  auto count_tets = [&]() {  // enqueued; the totals are read later
+    tc.stash.rows = A.take<TetRow>(tc.stash.cap);
+    if (A.failed) return fail(PH_ERR_CUDA, "ph_rips_persistence: device allocation failed");
+    return tet_count(graph, tin, nullptr, tc, tq_ws, tq_b, s);
+  };
+  if (tets) {
+    tc.row_cnt = A.take<i32>(T);
+    tc.row_off = A.take<int64_t>(T + 1);
+    tc.stash.cap = tet_stash_cap(T, 2 * T);  // about one and a half a triangle in dense complexes
+    tc.stash.totals = reinterpret_cast<LinkTotals*>(cnt + 11);
+    tq_ws = A.bytes(tq_b);
     if (A.failed) return alloc_fail();
-    int rc = ph_tets_count(tri_off, tri_w, E, adj_ptr, adj_idx, adj_rank, nullptr, tet_off, tq_ws, tq_b, s);
+    const int rc = count_tets();
     if (rc != PH_OK) return give_up(rc);
   }
   auto tets_limit = [&]() -> int {
@@ -542,11 +553,26 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
              (long long)Q, (long long)max_tetrahedra);
     return fail(PH_ERR_LIMIT, m);
   };
+  // the counts, once they are on the host: the limit, and a second pass where
+  // the stash was too small
+  auto take_tets = [&](i64 tets_, i64 rows_, i64 stash_) {
+    Q = tets_;
+    R2 = rows_;
+    int rc = tets_limit();
+    if (rc != PH_OK || stash_ <= tc.stash.cap) return rc;
+    tc.stash.cap = tet_stash_cap(T, R2);
+    ph::zero_async(cnt + 11, sizeof(LinkTotals), s);
+    rc = count_tets();
+    if (rc != PH_OK) return rc;
+    const int64_t* src[1] = {cnt + 13};
+    if (readback(src, 1, slots, s) != PH_OK) return (int)PH_ERR_CUDA;
+    return H[0] <= tc.stash.cap ? (int)PH_OK
+                                : fail(PH_ERR_CAPACITY, "ph_rips_persistence: the tetrahedron rows outgrew their buffer twice");
+  };
   if (tets_first) {
-    const int64_t* src[1] = {tet_off + E};
-    if (readback(src, 1, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
-    Q = H[0];
-    const int rc = tets_limit();
+    const int64_t* src[3] = {cnt + 11, cnt + 12, cnt + 13};
+    if (readback(src, 3, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
+    const int rc = take_tets(H[0], H[1], H[2]);
     if (rc != PH_OK) return give_up(rc);
   }
   if (E) {
@@ -561,8 +587,8 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
     int rc = reduce_rows(A, s, links.off, data1, E, 0, R1, (i32)E, mask, cmf1, filt, nullptr, row_m, pool1, st + 2,
                          res->rows[1], r1);
     if (rc != PH_OK) return give_up(rc);
-    const int64_t* src[4] = {cnt + 2, r1.nrows, r1.info + 1, max_dim == 2 ? tet_off + E : r1.nrows};
-    if (readback(src, 4, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
+    const int64_t* src[6] = {cnt + 2, r1.nrows, r1.info + 1, cnt + 11, cnt + 12, cnt + 13};
+    if (readback(src, 6, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
     const int st_red = (int)(H[0] & 0xffffffff);
     // the word beside it: the cofacet rows' status (the tetrahedra's only later)
     if ((int)(H[0] >> 32) != 0) return give_up(fail((int)(H[0] >> 32), "the triangle rows of the two passes differ"));
@@ -574,9 +600,8 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   }
   res->nrows[1] = H[1];
   res->stats[3] = H[2];
-  if (max_dim == 2 && !tets_first) {
-    Q = H[3];
-    const int rc = tets_limit();
+  if (tets && !tets_first) {
+    const int rc = take_tets(H[3], H[4], H[5]);
     if (rc != PH_OK) return give_up(rc);
   }
   if (max_dim == 1) {
@@ -592,38 +617,34 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
     return give_up(fail(PH_ERR_LIMIT, m));
   }
   res->stats[2] = Q;
-  i32* tet_m = A.take<i32>(Q);
-  i32* tet_faces = A.take<i32>(4 * Q);
+  i32* tet_m = A.take<i32>(R2);
+  i32* tet_faces = A.take<i32>(4 * R2);
   uint8_t* skip2 = A.take<uint8_t>(T);
-  i32* cmf2 = A.take<i32>(Q);
+  i32* cmf2 = A.take<i32>(R2);
   i32* off2 = A.take<i32>(T + 1);
-  i32* data2 = A.take<i32>(4 * Q);
-  const size_t c2_b = cofacet_lists_workspace_bytes(T);
-  void* c2_ws = A.bytes(c2_b);
+  i32* len2 = A.take<i32>(T);
+  i32* cursor2 = A.take<i32>(T);
+  i32* data2 = A.take<i32>(4 * R2);
   if (A.failed || cudaMallocAsync((void**)&res->rows[2], sizeof(float) * 2 * std::max<i64>(T, 1), s) != cudaSuccess)
     return alloc_fail();
   {
-    int rc = PH_OK;
-    if (Q)
-      rc = ph_tets_emit(si, sj, E, tri_off, tri_w, tri_fa, tri_fb, adj_ptr, adj_idx, adj_rank, nullptr, tet_off,
-                        tet_m, tet_faces, st + 3, s);
-    if (rc == PH_OK) rc = mark_pivots_mapped(r1.state, r1.piv, E, (i32)E, row_tri, skip2, T, s);
-    if (rc == PH_OK && Q) rc = ph_cof_max_face(tet_faces, nullptr, nullptr, nullptr, 4, Q, (i32)E, skip2, cmf2, s);
-    if (rc == PH_OK && Q)
-      rc = cofacet_lists(tet_faces, 4, Q, T, (i32)(E + T), off2, data2, st + 3, c2_ws, c2_b, s);
+    int rc = mark_pivots_mapped(r1.state, r1.piv, E, (i32)E, row_tri, skip2, T, s);
+    if (rc == PH_OK && tets)
+      rc = tet_rows(si, sj, tin, skip2, tc, (i32)E, (i32)(E + T), R2, tet_m, tet_faces, cmf2, len2, cursor2, off2,
+                    data2, tq_ws, tq_b, st + 3, s);
     if (rc != PH_OK) return give_up(rc);
-    if (!Q) ph::zero_async(off2, sizeof(i32) * (T + 1), s);
+    if (!tets) ph::zero_async(off2, sizeof(i32) * (T + 1), s);
   }
-  i64 pool2 = pool_capacity(4 * Q, T);
+  i64 pool2 = pool_capacity(4 * R2, T);
   RedOut r2{};
   for (int attempt = 0;; ++attempt) {
-    int rc = reduce_rows(A, s, off2, data2, T, (i32)E, Q, (i32)(E + T), skip2, cmf2, filt, tri_m, tet_m, pool2,
+    int rc = reduce_rows(A, s, off2, data2, T, (i32)E, R2, (i32)(E + T), skip2, cmf2, filt, tri_m, tet_m, pool2,
                          st + 4, res->rows[2], r2);
     if (rc != PH_OK) return give_up(rc);
     const int64_t* src[4] = {cnt + 2, cnt + 3, r2.nrows, r2.info + 1};
     if (readback(src, 4, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
     const int st_emit = (int)(H[0] >> 32), st_red = (int)(H[1] & 0xffffffff);
-    if (st_emit) return give_up(fail(st_emit, "ph_tets_emit failed"));
+    if (st_emit) return give_up(fail(st_emit, "the tetrahedron rows of the two passes differ"));
     if (st_red == PH_OK) break;
     if (st_red != PH_ERR_POOL || attempt >= 3 || pool2 >= POOL_MAX)
       return give_up(fail(st_red, "ph_reduce (H2) failed"));

@@ -88,7 +88,7 @@ float to_f32(double v);
 // records msg for ph_last_error() and returns code
 int fail(int code, const std::string& msg);
 
-// Brings count (<= 4) int64 values from the device into the pinned slots and
+// Brings count (<= 8) int64 values from the device into the pinned slots and
 // waits (spins briefly on a sequence word written after them, then blocks).
 int readback(const int64_t* const* src, int count, const Slots& dst, cudaStream_t s);
 // One part of a bulk readback: bytes from device src to host dst.

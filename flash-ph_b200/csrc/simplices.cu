@@ -402,29 +402,6 @@ __global__ void k_cof_scatter3(const i32* __restrict__ f0, const i32* __restrict
   }
 }
 
-// the cofacet rows of k-simplices given as k faces each (AoS): the row
-// lengths first (a count per face), then each simplex's rank into its faces'
-// rows; a write past its row's end is dropped and reported
-__global__ void k_cof_count_aos(const i32* __restrict__ faos, i64 H, i32* __restrict__ cnt) {
-  ph::pdl_wait();
-  ph::pdl_trigger();
-  for (i64 x = (i64)blockIdx.x * blockDim.x + threadIdx.x; x < H; x += (i64)gridDim.x * blockDim.x)
-    atomicAdd(&cnt[faos[x]], 1);
-}
-
-__global__ void k_cof_scatter_aos(const i32* __restrict__ faos, i64 H, int k, i32 row_base,
-                                  const i32* __restrict__ off, i32* __restrict__ cursor, i32* __restrict__ data,
-                                  int* status) {
-  ph::pdl_wait();
-  ph::pdl_trigger();
-  for (i64 x = (i64)blockIdx.x * blockDim.x + threadIdx.x; x < H; x += (i64)gridDim.x * blockDim.x) {
-    const i32 f = faos[x];
-    const i32 pos = off[f] + atomicAdd(&cursor[f], 1);
-    if (pos < off[f + 1]) data[pos] = row_base + (i32)(x / k);
-    else set_status(status, PH_ERR_ARG);
-  }
-}
-
 // ascending bitonic sort of n <= len2 (a power of two) values in shared memory
 // by the threads tid = 0..nthreads-1 of a group that synchronises with sync()
 template <typename Sync>
@@ -824,44 +801,3 @@ extern "C" int ph_cof_max_face(const int32_t* faces_aos, const int32_t* f0, cons
   PH_CHECK_LAUNCH();
   return PH_OK;
 }
-
-namespace ph {
-size_t cofacet_lists_workspace_bytes(int64_t n_faces) {
-  const i64 nf = std::max<i64>(n_faces, 1);
-  return Carve::need(sizeof(i32) * (size_t)(nf + 1)) + Carve::need(sizeof(i32) * (size_t)nf) +
-         Carve::need(scan_workspace_bytes(nf));
-}
-
-// The cofacet lists of S simplices with k faces each (AoS, the tetrahedra's
-// four triangles): lengths counted, offsets scanned, ranks scattered into
-// their lists in any order (reduce_lists orders them).
-int cofacet_lists(const int32_t* faos, int32_t k, int64_t S, int64_t n_faces, int32_t row_base, int32_t* cof_off,
-                  int32_t* cof_data, int* d_status, void* workspace, size_t workspace_bytes, cudaStream_t s) {
-  const i64 H = S * k;
-  if (k < 1 || S < 0 || n_faces < 0 || H >= (int64_t(1) << 31)) return PH_ERR_ARG;
-  Carve c(workspace, workspace_bytes);
-  const i64 nf = std::max<i64>(n_faces, 1);
-  i32* cnt = c.take<i32>(nf + 1);
-  i32* cursor = c.take<i32>(nf);
-  void* sws = c.take<char>((i64)scan_workspace_bytes(nf));
-  if (!cnt || !cursor || !sws) return PH_ERR_ARG;
-  if (n_faces == 0) {
-    ph::zero_async(cof_off, sizeof(i32), s);
-    PH_CHECK_LAUNCH();
-    return PH_OK;
-  }
-  ph::zero_async(cnt, sizeof(i32) * (size_t)n_faces, s, cursor, sizeof(i32) * (size_t)n_faces);
-  if (H > 0) {
-    ph::count_launch();
-    ph::launch_pdl(k_cof_count_aos, dim3(grid_for(H)), dim3(256), 0, s, faos, H, cnt);
-  }
-  PH_TRY(scan_exclusive_i32_i32(cnt, cof_off, n_faces, sws, scan_workspace_bytes(nf), s));
-  if (H > 0) {
-    ph::count_launch();
-    ph::launch_pdl(k_cof_scatter_aos, dim3(grid_for(H)), dim3(256), 0, s, faos, H, (int)k, row_base,
-                   (const i32*)cof_off, cursor, cof_data, d_status);
-  }
-  PH_CHECK_LAUNCH();
-  return PH_OK;
-}
-}  // namespace ph

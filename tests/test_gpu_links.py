@@ -57,6 +57,51 @@ def test_long_link_matches_oracle(points, pairs, cluster):
             assert np.array_equal(_bits(sorted_rows(d[2])), _bits(sorted_rows(ref["h2"])))
 
 
+# four hubs joined to each other and to every leaf, the last two after the
+# leaves: the triangle of the longest edge and the third hub has every leaf
+# among its earlier neighbours (the list holds 768); with 1300 leaves the graph
+# is too sparse for the rank table
+@pytest.mark.parametrize("leaves", [767, 768, 900, 1300])
+def test_many_earlier_neighbours_of_a_triangle(leaves):
+    from flashph_b200 import rips_persistence
+    rng = np.random.default_rng(leaves)
+    x = np.zeros((leaves + 4, leaves + 2), dtype=np.float32)
+    x[2 + np.arange(leaves), np.arange(leaves)] = rng.uniform(1.0, 1.02, leaves)
+    x[[0, 1, leaves + 2, leaves + 3], leaves:] = [(-0.7, 0), (0.7, 0), (0, 0.3), (0, -0.31)]
+    ref = oracle.run(x, T, 2, fused=True)
+    got = [d.cpu().numpy() for d in rips_persistence(torch.from_numpy(x).cuda(), T, max_dim=2)]
+    assert ref["Q"] > 4 * leaves
+    assert np.array_equal(_bits(got[1]), _bits(ref["h1"].reshape(-1, 2)))
+    assert np.array_equal(_bits(sorted_rows(got[2])), _bits(sorted_rows(ref["h2"])))
+
+
+def _staged(monkeypatch, x, t, dim):
+    from flashph_b200 import rips_persistence
+    monkeypatch.setenv("FLASHPH_PIPELINE", "staged")
+    out = rips_persistence(x, t, max_dim=dim)
+    monkeypatch.delenv("FLASHPH_PIPELINE")
+    return out
+
+
+# H2 in the native call keeps the tetrahedra that can be pivots, the stage by
+# stage form all of them: the same rows in the same order, ties (the lattice)
+# and the sparse end included
+@pytest.mark.parametrize("n,d,t", [(120, 4, 3.0), (300, 3, 1.1), (900, 10, 2.6), (3000, 10, 1.7), (216, 0, 2.3)])
+def test_h2_rows_equal_the_staged_form(monkeypatch, n, d, t):
+    from flashph_b200 import rips_persistence
+    from flashph_b200.batch import rips_persistence_batch
+    if d:
+        x = np.random.default_rng(n).standard_normal((n, d)).astype(np.float32)
+    else:
+        x = np.stack(np.meshgrid(*[np.arange(6)] * 3), -1).reshape(-1, 3).astype(np.float32)
+    x = torch.from_numpy(x).cuda()
+    want = _staged(monkeypatch, x, t, 2)
+    batch = rips_persistence_batch([x[:50], x, x[: n // 2]], t, [1, 2, 0])[1]
+    for got in (rips_persistence(x, t, max_dim=2), batch):
+        for a, b in zip(got, want):
+            assert np.array_equal(_bits(a.cpu().numpy()), _bits(b.cpu().numpy()))
+
+
 def test_row_beyond_the_shared_memory_sort(monkeypatch):
     """More than 8192 rows in one column: the native call against the stage by
     stage form, whose cofacet rows come from the radix sort."""
