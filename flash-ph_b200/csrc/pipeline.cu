@@ -214,7 +214,7 @@ int readback_parts(const Part* parts, int nparts, const Slots& slots, cudaStream
 
 i64 pool_capacity(i64 nnz, i64 K) {
   const i64 mult = nnz < (i64(1) << 24) ? 8 : 3;
-  i64 cap = std::min<i64>(mult * nnz + 2 * K + (i64(1) << 23), POOL_MAX);
+  i64 cap = std::min<i64>(mult * nnz + 6 * K + (i64(1) << 23), POOL_MAX);
   // a test can make the first pool small to exercise the exhaustion retry
   const long long lim = reduce_first_pool_limit();
   if (lim > 0) cap = std::min<i64>(cap, lim);

@@ -101,7 +101,7 @@ struct Part {
 // readback does.
 int readback_parts(const Part* parts, int nparts, const Slots& slots, cudaStream_t s);
 
-// reduction pool (int32 entries): initial records (at most 2 nnz), per-warp
+// reduction pool (int32 entries): initial records (nnz + 4 a column), per-warp
 // chunks, reduced columns; bounded by the 33-bit record offsets
 constexpr i64 POOL_MAX = (i64(1) << 33) - 1;
 i64 pool_capacity(i64 nnz, i64 K);

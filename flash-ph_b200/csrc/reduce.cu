@@ -23,8 +23,9 @@
 // apparent column can contain its pivot).
 //
 // Memory layout. Every column content lives in an immutable record
-// [len, rank_0 < rank_1 < ...] in one pool (initial records are copies of the
-// cofacet lists; later ones are bump-allocated per warp). The owner word of a
+// [len, rank_0 < rank_1 < ...] in one pool, at a multiple of four entries
+// (initial records are copies of the cofacet lists; later ones are
+// bump-allocated per warp). The owner word of a
 // pivot row is (column + 1) << 33 | record offset, 0 when free, so one
 // atomicMax both orders claims by column and publishes the claimer's content:
 // a reader needs the owner word and the record, two dependent loads. Claims
@@ -111,7 +112,7 @@ __global__ void k_classify(const i32* __restrict__ off, const i32* __restrict__ 
     }
     const bool has = c < K && !skipped && len > 0;
     // warp prefix of record sizes
-    int need = has ? len + 1 : 0, incl = need;
+    int need = has ? (len + 4) & ~3 : 0, incl = need;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int v = __shfl_up_sync(FULL, incl, o);
@@ -147,14 +148,17 @@ __global__ void k_classify(const i32* __restrict__ off, const i32* __restrict__ 
 
 // ---- cofacet lists in any order ------------------------------------------------------
 // k_ready does k_classify's work on lists that are not sorted yet, so that
-// they need no pass of their own: column c's record lies at off[c] + c of the
-// pool (no allocation). A lane sorts a list of up to 8 entries in registers
+// they need no pass of their own: column c's record lies at ready_at(off[c], c)
+// of the pool (no allocation). A lane sorts a list of up to 8 entries in registers
 // (most lists: the rows number 1-1.6 an edge), a warp one of up to 32 across
 // its lanes and of up to RY_LIST in its shared memory, the block longer ones
 // in all of it, and where they are (in the pool) beyond that.
 constexpr int RY_NT = 256;
 constexpr int RY_WARPS = RY_NT / 32;
 constexpr int RY_LIST = 1024;
+
+// room for every column's length and entries at a multiple of four
+__device__ __forceinline__ i64 ready_at(i32 off, i64 c) { return 4 * ((i64)(off >> 2) + c); }
 
 __device__ __forceinline__ void order(i32& x, i32& y) {
   const i32 lo = min(x, y);
@@ -209,7 +213,7 @@ __global__ void __launch_bounds__(RY_NT) k_ready(const i32* __restrict__ off, co
   __shared__ i32 longs[RY_NT];
   __shared__ int nlong;
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const i64 top = (i64)off[K] + K;  // records of all columns
+  const i64 top = ready_at(off[K], K);  // records of all columns
   const bool fits = top <= pool_cap;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     ctl->pool_top = (unsigned long long)top;
@@ -253,12 +257,12 @@ __global__ void __launch_bounds__(RY_NT) k_ready(const i32* __restrict__ off, co
 #pragma unroll
       for (int k = 0; k < 8; ++k) v[k] = k < len ? cof[o + k] : INT_MAX;
       sort8(v);
-      i32* r = pool + (i64)o + c;
+      i32* r = pool + ready_at(o, c);
       r[0] = len;
 #pragma unroll
       for (int k = 0; k < 8; ++k)
         if (k < len) r[1 + k] = v[k];
-      nres += settle(c, v[0], (u64)((i64)o + c));
+      nres += settle(c, v[0], (u64)ready_at(o, c));
     }
     if (len > RY_LIST) longs[atomicAdd(&nlong, 1)] = (i32)threadIdx.x;
     u32 todo = __ballot_sync(FULL, len > 8 && len <= RY_LIST);
@@ -268,7 +272,7 @@ __global__ void __launch_bounds__(RY_NT) k_ready(const i32* __restrict__ off, co
       const i64 cc = c0 + l;
       const i32 oo = __shfl_sync(FULL, o, l);
       const int n = __shfl_sync(FULL, len, l);
-      i32* r = pool + (i64)oo + cc;
+      i32* r = pool + ready_at(oo, cc);
       i32 first;
       if (n <= 32) {
         i32 x = lane < n ? cof[oo + lane] : INT_MAX;
@@ -290,7 +294,7 @@ __global__ void __launch_bounds__(RY_NT) k_ready(const i32* __restrict__ off, co
       }
       if (lane == 0) {
         r[0] = n;
-        nres += settle(cc, first, (u64)((i64)oo + cc));
+        nres += settle(cc, first, (u64)ready_at(oo, cc));
       }
     }
     __syncthreads();  // the list of long columns is complete, and the warps are done with their buffers
@@ -299,7 +303,7 @@ __global__ void __launch_bounds__(RY_NT) k_ready(const i32* __restrict__ off, co
       const i64 cc = b0 + longs[q];
       const i32 oo = off[cc];
       const int n = off[cc + 1] - oo;
-      i32* r = pool + (i64)oo + cc;
+      i32* r = pool + ready_at(oo, cc);
       i32* w = n <= RY_WARPS * RY_LIST ? buf : r + 1;
       for (int i = threadIdx.x; i < n; i += RY_NT) w[i] = cof[oo + i];
       __syncthreads();
@@ -308,7 +312,7 @@ __global__ void __launch_bounds__(RY_NT) k_ready(const i32* __restrict__ off, co
         for (int i = threadIdx.x; i < n; i += RY_NT) r[1 + i] = w[i];
       if (threadIdx.x == 0) {
         r[0] = n;
-        nres += settle(cc, w[0], (u64)((i64)oo + cc));
+        nres += settle(cc, w[0], (u64)ready_at(oo, cc));
       }
       __syncthreads();
     }
@@ -574,6 +578,7 @@ struct PoolChunk {
 
 __device__ __forceinline__ unsigned long long pool_alloc(PoolChunk& ch, RedCtl* ctl, i64 cap, int n, int chunk,
                                                          int* status) {
+  n = (n + 3) & ~3;  // records start at a multiple of four
   unsigned long long at = 0;
   if ((threadIdx.x & 31) == 0) {
     if (ch.pos + (unsigned long long)n <= ch.end) {
@@ -601,10 +606,8 @@ __device__ __forceinline__ unsigned long long pool_alloc(PoolChunk& ch, RedCtl* 
 // bits, the next pivot is the first set bit at or after the current one (the
 // added column's entries are all >= the pivot it cancels), and the sorted
 // record is produced only when the column claims a pivot. Cost per addition
-// is the added column's length, not the working column's. When the row range
-// fits one of the warp's shared buffers (up to 32 * RD_CAP rows) every
-// working column is such a bitmap in shared memory; otherwise only a column
-// that outgrows its shared buffer becomes one, in a global slot per warp.
+// is the added column's length, not the working column's. A column that
+// outgrows its shared buffer becomes one, in a global slot per warp.
 //
 // A global bitmap spans the whole row range (millions of rows for dense
 // complexes), while a column's entries are a few thousand at most: scanning
@@ -619,11 +622,10 @@ constexpr int RD_SUM_WORDS = RD_CAPB;  // summary words (the added-column buffer
 
 struct DenseCol {
   u32* bits = nullptr;  // this warp's bitmap
-  u32* sum = nullptr;   // summary of a global bitmap (shared memory), null for a shared bitmap
+  u32* sum = nullptr;   // its summary (shared memory), null where that does not fit
   i32 rb = 0;           // rank of the bitmap's bit 0 (word-aligned, at or below the column's first pivot)
   i64 lo = 0, hi = -1;  // touched word range
   i32 piv = -1;         // lowest set bit (global rank)
-  bool sm = false;      // bits are in this warp's shared memory
 };
 
 // shared-memory forms of the bitmap accesses (explicit state space: the
@@ -632,12 +634,6 @@ __device__ __forceinline__ u32 sm_ld32(const u32* p) {
   u32 v;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"((u32)__cvta_generic_to_shared(p)) : "memory");
   return v;
-}
-__device__ __forceinline__ u32 sm_xor32(u32* p, u32 x) {
-  u32 old;
-  asm volatile("atom.shared.xor.b32 %0, [%1], %2;" : "=r"(old) : "r"((u32)__cvta_generic_to_shared(p)), "r"(x)
-               : "memory");
-  return old;
 }
 __device__ __forceinline__ void sm_red_xor32(u32* p, u32 x) {
   asm volatile("red.shared.xor.b32 [%0], %1;" ::"r"((u32)__cvta_generic_to_shared(p)), "r"(x) : "memory");
@@ -656,13 +652,6 @@ __device__ __forceinline__ void sm_st32(u32* p, u32 v) {
   asm volatile("st.shared.u32 [%0], %1;" ::"r"((u32)__cvta_generic_to_shared(p)), "r"(v) : "memory");
 }
 
-__device__ __forceinline__ u32 dense_word(const DenseCol& D, i64 w) { return D.sm ? sm_ld32(D.bits + w) : __ldcg(D.bits + w); }
-__device__ __forceinline__ u32 dense_xor(const DenseCol& D, i64 w, u32 b) {
-  return D.sm ? sm_xor32(D.bits + w, b) : atomicXor(D.bits + w, b);
-}
-
-// flips the sorted entries src[0..len) (global ranks); returns the change in
-// the number of set bits (warp-uniform) and widens the touched range
 // flips the sorted entries held one per lane (lanes < len <= 32); the set-bit
 // count is not tracked here (the flips need not return their old words): a
 // vanished column shows as no set bit at the pivot scan, and the count of a
@@ -671,15 +660,10 @@ __device__ void dense_flip_regs(DenseCol& D, i32 v, int len, i32 row_base) {
   const int lane = threadIdx.x & 31;
   if (lane < len) {
     const i32 e = v - row_base;
-    const u32 b = 1u << (e & 31);
-    if (D.sm) {
-      sm_red_xor32(D.bits + (e >> 5), b);
-    } else {
-      gl_red_xor32(D.bits + (e >> 5), b);
-      if (D.sum) sm_red_or32(D.sum + (e >> 15), 1u << ((e >> 10) & 31));
-    }
+    gl_red_xor32(D.bits + (e >> 5), 1u << (e & 31));
+    if (D.sum) sm_red_or32(D.sum + (e >> 15), 1u << ((e >> 10) & 31));
   }
-  if (!D.sm) __threadfence_block();
+  __threadfence_block();
   const i32 first = __shfl_sync(FULL, v, 0), last = __shfl_sync(FULL, v, (len - 1) & 31);
   if (len > 0) {
     const i64 w0 = (i64)((first - row_base) >> 5), w1 = (i64)((last - row_base) >> 5);
@@ -766,19 +750,14 @@ __device__ int dense_count(const DenseCol& D, i32 row_base) {
     });
     return __reduce_add_sync(FULL, c);
   }
-  for (i64 w = w0 + lane; w <= D.hi; w += 32) c += __popc(dense_word(D, w));
+  for (i64 w = w0 + lane; w <= D.hi; w += 32) c += __popc(__ldcg(D.bits + w));
   return __reduce_add_sync(FULL, c);
 }
 
 // one entry's flip: the bitmap bit, and the summary bit of its block
 __device__ __forceinline__ void dense_flip1(const DenseCol& D, i32 e) {
-  const u32 b = 1u << (e & 31);
-  if (D.sm) {
-    sm_red_xor32(D.bits + (e >> 5), b);
-  } else {
-    gl_red_xor32(D.bits + (e >> 5), b);
-    if (D.sum) sm_red_or32(D.sum + (e >> 15), 1u << ((e >> 10) & 31));
-  }
+  gl_red_xor32(D.bits + (e >> 5), 1u << (e & 31));
+  if (D.sum) sm_red_or32(D.sum + (e >> 15), 1u << ((e >> 10) & 31));
 }
 
 // flips the sorted entries src[0..len) (global ranks) and widens the touched
@@ -803,7 +782,7 @@ __device__ void dense_flip(DenseCol& D, const i32* src, bool srcg, int len, i32 
     D.hi = max(D.hi, w1);
   }
   // the flips are visible to the warp's later loads of the bitmap
-  if (!D.sm) __threadfence_block();
+  __threadfence_block();
   __syncwarp();
 }
 
@@ -832,7 +811,7 @@ __device__ i32 dense_first(const DenseCol& D, i64 from, i32 row_base) {
   }
   for (i64 w0 = from; w0 <= D.hi; w0 += 32) {
     const i64 w = w0 + lane;
-    const u32 v = w <= D.hi ? dense_word(D, w) : 0u;
+    const u32 v = w <= D.hi ? __ldcg(D.bits + w) : 0u;
     const u32 m = __ballot_sync(FULL, v != 0);
     if (m) {
       const int f = __ffs(m) - 1;
@@ -881,7 +860,7 @@ __device__ void dense_to_list(const DenseCol& D, i32 row_base, i32* out) {
   }
   for (i64 w0 = wp; w0 <= D.hi; w0 += 32) {
     const i64 w = w0 + lane;
-    u32 v = w <= D.hi ? dense_word(D, w) : 0u;
+    u32 v = w <= D.hi ? __ldcg(D.bits + w) : 0u;
     const int c = __popc(v);
     int incl = c;
 #pragma unroll
@@ -922,10 +901,7 @@ __device__ void dense_clear(DenseCol& D, i64 lo, i64 hi) {
     D.piv = -1;
     return;
   }
-  if (D.sm)
-    for (i64 w = lo + lane; w <= hi; w += 32) sm_st32(D.bits + w, 0u);
-  else
-    for (i64 w = lo + lane; w <= hi; w += 32) __stcg(D.bits + w, 0u);
+  for (i64 w = lo + lane; w <= hi; w += 32) __stcg(D.bits + w, 0u);
   __syncwarp();
   D.lo = 0;
   D.hi = -1;
@@ -938,7 +914,7 @@ __device__ void dense_clear(DenseCol& D, i64 lo, i64 hi) {
 __global__ void __launch_bounds__(RD_NT, 1) k_reduce(i32 row_base, i64 K, const i32* __restrict__ state,
                                                  const u64* __restrict__ rec, u64* owner, i32* pool, i64 pool_cap,
                                                  int chunk, RedCtl* ctl, int* status, int max_steps,
-                                                 u32* dense_bits, i64 dense_words, int sm_words) {
+                                                 u32* dense_bits, i64 dense_words) {
   ph::pdl_wait();
   ph::pdl_trigger();
   extern __shared__ i32 rd_smem[];
@@ -950,14 +926,9 @@ __global__ void __launch_bounds__(RD_NT, 1) k_reduce(i32 row_base, i64 K, const 
   unsigned long long n_merges = 0, n_takeovers = 0;
   DenseCol D;
   bool dense_ready = false;  // this warp's slot has been cleared once
-  // shared bitmap (in the second working buffer) when the rows fit, else the global slot
-  const bool dense_sm = sm_words > 0;
-  const bool dense_ok = dense_sm || dense_words > 0;
-  const i64 dwords = dense_sm ? (i64)sm_words : dense_words;
-  if (dense_sm) {
-    D.bits = reinterpret_cast<u32*>(sW0 + RD_CAP);
-    D.sm = true;
-  } else if (dense_ok) {
+  const bool dense_ok = dense_words > 0;
+  const i64 dwords = dense_words;
+  if (dense_ok) {
     D.bits = dense_bits + (size_t)(blockIdx.x * RD_WARPS + w) * (size_t)dense_words;
     // the summary needs one bit per 32 data words; a slot's word count is
     // bounded by the 1 GiB of slots, far below RD_SUM_WORDS * 1024 words
@@ -1000,10 +971,6 @@ __global__ void __launch_bounds__(RD_NT, 1) k_reduce(i32 row_base, i64 K, const 
       // the bitmap window starts at the first pivot's word
       D.rb = len > 0 ? row_base + (((D.piv - row_base) >> 5) << 5) : row_base;
       dense_flip(D, src, srcg, len, D.rb);
-      if (D.sm) {  // a shared bitmap is read and cleared whole: no touched range to track
-        D.lo = 0;
-        D.hi = dwords - 1;
-      }
       dense = true;
     };
     auto leave_dense = [&]() {
@@ -1013,7 +980,7 @@ __global__ void __launch_bounds__(RD_NT, 1) k_reduce(i32 row_base, i64 K, const 
     auto load_record = [&](u64 at) {
       const i32* src = pool + at + 1;
       k = __ldcg(pool + at);
-      if (dense_sm || (k > RD_CAP && dense_ok)) {
+      if (k > RD_CAP && dense_ok) {
         enter_dense(src, true, k);
       } else if (k <= RD_CAP) {
         for (int i = lane; i < k; i += 32) (sW0 + cur * RD_CAP)[i] = __ldcg(src + i);
@@ -1046,69 +1013,8 @@ __global__ void __launch_bounds__(RD_NT, 1) k_reduce(i32 row_base, i64 K, const 
       }
       if (k == 0) break;  // the column vanished: it owns nothing
       const bool take = pending != 0;
-      // The chain of additions of a shared-bitmap column, in a loop of its own:
-      // while its pivot's owner is a larger column, add that column's record
-      // (one owner-word and one record-head round trip), then find the new
-      // pivot from the old one's word on. Long columns spend their whole
-      // reduction here, and this loop's few branches and registers make a
-      // step about 1.5x shorter than one of the general loop below, which
-      // takes over at the first pivot the column must claim (its owner word
-      // already loaded).
-      u64 ow_known = 0;
-      bool have_ow = false, aborted = false;
-      if (dense && D.sm && !take) {
-        for (;;) {
-          const i32 pf = D.piv;
-          const u64 ow_f = ld_acquire(owner + (pf - row_base));
-          if (owner_col(ow_f) <= c) {
-            ow_known = ow_f;
-            have_ow = true;
-            break;
-          }
-          const u64 at_f = ow_f & OW_OFF;
-          const i32 head = (at_f + lane < (u64)pool_cap) ? __ldcg(pool + at_f + lane) : 0;
-          const int lb = __shfl_sync(FULL, head, 0);
-          const i32 bv = __shfl_down_sync(FULL, head, 1);  // entry `lane` (lanes < 31)
-          if (lane < lb && lane < 31) {
-            const i32 e = bv - D.rb;
-            sm_red_xor32(D.bits + (e >> 5), 1u << (e & 31));
-          }
-          if (lb > 31) dense_flip(D, pool + at_f + 32, true, lb - 31, D.rb);
-          __syncwarp();
-          ++n_merges;
-          published = false;
-          // the added record cleared the old pivot: the new one is the first set
-          // bit from its word on, almost always within the next 32 words
-          const i64 wp = (i64)((pf - D.rb) >> 5);
-          const i64 wl = wp + lane;
-          const u32 v = wl < dwords ? sm_ld32(D.bits + wl) : 0u;
-          const u32 m = __ballot_sync(FULL, v != 0);
-          i32 np;
-          if (m) {
-            const int f = __ffs(m) - 1;
-            const u32 vw = __shfl_sync(FULL, v, f);
-            np = (i32)(((wp + f) << 5) + (__ffs(vw) - 1)) + D.rb;
-          } else {
-            np = dense_first(D, wp + 32, D.rb);
-          }
-          D.piv = np;
-          if (np < 0) break;
-          if (++step >= max_steps) break;
-          if ((step & 63) == 63 && *vabort) {
-            aborted = true;
-            break;
-          }
-        }
-        if (aborted) break;
-        if (D.piv < 0) {  // the column vanished
-          k = 0;
-          leave_dense();
-          break;
-        }
-        if (!have_ow) continue;  // the step limit: the loop top reports it
-      }
       const i32 p = dense ? D.piv : (wg ? __ldcg(W) : W[0]);
-      u64 ow = take ? pending : (have_ow ? ow_known : ld_acquire(owner + (p - row_base)));
+      u64 ow = take ? pending : ld_acquire(owner + (p - row_base));
       pending = 0;
       i32 o = owner_col(ow);
       if (!take && o < c) {
@@ -1254,6 +1160,277 @@ __global__ void __launch_bounds__(RD_NT, 1) k_reduce(i32 row_base, i64 K, const 
   }
 }
 
+// ---- rows that fit shared memory ------------------------------------------------------
+// The reduction proper for all but the largest complexes: a working column is
+// a bitmap of its warp's shared memory over the rows it can reach, with a
+// summary (a bit per 32-row word that may hold set bits), so every pass over a
+// column costs its nonzero words, not the row range.
+//
+// A column's reduction is a chain of additions, each waiting for the owner word
+// of the pivot the last one left and then for that owner's record: two
+// dependent L2 loads, ~0.7 us a step however little is added. But a column may
+// receive any column processed before it, at any of its entries, not only at
+// its pivot. So a round takes the first 32 nonzero words, a lane each, loads
+// the owners of their lowest entries and then the owners' records all at once,
+// and adds those up to the first entry that is free or owned by a column not
+// yet processed. The lowest entry is always among them (no other record
+// reaches below its own pivot), so the pivot rises every round; the others are
+// entries the chain would mostly meet later. An entry cancelled by an earlier
+// record of the same round is set again by its own owner's and is met again: a
+// few percent more additions, for 10 to 20 times fewer rounds than steps
+// (longest chain of dependent additions -> of rounds, reduced serially:
+// 4001-point torus in 3-D 564 -> 29, 20,000 x 10 Gaussian at 1.4 411 -> 49,
+// 1501 x 8 at its default threshold 409 -> 48).
+// The kernel, one addition a step in the same bitmap (or sorted lists beyond
+// 196,608 rows) -> rounds: 740 -> 205 us, 334 -> 151 us, 500 -> 349 us; with
+// 200,000 x 10 at 1.1 4.16 -> 1.35 ms and 200,000 x 50 at 6.0 2.55 -> 0.77 ms.
+constexpr int RS_MAX_WARPS = 4;
+constexpr size_t RS_SMEM = 226 * 1024;
+
+// words of the window, of its summary, and of the list of words a round takes
+__host__ __device__ inline size_t rs_warp_words(i64 nw) { return (size_t)(nw + nw / 32 + 32); }
+
+struct SharedCol {
+  u32* bits;
+  u32* sum;
+  i32* words;  // the round's word list (32)
+  int ns;      // summary words
+  i32 rb;      // rank of bit 0
+  int from;    // no set bit below this summary word
+
+  __device__ __forceinline__ void flip(i32 rank) const {
+    const u32 e = (u32)(rank - rb);
+    sm_red_xor32(bits + (e >> 5), 1u << (e & 31));
+    sm_red_or32(sum + (e >> 10), 1u << ((e >> 5) & 31));
+  }
+
+  // flips the entries src[0..len) of a record, by the warp
+  __device__ __forceinline__ void flip_all(const i32* src, int len) const {
+    const int lane = threadIdx.x & 31;
+    int i = lane;
+    for (; i + 96 < len; i += 128) {
+      i32 e[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) e[q] = __ldcg(src + i + 32 * q);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) flip(e[q]);
+    }
+    for (; i < len; i += 32) flip(__ldcg(src + i));
+    __syncwarp();
+  }
+
+  // Takes up to 32 words in ascending order from the lanes' masks m of the
+  // summary words s + lane (the bits taken are dropped from m); words[0..n).
+  __device__ __forceinline__ int take(int s, u32& m) const {
+    const int lane = threadIdx.x & 31;
+    const int c = __popc(m);
+    int incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += v;
+    }
+    for (int at = incl - c; m && at < 32; ++at) {
+      words[at] = ((s + lane) << 5) + __ffs(m) - 1;
+      m &= m - 1;
+    }
+    __syncwarp();
+    return min(__shfl_sync(FULL, incl, 31), 32);
+  }
+
+  // The first words with set bits, ascending over the lanes: the lane's lowest
+  // set bit (the bitmap's bit index), -1 on lanes without a word; the first of
+  // them is the column's pivot. All -1 when the column is empty.
+  __device__ __forceinline__ int lowest() {
+    const int lane = threadIdx.x & 31;
+    for (int s = from; s < ns;) {
+      u32 m = s + lane < ns ? sm_ld32(sum + s + lane) : 0u;
+      const u32 some = __ballot_sync(FULL, m != 0);
+      if (!some) {
+        s += 32;
+        from = s;
+        continue;
+      }
+      s += __ffs(some) - 1;
+      from = s;
+      m = s + lane < ns ? sm_ld32(sum + s + lane) : 0u;
+      const int n = take(s, m);
+      const int w = lane < n ? words[lane] : 0;
+      const u32 v = lane < n ? sm_ld32(bits + w) : 0u;
+      // words flipped empty since: their summary bits go
+      if (lane < n && !v) sm_red_and32(sum + (w >> 5), ~(1u << (w & 31)));
+      if (__any_sync(FULL, v != 0)) return v ? (w << 5) + __ffs(v) - 1 : -1;
+      __syncwarp();
+    }
+    return -1;
+  }
+
+  __device__ __forceinline__ int count() const {
+    const int lane = threadIdx.x & 31;
+    int c = 0;
+    for (int s = from + lane; s < ns; s += 32)
+      for (u32 m = sm_ld32(sum + s); m; m &= m - 1) c += __popc(sm_ld32(bits + (s << 5) + __ffs(m) - 1));
+    return __reduce_add_sync(FULL, c);
+  }
+
+  // the entries, ascending, to out
+  __device__ __forceinline__ void list(i32* out) const {
+    const int lane = threadIdx.x & 31;
+    int pos = 0;
+    for (int s = from; s < ns; s += 32) {
+      u32 m = s + lane < ns ? sm_ld32(sum + s + lane) : 0u;
+      while (__any_sync(FULL, m != 0)) {
+        const int n = take(s, m);
+        const int w = lane < n ? words[lane] : 0;
+        u32 v = lane < n ? sm_ld32(bits + w) : 0u;
+        const int c = __popc(v);
+        int incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(FULL, incl, o);
+          if (lane >= o) incl += t;
+        }
+        for (int at = pos + incl - c; v; v &= v - 1) out[at++] = (w << 5) + __ffs(v) - 1 + rb;
+        pos += __shfl_sync(FULL, incl, 31);
+        __syncwarp();  // the word list is free
+      }
+    }
+    __syncwarp();
+  }
+
+  __device__ __forceinline__ void clear() {
+    const int lane = threadIdx.x & 31;
+    for (int s = lane; s < ns; s += 32) {
+      for (u32 m = sm_ld32(sum + s); m; m &= m - 1) sm_st32(bits + (s << 5) + __ffs(m) - 1, 0u);
+      sm_st32(sum + s, 0u);
+    }
+    from = 0;
+    __syncwarp();
+  }
+};
+
+__global__ void __launch_bounds__(32 * RS_MAX_WARPS, 1)
+    k_reduce_shared(i32 row_base, i64 K, const i32* __restrict__ state, const u64* __restrict__ rec, u64* owner,
+                    i32* pool, i64 pool_cap, int chunk, RedCtl* ctl, int* status, int max_steps, int nw) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  extern __shared__ i32 rd_smem[];
+  const int lane = threadIdx.x & 31;
+  SharedCol D;
+  D.bits = reinterpret_cast<u32*>(rd_smem) + (size_t)(threadIdx.x >> 5) * rs_warp_words(nw);
+  D.sum = D.bits + nw;
+  D.ns = nw / 32;
+  D.words = reinterpret_cast<i32*>(D.sum + D.ns);
+  D.from = 0;
+  for (int i = lane; i < nw + D.ns; i += 32) D.bits[i] = 0u;
+  __syncwarp();
+  volatile int* vabort = &ctl->abort;
+  PoolChunk chunk_state;
+  unsigned long long n_merges = 0, n_takeovers = 0;
+  for (;;) {
+    int base = 0;
+    if (lane == 0) base = atomicAdd(&ctl->next, RD_FETCH);
+    base = __shfl_sync(FULL, base, 0);
+    if ((i64)base >= K || *vabort) break;
+    const i64 cand = K - 1 - base - lane;
+    u32 todo = __ballot_sync(FULL, lane < RD_FETCH && cand >= 0 && state[cand] == 2);
+    while (todo && !*vabort) {
+      const int l = __ffs(todo) - 1;
+      todo &= todo - 1;
+      i32 c = (i32)(K - 1 - base - l);
+      u64 wrec = rec[c];      // the column's record while it is as published
+      bool published = true;
+      {
+        const int k = __ldcg(pool + wrec);
+        // entries stay within [first pivot, first pivot + span): the window
+        // starts at the first pivot's word
+        D.rb = row_base + (((__ldcg(pool + wrec + 1) - row_base) >> 5) << 5);
+        D.flip_all(pool + wrec + 1, k);
+      }
+      for (int step = 0;; ++step) {
+        if ((step & 63) == 63 && *vabort) break;
+        if (step >= max_steps) {
+          if (lane == 0) set_status(status, PH_ERR_ITER_LIMIT);
+          atomicExch(&ctl->abort, 1);
+          break;
+        }
+        const int e = D.lowest();
+        const u32 live = __ballot_sync(FULL, e >= 0);
+        if (!live) break;  // the column vanished: it owns nothing
+        const u64 ow = e >= 0 ? ld_acquire(owner + (e + D.rb - row_base)) : 0ull;
+        const u32 stop = __ballot_sync(FULL, e >= 0 && owner_col(ow) <= c);
+        const u32 adds = live & ((stop & (0u - stop)) - 1u);  // the lanes below the first that stops
+        if (!adds) {
+          // publish the column as a record, then claim the pivot
+          if (!published) {
+            const int k = D.count();
+            const unsigned long long at = pool_alloc(chunk_state, ctl, pool_cap, k + 1, chunk, status);
+            if (at == ~0ull) break;
+            if (lane == 0) pool[at] = k;
+            D.list(pool + at + 1);
+            wrec = at;
+            published = true;
+          }
+          __syncwarp();
+          const int first = __ffs(live) - 1;
+          u64 old = 0;
+          if (lane == first) old = atom_max_acq_rel(owner + (e + D.rb - row_base), owner_word(c, wrec));
+          old = __shfl_sync(FULL, old, first);
+          __syncwarp();
+          const i32 oc = owner_col(old);
+          if (oc < 0) break;  // claimed a free pivot: this work item is done
+          if (oc == c) {      // cannot happen: a column never owns a pivot it is still reducing
+            if (lane == 0) set_status(status, PH_ERR_ARG);
+            break;
+          }
+          if (oc > c) continue;  // a larger column got there first: it is added in the next round
+          // displaced a smaller column: take it over. The bitmap holds the
+          // claimer's content, which the displaced column adds first: its
+          // record goes into it.
+          ++n_takeovers;
+          c = oc;
+          const u64 at = old & OW_OFF;
+          D.flip_all(pool + at + 1, __ldcg(pool + at));
+          ++n_merges;
+          published = false;
+          continue;
+        }
+        // add the records: length and seven entries a lane in two loads
+        const u64 at = ow & OW_OFF;
+        int len = 0, got = 0;
+        if ((adds >> lane) & 1u) {
+          const int4 a = __ldcg(reinterpret_cast<const int4*>(pool + at));
+          const bool wide = at + 8 <= (u64)pool_cap;
+          int4 b = make_int4(0, 0, 0, 0);
+          if (wide) b = __ldcg(reinterpret_cast<const int4*>(pool + at + 4));
+          len = a.x;
+          got = min(len, wide ? 7 : 3);
+          const i32 v[7] = {a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+          for (int q = 0; q < 7; ++q)
+            if (q < got) D.flip(v[q]);
+        }
+        u32 rest = __ballot_sync(FULL, len > got);
+        while (rest) {  // longer records, by the warp
+          const int r = __ffs(rest) - 1;
+          rest &= rest - 1;
+          const u64 ra = __shfl_sync(FULL, at, r);
+          const int skip = __shfl_sync(FULL, got, r), n = __shfl_sync(FULL, len, r);
+          D.flip_all(pool + ra + 1 + skip, n - skip);
+        }
+        n_merges += __popc(adds);
+        published = false;
+        __syncwarp();
+      }
+      D.clear();  // every exit leaves the window clean for the next column
+    }
+  }
+  if (lane == 0) {
+    if (n_merges) atomicAdd(&ctl->merges, n_merges);
+    if (n_takeovers) atomicAdd(&ctl->takeovers, n_takeovers);
+  }
+}
+
 // residual columns default to empty (state 3) ...
 __global__ void k_finish_cols(i64 K, i32* __restrict__ state, i32* __restrict__ piv, const RedCtl* ctl, i64* info) {
   ph::pdl_wait();
@@ -1321,18 +1498,19 @@ int reduce_blocks(i64 K) {
 // rounded up to whole 32-word blocks (slots and blocks 128-byte aligned).
 i64 window_words(i64 span) { return ((span + 31) / 32 + 2 + 31) / 32 * 32; }
 
-// words of the shared-memory bitmap each warp uses for every working column,
-// 0 when the window does not fit one working buffer
-int sm_dense_words(i64 span) {
+// warps a block whose windows fit shared memory together (up to RS_MAX_WARPS),
+// 0 when not even one does: spans of up to 1.79M rows fit, of 0.45M four
+int shared_warps(i64 span) {
   const i64 words = window_words(span);
-  return words <= RD_CAP ? (int)words : 0;
+  if (words > (i64)(RS_SMEM / 4)) return 0;
+  return (int)std::min<size_t>(RS_MAX_WARPS, RS_SMEM / 4 / rs_warp_words(words));
 }
 
-// dense working-column slots in global memory (windows beyond the shared
-// bitmap): one window per warp of the grid, when they fit in 1 GiB (else long
-// columns stay sorted lists in the pool)
+// dense working-column slots in global memory (windows beyond shared memory):
+// one window per warp of the grid, when they fit in 1 GiB (else long columns
+// stay sorted lists in the pool)
 i64 dense_words(i64 K, i64 span) {
-  if (sm_dense_words(span)) return 0;
+  if (shared_warps(span)) return 0;
   const i64 words = window_words(span);
   const i64 warps = (i64)reduce_blocks(K) * RD_WARPS;
   return words * warps * 4 <= (i64(1) << 30) ? words : 0;
@@ -1362,6 +1540,10 @@ int reduce_run(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32
     PH_CHECK_LAUNCH();
     return PH_OK;
   }
+  // records lie at multiples of 16 bytes whatever the caller's alignment
+  const i64 pad = std::min<i64>(pool_cap, (i64)((0 - (uintptr_t)pool) & 15) / 4);
+  pool += pad;
+  pool_cap -= pad;
   Carve c(workspace, workspace_bytes);
   u64* owner = c.take<u64>(std::max<i64>(R, 1));
   u64* rec = c.take<u64>(K);
@@ -1375,21 +1557,31 @@ int reduce_run(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32
   else
     ph::launch_pdl(k_ready, dim3(grid_for(K, RY_NT)), dim3(RY_NT), 0, s, cof_off, cof_data, K, col_base, row_base,
                    skip, row_cmf, col_state, col_piv, owner, rec, pool, pool_cap, ctl, d_status);
-  if (ph::allow_dynamic_smem((const void*)k_reduce) != cudaSuccess) {
+  span = span_or_all(R, span);
+  const int sw = shared_warps(span);
+  const void* kernel = sw ? (const void*)k_reduce_shared : (const void*)k_reduce;
+  if (ph::allow_dynamic_smem(kernel) != cudaSuccess) {
     PH_CHECK_LAUNCH();
     return PH_ERR_CUDA;
   }
-  const int blocks = reduce_blocks(K);
-  span = span_or_all(R, span);
-  const i64 dw = dense_words(K, span);
-  u32* dense = dw ? c.take<u32>(dw * (i64)blocks * RD_WARPS) : nullptr;
-  if (dw && !dense) return PH_ERR_ARG;
+  const int max_steps = (int)std::min<long long>(ph::reduce_max_steps(), INT_MAX);
+  const int warps = sw ? sw : RD_WARPS;
+  const int blocks = sw ? (int)std::max<i64>(1, std::min<i64>((K + sw - 1) / sw, ph::device_sms())) : reduce_blocks(K);
   // pool chunk per warp: small enough that the chunks of all warps fit a quarter of the pool
-  const int chunk = (int)std::max<i64>(64, std::min<i64>(2048, pool_cap / (4 * (i64)blocks * RD_WARPS)));
+  const int chunk = (int)std::max<i64>(64, std::min<i64>(2048, pool_cap / (4 * (i64)blocks * warps)) & ~3);
   ph::count_launch();
-  ph::launch_pdl(k_reduce, dim3(blocks), dim3(RD_NT), RD_SMEM, s, row_base, K, col_state, rec, owner, pool, pool_cap, chunk, ctl, d_status,
-                                          (int)std::min<long long>(ph::reduce_max_steps(), INT_MAX), dense, dw,
-                                          sm_dense_words(span));
+  if (sw) {
+    const i64 words = window_words(span);
+    ph::launch_pdl(k_reduce_shared, dim3(blocks), dim3(32 * sw), sw * rs_warp_words(words) * sizeof(u32), s, row_base,
+                   K, (const i32*)col_state, (const u64*)rec, owner, pool, pool_cap, chunk, ctl, d_status, max_steps,
+                   (int)words);
+  } else {
+    const i64 dw = dense_words(K, span);
+    u32* dense = dw ? c.take<u32>(dw * (i64)blocks * RD_WARPS) : nullptr;
+    if (dw && !dense) return PH_ERR_ARG;
+    ph::launch_pdl(k_reduce, dim3(blocks), dim3(RD_NT), RD_SMEM, s, row_base, K, (const i32*)col_state,
+                   (const u64*)rec, owner, pool, pool_cap, chunk, ctl, d_status, max_steps, dense, dw);
+  }
   ph::count_launch();
   ph::launch_pdl(k_finish_cols, dim3(grid_for(K)), dim3(256), 0, s, K, col_state, col_piv, ctl, d_info);
   if (R > 0) {
