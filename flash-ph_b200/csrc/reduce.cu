@@ -1170,132 +1170,164 @@ __global__ void __launch_bounds__(RD_NT, 1) k_reduce(i32 row_base, i64 K, const 
 // of the pivot the last one left and then for that owner's record: two
 // dependent L2 loads, ~0.7 us a step however little is added. But a column may
 // receive any column processed before it, at any of its entries, not only at
-// its pivot. So a round takes the first 32 nonzero words, a lane each, loads
-// the owners of their lowest entries and then the owners' records all at once,
-// and adds those up to the first entry that is free or owned by a column not
-// yet processed. The lowest entry is always among them (no other record
-// reaches below its own pivot), so the pivot rises every round; the others are
-// entries the chain would mostly meet later. An entry cancelled by an earlier
-// record of the same round is set again by its own owner's and is met again: a
-// few percent more additions, for 10 to 20 times fewer rounds than steps
-// (longest chain of dependent additions -> of rounds, reduced serially:
-// 4001-point torus in 3-D 564 -> 29, 20,000 x 10 Gaussian at 1.4 411 -> 49,
-// 1501 x 8 at its default threshold 409 -> 48).
+// its pivot. So a round takes up to 32 entries, a lane each, loads their owners
+// and then the owners' records all at once, and adds those up to the first
+// entry that is free or owned by a column not yet processed. The entries are
+// the lowest of the first words with set bits: of the words of the first two
+// groups of 32 words where the first has four or more (a dense column), else of
+// the first two words of each of 32 groups (no scan across the lanes either
+// way). The lowest entry of all is among them (no other record reaches below
+// its own pivot), so the pivot rises every round; the others are entries the
+// chain would mostly meet later. An entry cancelled by an earlier record of the
+// same round is set again by its own owner's and is met again: a few percent
+// more additions, for 8 to 15 times fewer rounds than steps (longest chain of
+// dependent additions -> of rounds, reduced serially: 4001-point torus in 3-D
+// 564 -> 46, 20,000 x 10 Gaussian at 1.4 411 -> 55, 1501 x 8 at its default
+// threshold 409 -> 57).
 // The kernel, one addition a step in the same bitmap (or sorted lists beyond
-// 196,608 rows) -> rounds: 740 -> 205 us, 334 -> 151 us, 500 -> 349 us; with
-// 200,000 x 10 at 1.1 4.16 -> 1.35 ms and 200,000 x 50 at 6.0 2.55 -> 0.77 ms.
-constexpr int RS_MAX_WARPS = 4;
+// 196,608 rows) -> rounds: 740 -> 221 us, 334 -> 142 us, 500 -> 339 us; with
+// 200,000 x 10 at 1.1 4.16 -> 1.02 ms and 200,000 x 50 at 6.0 2.55 -> 0.61 ms.
+// What bounds it now is the longest column of one warp: ~4,000 cycles a round
+// (700 the entries, an acquire of the owners, the records, their flips), more
+// where records hold thousands of entries.
+// Eight warps an SM against four: 1.28 -> 1.02 ms and 0.73 -> 0.61 ms on the
+// two large sparse sets, within 3% elsewhere.
+constexpr int RS_MAX_WARPS = 8;
 constexpr size_t RS_SMEM = 226 * 1024;
 
-// words of the window, of its summary, and of the list of words a round takes
+constexpr int RS_DENSE = 4;         // words of the first group from which a column counts as dense
+constexpr i64 RS_LONG_SWEEP = i64(1) << 19;
+
+// words of the window, of its summary, and of a round's entries
 __host__ __device__ inline size_t rs_warp_words(i64 nw) { return (size_t)(nw + nw / 32 + 32); }
 
 struct SharedCol {
   u32* bits;
   u32* sum;
-  i32* words;  // the round's word list (32)
-  int ns;      // summary words
-  i32 rb;      // rank of bit 0
-  int from;    // no set bit below this summary word
+  i32* slot;  // a round's entries (32)
+  int ns;     // summary words
+  i32 rb;    // rank of bit 0
+  int from;  // no set bit below this summary word's 32 words (a group)
+  bool bad;  // an entry lay outside the window (inconsistent inputs): not flipped
 
-  __device__ __forceinline__ void flip(i32 rank) const {
+  __device__ __forceinline__ void flip(i32 rank) {
     const u32 e = (u32)(rank - rb);
+    if ((e >> 10) >= (u32)ns) {
+      bad = true;
+      return;
+    }
     sm_red_xor32(bits + (e >> 5), 1u << (e & 31));
     sm_red_or32(sum + (e >> 10), 1u << ((e >> 5) & 31));
   }
 
-  // flips the entries src[0..len) of a record, by the warp
-  __device__ __forceinline__ void flip_all(const i32* src, int len) const {
+  // flips the entries [begin, len) of a record (its length word at rec), by the
+  // warp: 16 bytes a load, four loads a lane in flight, from the first whole
+  // 16 bytes on
+  __device__ __forceinline__ void flip_record(const i32* rec, int begin, int len) {
     const int lane = threadIdx.x & 31;
-    int i = lane;
-    for (; i + 96 < len; i += 128) {
-      i32 e[4];
+    const int head = min(len, ((begin + 1 + 3) & ~3) - 1);  // entry k is word k + 1
+    if (begin + lane < head) flip(__ldcg(rec + 1 + begin + lane));
+    const int whole = (len - head) >> 2;
+    const int4* v = reinterpret_cast<const int4*>(rec + 1 + head);
+    for (int i = lane; i < whole; i += 128) {
+      int4 x[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) e[q] = __ldcg(src + i + 32 * q);
+      for (int q = 0; q < 4; ++q)
+        if (i + 32 * q < whole) x[q] = __ldcg(v + i + 32 * q);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) flip(e[q]);
+      for (int q = 0; q < 4; ++q)
+        if (i + 32 * q < whole) flip(x[q].x), flip(x[q].y), flip(x[q].z), flip(x[q].w);
     }
-    for (; i < len; i += 32) flip(__ldcg(src + i));
+    const int tail = head + 4 * whole + lane;
+    if (tail < len) flip(__ldcg(rec + 1 + tail));
     __syncwarp();
   }
 
-  // Takes up to 32 words in ascending order from the lanes' masks m of the
-  // summary words s + lane (the bits taken are dropped from m); words[0..n).
-  __device__ __forceinline__ int take(int s, u32& m) const {
-    const int lane = threadIdx.x & 31;
-    const int c = __popc(m);
-    int incl = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(FULL, incl, o);
-      if (lane >= o) incl += v;
-    }
-    for (int at = incl - c; m && at < 32; ++at) {
-      words[at] = ((s + lane) << 5) + __ffs(m) - 1;
-      m &= m - 1;
-    }
-    __syncwarp();
-    return min(__shfl_sync(FULL, incl, 31), 32);
-  }
+  static __device__ __forceinline__ int low(int w, u32 v) { return v ? (w << 5) + __ffs(v) - 1 : -1; }
 
-  // The first words with set bits, ascending over the lanes: the lane's lowest
-  // set bit (the bitmap's bit index), -1 on lanes without a word; the first of
-  // them is the column's pivot. All -1 when the column is empty.
-  __device__ __forceinline__ int lowest() {
+  // A round's entries, ascending over the lanes: bit indices, -1 beyond them;
+  // lane 0 holds the pivot, -1 when the column is empty. `dense`: the first
+  // group holds RS_DENSE words or more.
+  __device__ __forceinline__ int lowest(bool& dense) {
     const int lane = threadIdx.x & 31;
+    const u32 lt = lanemask_lt();
     for (int s = from; s < ns;) {
       u32 m = s + lane < ns ? sm_ld32(sum + s + lane) : 0u;
       const u32 some = __ballot_sync(FULL, m != 0);
       if (!some) {
-        s += 32;
-        from = s;
+        from = s += 32;
         continue;
       }
-      s += __ffs(some) - 1;
-      from = s;
-      m = s + lane < ns ? sm_ld32(sum + s + lane) : 0u;
-      const int n = take(s, m);
-      const int w = lane < n ? words[lane] : 0;
-      const u32 v = lane < n ? sm_ld32(bits + w) : 0u;
-      // words flipped empty since: their summary bits go
-      if (lane < n && !v) sm_red_and32(sum + (w >> 5), ~(1u << (w & 31)));
-      if (__any_sync(FULL, v != 0)) return v ? (w << 5) + __ffs(v) - 1 : -1;
+      const int g = __ffs(some) - 1;
+      from = s + g;
+      dense = __popc(__shfl_sync(FULL, m, g)) >= RS_DENSE;
+      int e0, e1, at0, at1;
+      u32 live0, live1;
+      if (dense) {
+        const u32 other = some & (some - 1);
+        const int w0 = ((s + g) << 5) + lane, g1 = __ffs(other) - 1, w1 = ((s + g1) << 5) + lane;
+        const u32 v0 = sm_ld32(bits + w0), v1 = other ? sm_ld32(bits + w1) : 0u;
+        live0 = __ballot_sync(FULL, v0 != 0);
+        live1 = __ballot_sync(FULL, v1 != 0);
+        if (lane == 0) {  // words flipped empty since: their summary bits go
+          sm_st32(sum + s + g, live0);
+          if (other) sm_st32(sum + s + g1, live1);
+        }
+        e0 = low(w0, v0);
+        e1 = low(w1, v1);
+        at0 = __popc(live0 & lt);
+        at1 = __popc(live0) + __popc(live1 & lt);
+        __syncwarp();
+      } else {
+        const int w0 = ((s + lane) << 5) + (m ? __ffs(m) - 1 : 0);
+        const u32 m1 = m & (m - 1);
+        const int w1 = ((s + lane) << 5) + (m1 ? __ffs(m1) - 1 : 0);
+        const u32 v0 = m ? sm_ld32(bits + w0) : 0u, v1 = m1 ? sm_ld32(bits + w1) : 0u;
+        const u32 gone = (m && !v0 ? m ^ m1 : 0u) | (m1 && !v1 ? m1 ^ (m1 & (m1 - 1)) : 0u);
+        if (gone) sm_st32(sum + s + lane, m & ~gone);
+        e0 = low(w0, v0);
+        e1 = low(w1, v1);
+        live0 = __ballot_sync(FULL, v0 != 0);
+        live1 = __ballot_sync(FULL, v1 != 0);
+        at0 = __popc(live0 & lt) + __popc(live1 & lt);
+        at1 = at0 + (v0 != 0);
+        __syncwarp();
+        // a group whose first two words were flipped empty may have bits in the
+        // next ones: it has to be looked at again before any later group counts
+        if (__any_sync(FULL, !(v0 | v1) && (m & ~gone))) continue;
+      }
+      const int n = __popc(live0) + __popc(live1);
+      if (!n) continue;
+      if (e0 >= 0 && at0 < 32) slot[at0] = e0;
+      if (e1 >= 0 && at1 < 32) slot[at1] = e1;
       __syncwarp();
+      const int e = lane < n ? slot[lane] : -1;
+      __syncwarp();
+      return e;
     }
     return -1;
   }
 
-  __device__ __forceinline__ int count() const {
+  // f(word, its bits) for every word that may hold set bits, each by one lane:
+  // a lane takes whole groups of a sparse column, its word of every group of a
+  // dense one. The same lane gets the same words in the same order each time.
+  template <typename F>
+  __device__ __forceinline__ void each_word(bool dense, F&& f) const {
     const int lane = threadIdx.x & 31;
-    int c = 0;
-    for (int s = from + lane; s < ns; s += 32)
-      for (u32 m = sm_ld32(sum + s); m; m &= m - 1) c += __popc(sm_ld32(bits + (s << 5) + __ffs(m) - 1));
-    return __reduce_add_sync(FULL, c);
-  }
-
-  // the entries, ascending, to out
-  __device__ __forceinline__ void list(i32* out) const {
-    const int lane = threadIdx.x & 31;
-    int pos = 0;
     for (int s = from; s < ns; s += 32) {
       u32 m = s + lane < ns ? sm_ld32(sum + s + lane) : 0u;
-      while (__any_sync(FULL, m != 0)) {
-        const int n = take(s, m);
-        const int w = lane < n ? words[lane] : 0;
-        u32 v = lane < n ? sm_ld32(bits + w) : 0u;
-        const int c = __popc(v);
-        int incl = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int t = __shfl_up_sync(FULL, incl, o);
-          if (lane >= o) incl += t;
+      if (!dense) {
+        for (; m; m &= m - 1) {
+          const int w = ((s + lane) << 5) + __ffs(m) - 1;
+          f(w, sm_ld32(bits + w));
         }
-        for (int at = pos + incl - c; v; v &= v - 1) out[at++] = (w << 5) + __ffs(v) - 1 + rb;
-        pos += __shfl_sync(FULL, incl, 31);
-        __syncwarp();  // the word list is free
+      } else {
+        for (u32 some = __ballot_sync(FULL, m != 0); some; some &= some - 1) {
+          const int w = ((s + __ffs(some) - 1) << 5) + lane;
+          f(w, sm_ld32(bits + w));
+        }
       }
     }
-    __syncwarp();
   }
 
   __device__ __forceinline__ void clear() {
@@ -1320,111 +1352,158 @@ __global__ void __launch_bounds__(32 * RS_MAX_WARPS, 1)
   D.bits = reinterpret_cast<u32*>(rd_smem) + (size_t)(threadIdx.x >> 5) * rs_warp_words(nw);
   D.sum = D.bits + nw;
   D.ns = nw / 32;
-  D.words = reinterpret_cast<i32*>(D.sum + D.ns);
+  D.slot = reinterpret_cast<i32*>(D.sum + D.ns);
   D.from = 0;
+  D.bad = false;
   for (int i = lane; i < nw + D.ns; i += 32) D.bits[i] = 0u;
   __syncwarp();
   volatile int* vabort = &ctl->abort;
   PoolChunk chunk_state;
   unsigned long long n_merges = 0, n_takeovers = 0;
-  for (;;) {
-    int base = 0;
-    if (lane == 0) base = atomicAdd(&ctl->next, RD_FETCH);
-    base = __shfl_sync(FULL, base, 0);
-    if ((i64)base >= K || *vabort) break;
-    const i64 cand = K - 1 - base - lane;
-    u32 todo = __ballot_sync(FULL, lane < RD_FETCH && cand >= 0 && state[cand] == 2);
-    while (todo && !*vabort) {
-      const int l = __ffs(todo) - 1;
-      todo &= todo - 1;
-      i32 c = (i32)(K - 1 - base - l);
-      u64 wrec = rec[c];      // the column's record while it is as published
-      bool published = true;
-      {
-        const int k = __ldcg(pool + wrec);
-        // entries stay within [first pivot, first pivot + span): the window
-        // starts at the first pivot's word
-        D.rb = row_base + (((__ldcg(pool + wrec + 1) - row_base) >> 5) << 5);
-        D.flip_all(pool + wrec + 1, k);
+  // Columns are taken from the sweep in descending order, a chunk at a time:
+  // the counter and the states are a round trip each, as long as a round of
+  // additions, so chunks are larger where few columns are residual.
+  // (and the columns many, or one warp would get several of the last, longest)
+  const int fetch = (i64)ctl->nres * 16 < K && K >= RS_LONG_SWEEP ? 32 : RD_FETCH;
+
+  // reduces column c, whose record at wrec holds len0 entries, the first of them first0
+  auto reduce_column = [&](i32 c, u64 wrec, int len0, i32 first0) {
+    bool published = true;  // the column is its record
+    // entries stay within [first pivot, first pivot + span): the window starts
+    // at the first pivot's word
+    D.rb = row_base + (((first0 - row_base) >> 5) << 5);
+    D.flip_record(pool + wrec, 0, len0);
+    for (int step = 0;; ++step) {
+      if ((step & 63) == 63 && *vabort) break;
+      if (step >= max_steps) {
+        if (lane == 0) set_status(status, PH_ERR_ITER_LIMIT);
+        atomicExch(&ctl->abort, 1);
+        break;
       }
-      for (int step = 0;; ++step) {
-        if ((step & 63) == 63 && *vabort) break;
-        if (step >= max_steps) {
-          if (lane == 0) set_status(status, PH_ERR_ITER_LIMIT);
-          atomicExch(&ctl->abort, 1);
+      bool dense = false;
+      const int e = D.lowest(dense);
+      const u32 live = __ballot_sync(FULL, e >= 0);
+      if (!live) break;  // the column vanished: it owns nothing
+      const u64 ow = e >= 0 ? ld_acquire(owner + (e + D.rb - row_base)) : 0ull;
+      // what comes before the first entry that is free or owned by a column
+      // not processed yet
+      const u32 stop = __ballot_sync(FULL, e >= 0 && owner_col(ow) <= c);
+      const u32 adds = live & ((stop & (0u - stop)) - 1u);
+      if (!adds) {
+        const i32 p = __shfl_sync(FULL, e, 0) + D.rb;
+        // publish the column as a record (the pivot first, the others in any
+        // order), then claim the pivot
+        if (!published) {
+          if (lane == 0) D.flip(p);
+          __syncwarp();
+          int n = 0;
+          D.each_word(dense, [&](int, u32 v) { n += __popc(v); });
+          int incl = n;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += v;
+          }
+          const int k = __shfl_sync(FULL, incl, 31) + 1;
+          const unsigned long long at = pool_alloc(chunk_state, ctl, pool_cap, k + 1, chunk, status);
+          if (at == ~0ull) break;
+          if (lane == 0) {
+            pool[at] = k;
+            pool[at + 1] = p;
+          }
+          i32* out = pool + at + 2 + (incl - n);
+          D.each_word(dense, [&](int w, u32 v) {
+            for (; v; v &= v - 1) *out++ = (w << 5) + __ffs(v) - 1 + D.rb;
+          });
+          __syncwarp();  // every lane has read its words
+          if (lane == 0) D.flip(p);
+          wrec = at;
+          published = true;
+        }
+        __syncwarp();
+        u64 old = 0;
+        if (lane == 0) old = atom_max_acq_rel(owner + (p - row_base), owner_word(c, wrec));
+        old = __shfl_sync(FULL, old, 0);
+        __syncwarp();
+        const i32 oc = owner_col(old);
+        if (oc < 0) break;  // claimed a free pivot: this work item is done
+        if (oc == c) {      // cannot happen: a column never owns a pivot it is still reducing
+          if (lane == 0) set_status(status, PH_ERR_ARG);
           break;
         }
-        const int e = D.lowest();
-        const u32 live = __ballot_sync(FULL, e >= 0);
-        if (!live) break;  // the column vanished: it owns nothing
-        const u64 ow = e >= 0 ? ld_acquire(owner + (e + D.rb - row_base)) : 0ull;
-        const u32 stop = __ballot_sync(FULL, e >= 0 && owner_col(ow) <= c);
-        const u32 adds = live & ((stop & (0u - stop)) - 1u);  // the lanes below the first that stops
-        if (!adds) {
-          // publish the column as a record, then claim the pivot
-          if (!published) {
-            const int k = D.count();
-            const unsigned long long at = pool_alloc(chunk_state, ctl, pool_cap, k + 1, chunk, status);
-            if (at == ~0ull) break;
-            if (lane == 0) pool[at] = k;
-            D.list(pool + at + 1);
-            wrec = at;
-            published = true;
-          }
-          __syncwarp();
-          const int first = __ffs(live) - 1;
-          u64 old = 0;
-          if (lane == first) old = atom_max_acq_rel(owner + (e + D.rb - row_base), owner_word(c, wrec));
-          old = __shfl_sync(FULL, old, first);
-          __syncwarp();
-          const i32 oc = owner_col(old);
-          if (oc < 0) break;  // claimed a free pivot: this work item is done
-          if (oc == c) {      // cannot happen: a column never owns a pivot it is still reducing
-            if (lane == 0) set_status(status, PH_ERR_ARG);
-            break;
-          }
-          if (oc > c) continue;  // a larger column got there first: it is added in the next round
-          // displaced a smaller column: take it over. The bitmap holds the
-          // claimer's content, which the displaced column adds first: its
-          // record goes into it.
-          ++n_takeovers;
-          c = oc;
-          const u64 at = old & OW_OFF;
-          D.flip_all(pool + at + 1, __ldcg(pool + at));
-          ++n_merges;
-          published = false;
-          continue;
-        }
-        // add the records: length and seven entries a lane in two loads
-        const u64 at = ow & OW_OFF;
-        int len = 0, got = 0;
-        if ((adds >> lane) & 1u) {
-          const int4 a = __ldcg(reinterpret_cast<const int4*>(pool + at));
-          const bool wide = at + 8 <= (u64)pool_cap;
-          int4 b = make_int4(0, 0, 0, 0);
-          if (wide) b = __ldcg(reinterpret_cast<const int4*>(pool + at + 4));
-          len = a.x;
-          got = min(len, wide ? 7 : 3);
-          const i32 v[7] = {a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-          for (int q = 0; q < 7; ++q)
-            if (q < got) D.flip(v[q]);
-        }
-        u32 rest = __ballot_sync(FULL, len > got);
-        while (rest) {  // longer records, by the warp
-          const int r = __ffs(rest) - 1;
-          rest &= rest - 1;
-          const u64 ra = __shfl_sync(FULL, at, r);
-          const int skip = __shfl_sync(FULL, got, r), n = __shfl_sync(FULL, len, r);
-          D.flip_all(pool + ra + 1 + skip, n - skip);
-        }
-        n_merges += __popc(adds);
+        if (oc > c) continue;  // a larger column got there first: it is added in the next round
+        // displaced a smaller column: take it over. The bitmap holds the
+        // claimer's content, which the displaced column adds first: its record
+        // goes into it.
+        ++n_takeovers;
+        c = oc;
+        const u64 at = old & OW_OFF;
+        D.flip_record(pool + at, 0, __ldcg(pool + at));
+        ++n_merges;
         published = false;
-        __syncwarp();
+        continue;
       }
-      D.clear();  // every exit leaves the window clean for the next column
+      // add the records: length and seven entries of each in two loads
+      const u64 at = ow & OW_OFF;
+      int len = 0, got = 0;
+      if ((adds >> lane) & 1u) {
+        const bool wide = at + 8 <= (u64)pool_cap;
+        const int4 x = __ldcg(reinterpret_cast<const int4*>(pool + at));
+        int4 y = make_int4(0, 0, 0, 0);
+        if (wide) y = __ldcg(reinterpret_cast<const int4*>(pool + at + 4));
+        len = x.x;
+        got = min(len, wide ? 7 : 3);
+        const i32 v[7] = {x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int k = 0; k < 7; ++k)
+          if (k < got) D.flip(v[k]);
+      }
+      // longer records: the next 32 entries of four of them in flight, then
+      // what is longer still
+      for (u32 rest = __ballot_sync(FULL, len > got); rest;) {
+        u64 ra[4];
+        int skip[4], n[4];
+        i32 x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int l = rest ? __ffs(rest) - 1 : 0;
+          ra[k] = __shfl_sync(FULL, at, l);
+          skip[k] = __shfl_sync(FULL, got, l);
+          n[k] = rest ? __shfl_sync(FULL, len, l) : 0;
+          rest &= rest - 1;
+          if (skip[k] + lane < n[k]) x[k] = __ldcg(pool + ra[k] + 1 + skip[k] + lane);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (skip[k] + lane < n[k]) D.flip(x[k]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (n[k] > skip[k] + 32) D.flip_record(pool + ra[k], skip[k] + 32, n[k]);
+      }
+      n_merges += __popc(adds);
+      published = false;
+      __syncwarp();
+    }
+    D.clear();  // every exit leaves the window clean for the next column
+  };
+
+  for (;;) {
+    int base = 0;
+    if (lane == 0) base = atomicAdd(&ctl->next, fetch);
+    base = __shfl_sync(FULL, base, 0);
+    if (base < 0 || (i64)base >= K || *vabort) break;
+    const i64 mine = K - 1 - base - lane;
+    const bool res = lane < fetch && mine >= 0 && state[mine] == 2;
+    // the records' places and heads of all of them at once
+    const u64 at = res ? rec[mine] : 0ull;
+    const int4 h = res ? __ldcg(reinterpret_cast<const int4*>(pool + at)) : make_int4(0, 0, 0, 0);
+    for (u32 todo = __ballot_sync(FULL, res); todo && !*vabort; todo &= todo - 1) {
+      const int l = __ffs(todo) - 1;
+      reduce_column((i32)(K - 1 - base - l), __shfl_sync(FULL, at, l), __shfl_sync(FULL, h.x, l),
+                    __shfl_sync(FULL, h.y, l));
     }
   }
+  if (D.bad) set_status(status, PH_ERR_ARG);
   if (lane == 0) {
     if (n_merges) atomicAdd(&ctl->merges, n_merges);
     if (n_takeovers) atomicAdd(&ctl->takeovers, n_takeovers);
@@ -1499,7 +1578,7 @@ int reduce_blocks(i64 K) {
 i64 window_words(i64 span) { return ((span + 31) / 32 + 2 + 31) / 32 * 32; }
 
 // warps a block whose windows fit shared memory together (up to RS_MAX_WARPS),
-// 0 when not even one does: spans of up to 1.79M rows fit, of 0.45M four
+// 0 when not even one does: spans of up to 1.79M rows fit, of 0.22M eight
 int shared_warps(i64 span) {
   const i64 words = window_words(span);
   if (words > (i64)(RS_SMEM / 4)) return 0;

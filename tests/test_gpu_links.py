@@ -112,3 +112,15 @@ def test_row_beyond_the_shared_memory_sort(monkeypatch):
     staged = rips_persistence(x, T, max_dim=1)
     for a, b in zip(native, staged):
         assert np.array_equal(_bits(a.cpu().numpy()), _bits(b.cpu().numpy()))
+
+
+def test_reduction_beyond_shared_memory_windows(monkeypatch):
+    """2.8M triangle rows in the stage by stage form (beyond the 1.79M that the
+    shared-memory reduction takes: the general kernel), 0.09M in the native
+    call: the same rows."""
+    from flashph_b200 import rips_persistence
+    x = torch.from_numpy(np.random.default_rng(0).standard_normal((1000, 3)).astype(np.float32)).cuda()
+    want = _staged(monkeypatch, x, 1.269, 1)
+    got = rips_persistence(x, 1.269, max_dim=1)
+    for a, b in zip(got, want):
+        assert np.array_equal(_bits(a.cpu().numpy()), _bits(b.cpu().numpy()))
