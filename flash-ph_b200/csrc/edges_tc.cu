@@ -37,25 +37,40 @@
 // (non-finite or huge points, |y^|^2 >= 2^120, or a huge threshold) skips
 // the screen and recomputes every pair exactly.
 //
-// Kernel anatomy (one persistent CTA per SM, 10 warps, a contiguous range of
-// work items; an item is row block I (128 points) against column blocks
-// J .. J + nb - 1, nb = 2 (MMA N = 256) unless the operand rings would not
-// fit shared memory, rows in order, clipped at the cloud's last block):
-//   warp 8 (producer) : TMA loads (cp.async.bulk.tensor, 2-D, swizzled, no
-//                       multicast) of the A tile (row block I, reused while I
-//                       is unchanged) and the B tile (column block J) into
-//                       shared-memory rings, completion on mbarriers
-//   warp 9 (MMA)      : one thread issues ceil((d + 4) / 16) tcgen05.mma
-//                       (M = N = 128, K = 16) into one of two TMEM
-//                       accumulator stages, tcgen05.commit frees the operand
-//                       stages and publishes the accumulator
-//   warps 0-7         : two warpgroups taking alternate tiles (one TMEM
-//                       stage each); a warp reads its 32 TMEM lanes x 128
-//                       columns (two tcgen05.ld in flight), a min pre-check
-//                       then one compare + ballot per column, candidates
-//                       compacted into a per-warp queue that spans tiles and
-//                       is recomputed with the exact chain 32 pairs at a
-//                       time, with warp-aggregated emission
+// Kernel anatomy (one persistent CTA per SM, 18 warps, a contiguous range of
+// work items; an item is nr row blocks of 128 points, I and I + 1, against nb
+// column blocks J and J + 1 (MMA N = 256), one accumulator a row block; one row
+// block an item, and one column block, where the operand rings would not fit
+// shared memory otherwise; rows in order, clipped at the cloud's last block):
+//   warp 16 (producer): TMA loads (cp.async.bulk.tensor, 2-D, swizzled, no
+//                       multicast) of the A tiles (row blocks, reused while
+//                       they are unchanged) and the B tile (column blocks,
+//                       read once for both row blocks) into shared-memory
+//                       rings, completion on mbarriers
+//   warp 17 (MMA)     : one thread issues ceil((d + 4) / 16) tcgen05.mma
+//                       (M = 128, N = 128 nb, K = 16) a row block, into the two
+//                       TMEM accumulators in turn; tcgen05.commit publishes the
+//                       accumulator and frees the operand stages
+//   warps 0-15        : four warpgroups, each one quarter of every accumulator's
+//                       columns (so that one accumulator is filled while the
+//                       other is read, and an item's thresholds are computed
+//                       once for its two row blocks); a warp reads its 32 TMEM
+//                       lanes x 64 columns in two loads (32 registers, no
+//                       spills at the 96 that 18 warps leave each), a tree of
+//                       three-input minima and one vote; only a chunk that
+//                       holds a candidate is read again, compared value by
+//                       value and compacted into a per-warp queue that spans
+//                       items and is recomputed with the exact chain 32 pairs
+//                       at a time, with warp-aggregated emission
+// What bounds it: an item (2 x 2 blocks) takes ~2,700 cycles at K = 16 and
+// ~3,100 at K = 64, in which a warp of the epilogue spends ~850 on loads and
+// minima, ~650 waiting for the accumulators, ~550 on the item's thresholds and
+// ~200 on candidates, and the MMA thread ~280 a row block and ~170 a K step on
+// issue. Eight warps with one row block an item (the epilogue's loads not
+// overlapped with the next item's MMAs): 200,000 x 10 at 1.1 3.86 ms, 200,000 x
+// 50 at 6.0 4.67 ms; this form 3.08 and 4.05 ms. Accumulators of N = 128, four
+// in TMEM: 4.3 and 6.3 ms (the operand reads bound the MMA); 64 columns in one
+// go in 64 registers: 4.5 and 7.5 ms (spills).
 // Each cloud's operand rows are padded to a multiple of 128 with rows whose
 // augmented columns carry 2^100, so padding never passes the screen. Every
 // wait is bounded (a few seconds of global time); a timeout sets
@@ -75,11 +90,11 @@ namespace {
 constexpr int TC_T = 128;                 // tile side (points)
 constexpr int TC_MAXK = 256;              // augmented K supported (d <= 252)
 constexpr int TC_AUG = 4;                 // augmented columns
-constexpr int TC_EPI_WARPS = 8;
-constexpr int TC_PRODUCER_WARP = 8;
-constexpr int TC_MMA_WARP = 9;
-constexpr int TC_THREADS = 320;
-constexpr int TC_QCAP = 512;              // candidate pairs queued per epilogue warp (across tiles)
+constexpr int TC_EPI_WARPS = 16;
+constexpr int TC_PRODUCER_WARP = 16;
+constexpr int TC_MMA_WARP = 17;
+constexpr int TC_THREADS = 576;
+constexpr int TC_QCAP = 256;              // candidate pairs queued per epilogue warp (across tiles)
 constexpr int TC_MAX_STAGES = 6;
 constexpr unsigned FULL = 0xffffffffu;
 constexpr unsigned long long TC_WAIT_NS = 4000000000ull;
@@ -91,12 +106,13 @@ struct TcShape {
   int box_k;         // K columns per TMA box and swizzle row: min(kq, 64)
   int natoms;        // K atoms (TMA boxes along K) per operand
   int row_bytes;     // box_k x 2
+  int nr;            // 128-point row blocks per work item (1 or 2)
   int nb;            // 128-point column blocks per work item (1 or 2: MMA N = 128 nb)
   int a_atom_bytes;  // 128 rows x row_bytes
   int b_atom_bytes;  // 128 nb rows x row_bytes
   int a_bytes;       // natoms x a_atom_bytes
   int b_bytes;       // natoms x b_atom_bytes
-  int ns, na;        // B and A ring stages
+  int ns, na;        // B and A ring stages (an A stage holds nr tiles)
   u32 layout;        // UMMA layout type: 6 = 32-byte, 4 = 64-byte, 2 = 128-byte swizzle
   u32 sbo;           // 8-row group stride (8 x row_bytes) >> 4
 };
@@ -118,35 +134,40 @@ __device__ __forceinline__ int find_off(const i64* off, int nsegs, i64 b) {
   return lo;
 }
 
-// Work items of a cloud with nt 128-point blocks: row block I against column
-// blocks J .. J + nb - 1 (clipped at nt), J = I, I + nb, ...; rows in order.
-// items(I) = ceil((nt - I) / nb); rows_before(I) = sum of items(r), r < I.
-__host__ __device__ inline i64 tc_rows_before(i64 I, i64 nt, int nb) {
-  if (nb == 1) return I * nt - I * (I - 1) / 2;
+// Work items of a cloud with nt 128-point blocks: row group P (blocks P nr ..
+// P nr + nr - 1, clipped at nt) against column blocks J .. J + nb - 1 (clipped
+// at nt), J = P nr, P nr + nb, ...; groups in order. items(P) = ceil((nt - P nr)
+// / nb); items_before(P) = sum of items(p), p < P. nr = 2 comes with nb = 2.
+__host__ __device__ inline i64 tc_items_before(i64 P, i64 nt, int nr, int nb) {
+  if (nr == 2) {
+    const i64 np = (nt + 1) / 2;
+    return P * np - P * (P - 1) / 2;
+  }
+  if (nb == 1) return P * nt - P * (P - 1) / 2;
   auto F = [](i64 M) { return (M & 1) ? ((M + 1) / 2) * ((M + 1) / 2) : (M / 2) * (M / 2 + 1); };
-  return F(nt) - F(nt - I);
+  return F(nt) - F(nt - P);
 }
 
-__host__ __device__ inline i64 tc_cloud_items(i64 n, int nb) {
+__host__ __device__ inline i64 tc_cloud_items(i64 n, int nr, int nb) {
   if (n < 2) return 0;
   const i64 nt = (n + TC_T - 1) / TC_T;
-  return tc_rows_before(nt, nt, nb);
+  return tc_items_before((nt + nr - 1) / nr, nt, nr, nb);
 }
 
-// walks the global item sequence: clouds in table order, rows I, column blocks J
+// walks the global item sequence: clouds in table order, row groups, column
+// blocks (block numbers fit 32 bits: the launch checks it)
 struct ItemIt {
   const ph_cloud_seg* segs;
   const i64* blk_off;
   const i64* item_off;
-  int nsegs, nb, c;
-  i64 I, J, nt, blk;
-  ph_cloud_seg sg;
-  __device__ int nh() const { return (nt - J) < nb ? (int)(nt - J) : nb; }  // column blocks in this item
+  int nsegs, nr, nb, c;
+  int I, J, nt, blk;  // first row block, first column block, blocks of the cloud, its first block
+  __device__ int nh() const { return nt - J < nb ? nt - J : nb; }     // column blocks in this item
+  __device__ int rows() const { return nt - I < nr ? nt - I : nr; }   // row blocks in this item
   __device__ bool row_end() const { return J + nb >= nt; }
   __device__ void load() {
-    sg = segs[c];
-    nt = (sg.n + TC_T - 1) / TC_T;
-    blk = blk_off[c];
+    nt = (segs[c].n + TC_T - 1) / TC_T;
+    blk = (int)blk_off[c];
   }
   __device__ void start(i64 q) {
     // clouds without items share their successor's offset; take the last such entry
@@ -159,20 +180,21 @@ struct ItemIt {
     c = lo;
     load();
     const i64 local = q - item_off[c];
-    i64 a = 0, b = nt - 1;  // largest I with rows_before(I) <= local
+    i64 a = 0, b = (nt + nr - 1) / nr - 1;  // largest P with items_before(P) <= local
     while (a < b) {
       const i64 mid = (a + b + 1) >> 1;
-      if (tc_rows_before(mid, nt, nb) <= local) a = mid;
+      if (tc_items_before(mid, nt, nr, nb) <= local) a = mid;
       else b = mid - 1;
     }
-    I = a;
-    J = I + (i64)nb * (local - tc_rows_before(I, nt, nb));
+    I = (int)a * nr;
+    J = I + nb * (int)(local - tc_items_before(a, nt, nr, nb));
   }
   // only called while another item exists
   __device__ void next() {
     J += nb;
     if (J < nt) return;
-    if (++I < nt) {
+    I += nr;
+    if (I < nt) {
       J = I;
       return;
     }
@@ -185,7 +207,7 @@ struct ItemIt {
 };
 
 // item_off[c] = items of clouds before c, item_off[nsegs] = total (one block)
-__global__ void k_tc_items(const ph_cloud_seg* __restrict__ segs, int nsegs, int nb, i64* __restrict__ item_off) {
+__global__ void k_tc_items(const ph_cloud_seg* __restrict__ segs, int nsegs, int nr, int nb, i64* __restrict__ item_off) {
   ph::pdl_wait();
   ph::pdl_trigger();
   __shared__ i64 part[1024];
@@ -193,7 +215,7 @@ __global__ void k_tc_items(const ph_cloud_seg* __restrict__ segs, int nsegs, int
   const int chunk = (nsegs + nt - 1) / nt;
   const int c0 = tid * chunk, c1 = min(nsegs, c0 + chunk);
   i64 sum = 0;
-  for (int c = c0; c < c1; ++c) sum += tc_cloud_items(segs[c].n, nb);
+  for (int c = c0; c < c1; ++c) sum += tc_cloud_items(segs[c].n, nr, nb);
   part[tid] = sum;
   __syncthreads();
   for (int o = 1; o < nt; o <<= 1) {  // inclusive scan
@@ -205,7 +227,7 @@ __global__ void k_tc_items(const ph_cloud_seg* __restrict__ segs, int nsegs, int
   i64 run = part[tid] - sum;
   for (int c = c0; c < c1; ++c) {
     item_off[c] = run;
-    run += tc_cloud_items(segs[c].n, nb);
+    run += tc_cloud_items(segs[c].n, nr, nb);
   }
   if (tid == nt - 1) item_off[nsegs] = part[tid];
 }
@@ -418,7 +440,36 @@ __device__ __forceinline__ void tmem_ld32_issue(u32 taddr, u32 (&r)[32]) {
       : "r"(taddr));
 }
 
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// waits for the loads issued, as a definition of the values loaded: no use of
+// them moves above it
+__device__ __forceinline__ void tmem_ld_wait(u32 (&r)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+                 "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]),
+                 "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]),
+                 "+r"(r[30]), "+r"(r[31])
+               :
+               : "memory");
+}
+
+// the smallest of three values, and of a lane's 32 (16 instructions)
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float least32(const u32 (&v)[32]) {
+  float m[12];
+#pragma unroll
+  for (int k = 0; k < 10; ++k)
+    m[k] = min3(__uint_as_float(v[3 * k]), __uint_as_float(v[3 * k + 1]), __uint_as_float(v[3 * k + 2]));
+  m[10] = __uint_as_float(v[30]);
+  m[11] = __uint_as_float(v[31]);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) m[k] = min3(m[3 * k], m[3 * k + 1], m[3 * k + 2]);
+  return fminf(min3(m[0], m[1], m[2]), m[3]);
+}
 
 // the exact FP32 chain of ph_edges_enumerate
 __device__ __forceinline__ float exact_dsq(const float* __restrict__ x, const float* __restrict__ y, int d) {
@@ -480,10 +531,57 @@ __device__ __noinline__ void flush_queue(const uint2* __restrict__ queue, int cn
   __syncwarp();
 }
 
+// What a warp of the epilogue keeps between candidates.
+struct Epilogue {
+  uint2* queue;  // cloud-local pairs
+  int cnt;
+  ph_cloud_seg qs;  // their cloud
+  const float* pts;
+  i32 *oi, *oj;
+  float* od;
+  i64 cap;
+  unsigned long long* count;
+  unsigned long long n_cand;
+
+  __device__ void flush() {
+    flush_queue(queue, cnt, qs, pts, oi, oj, od, cap, count);
+    n_cand += (unsigned long long)cnt;
+    cnt = 0;
+  }
+};
+
+// The candidates among a warp's columns of the accumulator (read again: few
+// chunks hold one), queued: one compare per pair into a lane mask, the set bits one
+// per lane and round. Out of line, as flush_queue.
+__device__ __noinline__ void screen_chunk(Epilogue& e, u32 taddr, u32 i, u32 j0, int cols, float bound) {
+  const u32 lt = lanemask_lt();
+#pragma unroll 1
+  for (int half = 0; half < cols; half += 32) {
+    u32 v[32];
+    tmem_ld32_issue(taddr + (u32)half, v);
+    tmem_ld_wait(v);
+    u32 mask = 0;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) mask |= (__uint_as_float(v[k]) < bound ? 1u : 0u) << k;
+#pragma unroll 1
+    while (__any_sync(FULL, mask != 0)) {
+      const bool has = mask != 0;
+      const u32 m = __ballot_sync(FULL, has);
+      if (e.cnt + 32 > TC_QCAP) e.flush();
+      if (has) {
+        e.queue[e.cnt + __popc(m & lt)] = make_uint2(i, j0 + half + (u32)__ffs(mask) - 1u);
+        mask &= mask - 1;
+      }
+      e.cnt += __popc(m);
+    }
+  }
+}
+
 // ---- main kernel ------------------------------------------------------------------------
 // barrier slots: B full [0, 6), B empty [6, 12), A full [12, 14), A empty [14, 16),
-// TMEM full [16, 18), TMEM empty [18, 20)
-constexpr int BAR_BF = 0, BAR_BE = 6, BAR_AF = 12, BAR_AE = 14, BAR_TF = 16, BAR_TE = 18, BAR_N = 20;
+// TMEM full [16, 18), TMEM empty [18, 20), the MMA thread's own 20
+constexpr int BAR_BF = 0, BAR_BE = 6, BAR_AF = 12, BAR_AE = 14, BAR_TF = 16, BAR_TE = 18, BAR_DRAIN = 20, BAR_N = 21;
+constexpr u32 TC_TMEM_COLS = 4 * TC_T;  // two accumulators of two column blocks
 
 __global__ void __launch_bounds__(TC_THREADS, 1)
     k_tc_edges(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -500,13 +598,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   __shared__ unsigned long long st_sh[2];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sA = smem;
-  unsigned char* sB = smem + sh.na * sh.a_bytes;
+  const int a_stage = sh.nr * sh.a_bytes;
+  unsigned char* sB = smem + sh.na * a_stage;
   uint2* qbase = reinterpret_cast<uint2*>(sB + sh.ns * sh.b_bytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const u32 bar0 = smem_u32(bars);
   auto bar = [bar0](int slot) { return bar0 + 8u * (u32)slot; };
   volatile int* abort_flag = &abort_sh;
-  const u32 stage_cols = (u32)(TC_T * sh.nb);  // TMEM columns per accumulator stage
 
   // contiguous item range of this CTA
   const i64 nitems = item_off[nsegs];
@@ -522,8 +620,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     for (int s = 0; s < 2; ++s) {
       mbar_init(bar(BAR_AF + s), 1);
       mbar_init(bar(BAR_AE + s), 1);
+    }
+    mbar_init(bar(BAR_DRAIN), 1);
+    for (int s = 0; s < 2; ++s) {
       mbar_init(bar(BAR_TF + s), 1);
-      mbar_init(bar(BAR_TE + s), TC_EPI_WARPS / 2);
+      mbar_init(bar(BAR_TE + s), TC_EPI_WARPS);
     }
     abort_sh = 0;
     st_sh[0] = st_sh[1] = 0;
@@ -531,7 +632,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   }
   if (warp == TC_MMA_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)),
-                 "r"(2 * stage_cols));
+                 "r"(TC_TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -541,7 +642,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 
   if (T > 0 && warp == TC_PRODUCER_WARP) {
     if (lane == 0) {
-      ItemIt it{segs, blk_off, item_off, nsegs, sh.nb};
+      ItemIt it{segs, blk_off, item_off, nsegs, sh.nr, sh.nb};
       it.start(b0);
       // ring positions kept incrementally (no divisions on this thread); a_ph /
       // b_ph = (use + 1) & 1 for the current use of the stage, which is the
@@ -563,10 +664,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             a_ph ^= 1;
           }
           if (u >= sh.na && !(ok = mbar_wait(bar(BAR_AE + as), a_ph, abort_flag))) break;
-          mbar_expect_tx(bar(BAR_AF + as), (u32)sh.a_bytes);
-          const int y = (int)(TC_T * (it.blk + it.I));
-          for (int a = 0; a < sh.natoms; ++a)
-            tma_load_2d(smem_u32(sA + as * sh.a_bytes + a * sh.a_atom_bytes), &tmA, a * 64, y, bar(BAR_AF + as));
+          const int rows = it.rows();
+          mbar_expect_tx(bar(BAR_AF + as), (u32)(rows * sh.a_bytes));
+          for (int r = 0; r < rows; ++r)
+            for (int a = 0; a < sh.natoms; ++a)
+              tma_load_2d(smem_u32(sA + as * a_stage + r * sh.a_bytes + a * sh.a_atom_bytes), &tmA, a * 64,
+                          TC_T * (it.blk + it.I + r), bar(BAR_AF + as));
         }
         if (++bs == sh.ns) {
           bs = 0;
@@ -575,7 +678,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         if (t >= sh.ns && !(ok = mbar_wait(bar(BAR_BE + bs), b_ph, abort_flag))) break;
         const int nh = it.nh();
         mbar_expect_tx(bar(BAR_BF + bs), (u32)(sh.natoms * nh * sh.a_atom_bytes));
-        const int y = (int)(TC_T * (it.blk + it.J));
+        const int y = TC_T * (it.blk + it.J);
         for (int a = 0; a < sh.natoms; ++a)
           for (int h = 0; h < nh; ++h)
             tma_load_2d(smem_u32(sB + bs * sh.b_bytes + a * sh.b_atom_bytes + h * sh.a_atom_bytes), &tmB, a * 64,
@@ -596,14 +699,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       const u32 idesc1 = umma_idesc_bf16_f32(TC_T, TC_T), idesc2 = umma_idesc_bf16_f32(TC_T, 2 * TC_T);
       const int spa = sh.box_k / 16;  // K slices per swizzle row
       const u64 a_step = (u64)(sh.a_atom_bytes >> 4), b_step = (u64)(sh.b_atom_bytes >> 4);
-      ItemIt it{segs, blk_off, item_off, nsegs, sh.nb};
+      ItemIt it{segs, blk_off, item_off, nsegs, sh.nr, sh.nb};
       it.start(b0);
       // as for the producer; the full-barrier phase of use v has parity v & 1
       int as = -1, bs = -1;
       u32 a_ph = 1, b_ph = 1;
       bool new_a = true;
-      i64 done = 0;
+      i64 unit = 0;  // row blocks issued: accumulator unit & 1, phase (unit >> 1) & 1
       bool ok = true;
+      int ks = 0, cloud = -1;
       for (i64 t = 0; t < T; ++t) {
         if (t) {
           new_a = it.row_end();
@@ -614,6 +718,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             as = 0;
             a_ph ^= 1;
           }
+          if (it.c != cloud) {
+            cloud = it.c;
+            ks = (segs[cloud].d + TC_AUG + 15) / 16;
+          }
           if (!(ok = mbar_wait(bar(BAR_AF + as), a_ph ^ 1, abort_flag))) break;
         }
         const bool last_a = (t + 1 == T) || it.row_end();
@@ -622,167 +730,150 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           b_ph ^= 1;
         }
         if (!(ok = mbar_wait(bar(BAR_BF + bs), b_ph ^ 1, abort_flag))) break;
-        const int ts = (int)(t & 1);
-        if (t >= 2 && !(ok = mbar_wait(bar(BAR_TE + ts), (u32)((t >> 1) - 1) & 1, abort_flag))) break;
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const int ks = (it.sg.d + TC_AUG + 15) / 16;
+        const int rows = it.rows();
         const u32 idesc = it.nh() == 2 ? idesc2 : idesc1;
-        const u64 da0 = umma_desc(smem_u32(sA + as * sh.a_bytes), sh.layout, sh.sbo);
         const u64 db0 = umma_desc(smem_u32(sB + bs * sh.b_bytes), sh.layout, sh.sbo);
-        // K slice s sits in swizzle atom s / spa at 32-byte step s % spa, kept
-        // incrementally: a division per MMA on this one thread cost more than
-        // the MMA itself
-        u64 da = da0, db = db0;
-        for (int s = 0, sub = 0; s < ks; ++s) {
-          umma_bf16(tmem + (u32)ts * stage_cols, da, db, idesc, s > 0 ? 1u : 0u);
-          if (++sub == spa) {
-            sub = 0;
-            da += a_step - (u64)(2 * (spa - 1));
-            db += b_step - (u64)(2 * (spa - 1));
-          } else {
-            da += 2;
-            db += 2;
+        for (int r = 0; r < sh.nr; ++r, ++unit) {
+          const int ts = (int)(unit & 1);
+          if (unit >= 2 && !(ok = mbar_wait(bar(BAR_TE + ts), (u32)((unit >> 1) - 1) & 1, abort_flag))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          // K slice s sits in swizzle atom s / spa at 32-byte step s % spa, kept
+          // incrementally: a division per MMA on this one thread cost more than
+          // the MMA itself
+          if (r < rows) {
+            u64 da = umma_desc(smem_u32(sA + as * a_stage + r * sh.a_bytes), sh.layout, sh.sbo), db = db0;
+            for (int s = 0, sub = 0; s < ks; ++s) {
+              umma_bf16(tmem + (u32)(2 * ts * TC_T), da, db, idesc, s > 0 ? 1u : 0u);
+              if (++sub == spa) {
+                sub = 0;
+                da += a_step - (u64)(2 * (spa - 1));
+                db += b_step - (u64)(2 * (spa - 1));
+              } else {
+                da += 2;
+                db += 2;
+              }
+            }
           }
+          umma_commit(bar(BAR_TF + ts));  // at once where the cloud has no such row block
         }
+        if (!ok) break;
         umma_commit(bar(BAR_BE + bs));
-        umma_commit(bar(BAR_TF + ts));
         if (last_a) umma_commit(bar(BAR_AE + as));
-        done = t + 1;
       }
       if (!ok) {
         set_status(status, PH_ERR_ITER_LIMIT);
-        // drain: the accumulators of the last MMAs issued
-        for (i64 k = (done > 2 ? done - 2 : 0); k < done; ++k)
-          mbar_wait(bar(BAR_TF + (int)(k & 1)), (u32)(k / 2) & 1, nullptr);
+        // drain: the MMAs issued (a commit after them arrives when they are done)
+        umma_commit(bar(BAR_DRAIN));
+        mbar_wait(bar(BAR_DRAIN), 0, nullptr);
       }
     }
     __syncwarp();
   } else if (T > 0 && warp < TC_EPI_WARPS) {
-    // warpgroup g takes the items t = g, g + 2, ... (TMEM stage g). Candidates
-    // are queued as cloud-local pairs across items and recomputed 32 at a
-    // time (when the queue fills, the cloud changes, or the range ends), so the
-    // latency of the exact chain's loads is paid once per 32 candidates.
+    // Warpgroup g takes the g-th quarter of every accumulator's columns: half a
+    // column block of an item, or a quarter of the only one. Candidates are
+    // queued as cloud-local pairs across items and recomputed 32 at a time (when
+    // the queue fills, the cloud changes, or the range ends), so the latency of
+    // the exact chain's loads is paid once per 32 candidates.
     const int q4 = warp & 3, g = warp >> 2;
-    const int row = q4 * 32 + lane;
-    const u32 lt = lanemask_lt();
-    uint2* queue = qbase + warp * TC_QCAP;
-    unsigned long long n_cand = 0, n_forced = 0;
-    int cnt = 0;
-    ph_cloud_seg qs{};  // cloud of the queued candidates
-    float sqthr = 0.0f;  // sqrt of the widened threshold of that cloud, rounded up
-    auto flush = [&]() {
-      flush_queue(queue, cnt, qs, pts_all, oi, oj, od, cap, count);
-      n_cand += (unsigned long long)cnt;
-      cnt = 0;
-    };
-    ItemIt it{segs, blk_off, item_off, nsegs, sh.nb};
+    const int cols = 32 * sh.nb;            // columns of this warp
+    const u32 col = (u32)(cols * g);        // the first of them
+    const int h = (int)(col / (u32)TC_T);   // their column block of the item
+    Epilogue ep{qbase + warp * TC_QCAP, 0, ph_cloud_seg{}, pts_all, oi, oj, od, cap, count, 0};
+    unsigned long long n_forced = 0;
+    float sqthr = 0.0f;          // sqrt of the widened threshold of the cloud, rounded up
+    float rt[2] = {0.0f, 0.0f};  // that plus the rounding radius of each row block
+    int cloud = -1, group = -1;
+    ItemIt it{segs, blk_off, item_off, nsegs, sh.nr, sh.nb};
     it.start(b0);
-    if (g == 1 && T > 1) it.next();
-    for (i64 t = g; t < T; t += 2) {
-      const ph_cloud_seg& sg = it.sg;
-      const bool new_cloud = sg.pt_off != qs.pt_off || sg.vbase != qs.vbase || t == g;
-      if (cnt && new_cloud) flush();
-      qs = sg;
-      const int nh = it.nh();
-      const i64 i0 = it.I * TC_T, j0 = it.J * TC_T;
-      // widened thresholds of the item's column blocks, computed while the MMAs
+    float rj = it.nh() > h ? blkrad[it.blk + it.J + h] : 0.0f;  // of the column block, loaded an item ahead
+    const u32 taddr = tmem + ((u32)(q4 * 32) << 16) + col;
+    u32 unit = 0;  // row blocks met: accumulator unit & 1, phase (unit >> 1) & 1
+    bool ok = true;
+    for (i64 t = 0; t < T; ++t) {
+      if (it.c != cloud || it.I != group) {
+        if (it.c != cloud) {
+          if (ep.cnt) ep.flush();
+          cloud = it.c;
+          ep.qs = segs[cloud];
+          sqthr = __double2float_ru(sqrt((double)ep.qs.thr_sq * thr_scale));
+        }
+        group = it.I;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) rt[r] = it.rows() > r ? __fadd_ru(sqthr, blkrad[it.blk + it.I + r]) : 0.0f;
+      }
+      const int rows = it.rows();
+      const bool here = it.nh() > h;  // the item has this warpgroup's column block
+      const u32 i0 = (u32)(it.I * TC_T), j0 = (u32)(it.J * TC_T) + col;
+      // widened thresholds of the item's row blocks, computed while the MMAs
       // run: (sqrt(thr') + r_I + r_J)^2 (1 + 2^-20) + 2^-96 with every FP32
       // operation rounded up (an upper bound of that value; the square root,
       // in FP64, once per cloud)
-      if (new_cloud) sqthr = __double2float_ru(sqrt((double)sg.thr_sq * thr_scale));
-      const float rt = __fadd_ru(sqthr, blkrad[it.blk + it.I]);
-      float base[2];
+      float bound[2];
       bool force[2];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float radius = __fadd_ru(rt, h < nh ? blkrad[it.blk + it.J + h] : 0.0f);
+      for (int r = 0; r < 2; ++r) {
+        const float radius = __fadd_ru(rt[r], rj);
         const float b = __fadd_ru(__fmul_ru(__fmul_ru(radius, radius), 1.0f + 0x1p-20f), 0x1p-96f);
-        force[h] = !(b < 3.0e38f);
-        base[h] = force[h] ? 0.0f : b;
+        force[r] = here && !(b < 3.0e38f);
+        bound[r] = force[r] ? -INFINITY : b;  // nothing passes: every pair is recomputed
       }
-      // one compare per pair into a lane mask; the set bits are queued one per
-      // lane per round (a round per candidate in the densest lane)
-      // the smallest of a lane's 32 values (a min tree)
-      auto vmin = [](const u32 (&v)[32]) {
-        float m16[16];
-#pragma unroll
-        for (int k = 0; k < 16; ++k) m16[k] = fminf(__uint_as_float(v[k]), __uint_as_float(v[k + 16]));
-#pragma unroll
-        for (int w = 8; w > 0; w >>= 1)
-#pragma unroll
-          for (int k = 0; k < w; ++k) m16[k] = fminf(m16[k], m16[k + w]);
-        return m16[0];
-      };
-      // the candidates among a lane's 32 values, queued
-      auto screen = [&](const u32 (&v)[32], int c0, float bs_) {
-        u32 mask = 0;
-#pragma unroll
-        for (int k = 0; k < 32; ++k) mask |= (__uint_as_float(v[k]) < bs_ ? 1u : 0u) << k;
+      if (t + 1 < T) {
+        it.next();
+        rj = it.nh() > h ? blkrad[it.blk + it.J + h] : 0.0f;
+      }
 #pragma unroll 1
-        while (__any_sync(FULL, mask != 0)) {
-          const bool has = mask != 0;
-          const u32 m = __ballot_sync(FULL, has);
-          if (cnt + 32 > TC_QCAP) flush();
-          if (has) {
-            const int k = __ffs(mask) - 1;
-            queue[cnt + __popc(m & lt)] = make_uint2((u32)(i0 + row), (u32)(j0 + c0 + k));
-            mask &= mask - 1;
+      for (int r = 0; r < sh.nr; ++r, ++unit) {
+        const int ts = (int)(unit & 1);
+        if (!(ok = __all_sync(FULL, mbar_wait(bar(BAR_TF + ts), (unit >> 1) & 1, abort_flag)) != 0)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const float b = r ? bound[1] : bound[0];
+        const u32 ta = taddr + (u32)(2 * ts * TC_T);
+        if (here && r < rows) {
+          float least;
+          {
+            u32 x[32];
+            tmem_ld32_issue(ta, x);
+            tmem_ld_wait(x);
+            least = least32(x);
           }
-          cnt += __popc(m);
+          if (sh.nb == 2) {
+            u32 x[32];
+            tmem_ld32_issue(ta + 32u, x);
+            tmem_ld_wait(x);
+            least = fminf(least, least32(x));
+          }
+          if (__any_sync(FULL, least < b))
+            screen_chunk(ep, ta, i0 + (u32)(r * TC_T + q4 * 32 + lane), j0, cols, b);
         }
-      };
-      int okw = 1;
-      if (lane == 0) okw = mbar_wait(bar(BAR_TF + g), (u32)(t >> 1) & 1, abort_flag) ? 1 : 0;
-      okw = __shfl_sync(FULL, okw, 0);
-      if (!okw) {
-        if (lane == 0) set_status(status, PH_ERR_ITER_LIMIT);
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(BAR_TE + ts));
+        if (r ? force[1] : force[0]) {
+          // no screen for this block: every pair of the warp's rows exactly
+          if (r >= rows) continue;
+          n_forced += 32 * cols;
+          const float* P = pts_all + ep.qs.pt_off;
+          const i64 gi = i0 + r * TC_T + q4 * 32 + lane;
+          for (int k = 0; k < cols; ++k) {
+            const i64 gj = (i64)j0 + k;
+            bool emit = false;
+            float acc = 0.0f;
+            if (gi < gj && gj < ep.qs.n) {
+              acc = exact_dsq(P + gi * ep.qs.d, P + gj * ep.qs.d, ep.qs.d);
+              emit = acc < ep.qs.thr_sq;
+            }
+            emit_warp(emit, ep.qs.vbase + gi, ep.qs.vbase + gj, acc, lane, oi, oj, od, cap, count);
+          }
+        }
+      }
+      if (!ok) {
+        set_status(status, PH_ERR_ITER_LIMIT);
         break;
       }
-      asm volatile("tcgen05.fence::after_thread_sync;");
-      const u32 taddr = tmem + (u32)g * stage_cols + ((u32)(q4 * 32) << 16);
-#pragma unroll 1
-      for (int c0 = 0; c0 < TC_T * nh; c0 += 64) {
-        const int h = c0 >> 7;
-        if (force[h]) continue;
-        u32 v0[32], v1[32];
-        tmem_ld32_issue(taddr + (u32)c0, v0);
-        tmem_ld32_issue(taddr + (u32)(c0 + 32), v1);
-        tmem_ld_wait();
-        // both min trees before one vote: independent chains side by side and
-        // one branch per 64 columns (almost always: no candidate)
-        const float mn = fminf(vmin(v0), vmin(v1));
-        if (!__any_sync(FULL, mn < base[h])) continue;
-        screen(v0, c0, base[h]);
-        screen(v1, c0 + 32, base[h]);
-      }
-      asm volatile("tcgen05.fence::before_thread_sync;");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(BAR_TE + g));
-      for (int h = 0; h < nh; ++h) {
-        if (!force[h]) continue;
-        // no screen for this column block: every pair of the warp's rows exactly
-        n_forced += 32 * TC_T;
-        const float* P = pts_all + sg.pt_off;
-        const i64 gi = i0 + row;
-        for (int col = 0; col < TC_T; ++col) {
-          const i64 gj = j0 + h * TC_T + col;
-          bool emit = false;
-          float acc = 0.0f;
-          if (gi < gj && gj < sg.n) {
-            acc = exact_dsq(P + gi * sg.d, P + gj * sg.d, sg.d);
-            emit = acc < sg.thr_sq;
-          }
-          emit_warp(emit, sg.vbase + gi, sg.vbase + gj, acc, lane, oi, oj, od, cap, count);
-        }
-      }
-      if (t + 2 < T) {
-        it.next();
-        it.next();
-      }
     }
-    if (cnt) flush();
+    if (ep.cnt) ep.flush();
     if (stats && lane == 0) {
-      atomicAdd(&st_sh[0], n_cand);
+      atomicAdd(&st_sh[0], ep.n_cand);
       atomicAdd(&st_sh[1], n_forced);
     }
   }
@@ -790,7 +881,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   if (warp == TC_MMA_WARP) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * stage_cols));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_TMEM_COLS));
   }
   if (stats && threadIdx.x == 0) {
     if (st_sh[0]) atomicAdd(&stats[0], st_sh[0]);
@@ -823,19 +914,23 @@ TcPlan plan_for(int max_d) {
   s.sbo = (u32)(8 * s.row_bytes) >> 4;
   const size_t queues = (size_t)TC_EPI_WARPS * TC_QCAP * sizeof(uint2);
   const size_t budget = 227 * 1024 - 1024 - queues;
-  // widest items (N = 256) whose rings still hold two B stages
-  for (int nb = 2; nb >= 1; --nb) {
-    s.nb = nb;
-    s.b_atom_bytes = nb * s.a_atom_bytes;
+  // the widest items whose rings still hold two B stages: two row blocks (they
+  // share the B tile, which halves its traffic) and two column blocks, then one
+  // row block, then one column block
+  for (int form = 0; form < 3; ++form) {
+    s.nr = form == 0 ? 2 : 1;
+    s.nb = form <= 1 ? 2 : 1;
+    s.b_atom_bytes = s.nb * s.a_atom_bytes;
     s.b_bytes = s.natoms * s.b_atom_bytes;
     for (int na = 2; na >= 1; --na) {
-      if (budget < (size_t)na * s.a_bytes) continue;
-      const int ns = (int)((budget - (size_t)na * s.a_bytes) / s.b_bytes);
+      const size_t a_ring = (size_t)na * s.nr * s.a_bytes;
+      if (budget < a_ring) continue;
+      const int ns = (int)((budget - a_ring) / s.b_bytes);
       if (ns >= 2) {
         s.na = na;
         s.ns = std::min(ns, TC_MAX_STAGES);
         // at least 120 KB so that one CTA (and its TMEM columns) holds an SM
-        p.smem = std::max<size_t>(1024 + (size_t)s.na * s.a_bytes + (size_t)s.ns * s.b_bytes + queues, 120 * 1024);
+        p.smem = std::max<size_t>(1024 + a_ring + (size_t)s.ns * s.b_bytes + queues, 120 * 1024);
         return p;
       }
     }
@@ -934,7 +1029,7 @@ extern "C" int ph_batch_edges_enumerate_screened(const float* pts, const ph_clou
   ph::count_launch();
   ph::launch_pdl(k_tc_points, dim3((unsigned)nblocks), dim3(TC_T), 0, s, pts, segs, nsegs, blk_off, sum, p.sh.kq, kappa, YA, YB, blkrad);
   ph::count_launch();
-  ph::launch_pdl(k_tc_items, dim3(1), dim3(1024), 0, s, segs, nsegs, p.sh.nb, item_off);
+  ph::launch_pdl(k_tc_items, dim3(1), dim3(1024), 0, s, segs, nsegs, p.sh.nr, p.sh.nb, item_off);
   const double thr_scale = 1.0 + (double)(max_d + 3) * 0x1p-24;
   // persistent: one CTA per SM, each a contiguous range of the items (counted on the device)
   const int grid = (int)std::min<i64>(ntiles, (i64)sms);
