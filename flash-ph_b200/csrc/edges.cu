@@ -16,15 +16,11 @@
 #include <algorithm>
 #include <cmath>
 
-#include "prim.cuh"
+#include "edges.cuh"
 
 namespace ph {
 namespace {
 
-constexpr int ET = 128;  // points per tile side
-constexpr int EK = 16;   // dimensions per shared-memory chunk
-constexpr int ENT = 256;
-constexpr unsigned FULL = 0xffffffffu;
 
 __device__ __forceinline__ void tile_coords(i64 b, i64 nt, i64& I, i64& J) {
   // b-th tile of the row-major upper triangle (I <= J) of an nt x nt grid
@@ -59,91 +55,17 @@ __global__ void __launch_bounds__(ENT, 2)
             i64 cap, unsigned long long* __restrict__ count) {
   ph::pdl_wait();
   ph::pdl_trigger();
-  __shared__ __align__(16) float xs[EK][ET];
-  __shared__ __align__(16) float ys[EK][ET];
+  __shared__ EdgeTile sh;
   const ph_cloud_seg sg = segs ? segs[find_seg(segs, nsegs, (i64)blockIdx.x)] : seg0;
-  const float* __restrict__ pts = pts_all + sg.pt_off;
-  const i64 n = sg.n;
-  const int d = sg.d;
-  const float thr_sq = sg.thr_sq;
-  const i64 nt = (n + ET - 1) / ET;
+  const i64 n = sg.n, nt = (n + ET - 1) / ET;
   i64 I, J;
   tile_coords((i64)blockIdx.x - sg.tile_off, nt, I, J);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const i64 i0 = I * ET, j0 = J * ET;
-  float acc[8][8];
-#pragma unroll
-  for (int r = 0; r < 8; ++r)
-#pragma unroll
-    for (int c = 0; c < 8; ++c) acc[r][c] = 0.0f;
-
-  for (int k0 = 0; k0 < d; k0 += EK) {
-    const int kc = min(EK, d - k0);
-    const int tot = ET * kc;
-    for (int idx = threadIdx.x; idx < tot; idx += ENT) {
-      const int p = idx / kc, k = idx - p * kc;
-      const i64 gi = i0 + p, gj = j0 + p;
-      xs[k][p] = gi < n ? pts[gi * d + k0 + k] : 0.0f;
-      ys[k][p] = gj < n ? pts[gj * d + k0 + k] : 0.0f;
-    }
-    __syncthreads();
-#pragma unroll 2
-    for (int k = 0; k < kc; ++k) {
-      const float4 xa = *reinterpret_cast<const float4*>(&xs[k][ty * 8]);
-      const float4 xb = *reinterpret_cast<const float4*>(&xs[k][ty * 8 + 4]);
-      const float4 ya = *reinterpret_cast<const float4*>(&ys[k][tx * 8]);
-      const float4 yb = *reinterpret_cast<const float4*>(&ys[k][tx * 8 + 4]);
-      const float xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-      const float yv[8] = {ya.x, ya.y, ya.z, ya.w, yb.x, yb.y, yb.z, yb.w};
-#pragma unroll
-      for (int r = 0; r < 8; ++r)
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const float df = __fsub_rn(xv[r], yv[c]);
-          acc[r][c] = __fmaf_rn(df, df, acc[r][c]);
-        }
-    }
-    __syncthreads();
-  }
-
-  // hits of this thread's 8x8 block as a 64-bit mask
-  u64 hit = 0;
-#pragma unroll
-  for (int r = 0; r < 8; ++r)
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const i64 gi = i0 + ty * 8 + r, gj = j0 + tx * 8 + c;
-      const bool ok = (gi < gj) && (gj < n) && (acc[r][c] < thr_sq);
-      hit |= (u64)ok << (r * 8 + c);
-    }
-  const int cnt = __popcll(hit);
-  if (!__any_sync(FULL, cnt != 0)) return;
-  // warp-aggregated reservation
-  const int lane = threadIdx.x & 31;
-  int incl = cnt;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += y;
-  }
-  const int wtot = __shfl_sync(FULL, incl, 31);
-  unsigned long long base = 0;
-  if (lane == 31) base = atomicAdd(count, (unsigned long long)wtot);
-  base = __shfl_sync(FULL, base, 31);
-  unsigned long long pos = base + (unsigned long long)(incl - cnt);
-#pragma unroll
-  for (int r = 0; r < 8; ++r)
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      if ((hit >> (r * 8 + c)) & 1ull) {
-        if (pos < (unsigned long long)cap) {
-          oi[pos] = (i32)(sg.vbase + i0 + ty * 8 + r);
-          oj[pos] = (i32)(sg.vbase + j0 + tx * 8 + c);
-          od[pos] = acc[r][c];
-        }
-        ++pos;
-      }
-    }
+  edge_tile(sh, pts_all + sg.pt_off, n, sg.d, sg.thr_sq, I * ET, J * ET, cap, count,
+            [&](unsigned long long at, i64 gi, i64 gj, float dsq) {
+              oi[at] = (i32)(sg.vbase + gi);
+              oj[at] = (i32)(sg.vbase + gj);
+              od[at] = dsq;
+            });
 }
 
 // ---- filtration sort -------------------------------------------------------

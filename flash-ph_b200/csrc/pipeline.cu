@@ -25,6 +25,7 @@
 #include <string>
 #include <vector>
 
+#include "edges.cuh"
 #include "links.cuh"
 #include "pipeline.cuh"
 
@@ -242,6 +243,27 @@ using namespace ph::pl;
 
 namespace {
 
+// The edge kernel of a single cloud. All give the same edges with the same
+// bits; which is fastest, measured with thresholds from 3 neighbours a point to
+// the default one (95th percentile of the 20-NN distances):
+//  * direct (k_edges) for small clouds, whose few tiles the persistent screen
+//    spreads badly and whose density leaves it many candidates: 331 x 50 28
+//    against 220 us, 2500 x 10 14-18 against 27-64, 4000 x 32 46-53 against
+//    36-157; past n^2 (d + 8) = 5e8 the screen wins on sparse clouds (8000 x 10
+//    76 against 37 us) and the dense ones come to equal (20,000 x 10 507, 534);
+//  * blocks in grid order (edges_near) for larger clouds of up to four
+//    dimensions;
+//  * the tensor-core screen for the others.
+enum class EdgeKernel { direct, screened, nearby };
+
+EdgeKernel edge_kernel(i64 n, int d, int edge_mode) {
+  if (edge_mode == 1) return EdgeKernel::screened;
+  if (edge_mode == 2 || d > 252) return EdgeKernel::direct;
+  if ((double)n * (double)n * (d + 8) <= 5e8) return EdgeKernel::direct;
+  if (d <= NEAR_MAX_D && n <= NEAR_MAX_N) return EdgeKernel::nearby;
+  return d >= 8 || n <= NEAR_MAX_N ? EdgeKernel::screened : EdgeKernel::direct;
+}
+
 // the segment record of a single cloud, and the run's counters cleared
 __global__ void k_single_seg(ph_cloud_seg* seg, int64_t* blk_off, int64_t n, int32_t d, float thr_sq,
                              int64_t nblocks, int64_t* cnt) {
@@ -306,7 +328,8 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   const float thr_sq = to_f32(max_edge_length * max_edge_length);
 
   // ---- 1. edges (rips.py:170-200; edge_kernel.py) ----------------------------------------
-  const bool screened = edge_mode == 1 || (edge_mode == 0 && d >= 8 && d <= 252);
+  const EdgeKernel ek = edge_kernel(n, d, edge_mode);
+  const bool screened = ek == EdgeKernel::screened;
   const i64 nblocks = (n + 127) / 128;
   const i64 ntiles = ph_cloud_tiles(n);
   ph_cloud_seg* seg = A.take<ph_cloud_seg>(1);
@@ -319,8 +342,10 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   int* st = reinterpret_cast<int*>(cnt + 1);
   count_launch();
   ph::launch_pdl(k_single_seg, dim3(1), dim3(1), 0, s, seg, blk, n, d, thr_sq, nblocks, cnt);
-  const size_t ews = screened ? ph_edges_screened_workspace_bytes(n, 1, d) : 0;
-  void* ew = screened ? A.bytes(ews) : nullptr;
+  const size_t ews = screened                   ? ph_edges_screened_workspace_bytes(n, 1, d)
+                     : ek == EdgeKernel::nearby ? edges_near_workspace_bytes(n, d)
+                                                : 0;
+  void* ew = ews ? A.bytes(ews) : nullptr;
   const i64 pairs = n * (n - 1) / 2;
   // first edge buffer: 256 edges a point, 2^22 at least, and up to an eighth
   // of the pairs (at most 2^27 edges, 1.5 GiB): dense clouds (thresholds at
@@ -340,6 +365,8 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
     if (screened)
       rc = ph_batch_edges_enumerate_screened(d_points, seg, 1, ntiles, d, n, blk, nblocks, ei, ej, ed, cap,
                                              reinterpret_cast<unsigned long long*>(cnt), st, nullptr, ew, ews, s);
+    else if (ek == EdgeKernel::nearby)
+      rc = edges_near(d_points, n, d, thr_sq, ei, ej, ed, cap, reinterpret_cast<unsigned long long*>(cnt), ew, ews, s);
     else
       rc = ph_batch_edges_enumerate(d_points, seg, 1, ntiles, ei, ej, ed, cap,
                                     reinterpret_cast<unsigned long long*>(cnt), s);
