@@ -193,6 +193,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   i64 N = 0, floats = 0, pairs = 0, ntiles = 0, nblocks = 0;
   int max_d = 1, dim_all = 0;
   bool any_wrap = false;
+  int64_t max_n = 0;
   std::vector<ph_cloud_seg> segs(K);
   std::vector<GatherItem> gather(K);
   std::vector<int64_t> blk(K + 1, 0);
@@ -214,6 +215,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
     ntiles += ph_cloud_tiles(n[c]);
     blk[c + 1] = blk[c] + (n[c] + 127) / 128;
     max_d = std::max(max_d, (int)d[c]);
+    max_n = std::max(max_n, n[c]);
     dim_all = std::max(dim_all, (int)max_dim[c]);
     any_wrap = any_wrap || n[c] > 92682;
   }
@@ -333,13 +335,12 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   // ---- 3. H0 per cloud ----------------------------------------------------------------------------
   uint8_t* mask = A.take<uint8_t>(E);
   i32* comp = A.take<i32>(N);
-  int64_t* ncomp = A.take<int64_t>(1);
   const size_t mst_b = ph_boruvka_workspace_bytes(N, E), h0_b = ph_batch_h0_rows_workspace_bytes(E);
   void* mst_ws = A.bytes(mst_b);
   void* h0_ws = A.bytes(h0_b);
   if (A.failed || cudaMallocAsync((void**)&res->rows[0], sizeof(float) * 2 * N, s) != cudaSuccess) return alloc_fail();
   {
-    int rc = ph_boruvka_mst(si, sj, E, N, mask, comp, ncomp, st + 1, mst_ws, mst_b, s);
+    int rc = batch_forest(si, sj, E, N, e_off, dsegs, K, max_n, mask, comp, cnt + 15, st + 1, mst_ws, mst_b, s);
     if (rc == PH_OK) rc = ph_batch_h0_rows(filt, mask, E, e_off, dsegs, K, vcloud, N, res->rows[0], h0_ws, h0_b, s);
     if (rc != PH_OK) return give_up(rc);
   }

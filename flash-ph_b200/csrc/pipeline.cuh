@@ -118,5 +118,13 @@ struct RedOut {
 int reduce_only(Arena& A, cudaStream_t s, const i32* off, const i32* data, i64 K, i32 col_base, i64 R,
                 i32 row_base, i64 span, const uint8_t* skip, const i32* cmf, i64 pool_cap, int* status, RedOut& o);
 
+// The forest of a batch's union graph: a block a cloud where every cloud fits
+// one, else ph_boruvka_mst over the union. Edges lie cloud by cloud (e_off);
+// max_n is the largest cloud's vertex count; *d_ncomp starts at zero; the
+// workspace is ph_boruvka_mst's.
+int batch_forest(const i32* edge_i, const i32* edge_j, i64 E, i64 n, const i64* e_off, const ph_cloud_seg* segs,
+                 int K, i64 max_n, uint8_t* mst_mask, i32* comp, i64* d_ncomp, int* d_status, void* workspace,
+                 size_t workspace_bytes, cudaStream_t s);
+
 }  // namespace pl
 }  // namespace ph
