@@ -403,7 +403,6 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   uint8_t* want = A.take<uint8_t>(K);
   uint8_t* tkeep = A.take<uint8_t>(K);
   unsigned long long* ttot = A.take<unsigned long long>(K);
-  int* tnext = A.take<int>(1);
   if (A.failed) return alloc_fail();
   const bool pre = max_triangles > 0 && E > 0 && N <= ph_triangles_total_max_vertices();
   if (pre) {
@@ -411,7 +410,10 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
     const i64 m_star = std::max<i64>(0, (i64)std::floor(bound_m) - 1);  // conservative: a few more clouds counted
     count_launch();
     ph::launch_pdl(k_tri_want, dim3(grid_for(K)), dim3(256), 0, s, (const int64_t*)e_off, K, m_star, want);
-    PH_TRY(ph_batch_triangles_total(adj_ptr, adj_idx, N, vcloud, want, K, ttot, tnext, s));
+    const size_t tt_b = ph_triangles_total_edges_workspace_bytes(E, N);
+    void* tt_ws = A.bytes(tt_b);
+    if (A.failed) return alloc_fail();
+    PH_TRY(batch_triangles_total(si, sj, E, adj_ptr, N, vcloud, want, dsegs, K, ttot, tt_ws, tt_b, s));
     count_launch();
     ph::launch_pdl(k_tri_keep, dim3(grid_for(K)), dim3(256), 0, s, (const uint8_t*)want,
                    (const unsigned long long*)ttot, K, (i64)max_triangles, tkeep);

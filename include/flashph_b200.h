@@ -223,8 +223,9 @@ int ph_triangles_total(const int32_t* adj_ptr, const int32_t* adj_idx, int64_t n
                        unsigned long long* d_total, int* d_next, void* stream);
 
 /* ph_triangles_total from the unsorted edges (i < j, any order), without the
- * adjacency: an upper adjacency (row i lists the j of every edge (i, j)) is
- * built by counting, then the same bitmap pass runs. The total the count pass
+ * adjacency: vertices are renumbered by descending degree, each edge goes to
+ * the row of its larger number, rows become masks of 64-vertex words, and a
+ * shared bitmap meets them word by word. The total the count pass
  * of triangle_kernel.py:288 triangle_enumerate checks against max_triangles
  * (triangle_kernel.py:377-381), for a call that may be over the limit, before
  * any filtration order exists. n <= ph_triangles_total_max_vertices(). */
