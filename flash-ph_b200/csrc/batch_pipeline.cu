@@ -324,7 +324,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   if (A.failed) return alloc_fail();
   if (E) {
     int rc = ph_batch_edges_sort(ei, ej, ed, E, vcloud, dsegs, K, any_wrap ? 1 : 0, si, sj, sd, sort_ws, sort_b, s);
-    if (rc == PH_OK) rc = ph_vertex_csr(si, sj, E, N, adj_ptr, adj_idx, adj_rank, csr_ws, csr_b, s);
+    if (rc == PH_OK && dim_all > 0) rc = ph_vertex_csr(si, sj, E, N, adj_ptr, adj_idx, adj_rank, csr_ws, csr_b, s);
     if (rc == PH_OK) rc = ph_sqrt_f32(sd, filt, E, s);
     if (rc != PH_OK) return give_up(rc);
   } else {

@@ -160,6 +160,279 @@ __global__ void k_csr_fill(const u64* __restrict__ keys, const u32* __restrict__
   }
 }
 
+// ---- adjacency without a sort of all half-edges ----------------------------------------
+// Degrees are counted (the counter's old value is the half-edge's slot in its
+// row), scanned, the half-edges (neighbour << 32 | 2 rank + side) scattered to
+// their rows, and each row sorted where it lies: three passes over memory
+// instead of a radix sort's two per digit. Slots come from atomics, in any
+// order; the keys of a row differ (the side bit tells a self-loop's two), so
+// the sorted row is the same whatever it was.
+// Radix sort -> this form: 20,000 vertices, 48,000 edges 57 -> 30 us; 1500,
+// 158,000 68 -> 42; 50,000, 300,000 109 -> 47; 200,000, 330,000 134 -> 35;
+// 186,000, 11M 3242 -> 944 (the row sorts' 64-bit exchanges; else bound by the
+// atomics' and the scattered stores' sectors).
+constexpr int CSR_NT = 256;
+constexpr int CSR_WARP = 1024;    // entries a warp sorts in its registers
+constexpr int CSR_BIG_NT = 1024;
+constexpr int CSR_BLOCK = 16384;  // entries a block sorts in shared memory
+constexpr int CSR_RANGE = 32768;  // neighbours a block counts at a time in a longer row
+constexpr u64 CSR_NONE = ~0ull;
+// half-edges: fewer are sorted by one cluster in less time than these six or
+// seven launches (16,000 edges 25 us by the sort, 36 us here; 24,000: 30, 31;
+// 48,000: 45, 30)
+constexpr i64 CSR_MIN = 48 * 1024;
+
+__device__ __forceinline__ i32 csr_rank(u64 half) { return (i32)((u32)half >> 1); }
+
+__global__ void k_csr_count(const i32* __restrict__ ei, const i32* __restrict__ ej, i64 E, i32* __restrict__ cnt,
+                            int2* __restrict__ slot) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  for (i64 e = (i64)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += (i64)gridDim.x * blockDim.x)
+    slot[e] = make_int2(atomicAdd(&cnt[ei[e]], 1), atomicAdd(&cnt[ej[e]], 1));
+}
+
+__global__ void k_csr_scatter(const i32* __restrict__ ei, const i32* __restrict__ ej, i64 E,
+                              const i32* __restrict__ ptr, const int2* __restrict__ slot, u64* __restrict__ half) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  for (i64 e = (i64)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += (i64)gridDim.x * blockDim.x) {
+    const i32 i = ei[e], j = ej[e];
+    const int2 at = slot[e];
+    half[ptr[i] + at.x] = (u64)(u32)j << 32 | (u64)(2 * e);
+    half[ptr[j] + at.y] = (u64)(u32)i << 32 | (u64)(2 * e + 1);
+  }
+}
+
+// bitonic sort of len2 (a power of two) keys by threads t of T
+template <typename Sync>
+__device__ __forceinline__ void csr_bitonic(u64* key, int len2, int t, int T, Sync sync) {
+  for (int k = 2; k <= len2; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int p = t; p < len2 / 2; p += T) {
+        const int a = 2 * p - (p & (j - 1)), b = a + j;  // a without bit j, b with it
+        const u64 x = key[a], y = key[b];
+        if ((x > y) == ((a & k) == 0)) {
+          key[a] = y;
+          key[b] = x;
+        }
+      }
+      sync();
+    }
+}
+
+__device__ __forceinline__ void csr_order(u64& lo, u64& hi, bool up) {
+  const u64 a = lo, b = hi;
+  const bool swap = (a > b) == up;
+  lo = swap ? b : a;
+  hi = swap ? a : b;
+}
+
+// One row of up to 32 K entries by a warp: a bitonic network over K registers
+// a lane (entry lane K + k), whose steps inside a lane need no shuffle, then
+// through the warp's shared memory (a pad word a lane) to coalesced stores.
+template <int K>
+__device__ __noinline__ void csr_warp_row(const u64* __restrict__ half, int len, i32* __restrict__ idx,
+                                          i32* __restrict__ rank, u64* buf) {
+  const int lane = threadIdx.x & 31;
+  u64 x[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) x[k] = k * 32 + lane < len ? half[k * 32 + lane] : CSR_NONE;
+  // runs of K: alternately up and down, the last stage by lane
+#pragma unroll
+  for (int size = 2; size <= K; size <<= 1)
+#pragma unroll
+    for (int j = size >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (!(k & j)) csr_order(x[k], x[k + j], size < K ? !(k & size) : !(lane & 1));
+  for (int m = 2; m <= 32; m <<= 1) {  // runs of m lanes
+    const bool up = !(lane & m);
+    for (int o = m >> 1; o > 0; o >>= 1) {
+      const bool small = !(lane & o) == up;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const u64 y = __shfl_xor_sync(0xffffffffu, x[k], o);
+        x[k] = (x[k] < y) == small ? x[k] : y;
+      }
+    }
+#pragma unroll
+    for (int j = K >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (!(k & j)) csr_order(x[k], x[k + j], up);
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) buf[lane * (K + 1) + k] = x[k];
+  __syncwarp();
+  for (int p = lane; p < len; p += 32) {
+    const u64 y = buf[(p / K) * (K + 1) + p % K];
+    idx[p] = (i32)(y >> 32);
+    rank[p] = csr_rank(y);
+  }
+  __syncwarp();
+}
+
+// a row of up to 32 entries: each key's place is the count of smaller ones
+__device__ __forceinline__ void csr_short_row(const u64* __restrict__ half, int len, i32* __restrict__ idx,
+                                              i32* __restrict__ rank) {
+  const int lane = threadIdx.x & 31;
+  const u64 x = lane < len ? half[lane] : CSR_NONE;
+  int at = 0;
+  for (int k = 0; k < len; ++k) at += __shfl_sync(0xffffffffu, x, k) < x;
+  if (lane < len) {
+    idx[at] = (i32)(x >> 32);
+    rank[at] = csr_rank(x);
+  }
+}
+
+// Short rows, for an average of up to 8 a row: up to 8 entries by 8 lanes, four
+// rows a warp at once, up to 32 by the warp; longer ones are listed.
+__global__ void __launch_bounds__(CSR_NT) k_csr_short(const u64* __restrict__ half, const i32* __restrict__ ptr, i64 n,
+                                                      i32* __restrict__ idx, i32* __restrict__ rank,
+                                                      i32* __restrict__ list, i32* __restrict__ nlist) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  const int lane = threadIdx.x & 31, l8 = lane & 7;
+  const i64 stride = ((i64)gridDim.x * CSR_NT >> 5) * 4;
+  for (i64 v0 = (((i64)blockIdx.x * CSR_NT + threadIdx.x) >> 5) * 4; v0 < n; v0 += stride) {
+    const i64 v = v0 + (lane >> 3);
+    const int s = v < n ? ptr[v] : 0, len = v < n ? ptr[v + 1] - s : 0;
+    const bool mine = len <= 8 && l8 < len;
+    const u64 x = mine ? half[s + l8] : CSR_NONE;
+    int at = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) at += __shfl_sync(0xffffffffu, x, k, 8) < x;
+    if (mine) {
+      idx[s + at] = (i32)(x >> 32);
+      rank[s + at] = csr_rank(x);
+    }
+    if (l8 == 0 && len > 32) list[atomicAdd(nlist, 1)] = (i32)v;
+    for (u32 todo = __ballot_sync(0xffffffffu, l8 == 0 && len > 8 && len <= 32); todo; todo &= todo - 1) {
+      const int from = __ffs(todo) - 1;
+      const int rs = __shfl_sync(0xffffffffu, s, from), rl = __shfl_sync(0xffffffffu, len, from);
+      csr_short_row(half + rs, rl, idx + rs, rank + rs);
+    }
+  }
+}
+
+// A warp a row of up to CSR_WARP entries: those listed, or (no list) all n;
+// longer ones are listed for k_csr_big.
+__global__ void __launch_bounds__(CSR_NT) k_csr_rows(const u64* __restrict__ half, const i32* __restrict__ ptr, i64 n,
+                                                     const i32* __restrict__ list, const i32* __restrict__ nlist,
+                                                     i32* __restrict__ idx, i32* __restrict__ rank,
+                                                     i32* __restrict__ big, i32* __restrict__ nbig) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  extern __shared__ u64 key[];
+  u64* buf = key + (size_t)(threadIdx.x >> 5) * (CSR_WARP + 32);
+  const i64 count = list ? *nlist : n, stride = (i64)gridDim.x * CSR_NT >> 5;
+  for (i64 r = ((i64)blockIdx.x * CSR_NT + threadIdx.x) >> 5; r < count; r += stride) {
+    const i64 v = list ? list[r] : r;
+    const int s = ptr[v], len = ptr[v + 1] - s;
+    if (len <= 32)
+      csr_short_row(half + s, len, idx + s, rank + s);
+    else if (len <= 64)
+      csr_warp_row<2>(half + s, len, idx + s, rank + s, buf);
+    else if (len <= 128)
+      csr_warp_row<4>(half + s, len, idx + s, rank + s, buf);
+    else if (len <= 256)
+      csr_warp_row<8>(half + s, len, idx + s, rank + s, buf);
+    else if (len <= 512)
+      csr_warp_row<16>(half + s, len, idx + s, rank + s, buf);
+    else if (len <= CSR_WARP)
+      csr_warp_row<32>(half + s, len, idx + s, rank + s, buf);
+    else if ((threadIdx.x & 31) == 0)
+      big[atomicAdd(nbig, 1)] = (i32)v;
+  }
+}
+
+// Rows beyond CSR_WARP, a block a row: in shared memory up to CSR_BLOCK
+// entries; beyond, by counting over ranges of neighbours (no row is too long),
+// where the entries of one neighbour (repeated edges) are put in rank order.
+__global__ void __launch_bounds__(CSR_BIG_NT) k_csr_big(const u64* __restrict__ half, const i32* __restrict__ ptr,
+                                                        i64 n, i32* __restrict__ idx, i32* __restrict__ rank,
+                                                        const i32* __restrict__ big, const i32* __restrict__ nbig) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  extern __shared__ u64 key[];
+  __shared__ int sums[32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  for (int r = blockIdx.x; r < *nbig; r += gridDim.x) {
+    const i32 v = big[r];
+    const int s = ptr[v], len = ptr[v + 1] - s;
+    if (len <= CSR_BLOCK) {
+      int len2 = 2 * CSR_WARP;
+      while (len2 < len) len2 <<= 1;
+      for (int k = t; k < len2; k += CSR_BIG_NT) key[k] = k < len ? half[s + k] : CSR_NONE;
+      __syncthreads();
+      csr_bitonic(key, len2, t, CSR_BIG_NT, [] { __syncthreads(); });
+      for (int k = t; k < len; k += CSR_BIG_NT) {
+        idx[s + k] = (i32)(key[k] >> 32);
+        rank[s + k] = csr_rank(key[k]);
+      }
+      __syncthreads();
+      continue;
+    }
+    i32* cnt = reinterpret_cast<i32*>(key);
+    int done = s;  // entries of the ranges before
+    for (i64 lo = 0; lo < n; lo += CSR_RANGE) {
+      for (int k = t; k < CSR_RANGE; k += CSR_BIG_NT) cnt[k] = 0;
+      __syncthreads();
+      for (int p = s + t; p < s + len; p += CSR_BIG_NT) {
+        const i64 w = (i64)(half[p] >> 32) - lo;
+        if (w >= 0 && w < CSR_RANGE) atomicAdd(&cnt[w], 1);
+      }
+      __syncthreads();
+      // each thread's CSR_RANGE / CSR_BIG_NT counters, the threads' sums, then starts in place of counts
+      constexpr int PER = CSR_RANGE / CSR_BIG_NT;
+      int sum = 0;
+      for (int k = 0; k < PER; ++k) sum += cnt[t * PER + k];
+      int incl = sum;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane == 31) sums[warp] = incl;
+      __syncthreads();
+      int before = 0, total = 0;
+      for (int w = 0; w < CSR_BIG_NT / 32; ++w) {
+        before += w < warp ? sums[w] : 0;
+        total += sums[w];
+      }
+      int at = done + before + incl - sum;
+      for (int k = 0; k < PER; ++k) {
+        const int c = cnt[t * PER + k];
+        cnt[t * PER + k] = at;
+        at += c;
+      }
+      __syncthreads();
+      for (int p = s + t; p < s + len; p += CSR_BIG_NT) {
+        const u64 x = half[p];
+        const i64 w = (i64)(x >> 32) - lo;
+        if (w >= 0 && w < CSR_RANGE) {
+          const int o = atomicAdd(&cnt[w], 1);
+          idx[o] = (i32)(x >> 32);
+          rank[o] = csr_rank(x);
+        }
+      }
+      __syncthreads();
+      // cnt[w] is now the end of w's entries: insertion sort of each run by rank
+      for (int k = 0; k < PER; ++k) {
+        const int w = t * PER + k, end = cnt[w], start = w ? cnt[w - 1] : done;
+        for (int a = start + 1; a < end; ++a) {
+          const i32 x = rank[a];
+          int b = a;
+          for (; b > start && rank[b - 1] > x; --b) rank[b] = rank[b - 1];
+          rank[b] = x;
+        }
+      }
+      done += total;
+      __syncthreads();
+    }
+  }
+}
+
 __global__ void k_sqrt(const float* __restrict__ in, float* __restrict__ out, i64 n) {
   ph::pdl_wait();
   ph::pdl_trigger();
@@ -265,8 +538,55 @@ extern "C" int ph_vertex_csr(const int32_t* edge_i, const int32_t* edge_j, int64
   Carve c(workspace, workspace_bytes);
   u64* keys = c.take<u64>(2 * E);
   u32* vals = c.take<u32>(2 * E);
+  const Carve rest = c;
   void* rws = c.take<char>((i64)radix_sort_workspace_bytes(2 * E));
   if (!keys || !vals || !rws) return PH_ERR_ARG;
+  // the counts, the scan's parts and the list of long rows lie where the radix
+  // sort's buffers would; vertices far beyond the edges do not fit there
+  Carve w = rest;
+  i32* cnt = w.take<i32>(n + 3);
+  i32* big = w.take<i32>(2 * E / CSR_WARP + 1);
+  void* sws = w.take<char>((i64)scan_workspace_bytes(n));
+  i32* list = w.take<i32>(2 * E / 32 + 1);
+  if (2 * E >= CSR_MIN && cnt && big && sws && list) {
+    if (ph::allow_dynamic_smem((const void*)k_csr_big) != cudaSuccess) {
+      PH_CHECK_LAUNCH();
+      return PH_ERR_CUDA;
+    }
+    int2* slot = reinterpret_cast<int2*>(vals);
+    i32 *nbig = cnt + n + 1, *nlist = cnt + n + 2;
+    ph::zero_async(cnt, sizeof(i32) * (size_t)(n + 3), s);
+    ph::count_launch();
+    ph::launch_pdl(k_csr_count, dim3(grid_for(E)), dim3(256), 0, s, edge_i, edge_j, E, cnt, slot);
+    PH_TRY(scan_exclusive_i32_i32(cnt, adj_ptr, n, sws, scan_workspace_bytes(n), s));
+    ph::count_launch();
+    ph::launch_pdl(k_csr_scatter, dim3(grid_for(E)), dim3(256), 0, s, edge_i, edge_j, E, (const i32*)adj_ptr,
+                   (const int2*)slot, keys);
+    const bool sparse = 2 * E <= 8 * n;
+    const size_t rows_smem = sizeof(u64) * (CSR_NT / 32) * (CSR_WARP + 32);
+    if (ph::allow_dynamic_smem((const void*)k_csr_rows) != cudaSuccess) {
+      PH_CHECK_LAUNCH();
+      return PH_ERR_CUDA;
+    }
+    const i64 sms = ph::device_sms();
+    if (sparse) {
+      ph::count_launch();
+      ph::launch_pdl(k_csr_short, dim3((unsigned)std::min<i64>((n + CSR_NT / 8 - 1) / (CSR_NT / 8), sms * 8)),
+                     dim3(CSR_NT), 0, s, (const u64*)keys, (const i32*)adj_ptr, n, adj_idx, adj_rank, list, nlist);
+    }
+    const i64 rows = sparse ? std::min<i64>(n, 2 * E / 33) : n;
+    ph::count_launch();
+    ph::launch_pdl(k_csr_rows, dim3((unsigned)std::max<i64>(1, std::min<i64>((rows + CSR_NT / 32 - 1) / (CSR_NT / 32), sms * 2))),
+                   dim3(CSR_NT), rows_smem, s, (const u64*)keys, (const i32*)adj_ptr, n,
+                   (const i32*)(sparse ? list : nullptr), (const i32*)nlist, adj_idx, adj_rank, big, nbig);
+    const i64 big_rows = std::min<i64>(n, 2 * E / (CSR_WARP + 1));
+    ph::count_launch();
+    ph::launch_pdl(k_csr_big, dim3((unsigned)std::max<i64>(1, std::min<i64>(big_rows, sms))),
+                   dim3(CSR_BIG_NT), sizeof(u64) * CSR_BLOCK, s, (const u64*)keys, (const i32*)adj_ptr, n, adj_idx,
+                   adj_rank, (const i32*)big, (const i32*)nbig);
+    PH_CHECK_LAUNCH();
+    return PH_OK;
+  }
   // sort only the key bits a vertex pair needs: 2 x bits(n - 1), in whole bytes
   int sh = 1;
   while (sh < 32 && (int64_t(1) << sh) < n) ++sh;

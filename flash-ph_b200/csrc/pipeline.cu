@@ -437,7 +437,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   if (A.failed) return alloc_fail();
   if (E) {
     int rc = ph_edges_sort(ei, ej, ed, E, n, si, sj, sd, sort_ws, sort_b, s);
-    if (rc == PH_OK) rc = ph_vertex_csr(si, sj, E, n, adj_ptr, adj_idx, adj_rank, csr_ws, csr_b, s);
+    if (rc == PH_OK && max_dim > 0) rc = ph_vertex_csr(si, sj, E, n, adj_ptr, adj_idx, adj_rank, csr_ws, csr_b, s);
     if (rc == PH_OK) rc = ph_sqrt_f32(sd, filt, E, s);
     if (rc != PH_OK) return give_up(rc);
   } else {
