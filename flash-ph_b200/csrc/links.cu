@@ -79,9 +79,18 @@ struct Graph {
   const i32* __restrict__ aptr;
   const i32* __restrict__ aidx;
   const i32* __restrict__ arank;
-  const i32* __restrict__ tab;  // null: no table
-  i64 ld;
-  i32 vb;  // the cloud's first vertex
+  const char* __restrict__ tab;  // rank of (0, 0), were the table of all vertices; null: no table
+  i32 row;                       // bytes of a table row (n <= 16384)
+
+  // The rank at (x, w), col the address of (0, w): one multiply-add and a load.
+  // The passes over links are bound by instruction issue (66% of the slots,
+  // 960 a dense edge, at 14% L1 and 97% L2 hits), not by the table's bytes.
+  // Index arithmetic in 64 bits and single list loads -> this: 1501 points in
+  // 8 dimensions 217 -> 202 us, tetrahedra of 331 in 50 214 -> 193 us.
+  __device__ __forceinline__ const char* col(i32 w) const { return tab + 4 * (i64)w; }
+  __device__ __forceinline__ i32 cell(const char* c, i32 x) const {
+    return *reinterpret_cast<const i32*>(c + (i64)x * row);
+  }
 
   // the ranks at key[q] of the adjacency rows [lo[q], hi[q]), NO_RANK where
   // there is no such entry (an empty range: not looked up), searches interleaved
@@ -118,8 +127,9 @@ struct Graph {
   template <int N>
   __device__ __forceinline__ void ranks(const i32 (&x)[N], const bool (&ask)[N], i32 w, i32 (&r)[N]) const {
     if (tab) {
+      const char* c = col(w);
 #pragma unroll
-      for (int q = 0; q < N; ++q) r[q] = ask[q] ? tab[(i64)(x[q] - vb) * ld + (w - vb)] : NO_RANK;
+      for (int q = 0; q < N; ++q) r[q] = ask[q] ? cell(c, x[q]) : NO_RANK;
       return;
     }
     int lo[N], hi[N];
@@ -143,19 +153,19 @@ struct Graph {
 };
 
 __device__ __forceinline__ Graph graph_of(const LinkGraph& g, i32 a) {
-  Graph r{g.adj_ptr, g.adj_idx, g.adj_rank, nullptr, 0, 0};
+  Graph r{g.adj_ptr, g.adj_idx, g.adj_rank, nullptr, 0};
   if (!g.table) return r;
   if (!g.table_off) {
-    r.tab = g.table;
-    r.ld = g.n;
+    r.tab = reinterpret_cast<const char*>(g.table);
+    r.row = (i32)(4 * g.n);
     return r;
   }
   const i32 c = g.vcloud[a];
   const i64 at = g.table_off[c];
   if (at < 0) return r;
-  r.tab = g.table + at;
-  r.ld = g.segs[c].n;
-  r.vb = (i32)g.segs[c].vbase;
+  const i64 vb = g.segs[c].vbase;
+  r.row = 4 * g.segs[c].n;
+  r.tab = reinterpret_cast<const char*>(g.table + at) - vb * r.row - 4 * vb;
   return r;
 }
 
@@ -191,6 +201,21 @@ __device__ __forceinline__ Ends ends_of(const LinkGraph& g, i32 m, i32 a, i32 b)
   return Ends{m, a, b, as ? sa : sb, as ? ea : eb, as ? sb : sa, as ? eb : ea, as};
 }
 
+// entries j, j + 1, ... of a group's list (j a multiple of their number); those
+// past its end are whatever the words hold, and are not looked up
+__device__ __forceinline__ void list_at(const i32* list, int j, i32 (&x)[4]) {
+  const int4 v = *reinterpret_cast<const int4*>(list + j);
+  x[0] = v.x;
+  x[1] = v.y;
+  x[2] = v.z;
+  x[3] = v.w;
+}
+__device__ __forceinline__ void list_at(const i32* list, int j, i32 (&x)[2]) {
+  const int2 v = *reinterpret_cast<const int2*>(list + j);
+  x[0] = v.x;
+  x[1] = v.y;
+}
+
 // The rows of an edge in ascending order, up to G at a time: f(mine, lanes, i,
 // fa, fb) by the whole group, where the lanes of the mask hold one each, the
 // one with link index i and other edges fa, fb. Returns the link's length
@@ -203,7 +228,7 @@ __device__ __forceinline__ int edge_rows(const Group<G>& gr, const Graph& g, con
   const int lane = gr.lane;
   const u32 lt = gr.below();
   const i32 m = e.m;
-  const i32* ltab = g.tab ? g.tab + (i64)((e.a_short ? e.b : e.a) - g.vb) * g.ld - g.vb : nullptr;
+  const i32* ltab = g.tab ? reinterpret_cast<const i32*>(g.tab + (i64)(e.a_short ? e.b : e.a) * g.row) : nullptr;
   // positions base + lane + G q of the shorter row: the vertex, its edges'
   // ranks, and whether it is in the link
   auto look = [&](int base, auto& w, auto& rs, auto& rl, auto& in) {
@@ -242,11 +267,9 @@ __device__ __forceinline__ int edge_rows(const Group<G>& gr, const Graph& g, con
       if (!gr.ballot(open && j < i)) break;
       i32 x[U], r[U];
       bool ask[U];
+      list_at(list, j, x);
 #pragma unroll
-      for (int q = 0; q < U; ++q) {
-        ask[q] = open && j + q < i;
-        x[q] = ask[q] ? list[j + q] : 0;
-      }
+      for (int q = 0; q < U; ++q) ask[q] = open && j + q < i;
       g.ranks(x, ask, w[0], r);
 #pragma unroll
       for (int q = 0; q < U; ++q) open &= r[q] >= m;
@@ -289,11 +312,9 @@ __device__ __forceinline__ int edge_rows(const Group<G>& gr, const Graph& g, con
     while (tested == 0 ? left != 0 : __popc(left) * (base / G + 1) > (top - tested) / U) {
       i32 x[U], r[U];
       bool ask[U];
+      list_at(list, tested, x);
 #pragma unroll
-      for (int q = 0; q < U; ++q) {
-        ask[q] = open && tested + q < i;
-        x[q] = ask[q] ? list[tested + q] : 0;
-      }
+      for (int q = 0; q < U; ++q) ask[q] = open && tested + q < i;
       g.ranks(x, ask, w, r);
 #pragma unroll
       for (int q = 0; q < U; ++q) open &= r[q] >= m;
@@ -435,7 +456,7 @@ __global__ void __launch_bounds__(LK_NT, LK_BLOCKS) k_links(const i32* __restric
   ph::pdl_wait();
   ph::pdl_trigger();
   constexpr int PER = 32 / G;  // edges a warp has in flight
-  __shared__ i32 lists[LK_WARPS][LK_LIST];
+  __shared__ __align__(16) i32 lists[LK_WARPS][LK_LIST];
   __shared__ unsigned long long sum[2];
   const Group<G> gr;
   const Group<32> wp;
@@ -559,7 +580,7 @@ __global__ void __launch_bounds__(LK_NT) k_tet_links(LinkGraph lg, TetArgs ta,
   ph::pdl_wait();
   ph::pdl_trigger();
   constexpr int U = 4;  // lookups a lane has in flight
-  __shared__ i32 lists[LK_WARPS][LK_LIST];
+  __shared__ __align__(16) i32 lists[LK_WARPS][LK_LIST];
   __shared__ unsigned long long sum[2];
   const Group<32> gr;
   const int lane = gr.lane;
@@ -602,9 +623,12 @@ __global__ void __launch_bounds__(LK_NT) k_tet_links(LinkGraph lg, TetArgs ta,
         tets += __popc(left);
         int tested = 0;
         while (tested < held && __popc(left) * ((held - tested + 31) / 32) > (tested ? (held - tested) / U : 0)) {
-          i32 r[U];
+          i32 x[U], r[U];
+          bool ask[U];
+          list_at(list, tested, x);
 #pragma unroll
-          for (int u = 0; u < U; ++u) r[u] = open && tested + u < held ? g.rank(list[tested + u], q) : NO_RANK;
+          for (int u = 0; u < U; ++u) ask[u] = open && tested + u < held;
+          g.ranks(x, ask, q, r);
 #pragma unroll
           for (int u = 0; u < U; ++u) open &= r[u] >= m;
           tested += U;
