@@ -195,6 +195,57 @@ __global__ void __launch_bounds__(SCAN_NT) k_scan_coop(const In* __restrict__ in
   }
 }
 
+// Short scans (up to SCAN_SMALL values): every block sums all values before
+// its tile again and scans the tile. Nothing passes between blocks, so it is an
+// ordinary dependent launch: the cooperative form's barrier and its launch,
+// which waits for the whole chip, cost more than the reads (at most 240 KB of
+// L2 hits a block). 5.1-6.3 us -> 3.2-5 us up to 10,000 values, 4.5-6 us at
+// 31,000, and the launches before and after overlap it: calls of 211, 500 and
+// 20,000 points 324 -> 308, 578 -> 555 and 686 -> 667 us.
+constexpr int SMALL_NT = 1024;
+constexpr int SMALL_ITEMS = 4;
+constexpr i64 SMALL_TILE = SMALL_NT * SMALL_ITEMS;
+constexpr i64 SCAN_SMALL = 65536;
+
+template <typename In, typename Out>
+__global__ void __launch_bounds__(SMALL_NT) k_scan_small(const In* __restrict__ in, i64 n, Out* __restrict__ out,
+                                                        const int* active) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  if (active && !*active) return;
+  __shared__ Out sm[SMALL_NT / 32];
+  __shared__ Out tile[SMALL_TILE];
+  const i64 base = (i64)blockIdx.x * SMALL_TILE;
+  Out before = 0;
+#pragma unroll 8
+  for (i64 i = threadIdx.x; i < base; i += SMALL_NT) before += (Out)in[i];
+#pragma unroll
+  for (int k = 0; k < SMALL_ITEMS; ++k) {
+    const int j = k * SMALL_NT + threadIdx.x;
+    tile[j] = base + j < n ? (Out)in[base + j] : Out(0);
+  }
+  Out carry;
+  block_excl_scan<Out, SMALL_NT>(before, sm, &carry);  // also: the tile is filled
+  Out loc[SMALL_ITEMS];
+  Out sum = 0;
+#pragma unroll
+  for (int k = 0; k < SMALL_ITEMS; ++k) {
+    loc[k] = sum;
+    sum += tile[threadIdx.x * SMALL_ITEMS + k];
+  }
+  Out tot;
+  const Out ex = block_excl_scan<Out, SMALL_NT>(sum, sm, &tot) + carry;
+#pragma unroll
+  for (int k = 0; k < SMALL_ITEMS; ++k) tile[threadIdx.x * SMALL_ITEMS + k] = ex + loc[k];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < SMALL_ITEMS; ++k) {
+    const int j = k * SMALL_NT + threadIdx.x;
+    if (base + j < n) out[base + j] = tile[j];
+  }
+  if (threadIdx.x == 0 && base + SMALL_TILE >= n) out[n] = carry + tot;
+}
+
 template <typename In, typename Out>
 int scan_impl(const In* in, Out* out, i64 n, void* ws, size_t ws_bytes, cudaStream_t s,
               const int* active) {
@@ -208,6 +259,15 @@ int scan_impl(const In* in, Out* out, i64 n, void* ws, size_t ws_bytes, cudaStre
   Carve c(ws, ws_bytes);
   Out* part = c.take<Out>(nparts);
   if (!part) return PH_ERR_ARG;
+  // blocks read their predecessors' values again: not for a scan in place
+  const uintptr_t i0 = (uintptr_t)in, o0 = (uintptr_t)out;
+  if (n <= SCAN_SMALL && (i0 + n * sizeof(In) <= o0 || o0 + (n + 1) * sizeof(Out) <= i0)) {
+    ph::count_launch();
+    ph::launch_pdl(k_scan_small<In, Out>, dim3((unsigned)((n + SMALL_TILE - 1) / SMALL_TILE)), dim3(SMALL_NT), 0, s,
+                   in, n, out, active);
+    PH_CHECK_LAUNCH();
+    return PH_OK;
+  }
   if (nparts <= COOP_MAX_PARTS) {
     const int per_sm = ph::occupancy((const void*)k_scan_coop<In, Out>, SCAN_NT, 0);
     const i64 resident = (i64)ph::device_sms() * per_sm;
