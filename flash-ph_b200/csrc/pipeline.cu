@@ -399,7 +399,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   // On dense graphs the per-edge triangle count costs sum(deg^2), and a call
   // over the triangle limit (the reference's ValueError, with the exact total
   // in its text) needs nothing but that total: it comes from the unsorted
-  // edges (an upper adjacency built by counting, no sort) and a shared-bitmap
+  // edges (degree-ordered words of 64 vertices, by counting) and a shared-bitmap
   // pass, before the filtration order and the forest are built.
   const bool total_first = max_dim >= 1 && 4.0 * (double)E * (double)E / (double)n > 2e8 &&
                            n <= ph_triangles_total_max_vertices();
