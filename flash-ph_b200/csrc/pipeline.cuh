@@ -12,30 +12,53 @@
 namespace ph {
 namespace pl {
 
-// stream-ordered allocations released together when the run ends
+// Stream-ordered allocations released together when the run ends. A call takes
+// some 50 buffers, most of them small, and an allocation with its release costs
+// the host about a microsecond while a small call's kernels, of 2 to 5 us each,
+// wait for their launches: requests of up to ARENA_SMALL bytes share slabs.
+// Calls of 211, 500, 4001 and 20,000 points 311 -> 293 us, 577 -> 549, 667 -> 652,
+// 685 -> 651.
+constexpr size_t ARENA_SMALL = 512 << 10;
+constexpr size_t ARENA_SLAB = 4 << 20;
 struct Arena {
   cudaStream_t s;
   std::vector<void*> ptrs;
+  char* slab = nullptr;  // the newest slab's unused part
+  size_t left = 0;
   bool failed = false;
   explicit Arena(cudaStream_t st) : s(st) {}
   Arena(const Arena&) = delete;
   Arena& operator=(const Arena&) = delete;
-  template <typename T>
-  T* take(i64 count) {
+  void* raw(size_t bytes) {
     void* p = nullptr;
-    const size_t bytes = (size_t)std::max<i64>(count, 1) * sizeof(T);
     if (cudaMallocAsync(&p, bytes, s) != cudaSuccess) {
       failed = true;
       return nullptr;
     }
     ptrs.push_back(p);
-    return static_cast<T*>(p);
+    return p;
+  }
+  template <typename T>
+  T* take(i64 count) {
+    const size_t bytes = (size_t)std::max<i64>(count, 1) * sizeof(T);
+    if (bytes > ARENA_SMALL) return static_cast<T*>(raw(bytes));
+    const size_t need = (bytes + 255) & ~size_t(255);
+    if (need > left) {
+      slab = static_cast<char*>(raw(ARENA_SLAB));
+      left = slab ? ARENA_SLAB : 0;
+      if (!slab) return nullptr;
+    }
+    char* p = slab;
+    slab += need;
+    left -= need;
+    return reinterpret_cast<T*>(p);
   }
   void* bytes(size_t n) { return take<unsigned char>((i64)std::max<size_t>(n, 1)); }
   // hands the buffers to a result, which frees them later
   void release_to(std::vector<void*>& keep) {
     keep.swap(ptrs);
     ptrs.clear();
+    left = 0;
   }
   ~Arena() {
     for (void* p : ptrs) cudaFreeAsync(p, s);
