@@ -18,7 +18,8 @@
 // 3-6% of the triangles of dense clouds and 10-25% of sparser ones, 1.0-1.6
 // rows an edge, so the cofacet rows, their order and the reducer's columns
 // shrink by that factor, and only these triangles need storing for H1.
-// Measured, all triangles as rows -> these rows: 1501 x 8 Gaussian (6.1M
+// Measured with the reducer of one addition a step (present calls are faster on
+// both sides), all triangles as rows -> these rows: 1501 x 8 Gaussian (6.1M
 // triangles, 209K rows) 8.8 -> 2.0 ms a call; 4001-point torus in 3-D (0.94M,
 // 90K) 3.8 -> 1.0 ms; a union of 192 clouds of 64-4096 points 119 -> 27 ms;
 // 20,000 x 10 at 1.4 (17.6K, 13.4K) unchanged, 0.88 ms.
