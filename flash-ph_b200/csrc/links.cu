@@ -51,6 +51,7 @@
 #include <algorithm>
 #include <climits>
 
+#include "arith.cuh"
 #include "links.cuh"
 
 namespace ph {
@@ -64,15 +65,6 @@ constexpr int LK_BLOCKS = 4;   // resident blocks an SM
 constexpr int LK_CHUNK = 8;    // stash rows a group takes at a time
 constexpr u32 FULL = 0xffffffffu;
 constexpr i32 NO_RANK = INT_MAX;
-
-__device__ __forceinline__ int lower_bound_i32(const i32* __restrict__ a, int lo, int hi, i32 x) {
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (a[mid] < x) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
 
 // the graph as one warp sees it for an edge: adjacency rows, and the rank
 // table of the edge's cloud where there is one
@@ -107,7 +99,7 @@ struct Graph {
       bool more = false;
 #pragma unroll
       for (int q = 0; q < N; ++q) {
-        mid[q] = (lo[q] + hi[q]) >> 1;
+        mid[q] = midpoint(lo[q], hi[q]);
         more |= lo[q] < hi[q];
       }
       if (!more) break;
@@ -229,17 +221,19 @@ __device__ __forceinline__ int edge_rows(const Group<G>& gr, const Graph& g, con
   const int lane = gr.lane;
   const u32 lt = gr.below();
   const i32 m = e.m;
+  const u32 end = e.s1;
   const i32* ltab = g.tab ? reinterpret_cast<const i32*>(g.tab + (i64)(e.a_short ? e.b : e.a) * g.row) : nullptr;
   // positions base + lane + G q of the shorter row: the vertex, its edges'
-  // ranks, and whether it is in the link
-  auto look = [&](int base, auto& w, auto& rs, auto& rl, auto& in) {
+  // ranks, and whether it is in the link (positions past the row's end may
+  // pass 2^31: unsigned)
+  auto look = [&](u32 base, auto& w, auto& rs, auto& rl, auto& in) {
     constexpr int N = sizeof(w) / sizeof(w[0]);
     int lo[N], hi[N];
 #pragma unroll
     for (int q = 0; q < N; ++q) {
-      const int p = base + lane + G * q;
-      rs[q] = p < e.s1 ? g.arank[p] : NO_RANK;
-      w[q] = p < e.s1 ? g.aidx[p] : 0;
+      const u32 p = base + lane + G * q;
+      rs[q] = p < end ? g.arank[p] : NO_RANK;
+      w[q] = p < end ? g.aidx[p] : 0;
     }
     if (ltab) {
 #pragma unroll
@@ -280,8 +274,9 @@ __device__ __forceinline__ int edge_rows(const Group<G>& gr, const Graph& g, con
     gr.sync();  // the list is free for the next edge
     return nl;
   }
-  int nl = 0, held = 0, stop = e.s1;  // link length, vertices in the list, row position after the last of them
-  for (int base = e.s0; base < e.s1; base += U * G) {
+  int nl = 0, held = 0;
+  u32 stop = end;  // vertices in the link and in the list, row position after the last of the list's
+  for (u32 base = e.s0; base < end; base += U * G) {
     i32 w[U], rs[U], rl[U];
     bool in[U];
     look(base, w, rs, rl, in);
@@ -289,7 +284,7 @@ __device__ __forceinline__ int edge_rows(const Group<G>& gr, const Graph& g, con
     for (int q = 0; q < U; ++q) {
       const u32 vb = gr.ballot(in[q]);
       const int cnt = __popc(vb);
-      if (stop == e.s1) {
+      if (stop == end) {
         if (nl + cnt <= LIST) {
           if (in[q]) list[nl + __popc(vb & lt)] = w[q];
           held = nl + cnt;
@@ -340,7 +335,7 @@ __device__ __forceinline__ int edge_rows(const Group<G>& gr, const Graph& g, con
   }
   if (nl > held) {  // a link longer than the list: its tail against the list, then against the row
     int at = held;
-    for (int base = stop; base < e.s1; base += G) {
+    for (u32 base = stop; base < end; base += G) {
       i32 w[1], rs[1], rl[1];
       bool in[1];
       look(base, w, rs, rl, in);
@@ -350,7 +345,7 @@ __device__ __forceinline__ int edge_rows(const Group<G>& gr, const Graph& g, con
         if (!gr.ballot(open)) break;
         if (open && g.rank(list[j], w[0]) < m) open = false;
       }
-      for (int x = stop; open && x < base + lane; ++x) {
+      for (u32 x = stop; open && x < base + lane; ++x) {
         const i32 v = g.aidx[x];
         if (g.arank[x] < m && g.rank(e.a_short ? e.b : e.a, v) < m && g.rank(v, w[0]) < m) open = false;
       }

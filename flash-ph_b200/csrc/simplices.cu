@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <climits>
 
+#include "arith.cuh"
 #include "pipeline.cuh"
 
 namespace ph {
@@ -34,15 +35,6 @@ constexpr int SX_WARPS = SX_NT / 32;
 // entries x (index, rank) = 36 KB a block.
 constexpr int SX_STAGE = 576;
 constexpr unsigned FULL = 0xffffffffu;
-
-__device__ __forceinline__ int lower_bound_i32(const i32* __restrict__ a, int lo, int hi, i32 x) {
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (a[mid] < x) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
 
 // EMIT = false: count; EMIT = true: write triangles.
 template <bool EMIT>
@@ -87,11 +79,11 @@ __global__ void __launch_bounds__(SX_NT) k_triangles(const i32* __restrict__ ei,
       }
       __syncwarp();
     }
-    for (int base = s0; base < s1; base += 32) {
-      const int p = base + lane;
+    for (u32 base = s0; base < (u32)s1; base += 32) {
+      const u32 p = base + lane;  // past the row's end: up to 2^31 + 29
       bool common = false, valid = false;
       i32 w = 0, rs = 0, rl = 0;
-      if (p < s1) {
+      if (p < (u32)s1) {
         w = aidx[p];
         rs = arank[p];
         if (staged) {
