@@ -305,7 +305,9 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
     E = H[0];
     if (E <= cap || E >= (int64_t(1) << 31)) break;
     cap = E;
+    for (void* p : {(void*)ei, (void*)ej, (void*)ed}) A.spare(p);
   }
+  A.spare(ew);
   if (E >= (int64_t(1) << 31)) return give_up(fail(PH_ERR_CAPACITY, "ph_rips_persistence_batch: union edge count exceeds the int32 range"));
   if (E > cap) return give_up(fail(PH_ERR_CAPACITY, "ph_rips_persistence_batch: edge counts of the two passes differ"));
 
@@ -332,13 +334,15 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   }
   PH_TRY(ph_batch_item_offsets(si, E, vcloud, K, e_off, s));
 
+  for (void* p : {(void*)ei, (void*)ej, (void*)ed, sort_ws, csr_ws}) A.spare(p);
+
   // ---- 3. H0 per cloud ----------------------------------------------------------------------------
   uint8_t* mask = A.take<uint8_t>(E);
   i32* comp = A.take<i32>(N);
   const size_t mst_b = ph_boruvka_workspace_bytes(N, E), h0_b = ph_batch_h0_rows_workspace_bytes(E);
   void* mst_ws = A.bytes(mst_b);
   void* h0_ws = A.bytes(h0_b);
-  if (A.failed || cudaMallocAsync((void**)&res->rows[0], sizeof(float) * 2 * N, s) != cudaSuccess) return alloc_fail();
+  if (A.failed || !(res->rows[0] = static_cast<float*>(A.get(sizeof(float) * 2 * N)))) return alloc_fail();
   {
     int rc = batch_forest(si, sj, E, N, e_off, dsegs, K, max_n, mask, comp, cnt + 15, st + 1, mst_ws, mst_b, s);
     if (rc == PH_OK) rc = ph_batch_h0_rows(filt, mask, E, e_off, dsegs, K, vcloud, N, res->rows[0], h0_ws, h0_b, s);
@@ -385,12 +389,10 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   links.stash.cap = link_stash_cap(E, N, 2 * E);  // 1.0 to 1.6 rows an edge are usual
   links.stash.totals = reinterpret_cast<LinkTotals*>(cnt + 8);
   // rank tables of the dense clouds, as far as 2 GiB go
-  i64 table_cap = 0;
-  for (int c = 0; c < K; ++c)
-    if (max_dim[c] >= 1 && n[c] <= LINK_TABLE_MAX_N) table_cap += n[c] * n[c];
-  table_cap = std::min<i64>(table_cap, i64(1) << 29);
-  i32* table = table_cap ? A.take<i32>(table_cap) : nullptr;
-  int64_t* table_off = table ? A.take<int64_t>(K) : nullptr;
+  const i64 table_cap = E ? std::min<i64>(link_tables_bound(n, K, E), i64(1) << 29) : 0;
+  graph.table = table_cap ? A.optional<i32>(table_cap) : nullptr;
+  A.spare(const_cast<i32*>(graph.table), &graph.table);
+  int64_t* table_off = A.take<int64_t>(K);
   int64_t* per = A.take<int64_t>(K);
   int64_t* per_rows = A.take<int64_t>(K);
   uint8_t* cflag = A.take<uint8_t>(2 * K);  // per-cloud flags: [0, K) H1 kept, [K, 2K) H2 kept
@@ -404,33 +406,32 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   uint8_t* tkeep = A.take<uint8_t>(K);
   unsigned long long* ttot = A.take<unsigned long long>(K);
   if (A.failed) return alloc_fail();
-  const bool pre = max_triangles > 0 && E > 0 && N <= ph_triangles_total_max_vertices();
+  bool pre = max_triangles > 0 && E > 0 && N <= ph_triangles_total_max_vertices();
+  const size_t tt_b = pre ? ph_triangles_total_edges_workspace_bytes(E, N) : 0;
+  void* tt_ws = pre ? A.optional<char>((i64)tt_b) : nullptr;
+  pre = tt_ws != nullptr;  // without it the per-edge pass counts them all
   if (pre) {
     const double bound_m = std::pow(3.0 * (double)max_triangles / std::sqrt(2.0), 2.0 / 3.0);
     const i64 m_star = std::max<i64>(0, (i64)std::floor(bound_m) - 1);  // conservative: a few more clouds counted
     count_launch();
     ph::launch_pdl(k_tri_want, dim3(grid_for(K)), dim3(256), 0, s, (const int64_t*)e_off, K, m_star, want);
-    const size_t tt_b = ph_triangles_total_edges_workspace_bytes(E, N);
-    void* tt_ws = A.bytes(tt_b);
-    if (A.failed) return alloc_fail();
     PH_TRY(batch_triangles_total(si, sj, E, adj_ptr, N, vcloud, want, dsegs, K, ttot, tt_ws, tt_b, s));
     count_launch();
     ph::launch_pdl(k_tri_keep, dim3(grid_for(K)), dim3(256), 0, s, (const uint8_t*)want,
                    (const unsigned long long*)ttot, K, (i64)max_triangles, tkeep);
+    A.spare(tt_ws);
   }
-  {
-    int rc = PH_OK;
-    if (table) {
-      rc = link_table_offsets(dsegs, e_off, K, table_cap, table_off, s);
-      graph.table = table;
-      graph.table_off = table_off;
-      if (rc == PH_OK) rc = link_table(graph, table, s);
-    }
+  if (graph.table) {
+    int rc = link_table_offsets(dsegs, e_off, K, table_cap, table_off, s);
+    graph.table_off = table_off;
+    if (rc == PH_OK) rc = link_table(graph, const_cast<i32*>(graph.table), s);
     if (rc != PH_OK) return give_up(rc);
   }
   for (int attempt = 0; attempt < 2; ++attempt) {
-    links.stash.rows = A.take<LinkRow>(links.stash.cap);
+    // without room for the guess the rows are counted first
+    links.stash.rows = attempt ? A.take<LinkRow>(links.stash.cap) : A.optional<LinkRow>(links.stash.cap);
     if (A.failed) return alloc_fail();
+    if (!links.stash.rows) links.stash.cap = 0;
     if (E) {
       const int rc = link_count(si, sj, E, graph, pre ? tkeep : nullptr, mask, links, lk_ws, lk_b, s);
       if (rc != PH_OK) return give_up(rc);
@@ -452,6 +453,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
     if (readback_parts(parts, pre ? 6 : 4, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
     if (hcnt[10] <= links.stash.cap) break;
     links.stash.cap = link_stash_cap(E, N, hcnt[9]);
+    A.spare(links.stash.rows);
     ph::zero_async(cnt + 8, sizeof(LinkTotals), s);
   }
   if (hcnt[10] > links.stash.cap)
@@ -522,7 +524,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   int64_t* nrows1 = A.take<int64_t>(1);
   const size_t r1_b = ph_batch_persistence_rows_workspace_bytes(E);
   void* r1_ws = A.bytes(r1_b);
-  if (A.failed || cudaMallocAsync((void**)&res->rows[1], sizeof(float) * 2 * std::max<i64>(E, 1), s) != cudaSuccess)
+  if (A.failed || !(res->rows[1] = static_cast<float*>(A.get(sizeof(float) * 2 * std::max<i64>(E, 1)))))
     return alloc_fail();
   if (E) {
     int rc = PH_OK;
@@ -530,6 +532,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
       rc = ph_triangles_emit(si, sj, E, adj_ptr, adj_idx, adj_rank, tri_off, tri_m, tri_w, tri_fa, tri_fb, s);
     if (rc == PH_OK) rc = link_rows(R1, mask, links, (i32)E, row_m, row_tri, cmf1, data1, st + 5, s);
     if (rc != PH_OK) return give_up(rc);
+    A.spare(links.stash.rows);
   }
   // H1 columns: the non-forest edges of the clouds kept for H1
   if (E) {
@@ -564,8 +567,9 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
                    (const int64_t*)e_off, K, t_off);
   }
   // tetrahedra of the clouds kept (all of them at first), and their rows, per cloud
-  auto count_tets = [&](const uint8_t* keep) {
-    tc.stash.rows = A.take<TetRow>(tc.stash.cap);
+  auto count_tets = [&](const uint8_t* keep, bool guess) {
+    tc.stash.rows = guess ? A.optional<TetRow>(tc.stash.cap) : A.take<TetRow>(tc.stash.cap);
+    if (!tc.stash.rows) tc.stash.cap = 0;
     if (A.failed) return fail(PH_ERR_CUDA, "ph_rips_persistence_batch: device allocation failed");
     const int rc = tet_count(graph, tin, keep, tc, tq_ws, tq_b, s);
     if (rc != PH_OK) return rc;
@@ -584,7 +588,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
                                      row_off1, nrows1, r1_ws, r1_b, s);
     if (rc != PH_OK) return give_up(rc);
     if (tets && attempt == 0) {  // counted before waiting
-      rc = count_tets(nullptr);
+      rc = count_tets(nullptr, true);
       if (rc != PH_OK) return give_up(rc);
     }
     Part parts[4] = {{cnt, hcnt, 16 * sizeof(int64_t)},
@@ -643,8 +647,9 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
     i64 rows = 0;
     for (int c = 0; c < K; ++c) rows += keep2[c] ? hrows[c] : 0;
     tc.stash.cap = tet_stash_cap(T2, rows);
+    A.spare(tc.stash.rows);
     ph::zero_async(cnt + 11, sizeof(LinkTotals), s);
-    const int rc = count_tets(any_cleared2 ? cflag + K : nullptr);
+    const int rc = count_tets(any_cleared2 ? cflag + K : nullptr, false);
     if (rc != PH_OK) return give_up(rc);
     Part parts[2] = {{cnt, hcnt, 16 * sizeof(int64_t)}, {per_rows, hrows, sizeof(int64_t) * K}};
     if (readback_parts(parts, 2, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
@@ -666,7 +671,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   int64_t* nrows2 = A.take<int64_t>(1);
   const size_t r2_b = ph_batch_persistence_rows_workspace_bytes(T2);
   void* r2_ws = A.bytes(r2_b);
-  if (A.failed || cudaMallocAsync((void**)&res->rows[2], sizeof(float) * 2 * std::max<i64>(T2, 1), s) != cudaSuccess)
+  if (A.failed || !(res->rows[2] = static_cast<float*>(A.get(sizeof(float) * 2 * std::max<i64>(T2, 1)))))
     return alloc_fail();
   {
     int rc = mark_pivots_mapped(r1.state, r1.piv, E, (i32)E, row_tri, skip2, T2, s);
@@ -681,6 +686,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
       rc = tet_rows(si, sj, tin, skip2, tc, (i32)E, (i32)(E + T2), R2, tet_m, tet_faces, cmf2, len2, cursor2, off2,
                     data2, tq_ws, tq_b, st + 3, s);
     if (rc != PH_OK) return give_up(rc);
+    A.spare(tc.stash.rows);
     if (!tets) ph::zero_async(off2, sizeof(i32) * (T2 + 1), s);
   }
   i64 pool2 = pool_capacity(4 * R2, T2);

@@ -12,6 +12,7 @@ namespace {
 thread_local std::string g_last_error;
 std::atomic<unsigned long long> g_launches{0};
 thread_local bool g_dependent_launch = true;
+thread_local long long g_optional_limit = 0;
 std::atomic<long long> g_reduce_max_steps{0};
 std::atomic<long long> g_reduce_first_pool{0};
 }  // namespace
@@ -20,6 +21,7 @@ long long reduce_max_steps() {
   return v > 0 ? v : (1ll << 24);
 }
 long long reduce_first_pool_limit() { return g_reduce_first_pool.load(std::memory_order_relaxed); }
+long long optional_buffer_limit() { return g_optional_limit; }
 void record_error(cudaError_t e) { g_last_error = cudaGetErrorString(e); }
 void record_message(const char* msg) { g_last_error = msg; }
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
@@ -127,6 +129,8 @@ extern "C" void ph_set_reduce_limits(int64_t max_steps, int64_t first_pool_entri
   ph::g_reduce_max_steps.store(max_steps > 0 ? max_steps : 0, std::memory_order_relaxed);
   ph::g_reduce_first_pool.store(first_pool_entries > 0 ? first_pool_entries : 0, std::memory_order_relaxed);
 }
+
+extern "C" void ph_set_optional_buffer_limit(int64_t bytes) { ph::g_optional_limit = bytes > 0 ? bytes : 0; }
 
 // ---- a measurement probe: the latency of one dependent L2 load ------------------------
 namespace {

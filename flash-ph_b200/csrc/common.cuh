@@ -51,6 +51,9 @@ int reduce_lists(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int
 int mark_pivots_mapped(const int32_t* col_state, const int32_t* col_piv, int64_t K, int32_t row_base,
                        const int32_t* map, uint8_t* row_flag, int64_t R, cudaStream_t s);
 long long reduce_first_pool_limit();
+// The most bytes of a buffer that a call can do without
+// (ph_set_optional_buffer_limit; 0: no limit).
+long long optional_buffer_limit();
 
 // Raises a kernel's dynamic shared memory limit to the device's opt-in
 // maximum (minus the kernel's static shared memory). Always the same value,

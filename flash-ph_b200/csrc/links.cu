@@ -50,6 +50,9 @@
 // together first and one after another then, as above.
 #include <algorithm>
 #include <climits>
+#include <cmath>
+#include <functional>
+#include <vector>
 
 #include "arith.cuh"
 #include "links.cuh"
@@ -760,6 +763,25 @@ inline int links_grid(i64 E, int lanes) {
 i64 link_stash_cap(i64 E, i64 n, i64 rows) {
   const int lanes = lanes_for(E, n);
   return rows + (i64)links_grid(E, lanes) * (LK_NT / lanes + LK_WARPS) * LK_CHUNK;
+}
+
+i64 link_tables_bound(const int64_t* n, int K, i64 E) {
+  std::vector<i64> sizes;
+  for (int c = 0; c < K; ++c)
+    if (n[c] <= LINK_TABLE_MAX_N) sizes.push_back(n[c]);
+  std::sort(sizes.begin(), sizes.end(), std::greater<i64>());
+  i64 entries = 0;
+  double left = (double)E;
+  for (const i64 m : sizes) {
+    const double edges = std::sqrt((double)m) * (double)m / 8.0;
+    if (left < edges) {  // the next one's share: an upper bound for any smaller ones in its place
+      entries += (i64)std::ceil((double)m * (double)m * (left / edges));
+      break;
+    }
+    left -= edges;
+    entries += m * m;
+  }
+  return entries;
 }
 
 int link_table(const LinkGraph& g, i32* table, cudaStream_t s) {

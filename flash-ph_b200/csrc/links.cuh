@@ -58,6 +58,11 @@ __host__ __device__ inline bool link_table_pays(i64 n, i64 E) {
   return n <= LINK_TABLE_MAX_N && 64.0 * (double)E * (double)E > (double)n * (double)n * (double)n;
 }
 
+// The most entries that the tables of K clouds can take together, with E edges
+// in all: a table of n^2 entries needs a cloud of n^1.5 / 8 edges, so the
+// largest clouds first, as far as the edges go.
+i64 link_tables_bound(const int64_t* n, int K, i64 E);
+
 // Buffers of the two passes, E entries each (offsets E + 1). tri_off may be
 // null where the triangles' numbering is not needed.
 struct LinkCounts {

@@ -328,8 +328,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   const float thr_sq = to_f32(max_edge_length * max_edge_length);
 
   // ---- 1. edges (rips.py:170-200; edge_kernel.py) ----------------------------------------
-  const EdgeKernel ek = edge_kernel(n, d, edge_mode);
-  const bool screened = ek == EdgeKernel::screened;
+  EdgeKernel ek = edge_kernel(n, d, edge_mode);
   const i64 nblocks = (n + 127) / 128;
   const i64 ntiles = ph_cloud_tiles(n);
   ph_cloud_seg* seg = A.take<ph_cloud_seg>(1);
@@ -342,10 +341,16 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   int* st = reinterpret_cast<int*>(cnt + 1);
   count_launch();
   ph::launch_pdl(k_single_seg, dim3(1), dim3(1), 0, s, seg, blk, n, d, thr_sq, nblocks, cnt);
-  const size_t ews = screened                   ? ph_edges_screened_workspace_bytes(n, 1, d)
+  const size_t ews = ek == EdgeKernel::screened ? ph_edges_screened_workspace_bytes(n, 1, d)
                      : ek == EdgeKernel::nearby ? edges_near_workspace_bytes(n, d)
                                                 : 0;
-  void* ew = ews ? A.bytes(ews) : nullptr;
+  void* ew = nullptr;
+  if (edge_mode == 1) {
+    ew = A.bytes(ews);
+  } else if (ews && !(ew = A.optional<char>((i64)ews))) {
+    ek = EdgeKernel::direct;  // needs no scratch
+  }
+  const bool screened = ek == EdgeKernel::screened;
   const i64 pairs = n * (n - 1) / 2;
   // first edge buffer: 256 edges a point, 2^22 at least, and up to an eighth
   // of the pairs (at most 2^27 edges, 1.5 GiB): dense clouds (thresholds at
@@ -378,7 +383,9 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
     E = H[0];
     if (E <= cap || E >= (int64_t(1) << 31)) break;
     cap = E;
+    for (void* p : {(void*)ei, (void*)ej, (void*)ed}) A.spare(p);
   }
+  A.spare(ew);
   if (E >= (int64_t(1) << 31)) {
     char m[160];
     snprintf(m, sizeof m, "Edge count %lld exceeds int32 range; reduce max_edge_length", (long long)E);
@@ -404,15 +411,15 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   const bool total_first = max_dim >= 1 && 4.0 * (double)E * (double)E / (double)n > 2e8 &&
                            n <= ph_triangles_total_max_vertices();
   i64 T_total = -1;
-  if (total_first) {
-    const size_t tt_b = ph_triangles_total_edges_workspace_bytes(E, n);
-    void* tt_ws = A.bytes(tt_b);
-    if (A.failed) return alloc_fail();
+  const size_t tt_b = total_first ? ph_triangles_total_edges_workspace_bytes(E, n) : 0;
+  void* tt_ws = total_first ? A.optional<char>((i64)tt_b) : nullptr;
+  if (tt_ws) {  // else the per-edge pass counts them
     const int rc = ph_triangles_total_edges(ei, ej, E, n, reinterpret_cast<unsigned long long*>(cnt + 5), tt_ws,
                                             tt_b, s);
     if (rc != PH_OK) return give_up(rc);
     const int64_t* src[1] = {cnt + 5};
     if (readback(src, 1, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
+    A.spare(tt_ws);
     T_total = H[0];
     if (T_total > max_triangles) {
       char m[200];
@@ -444,6 +451,8 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
     ph::zero_async(adj_ptr, sizeof(i32) * (n + 1), s);
   }
 
+  for (void* p : {(void*)ei, (void*)ej, (void*)ed, sort_ws, csr_ws}) A.spare(p);
+
   // ---- 3. H0 (boruvka.py, persistence.py:169-192) ---------------------------------------------
   uint8_t* mask = A.take<uint8_t>(E);
   i32* comp = A.take<i32>(n);
@@ -451,7 +460,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   const size_t mst_b = ph_boruvka_workspace_bytes(n, E), h0_b = ph_h0_rows_workspace_bytes(E);
   void* mst_ws = A.bytes(mst_b);
   void* h0_ws = A.bytes(h0_b);
-  if (A.failed || cudaMallocAsync((void**)&res->rows[0], sizeof(float) * 2 * n, s) != cudaSuccess)
+  if (A.failed || !(res->rows[0] = static_cast<float*>(A.get(sizeof(float) * 2 * n))))
     return alloc_fail();
   {
     int rc = ph_boruvka_mst(si, sj, E, n, mask, comp, ncomp, st + 1, mst_ws, mst_b, s);
@@ -485,23 +494,24 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   links.stash.totals = reinterpret_cast<LinkTotals*>(cnt + 8);
   const size_t lk_b = link_count_workspace_bytes(E);
   void* lk_ws = A.bytes(lk_b);
-  i32* table = link_table_pays(n, E) ? A.take<i32>(n * n) : nullptr;
+  graph.table = link_table_pays(n, E) ? A.optional<i32>(n * n) : nullptr;
+  A.spare(const_cast<i32*>(graph.table), &graph.table);
   if (A.failed) return alloc_fail();
   {
     int rc = PH_OK;
-    if (table) {
-      graph.table = table;
-      rc = link_table(graph, table, s);
-    }
+    if (graph.table) rc = link_table(graph, const_cast<i32*>(graph.table), s);
     for (int attempt = 0; attempt < 2; ++attempt) {
-      links.stash.rows = A.take<LinkRow>(links.stash.cap);
+      // without room for the guess the rows are counted first
+      links.stash.rows = attempt ? A.take<LinkRow>(links.stash.cap) : A.optional<LinkRow>(links.stash.cap);
       if (A.failed) return alloc_fail();
+      if (!links.stash.rows) links.stash.cap = 0;
       if (rc == PH_OK && E) rc = link_count(si, sj, E, graph, nullptr, mask, links, lk_ws, lk_b, s);
       if (rc != PH_OK) return give_up(rc);
       const int64_t* src[4] = {cnt + 8, cnt + 1, cnt + 9, cnt + 10};
       if (readback(src, 4, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
       if (H[3] <= links.stash.cap || H[0] > max_triangles) break;
       links.stash.cap = link_stash_cap(E, n, H[2]);
+      A.spare(links.stash.rows);
       ph::zero_async(cnt + 8, sizeof(LinkTotals), s);
     }
   }
@@ -541,7 +551,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   i32* row_m = A.take<i32>(R1);
   i32* data1 = A.take<i32>(3 * R1);
   i32* cmf1 = A.take<i32>(R1);
-  if (A.failed || cudaMallocAsync((void**)&res->rows[1], sizeof(float) * 2 * std::max<i64>(E, 1), s) != cudaSuccess)
+  if (A.failed || !(res->rows[1] = static_cast<float*>(A.get(sizeof(float) * 2 * std::max<i64>(E, 1)))))
     return alloc_fail();
   if (T && max_dim == 2) {
     const int rc = ph_triangles_emit(si, sj, E, adj_ptr, adj_idx, adj_rank, tri_off, tri_m, tri_w, tri_fa, tri_fb, s);
@@ -557,8 +567,9 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   TetCounts tc{};
   void* tq_ws = nullptr;
   const size_t tq_b = link_count_workspace_bytes(T);
-  auto count_tets = [&]() {  // enqueued; the totals are read later
-    tc.stash.rows = A.take<TetRow>(tc.stash.cap);
+  auto count_tets = [&](bool guess) {  // enqueued; the totals are read later
+    tc.stash.rows = guess ? A.optional<TetRow>(tc.stash.cap) : A.take<TetRow>(tc.stash.cap);
+    if (!tc.stash.rows) tc.stash.cap = 0;
     if (A.failed) return fail(PH_ERR_CUDA, "ph_rips_persistence: device allocation failed");
     return tet_count(graph, tin, nullptr, tc, tq_ws, tq_b, s);
   };
@@ -569,7 +580,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
     tc.stash.totals = reinterpret_cast<LinkTotals*>(cnt + 11);
     tq_ws = A.bytes(tq_b);
     if (A.failed) return alloc_fail();
-    const int rc = count_tets();
+    const int rc = count_tets(true);
     if (rc != PH_OK) return give_up(rc);
   }
   auto tets_limit = [&]() -> int {
@@ -588,8 +599,9 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
     int rc = tets_limit();
     if (rc != PH_OK || stash_ <= tc.stash.cap) return rc;
     tc.stash.cap = tet_stash_cap(T, R2);
+    A.spare(tc.stash.rows);
     ph::zero_async(cnt + 11, sizeof(LinkTotals), s);
-    rc = count_tets();
+    rc = count_tets(false);
     if (rc != PH_OK) return rc;
     const int64_t* src[1] = {cnt + 13};
     if (readback(src, 1, slots, s) != PH_OK) return (int)PH_ERR_CUDA;
@@ -605,6 +617,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   if (E) {
     const int rc = link_rows(R1, mask, links, (i32)E, row_m, row_tri, cmf1, data1, st + 3, s);
     if (rc != PH_OK) return give_up(rc);
+    A.spare(links.stash.rows);
   }
 
   // ---- 5. H1 reduction and rows (reduce_h1_gpu.py:159-223, 574-604) --------------------------
@@ -652,7 +665,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   i32* len2 = A.take<i32>(T);
   i32* cursor2 = A.take<i32>(T);
   i32* data2 = A.take<i32>(4 * R2);
-  if (A.failed || cudaMallocAsync((void**)&res->rows[2], sizeof(float) * 2 * std::max<i64>(T, 1), s) != cudaSuccess)
+  if (A.failed || !(res->rows[2] = static_cast<float*>(A.get(sizeof(float) * 2 * std::max<i64>(T, 1)))))
     return alloc_fail();
   {
     int rc = mark_pivots_mapped(r1.state, r1.piv, E, (i32)E, row_tri, skip2, T, s);
@@ -660,6 +673,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
       rc = tet_rows(si, sj, tin, skip2, tc, (i32)E, (i32)(E + T), R2, tet_m, tet_faces, cmf2, len2, cursor2, off2,
                     data2, tq_ws, tq_b, st + 3, s);
     if (rc != PH_OK) return give_up(rc);
+    A.spare(tc.stash.rows);
     if (!tets) ph::zero_async(off2, sizeof(i32) * (T + 1), s);
   }
   i64 pool2 = pool_capacity(4 * R2, T);

@@ -22,29 +22,50 @@ constexpr size_t ARENA_SMALL = 512 << 10;
 constexpr size_t ARENA_SLAB = 4 << 20;
 struct Arena {
   cudaStream_t s;
-  std::vector<void*> ptrs;
+  std::vector<void*> ptrs, slabs;
   char* slab = nullptr;  // the newest slab's unused part
   size_t left = 0;
   bool failed = false;
+  // buffers to give back where memory runs out, with the pointer to clear
+  // (null: nothing reads them any more)
+  struct Spare {
+    void* p;
+    const i32** slot;
+  };
+  std::vector<Spare> spares;
   explicit Arena(cudaStream_t st) : s(st) {}
   Arena(const Arena&) = delete;
   Arena& operator=(const Arena&) = delete;
-  void* raw(size_t bytes) {
+  // null where it is not to be had, spares given back or not (the error is the
+  // caller's to report, not the next launch's)
+  void* get(size_t bytes) {
     void* p = nullptr;
-    if (cudaMallocAsync(&p, bytes, s) != cudaSuccess) {
-      failed = true;
-      return nullptr;
+    if (cudaMallocAsync(&p, bytes, s) == cudaSuccess) return p;
+    cudaGetLastError();
+    if (spares.empty()) return nullptr;
+    for (const Spare& x : spares) {
+      ptrs.erase(std::find(ptrs.begin(), ptrs.end(), x.p));
+      cudaFreeAsync(x.p, s);
+      if (x.slot) *x.slot = nullptr;
     }
-    ptrs.push_back(p);
+    spares.clear();
+    if (cudaMallocAsync(&p, bytes, s) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+  }
+  void* raw(size_t bytes, std::vector<void*>& kept) {
+    void* p = get(bytes);
+    if (p) kept.push_back(p);
+    else failed = true;
     return p;
   }
   template <typename T>
   T* take(i64 count) {
     const size_t bytes = (size_t)std::max<i64>(count, 1) * sizeof(T);
-    if (bytes > ARENA_SMALL) return static_cast<T*>(raw(bytes));
+    if (bytes > ARENA_SMALL) return static_cast<T*>(raw(bytes, ptrs));
     const size_t need = (bytes + 255) & ~size_t(255);
     if (need > left) {
-      slab = static_cast<char*>(raw(ARENA_SLAB));
+      slab = static_cast<char*>(raw(ARENA_SLAB, slabs));
       left = slab ? ARENA_SLAB : 0;
       if (!slab) return nullptr;
     }
@@ -54,14 +75,33 @@ struct Arena {
     return reinterpret_cast<T*>(p);
   }
   void* bytes(size_t n) { return take<unsigned char>((i64)std::max<size_t>(n, 1)); }
+  // A buffer that the call can do without (a table, the first guess of a size):
+  // null where it is not to be had, or is over ph_set_optional_buffer_limit,
+  // and the call goes on.
+  template <typename T>
+  T* optional(i64 count) {
+    const long long limit = optional_buffer_limit();
+    if (limit > 0 && std::max<i64>(count, 1) * (i64)sizeof(T) > limit) return nullptr;
+    T* p = take<T>(count);
+    if (!p) failed = false;
+    return p;
+  }
+  // p may go where memory runs out (nothing happens to one that lies in a slab)
+  void spare(void* p, const i32** slot = nullptr) {
+    if (p && std::find(ptrs.begin(), ptrs.end(), p) != ptrs.end()) spares.push_back(Spare{p, slot});
+  }
   // hands the buffers to a result, which frees them later
   void release_to(std::vector<void*>& keep) {
     keep.swap(ptrs);
+    keep.insert(keep.end(), slabs.begin(), slabs.end());
     ptrs.clear();
+    slabs.clear();
+    spares.clear();
     left = 0;
   }
   ~Arena() {
     for (void* p : ptrs) cudaFreeAsync(p, s);
+    for (void* p : slabs) cudaFreeAsync(p, s);
   }
 };
 

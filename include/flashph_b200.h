@@ -63,6 +63,14 @@ void ph_set_dependent_launch(int32_t enable);
  * without a device fault. */
 void ph_set_reduce_limits(int64_t max_steps, int64_t first_pool_entries);
 
+/* Test-only, for the calling host thread: buffers that a native call can do
+ * without (the rank table of the triangle pass, the scratch of the faster edge
+ * kernels, the first guess of the triangle and tetrahedron rows) are taken as
+ * not to be had when they are larger than `bytes`. The call then runs the form
+ * that needs none, as it does when the device is out of memory, with the same
+ * results. 0 restores the default. No counterpart in the reference. */
+void ph_set_optional_buffer_limit(int64_t bytes);
+
 /* Measurement probe: one thread follows `hops` links of the cycle `next`
  * (next[i] is the index of the next entry; a random cycle over a buffer that
  * fits L2) from `start`, once to warm L2 and once timed; d_out[0] receives
