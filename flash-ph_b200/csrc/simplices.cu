@@ -215,7 +215,8 @@ __global__ void k_tri_degrees(const i32* __restrict__ ei, const i32* __restrict_
   }
 }
 
-// Counting sort by descending degree: bin vbase + n_c - 1 - degree, so the new
+// Counting sort by descending degree: bin vbase + n_c - 1 - degree (the first
+// one for more half-edges than that, which only repeated edges give), so the new
 // numbers of a cloud's vertices are its old ones in another order. PLACE:
 // start holds the bins' prefix and count runs from zero again. Lanes of one
 // bin count together (most vertices of a sparse graph share a few degrees).
@@ -231,12 +232,13 @@ __global__ void k_tri_bins(const i32* __restrict__ deg, const i32* __restrict__ 
     i32 bin = -1;
     if (v < n) {
       const i32 d = aptr ? aptr[v + 1] - aptr[v] : deg[v];
-      i64 top = n - 1;
+      i64 first = 0, top = n - 1;
       if (g.vcloud) {
         const ph_cloud_seg* c = g.segs + g.vcloud[v];
+        first = c->vbase;
         top = c->vbase + c->n - 1;
       }
-      bin = (i32)(top - d);
+      bin = (i32)max(first, top - d);
     }
     const u32 same = __match_any_sync(FULL, bin);
     const int first = __ffs(same) - 1;
@@ -265,9 +267,10 @@ __global__ void k_tri_rows(const i32* __restrict__ ei, const i32* __restrict__ e
 }
 
 // The nonzero words of each row, a warp a row: bits into the warp's bitmap
-// (with a bit a word beside it, so that only words in use are visited).
-__global__ void k_tri_words(const i32* __restrict__ ptr, const i32* __restrict__ idx, i64 n, int nwords,
-                            u64* __restrict__ mask, uint16_t* __restrict__ at, i32* __restrict__ len) {
+// (with a bit a word beside it, so that only words in use are visited). A row
+// with repeated entries is rewritten with each of them once, -1 after the last.
+__global__ void k_tri_words(const i32* __restrict__ ptr, i32* idx, i64 n, int nwords,
+                            u64* mask, uint16_t* at, i32* __restrict__ len) {
   ph::pdl_wait();
   ph::pdl_trigger();
   extern __shared__ u64 wbits[];
@@ -286,7 +289,7 @@ __global__ void k_tri_words(const i32* __restrict__ ptr, const i32* __restrict__
       atomicOr(&used[b >> 11], 1u << ((b >> 6) & 31));
     }
     __syncwarp();
-    int out = s;
+    int out = s, distinct = 0;
     if (e > s)
       for (int s0 = 0; s0 < nsum; s0 += 32) {
         const u32 mine = s0 + lane < nsum ? used[s0 + lane] : 0;
@@ -295,9 +298,11 @@ __global__ void k_tri_words(const i32* __restrict__ ptr, const i32* __restrict__
           const u32 set = __shfl_sync(FULL, mine, l);
           if ((set >> lane) & 1u) {
             const int w = (s0 + l) * 32 + lane, o = out + __popc(set & lanemask_lt());
-            mask[o] = bits[w];
+            const u64 v = bits[w];
+            mask[o] = v;
             at[o] = (uint16_t)w;
             bits[w] = 0;
+            distinct += __popcll(v);
           }
           out += __popc(set);
         }
@@ -305,6 +310,16 @@ __global__ void k_tri_words(const i32* __restrict__ ptr, const i32* __restrict__
       }
     if (lane == 0) len[a] = out - s;
     __syncwarp();
+    if (__reduce_add_sync(FULL, distinct) != e - s) {
+      int p = s;
+      for (int o = s; o < out; ++o)
+        for (int half = 0; half < 2; ++half) {
+          const u32 h = (u32)(mask[o] >> (32 * half));
+          if ((h >> lane) & 1u) idx[p + __popc(h & lanemask_lt())] = (i32)at[o] * 64 + 32 * half + lane;
+          p += __popc(h);
+        }
+      for (p += lane; p < e; p += 32) idx[p] = -1;
+    }
   }
 }
 
@@ -348,8 +363,8 @@ __global__ void __launch_bounds__(SX_NT) k_tri_count(const i32* __restrict__ ptr
     for (int p0 = s; p0 < e; p0 += SX_NT) {
       __syncthreads();
       if (p0 + (int)threadIdx.x < e) {
-        const i32 b = idx[p0 + threadIdx.x];
-        rows[threadIdx.x] = make_int2(ptr[b], len[b]);
+        const i32 b = idx[p0 + threadIdx.x];  // -1: a repeated entry
+        rows[threadIdx.x] = b < 0 ? make_int2(0, 0) : make_int2(ptr[b], len[b]);
       }
       __syncthreads();
       const int m = min(SX_NT, e - p0);
@@ -796,7 +811,7 @@ int tri_total_run(const i32* ei, const i32* ej, i64 E, i64 n, const i32* aptr, c
   const i64 occ_w = std::max(1, ph::occupancy((const void*)k_tri_words, warps * 32, words_smem));
   ph::count_launch();
   ph::launch_pdl(k_tri_words, dim3((unsigned)std::min<i64>((n + warps - 1) / warps, sms * occ_w)), dim3(warps * 32),
-                 words_smem, s, (const i32*)ptr, (const i32*)idx, n, nwords, mask, at, len);
+                 words_smem, s, (const i32*)ptr, idx, n, nwords, mask, at, len);
   const i64 occ_c = std::max(1, ph::occupancy((const void*)k_tri_count, SX_NT, count_smem));
   ph::count_launch();
   ph::launch_pdl(k_tri_count, dim3((unsigned)std::min<i64>(n, sms * occ_c)), dim3(SX_NT), count_smem, s,

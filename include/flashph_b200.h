@@ -236,7 +236,8 @@ int ph_triangles_total(const int32_t* adj_ptr, const int32_t* adj_idx, int64_t n
  * shared bitmap meets them word by word. The total the count pass
  * of triangle_kernel.py:288 triangle_enumerate checks against max_triangles
  * (triangle_kernel.py:377-381), for a call that may be over the limit, before
- * any filtration order exists. n <= ph_triangles_total_max_vertices(). */
+ * any filtration order exists. An edge given more than once counts once.
+ * n <= ph_triangles_total_max_vertices(). */
 size_t ph_triangles_total_edges_workspace_bytes(int64_t E, int64_t n);
 int ph_triangles_total_edges(const int32_t* edge_i, const int32_t* edge_j, int64_t E, int64_t n,
                              unsigned long long* d_total, void* workspace, size_t workspace_bytes, void* stream);
