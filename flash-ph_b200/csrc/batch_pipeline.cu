@@ -406,16 +406,18 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   uint8_t* tkeep = A.take<uint8_t>(K);
   unsigned long long* ttot = A.take<unsigned long long>(K);
   if (A.failed) return alloc_fail();
-  bool pre = max_triangles > 0 && E > 0 && N <= ph_triangles_total_max_vertices();
+  const double bound_m = std::pow(3.0 * (double)std::max<int64_t>(max_triangles, 0) / std::sqrt(2.0), 2.0 / 3.0);
+  const i64 m_star = std::max<i64>(0, (i64)std::floor(bound_m) - 1);  // conservative: a few more clouds counted
+  // (no cloud has more edges than all of them, or than the largest one's pairs)
+  bool pre = max_triangles > 0 && std::min<i64>(E, max_n * (max_n - 1) / 2) > m_star &&
+             N <= ph_triangles_total_max_vertices();
   const size_t tt_b = pre ? ph_triangles_total_edges_workspace_bytes(E, N) : 0;
   void* tt_ws = pre ? A.optional<char>((i64)tt_b) : nullptr;
   pre = tt_ws != nullptr;  // without it the per-edge pass counts them all
   if (pre) {
-    const double bound_m = std::pow(3.0 * (double)max_triangles / std::sqrt(2.0), 2.0 / 3.0);
-    const i64 m_star = std::max<i64>(0, (i64)std::floor(bound_m) - 1);  // conservative: a few more clouds counted
     count_launch();
     ph::launch_pdl(k_tri_want, dim3(grid_for(K)), dim3(256), 0, s, (const int64_t*)e_off, K, m_star, want);
-    PH_TRY(batch_triangles_total(si, sj, E, adj_ptr, N, vcloud, want, dsegs, K, ttot, tt_ws, tt_b, s));
+    PH_TRY(batch_triangles_total(si, sj, E, adj_ptr, N, max_n, vcloud, want, dsegs, K, ttot, tt_ws, tt_b, s));
     count_launch();
     ph::launch_pdl(k_tri_keep, dim3(grid_for(K)), dim3(256), 0, s, (const uint8_t*)want,
                    (const unsigned long long*)ttot, K, (i64)max_triangles, tkeep);

@@ -190,9 +190,10 @@ int batch_forest(const i32* edge_i, const i32* edge_j, i64 E, i64 n, const i64* 
                  size_t workspace_bytes, cudaStream_t s);
 
 // Triangles per cloud of a batch's union graph, of the clouds with want set
-// (the others' are zero); the workspace is ph_triangles_total_edges's.
-int batch_triangles_total(const i32* edge_i, const i32* edge_j, i64 E, const i32* adj_ptr, i64 n, const i32* vcloud,
-                          const uint8_t* want, const ph_cloud_seg* segs, int K, unsigned long long* d_per,
+// (the others' are zero); max_n is the largest cloud's vertex count; the
+// workspace is ph_triangles_total_edges's.
+int batch_triangles_total(const i32* edge_i, const i32* edge_j, i64 E, const i32* adj_ptr, i64 n, i64 max_n,
+                          const i32* vcloud, const uint8_t* want, const ph_cloud_seg* segs, int K, unsigned long long* d_per,
                           void* workspace, size_t workspace_bytes, cudaStream_t s);
 
 }  // namespace pl

@@ -266,11 +266,14 @@ __global__ void k_tri_rows(const i32* __restrict__ ei, const i32* __restrict__ e
   }
 }
 
-// The nonzero words of each row, a warp a row: bits into the warp's bitmap
+// The nonzero words of each row, a warp a row: bits into the warp's bitmap, which
+// spans the largest cloud (words count from the row's cloud on, so that a batch
+// of small clouds keeps its warps and blocks: 3000 clouds of 300 points, none
+// over its limit, 2.5 ms for this and the count with bitmaps of the union)
 // (with a bit a word beside it, so that only words in use are visited). A row
 // with repeated entries is rewritten with each of them once, -1 after the last.
-__global__ void k_tri_words(const i32* __restrict__ ptr, i32* idx, i64 n, int nwords,
-                            u64* mask, uint16_t* at, i32* __restrict__ len) {
+__global__ void k_tri_words(const i32* __restrict__ ptr, i32* idx, i64 n, int nwords, u64* mask, uint16_t* at,
+                            i32* __restrict__ len, TriClouds g) {
   ph::pdl_wait();
   ph::pdl_trigger();
   extern __shared__ u64 wbits[];
@@ -283,31 +286,35 @@ __global__ void k_tri_words(const i32* __restrict__ ptr, i32* idx, i64 n, int nw
   __syncwarp();
   for (i64 a = (i64)blockIdx.x * warps + wl; a < n; a += (i64)gridDim.x * warps) {
     const int s = ptr[a], e = ptr[a + 1];
+    if (s == e) {
+      if (lane == 0) len[a] = 0;
+      continue;
+    }
+    const i32 first = g.vcloud ? (i32)g.segs[g.vcloud[a]].vbase : 0;
     for (int p = s + lane; p < e; p += 32) {
-      const i32 b = idx[p];
+      const i32 b = idx[p] - first;
       atomicOr(reinterpret_cast<u32*>(bits) + (b >> 5), 1u << (b & 31));
       atomicOr(&used[b >> 11], 1u << ((b >> 6) & 31));
     }
     __syncwarp();
     int out = s, distinct = 0;
-    if (e > s)
-      for (int s0 = 0; s0 < nsum; s0 += 32) {
-        const u32 mine = s0 + lane < nsum ? used[s0 + lane] : 0;
-        for (u32 some = __ballot_sync(FULL, mine != 0); some; some &= some - 1) {
-          const int l = __ffs(some) - 1;
-          const u32 set = __shfl_sync(FULL, mine, l);
-          if ((set >> lane) & 1u) {
-            const int w = (s0 + l) * 32 + lane, o = out + __popc(set & lanemask_lt());
-            const u64 v = bits[w];
-            mask[o] = v;
-            at[o] = (uint16_t)w;
-            bits[w] = 0;
-            distinct += __popcll(v);
-          }
-          out += __popc(set);
+    for (int s0 = 0; s0 < nsum; s0 += 32) {
+      const u32 mine = s0 + lane < nsum ? used[s0 + lane] : 0;
+      for (u32 some = __ballot_sync(FULL, mine != 0); some; some &= some - 1) {
+        const int l = __ffs(some) - 1;
+        const u32 set = __shfl_sync(FULL, mine, l);
+        if ((set >> lane) & 1u) {
+          const int w = (s0 + l) * 32 + lane, o = out + __popc(set & lanemask_lt());
+          const u64 v = bits[w];
+          mask[o] = v;
+          at[o] = (uint16_t)w;
+          bits[w] = 0;
+          distinct += __popcll(v);
         }
-        if (mine) used[s0 + lane] = 0;
+        out += __popc(set);
       }
+      if (mine) used[s0 + lane] = 0;
+    }
     if (lane == 0) len[a] = out - s;
     __syncwarp();
     if (__reduce_add_sync(FULL, distinct) != e - s) {
@@ -315,7 +322,7 @@ __global__ void k_tri_words(const i32* __restrict__ ptr, i32* idx, i64 n, int nw
       for (int o = s; o < out; ++o)
         for (int half = 0; half < 2; ++half) {
           const u32 h = (u32)(mask[o] >> (32 * half));
-          if ((h >> lane) & 1u) idx[p + __popc(h & lanemask_lt())] = (i32)at[o] * 64 + 32 * half + lane;
+          if ((h >> lane) & 1u) idx[p + __popc(h & lanemask_lt())] = first + (i32)at[o] * 64 + 32 * half + lane;
           p += __popc(h);
         }
       for (p += lane; p < e; p += 32) idx[p] = -1;
@@ -762,8 +769,9 @@ extern "C" int ph_batch_triangles_total(const int32_t* adj_ptr, const int32_t* a
 
 namespace {
 
-// E edges in any order (i < j not needed); aptr: row pointers of their adjacency, or null
-int tri_total_run(const i32* ei, const i32* ej, i64 E, i64 n, const i32* aptr, const TriClouds& g,
+// E edges in any order (i < j not needed); span: vertices of the largest cloud;
+// aptr: row pointers of their adjacency, or null
+int tri_total_run(const i32* ei, const i32* ej, i64 E, i64 n, i64 span, const i32* aptr, const TriClouds& g,
                   unsigned long long* d_total, void* workspace, size_t workspace_bytes, cudaStream_t s) {
   Carve c(workspace, workspace_bytes);
   i32* zeroed = c.take<i32>(5 * (n + 1));
@@ -797,7 +805,7 @@ int tri_total_run(const i32* ei, const i32* ej, i64 E, i64 n, const i32* aptr, c
   ph::count_launch();
   ph::launch_pdl(k_tri_rows<true>, dim3(grid_for(E)), dim3(256), 0, s, ei, ej, E, (const i32*)rank, g,
                  (const i32*)ptr, filled, idx);
-  const int nwords = (int)((n + 63) / 64), nsum = (nwords + 31) / 32;
+  const int nwords = (int)((span + 63) / 64), nsum = (nwords + 31) / 32;
   const size_t per_warp = 8 * (size_t)nwords + 4 * (size_t)nsum, count_smem = 8 * (size_t)nwords;
   if (ph::allow_dynamic_smem((const void*)k_tri_words) != cudaSuccess ||
       ph::allow_dynamic_smem((const void*)k_tri_count) != cudaSuccess) {
@@ -811,7 +819,7 @@ int tri_total_run(const i32* ei, const i32* ej, i64 E, i64 n, const i32* aptr, c
   const i64 occ_w = std::max(1, ph::occupancy((const void*)k_tri_words, warps * 32, words_smem));
   ph::count_launch();
   ph::launch_pdl(k_tri_words, dim3((unsigned)std::min<i64>((n + warps - 1) / warps, sms * occ_w)), dim3(warps * 32),
-                 words_smem, s, (const i32*)ptr, idx, n, nwords, mask, at, len);
+                 words_smem, s, (const i32*)ptr, idx, n, nwords, mask, at, len, g);
   const i64 occ_c = std::max(1, ph::occupancy((const void*)k_tri_count, SX_NT, count_smem));
   ph::count_launch();
   ph::launch_pdl(k_tri_count, dim3((unsigned)std::min<i64>(n, sms * occ_c)), dim3(SX_NT), count_smem, s,
@@ -844,11 +852,11 @@ extern "C" int ph_triangles_total_edges(const int32_t* edge_i, const int32_t* ed
     PH_CHECK_LAUNCH();
     return PH_OK;
   }
-  return tri_total_run(edge_i, edge_j, E, n, nullptr, TriClouds{}, d_total, workspace, workspace_bytes, s);
+  return tri_total_run(edge_i, edge_j, E, n, n, nullptr, TriClouds{}, d_total, workspace, workspace_bytes, s);
 }
 
 int ph::pl::batch_triangles_total(const i32* edge_i, const i32* edge_j, i64 E, const i32* adj_ptr, i64 n,
-                                  const i32* vcloud, const uint8_t* want, const ph_cloud_seg* segs, int K,
+                                  i64 max_n, const i32* vcloud, const uint8_t* want, const ph_cloud_seg* segs, int K,
                                   unsigned long long* d_per, void* workspace, size_t workspace_bytes,
                                   cudaStream_t s) {
   if (n > ph_triangles_total_max_vertices()) return PH_ERR_ARG;
@@ -857,7 +865,7 @@ int ph::pl::batch_triangles_total(const i32* edge_i, const i32* edge_j, i64 E, c
     PH_CHECK_LAUNCH();
     return PH_OK;
   }
-  return tri_total_run(edge_i, edge_j, E, n, adj_ptr, TriClouds{vcloud, want, segs, d_per}, nullptr, workspace,
+  return tri_total_run(edge_i, edge_j, E, n, max_n, adj_ptr, TriClouds{vcloud, want, segs, d_per}, nullptr, workspace,
                        workspace_bytes, s);
 }
 
