@@ -176,6 +176,8 @@ constexpr int CSR_WARP = 1024;    // entries a warp sorts in its registers
 constexpr int CSR_BIG_NT = 1024;
 constexpr int CSR_BLOCK = 16384;  // entries a block sorts in shared memory
 constexpr int CSR_RANGE = 32768;  // neighbours a block counts at a time in a longer row
+constexpr int CSR_FEW = 32;       // entries of one neighbour that a thread puts in order
+constexpr int CSR_RUN = 4096;     // and that a warp does
 constexpr u64 CSR_NONE = ~0ull;
 // half-edges: fewer are sorted by one cluster in less time than these six or
 // seven launches (16,000 edges 25 us by the sort, 36 us here; 24,000: 30, 31;
@@ -349,7 +351,9 @@ __global__ void __launch_bounds__(CSR_NT) k_csr_rows(const u64* __restrict__ hal
 
 // Rows beyond CSR_WARP, a block a row: in shared memory up to CSR_BLOCK
 // entries; beyond, by counting over ranges of neighbours (no row is too long),
-// where the entries of one neighbour (repeated edges) are put in rank order.
+// where the entries of one neighbour (repeated edges) are put in rank order: a
+// few by a thread, up to CSR_RUN by a warp, more by the block, since an edge may
+// be given any number of times and one thread's moves grow with its square.
 __global__ void __launch_bounds__(CSR_BIG_NT) k_csr_big(const u64* __restrict__ half, const i32* __restrict__ ptr,
                                                         i64 n, i32* __restrict__ idx, i32* __restrict__ rank,
                                                         const i32* __restrict__ big, const i32* __restrict__ nbig) {
@@ -357,6 +361,7 @@ __global__ void __launch_bounds__(CSR_BIG_NT) k_csr_big(const u64* __restrict__ 
   ph::pdl_trigger();
   extern __shared__ u64 key[];
   __shared__ int sums[32];
+  __shared__ int pick, run[2];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   for (int r = blockIdx.x; r < *nbig; r += gridDim.x) {
     const i32 v = big[r];
@@ -417,15 +422,37 @@ __global__ void __launch_bounds__(CSR_BIG_NT) k_csr_big(const u64* __restrict__ 
         }
       }
       __syncthreads();
-      // cnt[w] is now the end of w's entries: insertion sort of each run by rank
+      // cnt[w] is now the end of w's entries, which are put in rank order
+      static_assert(PER == 32, "a bit a counter");
+      u32 many = 0;  // the thread's neighbours left to the block
       for (int k = 0; k < PER; ++k) {
         const int w = t * PER + k, end = cnt[w], start = w ? cnt[w - 1] : done;
-        for (int a = start + 1; a < end; ++a) {
-          const i32 x = rank[a];
-          int b = a;
-          for (; b > start && rank[b - 1] > x; --b) rank[b] = rank[b - 1];
-          rank[b] = x;
+        if (end - start <= CSR_FEW)
+          for (int a = start + 1; a < end; ++a) {
+            const i32 x = rank[a];
+            int b = a;
+            for (; b > start && rank[b - 1] > x; --b) rank[b] = rank[b - 1];
+            rank[b] = x;
+          }
+        many |= (end - start > CSR_RUN ? 1u : 0u) << k;
+        for (u32 todo = __ballot_sync(0xffffffffu, end - start > CSR_FEW && end - start <= CSR_RUN); todo;
+             todo &= todo - 1) {
+          const int l = __ffs(todo) - 1;
+          const int rs = __shfl_sync(0xffffffffu, start, l), re = __shfl_sync(0xffffffffu, end, l);
+          bitonic_group(rank + rs, re - rs, lane, 32, [] { __syncwarp(); });
         }
+      }
+      while (__syncthreads_or(many != 0)) {
+        if (many) pick = t;  // one of them
+        __syncthreads();
+        if (pick == t) {
+          const int w = t * PER + __ffs(many) - 1;
+          many &= many - 1;
+          run[0] = w ? cnt[w - 1] : done;
+          run[1] = cnt[w];
+        }
+        __syncthreads();
+        bitonic_group(rank + run[0], run[1] - run[0], t, CSR_BIG_NT, [] { __syncthreads(); });
       }
       done += total;
       __syncthreads();

@@ -40,6 +40,31 @@ int rows_nosort(const i32* state, const i32* piv, i64 K, i32 row_base, const flo
                 const i32* row_m, const i64* col_off, int nsegs, float* out_rows, i64* row_off, i64* d_nrows,
                 void* ws, size_t ws_bytes, cudaStream_t s);
 
+// Ascending bitonic sort of n values (any 31-bit count) by a group of threads:
+// every comparison ascending (each merge starts with a mirrored step), so that
+// the missing values past n, larger than all others, never move.
+template <typename Sync>
+__device__ __forceinline__ void bitonic_group(i32* v, int n, int tid, int nthreads, Sync sync) {
+  u32 len2 = 2;
+  while (len2 < (u32)n) len2 <<= 1;
+  for (u32 size = 2; size && size <= len2; size <<= 1) {
+    for (u32 stride = size >> 1; stride > 0; stride >>= 1) {
+      const bool mirror = stride == (size >> 1);
+      for (u32 i = tid; i < (len2 >> 1); i += nthreads) {
+        const u32 lo = 2 * i - (i & (stride - 1));
+        const u32 hi = mirror ? (lo & ~(size - 1)) + size - 1 - (lo & (size - 1)) : lo + stride;
+        if (hi >= (u32)n) continue;
+        const i32 x = v[lo], y = v[hi];
+        if (x > y) {
+          v[lo] = y;
+          v[hi] = x;
+        }
+      }
+      sync();
+    }
+  }
+}
+
 // Workspace carving helper: aligned bump allocation inside a caller buffer.
 struct Carve {
   char* base;

@@ -176,31 +176,6 @@ __device__ __forceinline__ void sort8(i32 (&v)[8]) {
   order(v[1], v[2]), order(v[3], v[4]), order(v[5], v[6]);
 }
 
-// ascending bitonic sort of n values by a group of threads: every comparison
-// ascending (each merge starts with a mirrored step), so that the missing
-// values past n, larger than all others, never move
-template <typename Sync>
-__device__ __forceinline__ void bitonic_group(i32* v, int n, int tid, int nthreads, Sync sync) {
-  int len2 = 2;
-  while (len2 < n) len2 <<= 1;
-  for (int size = 2; size <= len2; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      const bool mirror = stride == (size >> 1);
-      for (int i = tid; i < (len2 >> 1); i += nthreads) {
-        const int lo = 2 * i - (i & (stride - 1));
-        const int hi = mirror ? (lo & ~(size - 1)) + size - 1 - (lo & (size - 1)) : lo + stride;
-        if (hi >= n) continue;
-        const i32 x = v[lo], y = v[hi];
-        if (x > y) {
-          v[lo] = y;
-          v[hi] = x;
-        }
-      }
-      sync();
-    }
-  }
-}
-
 __global__ void __launch_bounds__(RY_NT) k_ready(const i32* __restrict__ off, const i32* __restrict__ cof, i64 K,
                                                 i32 col_base, i32 row_base, const uint8_t* __restrict__ skip,
                                                 const i32* __restrict__ cmf, i32* __restrict__ state,
