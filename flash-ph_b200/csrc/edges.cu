@@ -186,12 +186,30 @@ constexpr i64 CSR_MIN = 48 * 1024;
 
 __device__ __forceinline__ i32 csr_rank(u64 half) { return (i32)((u32)half >> 1); }
 
+// A place in v's row, by a whole warp (v < 0: none). Where most lanes hold the
+// vertex of the lane before them (edges of one vertex in a run), lanes of one
+// vertex count together: the atomics of one address are served one by one.
+__device__ __forceinline__ int csr_place(i32 v, i32* __restrict__ cnt) {
+  const int lane = threadIdx.x & 31;
+  const i32 up = __shfl_up_sync(0xffffffffu, v, 1);
+  if (__popc(__ballot_sync(0xffffffffu, lane > 0 && v == up)) < 16) return v >= 0 ? atomicAdd(&cnt[v], 1) : 0;
+  const u32 same = __match_any_sync(0xffffffffu, v);
+  const int first = __ffs(same) - 1;
+  int at = 0;
+  if (lane == first && v >= 0) at = atomicAdd(&cnt[v], __popc(same));
+  return __shfl_sync(0xffffffffu, at, first) + __popc(same & lanemask_lt());
+}
+
 __global__ void k_csr_count(const i32* __restrict__ ei, const i32* __restrict__ ej, i64 E, i32* __restrict__ cnt,
                             int2* __restrict__ slot) {
   ph::pdl_wait();
   ph::pdl_trigger();
-  for (i64 e = (i64)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += (i64)gridDim.x * blockDim.x)
-    slot[e] = make_int2(atomicAdd(&cnt[ei[e]], 1), atomicAdd(&cnt[ej[e]], 1));
+  const i64 first = (i64)blockIdx.x * blockDim.x + threadIdx.x - (threadIdx.x & 31);
+  for (i64 e0 = first; e0 < E; e0 += (i64)gridDim.x * blockDim.x) {
+    const i64 e = e0 + (threadIdx.x & 31);
+    const int a = csr_place(e < E ? ei[e] : -1, cnt), b = csr_place(e < E ? ej[e] : -1, cnt);
+    if (e < E) slot[e] = make_int2(a, b);
+  }
 }
 
 __global__ void k_csr_scatter(const i32* __restrict__ ei, const i32* __restrict__ ej, i64 E,
@@ -319,11 +337,12 @@ __global__ void __launch_bounds__(CSR_NT) k_csr_short(const u64* __restrict__ ha
 }
 
 // A warp a row of up to CSR_WARP entries: those listed, or (no list) all n;
-// longer ones are listed for k_csr_big.
+// longer ones are listed for k_csr_big, in one list from both its ends.
 __global__ void __launch_bounds__(CSR_NT) k_csr_rows(const u64* __restrict__ half, const i32* __restrict__ ptr, i64 n,
                                                      const i32* __restrict__ list, const i32* __restrict__ nlist,
                                                      i32* __restrict__ idx, i32* __restrict__ rank,
-                                                     i32* __restrict__ big, i32* __restrict__ nbig) {
+                                                     i32* __restrict__ big, i32* __restrict__ nbig,
+                                                     i32* __restrict__ longs, i32* __restrict__ nlongs) {
   ph::pdl_wait();
   ph::pdl_trigger();
   extern __shared__ u64 key[];
@@ -344,119 +363,136 @@ __global__ void __launch_bounds__(CSR_NT) k_csr_rows(const u64* __restrict__ hal
       csr_warp_row<16>(half + s, len, idx + s, rank + s, buf);
     else if (len <= CSR_WARP)
       csr_warp_row<32>(half + s, len, idx + s, rank + s, buf);
-    else if ((threadIdx.x & 31) == 0)
-      big[atomicAdd(nbig, 1)] = (i32)v;
+    else if ((threadIdx.x & 31) == 0) {
+      if (len <= CSR_BLOCK) big[atomicAdd(nbig, 1)] = (i32)v;
+      else longs[-atomicAdd(nlongs, 1)] = (i32)v;
+    }
   }
 }
 
-// Rows beyond CSR_WARP, a block a row: in shared memory up to CSR_BLOCK
-// entries; beyond, by counting over ranges of neighbours (no row is too long),
-// where the entries of one neighbour (repeated edges) are put in rank order: a
-// few by a thread, up to CSR_RUN by a warp, more by the block, since an edge may
-// be given any number of times and one thread's moves grow with its square.
+// The entries of one row whose neighbours are in [lo, lo + CSR_RANGE), to their
+// places, by a block: counted, with those of smaller neighbours, and placed from
+// the counters' scan; the entries of one neighbour (repeated edges) are then put
+// in rank order: a few by a thread, up to CSR_RUN by a warp, more by the block,
+// since an edge may be given any number of times and one thread's moves grow
+// with its square.
+__device__ void csr_range(const u64* __restrict__ half, int s, int len, i64 lo, i32* cnt, i32* __restrict__ idx,
+                          i32* __restrict__ rank) {
+  __shared__ int sums[32];
+  __shared__ int before_lo, pick, run[2];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  for (int k = t; k < CSR_RANGE; k += CSR_BIG_NT) cnt[k] = 0;
+  if (t == 0) before_lo = 0;
+  __syncthreads();
+  int below = 0;
+#pragma unroll 4
+  for (int p = t; p < len; p += CSR_BIG_NT) {
+    const i64 w = (i64)(half[s + p] >> 32) - lo;
+    below += w < 0;
+    if (w >= 0 && w < CSR_RANGE) atomicAdd(&cnt[w], 1);
+  }
+  below = __reduce_add_sync(0xffffffffu, below);
+  if (lane == 0 && below) atomicAdd(&before_lo, below);
+  __syncthreads();
+  // each thread's CSR_RANGE / CSR_BIG_NT counters, the threads' sums, then starts in place of counts
+  constexpr int PER = CSR_RANGE / CSR_BIG_NT;
+  int sum = 0;
+  for (int k = 0; k < PER; ++k) sum += cnt[t * PER + k];
+  int incl = sum;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) sums[warp] = incl;
+  __syncthreads();
+  const int done = s + before_lo;
+  int before = 0;
+  for (int w = 0; w < warp; ++w) before += sums[w];
+  int at = done + before + incl - sum;
+  for (int k = 0; k < PER; ++k) {
+    const int c = cnt[t * PER + k];
+    cnt[t * PER + k] = at;
+    at += c;
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int p = t; p < len; p += CSR_BIG_NT) {
+    const u64 x = half[s + p];
+    const i64 w = (i64)(x >> 32) - lo;
+    if (w >= 0 && w < CSR_RANGE) {
+      const int o = atomicAdd(&cnt[w], 1);
+      idx[o] = (i32)(x >> 32);
+      rank[o] = csr_rank(x);
+    }
+  }
+  __syncthreads();
+  // cnt[w] is now the end of w's entries, which are put in rank order
+  static_assert(PER == 32, "a bit a counter");
+  u32 many = 0;  // the thread's neighbours left to the block
+  for (int k = 0; k < PER; ++k) {
+    const int w = t * PER + k, end = cnt[w], start = w ? cnt[w - 1] : done;
+    if (end - start <= CSR_FEW)
+      for (int a = start + 1; a < end; ++a) {
+        const i32 x = rank[a];
+        int b = a;
+        for (; b > start && rank[b - 1] > x; --b) rank[b] = rank[b - 1];
+        rank[b] = x;
+      }
+    many |= (end - start > CSR_RUN ? 1u : 0u) << k;
+    for (u32 todo = __ballot_sync(0xffffffffu, end - start > CSR_FEW && end - start <= CSR_RUN); todo; todo &= todo - 1) {
+      const int l = __ffs(todo) - 1;
+      const int rs = __shfl_sync(0xffffffffu, start, l), re = __shfl_sync(0xffffffffu, end, l);
+      bitonic_group(rank + rs, re - rs, lane, 32, [] { __syncwarp(); });
+    }
+  }
+  while (__syncthreads_or(many != 0)) {
+    if (many) pick = t;  // one of them
+    __syncthreads();
+    if (pick == t) {
+      const int w = t * PER + __ffs(many) - 1;
+      many &= many - 1;
+      run[0] = w ? cnt[w - 1] : done;
+      run[1] = cnt[w];
+    }
+    __syncthreads();
+    bitonic_group(rank + run[0], run[1] - run[0], t, CSR_BIG_NT, [] { __syncthreads(); });
+  }
+}
+
+// Rows beyond CSR_WARP: a block a row in shared memory up to CSR_BLOCK entries
+// (big); longer ones (longs, descending from the list's end) by counting, a
+// block a range of CSR_RANGE neighbours, so that one long row is shared by many
+// blocks (no row is too long). One vertex joined to 2,000,000 others: 0.56 ms
+// by the radix sort, 38 by one block a row, 0.66 this way and with k_csr_count's
+// joint counts; 40 joined to 99,000 each: 1.05, 3.04, 0.50.
 __global__ void __launch_bounds__(CSR_BIG_NT) k_csr_big(const u64* __restrict__ half, const i32* __restrict__ ptr,
                                                         i64 n, i32* __restrict__ idx, i32* __restrict__ rank,
-                                                        const i32* __restrict__ big, const i32* __restrict__ nbig) {
+                                                        const i32* __restrict__ big, const i32* __restrict__ nbig,
+                                                        const i32* __restrict__ longs,
+                                                        const i32* __restrict__ nlongs) {
   ph::pdl_wait();
   ph::pdl_trigger();
   extern __shared__ u64 key[];
-  __shared__ int sums[32];
-  __shared__ int pick, run[2];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int t = threadIdx.x;
   for (int r = blockIdx.x; r < *nbig; r += gridDim.x) {
     const i32 v = big[r];
     const int s = ptr[v], len = ptr[v + 1] - s;
-    if (len <= CSR_BLOCK) {
-      int len2 = 2 * CSR_WARP;
-      while (len2 < len) len2 <<= 1;
-      for (int k = t; k < len2; k += CSR_BIG_NT) key[k] = k < len ? half[s + k] : CSR_NONE;
-      __syncthreads();
-      csr_bitonic(key, len2, t, CSR_BIG_NT, [] { __syncthreads(); });
-      for (int k = t; k < len; k += CSR_BIG_NT) {
-        idx[s + k] = (i32)(key[k] >> 32);
-        rank[s + k] = csr_rank(key[k]);
-      }
-      __syncthreads();
-      continue;
+    int len2 = 2 * CSR_WARP;
+    while (len2 < len) len2 <<= 1;
+    for (int k = t; k < len2; k += CSR_BIG_NT) key[k] = k < len ? half[s + k] : CSR_NONE;
+    __syncthreads();
+    csr_bitonic(key, len2, t, CSR_BIG_NT, [] { __syncthreads(); });
+    for (int k = t; k < len; k += CSR_BIG_NT) {
+      idx[s + k] = (i32)(key[k] >> 32);
+      rank[s + k] = csr_rank(key[k]);
     }
-    i32* cnt = reinterpret_cast<i32*>(key);
-    int done = s;  // entries of the ranges before
-    for (i64 lo = 0; lo < n; lo += CSR_RANGE) {
-      for (int k = t; k < CSR_RANGE; k += CSR_BIG_NT) cnt[k] = 0;
-      __syncthreads();
-      for (int p = s + t; p < s + len; p += CSR_BIG_NT) {
-        const i64 w = (i64)(half[p] >> 32) - lo;
-        if (w >= 0 && w < CSR_RANGE) atomicAdd(&cnt[w], 1);
-      }
-      __syncthreads();
-      // each thread's CSR_RANGE / CSR_BIG_NT counters, the threads' sums, then starts in place of counts
-      constexpr int PER = CSR_RANGE / CSR_BIG_NT;
-      int sum = 0;
-      for (int k = 0; k < PER; ++k) sum += cnt[t * PER + k];
-      int incl = sum;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-      }
-      if (lane == 31) sums[warp] = incl;
-      __syncthreads();
-      int before = 0, total = 0;
-      for (int w = 0; w < CSR_BIG_NT / 32; ++w) {
-        before += w < warp ? sums[w] : 0;
-        total += sums[w];
-      }
-      int at = done + before + incl - sum;
-      for (int k = 0; k < PER; ++k) {
-        const int c = cnt[t * PER + k];
-        cnt[t * PER + k] = at;
-        at += c;
-      }
-      __syncthreads();
-      for (int p = s + t; p < s + len; p += CSR_BIG_NT) {
-        const u64 x = half[p];
-        const i64 w = (i64)(x >> 32) - lo;
-        if (w >= 0 && w < CSR_RANGE) {
-          const int o = atomicAdd(&cnt[w], 1);
-          idx[o] = (i32)(x >> 32);
-          rank[o] = csr_rank(x);
-        }
-      }
-      __syncthreads();
-      // cnt[w] is now the end of w's entries, which are put in rank order
-      static_assert(PER == 32, "a bit a counter");
-      u32 many = 0;  // the thread's neighbours left to the block
-      for (int k = 0; k < PER; ++k) {
-        const int w = t * PER + k, end = cnt[w], start = w ? cnt[w - 1] : done;
-        if (end - start <= CSR_FEW)
-          for (int a = start + 1; a < end; ++a) {
-            const i32 x = rank[a];
-            int b = a;
-            for (; b > start && rank[b - 1] > x; --b) rank[b] = rank[b - 1];
-            rank[b] = x;
-          }
-        many |= (end - start > CSR_RUN ? 1u : 0u) << k;
-        for (u32 todo = __ballot_sync(0xffffffffu, end - start > CSR_FEW && end - start <= CSR_RUN); todo;
-             todo &= todo - 1) {
-          const int l = __ffs(todo) - 1;
-          const int rs = __shfl_sync(0xffffffffu, start, l), re = __shfl_sync(0xffffffffu, end, l);
-          bitonic_group(rank + rs, re - rs, lane, 32, [] { __syncwarp(); });
-        }
-      }
-      while (__syncthreads_or(many != 0)) {
-        if (many) pick = t;  // one of them
-        __syncthreads();
-        if (pick == t) {
-          const int w = t * PER + __ffs(many) - 1;
-          many &= many - 1;
-          run[0] = w ? cnt[w - 1] : done;
-          run[1] = cnt[w];
-        }
-        __syncthreads();
-        bitonic_group(rank + run[0], run[1] - run[0], t, CSR_BIG_NT, [] { __syncthreads(); });
-      }
-      done += total;
-      __syncthreads();
-    }
+    __syncthreads();
+  }
+  const i64 ranges = (n + CSR_RANGE - 1) / CSR_RANGE, items = *nlongs * ranges;
+  for (i64 q = blockIdx.x; q < items; q += gridDim.x) {
+    const i32 v = longs[-(q / ranges)];
+    csr_range(half, ptr[v], ptr[v + 1] - ptr[v], (q % ranges) * CSR_RANGE, reinterpret_cast<i32*>(key), idx, rank);
+    __syncthreads();
   }
 }
 
@@ -571,8 +607,9 @@ extern "C" int ph_vertex_csr(const int32_t* edge_i, const int32_t* edge_j, int64
   // the counts, the scan's parts and the list of long rows lie where the radix
   // sort's buffers would; vertices far beyond the edges do not fit there
   Carve w = rest;
-  i32* cnt = w.take<i32>(n + 3);
-  i32* big = w.take<i32>(2 * E / CSR_WARP + 1);
+  i32* cnt = w.take<i32>(n + 4);
+  const i64 nlist_big = 2 * E / CSR_WARP + 1;
+  i32* big = w.take<i32>(nlist_big);
   void* sws = w.take<char>((i64)scan_workspace_bytes(n));
   i32* list = w.take<i32>(2 * E / 32 + 1);
   if (2 * E >= CSR_MIN && cnt && big && sws && list) {
@@ -581,8 +618,8 @@ extern "C" int ph_vertex_csr(const int32_t* edge_i, const int32_t* edge_j, int64
       return PH_ERR_CUDA;
     }
     int2* slot = reinterpret_cast<int2*>(vals);
-    i32 *nbig = cnt + n + 1, *nlist = cnt + n + 2;
-    ph::zero_async(cnt, sizeof(i32) * (size_t)(n + 3), s);
+    i32 *nbig = cnt + n + 1, *nlist = cnt + n + 2, *nlongs = cnt + n + 3, *longs = big + nlist_big - 1;
+    ph::zero_async(cnt, sizeof(i32) * (size_t)(n + 4), s);
     ph::count_launch();
     ph::launch_pdl(k_csr_count, dim3(grid_for(E)), dim3(256), 0, s, edge_i, edge_j, E, cnt, slot);
     PH_TRY(scan_exclusive_i32_i32(cnt, adj_ptr, n, sws, scan_workspace_bytes(n), s));
@@ -605,12 +642,14 @@ extern "C" int ph_vertex_csr(const int32_t* edge_i, const int32_t* edge_j, int64
     ph::count_launch();
     ph::launch_pdl(k_csr_rows, dim3((unsigned)std::max<i64>(1, std::min<i64>((rows + CSR_NT / 32 - 1) / (CSR_NT / 32), sms * 2))),
                    dim3(CSR_NT), rows_smem, s, (const u64*)keys, (const i32*)adj_ptr, n,
-                   (const i32*)(sparse ? list : nullptr), (const i32*)nlist, adj_idx, adj_rank, big, nbig);
-    const i64 big_rows = std::min<i64>(n, 2 * E / (CSR_WARP + 1));
+                   (const i32*)(sparse ? list : nullptr), (const i32*)nlist, adj_idx, adj_rank, big, nbig,
+                   longs, nlongs);
+    // (not bounded by n: few vertices may share a long row's ranges, or have one edge many times)
+    const i64 big_rows = 2 * E / (CSR_WARP + 1);
     ph::count_launch();
     ph::launch_pdl(k_csr_big, dim3((unsigned)std::max<i64>(1, std::min<i64>(big_rows, sms))),
                    dim3(CSR_BIG_NT), sizeof(u64) * CSR_BLOCK, s, (const u64*)keys, (const i32*)adj_ptr, n, adj_idx,
-                   adj_rank, (const i32*)big, (const i32*)nbig);
+                   adj_rank, (const i32*)big, (const i32*)nbig, (const i32*)longs, (const i32*)nlongs);
     PH_CHECK_LAUNCH();
     return PH_OK;
   }
