@@ -344,7 +344,8 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   void* h0_ws = A.bytes(h0_b);
   if (A.failed || !(res->rows[0] = static_cast<float*>(A.get(sizeof(float) * 2 * N)))) return alloc_fail();
   {
-    int rc = batch_forest(si, sj, E, N, e_off, dsegs, K, max_n, mask, comp, cnt + 15, st + 1, mst_ws, mst_b, s);
+    int rc = batch_forest(si, sj, E, N, e_off, dsegs, K, max_n, mask, comp, cnt + 15, reinterpret_cast<int*>(cnt + 14), st + 1,
+                          mst_ws, mst_b, s);
     if (rc == PH_OK) rc = ph_batch_h0_rows(filt, mask, E, e_off, dsegs, K, vcloud, N, res->rows[0], h0_ws, h0_b, s);
     if (rc != PH_OK) return give_up(rc);
   }

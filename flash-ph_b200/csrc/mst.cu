@@ -71,7 +71,17 @@ constexpr u64 NO_OFFER = ~0ull;
 struct MstCtl {
   int offered;  // the last tick (round of all passes) in which some edge was live
   int hooked;   // roots that became children so far
+  i32 rest[8];  // clouds of a batch left to the grid
 };
+
+// A block passes a connected cloud's edges once its first few n are done with,
+// but looks at all of them where several components stay, 1 us for 1000. A
+// cloud of a batch with more than MST_MANY edges, and more than an eighth of
+// all, is given up after MST_TRY of them and left to the grid (0.1 ms and more a
+// cloud, one after another: two clouds of 0.4M edges lose by it, 1265 -> 1365 us
+// a call).
+constexpr i64 MST_TRY = i64(1) << 16, MST_MANY = i64(1) << 19;
+__host__ __device__ inline i64 mst_many(i64 E) { return E / 8 > MST_MANY ? E / 8 : MST_MANY; }
 
 // barriers; any(): whether some thread passed true (tick: the same for all, new each time)
 struct BlockBar {
@@ -126,11 +136,12 @@ struct MstArgs {
   i64* ncomp;
   int* status;
   int max_rounds;
+  i64 give_up;  // edges after which to leave off
 };
 
-// thread t of T
+// thread t of T; false where it left off
 template <typename Bar>
-__device__ void forest(Bar bar, i64 t, i64 T, const MstArgs& a, volatile i32* par, u64* offer) {
+__device__ bool forest(Bar bar, i64 t, i64 T, const MstArgs& a, volatile i32* par, u64* offer) {
   volatile u64* voff = offer;
   const i64 n = a.n, E = a.E;
   for (i64 v = t; v < n; v += T) {
@@ -166,6 +177,7 @@ __device__ void forest(Bar bar, i64 t, i64 T, const MstArgs& a, volatile i32* pa
   bar.sync();
   bool one = n == 1;  // a single component: no later edge can join two
   for (int tick = 0; lo < E && !one;) {
+    if (lo >= a.give_up) return false;
     i32 u[MST_SLOTS], v[MST_SLOTS];
     u32 live = 0;
 #pragma unroll
@@ -181,7 +193,7 @@ __device__ void forest(Bar bar, i64 t, i64 T, const MstArgs& a, volatile i32* pa
     for (int round = 0;; ++round, ++tick) {
       if (round >= a.max_rounds) {  // the same for all threads
         if (t == 0) set_status(a.status, PH_ERR_ITER_LIMIT);
-        return;
+        return true;
       }
       // offers: the lowest-ranked edge leaving each root; parents of the
       // vertices held are flat (all at a pass's start, roots after a round)
@@ -277,7 +289,7 @@ __device__ void forest(Bar bar, i64 t, i64 T, const MstArgs& a, volatile i32* pa
     for (i64 x = t; x < n; x += T) a.comp[x] = a.vbase;
     if (t == 0) atomicAdd((unsigned long long*)a.ncomp, 1ull);
     if (bad) set_status(a.status, PH_ERR_ITER_LIMIT);
-    return;
+    return true;
   }
   // labels: the smallest vertex of each component, and the component count.
   // Vertices ascend over the lanes, so the first lane of those with one root
@@ -295,6 +307,7 @@ __device__ void forest(Bar bar, i64 t, i64 T, const MstArgs& a, volatile i32* pa
   bar.sync();
   for (i64 x = t; x < n; x += T) a.comp[x] = a.vbase + *(volatile i32*)(a.minv + par[x]);
   if (bad) set_status(a.status, PH_ERR_ITER_LIMIT);
+  return true;
 }
 
 __global__ void __launch_bounds__(MST_NT, 1) k_mst_block(const MstArgs a) {
@@ -306,24 +319,34 @@ __global__ void __launch_bounds__(MST_NT, 1) k_mst_block(const MstArgs a) {
   forest(BlockBar{&ctl}, (i64)threadIdx.x, (i64)MST_NT, a, reinterpret_cast<i32*>(mst_smem + 2 * a.n), mst_smem);
 }
 
-// a block a cloud: edges [e_off[c], e_off[c + 1]), vertices from its segment; ncomp starts at zero
-__global__ void __launch_bounds__(MST_NT, 1) k_mst_clouds(MstArgs a, const i64* __restrict__ e_off,
-                                                          const ph_cloud_seg* __restrict__ segs) {
-  ph::pdl_wait();
-  ph::pdl_trigger();
-  extern __shared__ u64 mst_smem[];
-  __shared__ MstCtl ctl;
-  const i64 e0 = e_off[blockIdx.x];
-  const ph_cloud_seg g = segs[blockIdx.x];
+// one cloud of a batch: edges [e_off[c], e_off[c + 1]), vertices from its segment
+__device__ __forceinline__ MstArgs cloud_args(MstArgs a, const i64* __restrict__ e_off,
+                                              const ph_cloud_seg* __restrict__ segs, int c) {
+  const i64 e0 = e_off[c];
+  const ph_cloud_seg g = segs[c];
   a.ei += e0;
   a.ej += e0;
-  a.E = e_off[blockIdx.x + 1] - e0;
+  a.E = e_off[c + 1] - e0;
   a.n = g.n;
   a.vbase = (i32)g.vbase;
   a.minv += g.vbase;
   a.mst += e0;
   a.comp += g.vbase;
-  forest(BlockBar{&ctl}, (i64)threadIdx.x, (i64)MST_NT, a, reinterpret_cast<i32*>(mst_smem + 2 * a.n), mst_smem);
+  return a;
+}
+
+// a block a cloud; ncomp and nrest start at zero
+__global__ void __launch_bounds__(MST_NT, 1) k_mst_clouds(const MstArgs all, const i64* __restrict__ e_off,
+                                                          const ph_cloud_seg* __restrict__ segs, MstCtl* rest,
+                                                          int* nrest) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  extern __shared__ u64 mst_smem[];
+  __shared__ MstCtl ctl;
+  MstArgs a = cloud_args(all, e_off, segs, blockIdx.x);
+  a.give_up = a.E > mst_many(all.E) ? MST_TRY : LLONG_MAX;
+  const bool done = forest(BlockBar{&ctl}, (i64)threadIdx.x, (i64)MST_NT, a, reinterpret_cast<i32*>(mst_smem + 2 * a.n), mst_smem);
+  if (!done && threadIdx.x == 0) rest->rest[atomicAdd(nrest, 1)] = blockIdx.x;  // fewer than eight
 }
 
 __global__ void __launch_bounds__(MST_NT, 1) k_mst_cluster(const MstArgs a, i32* par, u64* offer, MstCtl* ctl) {
@@ -341,6 +364,20 @@ __global__ void __launch_bounds__(MST_NT, 1) k_mst_grid(const MstArgs a, i32* pa
   if (blockIdx.x == 0 && threadIdx.x == 0) *a.ncomp = 0;
   forest(GroupBar<cg::grid_group>{cg::this_grid(), ctl}, (i64)blockIdx.x * MST_NT + threadIdx.x,
          (i64)gridDim.x * MST_NT, a, par, offer);
+}
+
+// the clouds that the blocks left off, one after another
+__global__ void __launch_bounds__(MST_NT, 1) k_mst_rest(const MstArgs all, const i64* __restrict__ e_off,
+                                                        const ph_cloud_seg* __restrict__ segs, i32* par, u64* offer,
+                                                        MstCtl* ctl, const int* nrest) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  cg::grid_group g = cg::this_grid();
+  for (int q = 0; q < *nrest; ++q) {
+    forest(GroupBar<cg::grid_group>{g, ctl}, (i64)blockIdx.x * MST_NT + threadIdx.x, (i64)gridDim.x * MST_NT,
+           cloud_args(all, e_off, segs, ctl->rest[q]), par, offer);
+    g.sync();
+  }
 }
 
 __global__ void k_h0_rows(const float* __restrict__ filt, const uint8_t* __restrict__ mst,
@@ -439,7 +476,7 @@ extern "C" int ph_boruvka_mst(const int32_t* edge_i, const int32_t* edge_j, int6
   u64* offer = c.take<u64>(2 * n);
   if (!parent || !minv || !ctl || !offer) return PH_ERR_ARG;
   const int max_rounds = rounds_bound(n);
-  MstArgs a{edge_i, edge_j, E, n, 0, minv, mst_mask, comp, d_ncomp, d_status, max_rounds};
+  MstArgs a{edge_i, edge_j, E, n, 0, minv, mst_mask, comp, d_ncomp, d_status, max_rounds, LLONG_MAX};
   const i64 work = std::max<i64>(n, E);
   const int cs = takes_cluster(n, E) ? cluster_size() : 0;
   ph::count_launch();
@@ -476,25 +513,39 @@ extern "C" int ph_boruvka_mst(const int32_t* edge_i, const int32_t* edge_j, int6
 
 int ph::pl::batch_forest(const i32* edge_i, const i32* edge_j, i64 E, i64 n, const i64* e_off,
                          const ph_cloud_seg* segs, int K, i64 max_n, uint8_t* mst_mask, i32* comp, i64* d_ncomp,
-                         int* d_status, void* workspace, size_t workspace_bytes, cudaStream_t s) {
+                         int* d_left, int* d_status, void* workspace, size_t workspace_bytes, cudaStream_t s) {
   // A block takes 1 us for 1000 edges, the grid 0.26 us for 1000 of the union's
   // (many passes, each with its rounds): blocks where the largest cloud, by its
   // share of the vertices, has less than a quarter of the edges, or where a
   // block would take it on its own. 192 clouds of 64 to 4096 points, 11.0M
-  // edges: 2500 us by the grid -> 601 us.
+  // edges: 2500 us by the grid -> 601 us. The share is a guess: a cloud that
+  // turns out dense and in several components goes to the grid after all (40
+  // sparse clouds and one of two times 4000 points, 16M edges: whole call 14.5 ms by the
+  // grid, 16.2 by blocks alone, 6.6 this way).
   const i64 most = (i64)((double)E * max_n / n);
   if (max_n > MST_BLOCK_N || !(4 * max_n <= n || takes_block(max_n, most)))
     return ph_boruvka_mst(edge_i, edge_j, E, n, mst_mask, comp, d_ncomp, d_status, workspace, workspace_bytes, s);
   Carve c(workspace, workspace_bytes);
+  i32* parent = c.take<i32>(n);
   i32* minv = c.take<i32>(n);
-  if (!minv) return PH_ERR_ARG;
+  MstCtl* ctl = c.take<MstCtl>(1);
+  u64* offer = c.take<u64>(2 * n);
+  if (!parent || !minv || !ctl || !offer) return PH_ERR_ARG;
   if (ph::allow_dynamic_smem((const void*)k_mst_clouds) != cudaSuccess) {
     PH_CHECK_LAUNCH();
     return PH_ERR_CUDA;
   }
-  const MstArgs a{edge_i, edge_j, 0, 0, 0, minv, mst_mask, comp, d_ncomp, d_status, rounds_bound(max_n)};
+  const MstArgs a{edge_i, edge_j, E, 0, 0, minv, mst_mask, comp, d_ncomp, d_status, rounds_bound(max_n), LLONG_MAX};
   ph::count_launch();
-  ph::launch_pdl(k_mst_clouds, dim3((unsigned)K), dim3(MST_NT), block_smem(max_n), s, a, e_off, segs);
+  ph::launch_pdl(k_mst_clouds, dim3((unsigned)K), dim3(MST_NT), block_smem(max_n), s, a, e_off, segs, ctl,
+                 d_left);
+  if (std::min<i64>(E, max_n * (max_n - 1) / 2) > mst_many(E)) {  // else no cloud can have been given up
+    if (ph::occupancy((const void*)k_mst_rest, MST_NT, 0) < 1) return PH_ERR_CUDA;
+    void* args[] = {(void*)&a, (void*)&e_off, (void*)&segs, (void*)&parent, (void*)&offer, (void*)&ctl, (void*)&d_left};
+    ph::count_launch();
+    if (cudaLaunchCooperativeKernel((const void*)k_mst_rest, ph::device_sms(), MST_NT, args, 0, s) != cudaSuccess)
+      return PH_ERR_CUDA;
+  }
   PH_CHECK_LAUNCH();
   return PH_OK;
 }

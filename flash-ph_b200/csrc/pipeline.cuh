@@ -182,12 +182,13 @@ int reduce_only(Arena& A, cudaStream_t s, const i32* off, const i32* data, i64 K
                 i32 row_base, i64 span, const uint8_t* skip, const i32* cmf, i64 pool_cap, int* status, RedOut& o);
 
 // The forest of a batch's union graph: a block a cloud where every cloud fits
-// one, else ph_boruvka_mst over the union. Edges lie cloud by cloud (e_off);
-// max_n is the largest cloud's vertex count; *d_ncomp starts at zero; the
-// workspace is ph_boruvka_mst's.
+// one (those that it turns out too slow for by the grid then), else
+// ph_boruvka_mst over the union. Edges lie cloud by cloud (e_off); max_n is the
+// largest cloud's vertex count; *d_ncomp and *d_left (the clouds left to the
+// grid) start at zero; the workspace is ph_boruvka_mst's.
 int batch_forest(const i32* edge_i, const i32* edge_j, i64 E, i64 n, const i64* e_off, const ph_cloud_seg* segs,
-                 int K, i64 max_n, uint8_t* mst_mask, i32* comp, i64* d_ncomp, int* d_status, void* workspace,
-                 size_t workspace_bytes, cudaStream_t s);
+                 int K, i64 max_n, uint8_t* mst_mask, i32* comp, i64* d_ncomp, int* d_left, int* d_status,
+                 void* workspace, size_t workspace_bytes, cudaStream_t s);
 
 // Triangles per cloud of a batch's union graph, of the clouds with want set
 // (the others' are zero); max_n is the largest cloud's vertex count; the
