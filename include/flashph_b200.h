@@ -498,8 +498,10 @@ int ph_or_gather_mask(uint8_t* dst, const uint8_t* src, const int32_t* idx, int6
                       void* stream);
 
 /* k-th nearest-neighbour distance of every point of every cloud, k clamped
- * to n_c - 1 per cloud (threshold.py:133-176 _tiled_knn per cloud). qb_off (nsegs+1): per-cloud offsets of 128-point
- * query blocks; nqb their total; max_d the largest d. out: N floats. */
+ * to n_c - 1 per cloud (threshold.py:133-176 _tiled_knn per cloud). qb_off
+ * (nsegs+1): per-cloud offsets of 128-point query blocks; nqb their total;
+ * max_d the largest d (checked only: k alone chooses the form, as in
+ * ph_knn_kth). out: N floats. */
 int ph_batch_knn_kth(const float* pts, const ph_cloud_seg* segs, int32_t nsegs, const int64_t* qb_off,
                      int64_t nqb, int32_t max_d, int32_t k, float* out, void* stream);
 
@@ -513,7 +515,8 @@ int ph_batch_quantile(const float* values, int64_t N, const int32_t* vcloud, con
 /* ---- thresholds ---------------------------------------------------------- */
 
 /* k-th nearest-neighbour Euclidean distance of every point (self excluded),
- * threshold.py:133-176 _tiled_knn. k <= 64. out: n float32. */
+ * threshold.py:133-176 _tiled_knn: a buffer of the nearest up to k = 64, a
+ * radix select beyond, for any d. out: n float32. */
 int ph_knn_kth(const float* pts, int64_t n, int32_t d, int32_t k, float* out, void* stream);
 
 /* Linear-interpolation quantile of n values (torch.quantile semantics, as
