@@ -24,6 +24,7 @@ from .cohomology import h1_diagram, h2_diagram
 from .rips import edge_filtration_values, rips_filtration
 
 _VERTEX_PACK_BITS = 16
+_MAX_SIMPLICES = 10_000_000  # the reference's limits
 _VALID_BACKENDS = ("auto", "gpu", "giotto")
 
 
@@ -56,6 +57,13 @@ def rips_persistence(
     list[Tensor]
         [H0, H1, ...], each (K, 2) float32 on the input's device.
     """
+    return limited_persistence(points, max_edge_length, max_dim, backend)
+
+
+def limited_persistence(points, max_edge_length: float, max_dim: int = 1, backend: str = "auto",
+                        max_triangles: int = _MAX_SIMPLICES, max_tetrahedra: int = _MAX_SIMPLICES) -> list[Tensor]:
+    """``rips_persistence`` with the reference's limits (triangle_kernel.py,
+    cohomology_general.py) as arguments, which its public call does not have."""
     if isinstance(points, np.ndarray):
         points = torch.from_numpy(points).float()
         if torch.cuda.is_available():
@@ -88,9 +96,10 @@ def rips_persistence(
     dev = points.device
     with torch.cuda.device(dev):
         if os.environ.get("FLASHPH_PIPELINE", "native") == "staged":
-            dgms = _compute_staged(points, float(max_edge_length), max_dim)
+            dgms = _compute_staged(points, float(max_edge_length), max_dim, max_triangles, max_tetrahedra)
         else:
-            return _compute_native(points.float().contiguous(), float(max_edge_length), max_dim, out_device)
+            return _compute_native(points.float().contiguous(), float(max_edge_length), max_dim, out_device,
+                                   max_triangles, max_tetrahedra)
     if out_device != dev:
         dgms = [d.to(out_device) for d in dgms]
     return dgms
@@ -99,8 +108,8 @@ def rips_persistence(
 _EDGE_MODES = {"auto": 0, "on": 1, "off": 2}
 
 
-def _compute_native(points: Tensor, t: float, max_dim: int, out_device, max_triangles: int = 10_000_000,
-                    max_tetrahedra: int = 10_000_000) -> list[Tensor]:
+def _compute_native(points: Tensor, t: float, max_dim: int, out_device, max_triangles: int = _MAX_SIMPLICES,
+                    max_tetrahedra: int = _MAX_SIMPLICES) -> list[Tensor]:
     """The whole call in the CUDA library (ph_rips_persistence); diagrams are
     copied straight to the caller's device (pinned host memory for CPU
     callers)."""
@@ -137,7 +146,8 @@ def _compute_native(points: Tensor, t: float, max_dim: int, out_device, max_tria
     return outs
 
 
-def _compute_staged(points: Tensor, t: float, max_dim: int) -> list[Tensor]:
+def _compute_staged(points: Tensor, t: float, max_dim: int, max_triangles: int = _MAX_SIMPLICES,
+                    max_tetrahedra: int = _MAX_SIMPLICES) -> list[Tensor]:
     """The same computation stage by stage from Python (each stage its own
     library call); kept as a cross-check of the native pipeline and for the
     stage-level timers."""
@@ -152,9 +162,10 @@ def _compute_staged(points: Tensor, t: float, max_dim: int) -> list[Tensor]:
         check_status("ph_boruvka_mst", mst_status)
         return [h0]
     with _timing.stage("h1"):
-        h1, tris, red1, _ = h1_diagram(filt, edge_filt, mst_mask, checks=[("ph_boruvka_mst", mst_status)])
+        h1, tris, red1, _ = h1_diagram(filt, edge_filt, mst_mask, max_triangles,
+                                       checks=[("ph_boruvka_mst", mst_status)])
     if max_dim == 1:
         return [h0, h1]
     with _timing.stage("h2"):
-        h2, _, _, _ = h2_diagram(filt, edge_filt, tris, red1)
+        h2, _, _, _ = h2_diagram(filt, edge_filt, tris, red1, max_tetrahedra)
     return [h0, h1, h2]

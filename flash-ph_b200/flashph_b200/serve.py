@@ -41,7 +41,7 @@ import torch
 
 from . import _lib as L
 from .batch import rips_persistence_batch, worker_stream as slot_stream
-from .persistence import rips_persistence
+from .persistence import limited_persistence
 
 
 class _Request:
@@ -161,7 +161,8 @@ class PersistenceServer:
                     if len(batch) == 1 and batch[0].n >= self.solo_min_points:
                         r = batch[0]
                         try:
-                            res = [rips_persistence(r.points, r.t, max_dim=r.max_dim)]
+                            res = [limited_persistence(r.points, r.t, r.max_dim, max_triangles=self.max_triangles,
+                                                       max_tetrahedra=self.max_tetrahedra)]
                         except ValueError as ex:  # the reference's per-call errors
                             res = [ex]
                     else:
