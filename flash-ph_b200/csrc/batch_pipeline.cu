@@ -35,7 +35,7 @@ struct ph_batch_result {
   cudaStream_t stream = nullptr;
   std::vector<int32_t> status;        // per cloud: PH_OK or PH_ERR_LIMIT
   std::vector<std::string> message;   // per cloud: the ValueError text of a limit
-  std::vector<int64_t> stat[3];       // per cloud: edges, triangles, tetrahedra (-1: not counted)
+  std::vector<int64_t> stat[4];       // per cloud: edges, triangles, tetrahedra, H1 rows (-1: not counted)
   float* rows[3] = {nullptr, nullptr, nullptr};
   std::vector<int64_t> off[3];        // per dim: nclouds + 1 row offsets into rows[dim]
   std::vector<void*> scratch;
@@ -475,6 +475,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   for (int c = 0; c < K; ++c) {
     res->stat[0][c] = hoff[c + 1] - hoff[c];
     res->stat[1][c] = hper[c];
+    res->stat[3][c] = hrows[c];
     R1 += hrows[c];
     if (max_dim[c] < 1) continue;
     if (hper[c] > max_triangles) {
@@ -727,7 +728,7 @@ extern "C" const char* ph_batch_result_message(const ph_batch_result* r, int32_t
 }
 
 extern "C" int64_t ph_batch_result_stat(const ph_batch_result* r, int32_t cloud, int32_t k) {
-  if (!r || cloud < 0 || cloud >= r->nclouds || k < 0 || k > 2) return -1;
+  if (!r || cloud < 0 || cloud >= r->nclouds || k < 0 || k > 3) return -1;
   return r->stat[k][cloud];
 }
 

@@ -368,8 +368,9 @@ def _chunks(order, sizes, max_points=_CHUNK_POINTS, max_pairs=_CHUNK_PAIRS):
 
 
 class _Split(Exception):
-    """The chunk is over the rank range or the simplex budget; per-cloud
-    simplex counts (triangles + tetrahedra where counted) come with it."""
+    """The chunk is over the rank range or the simplex budget; what each
+    cloud takes of the budget comes with it: its H1 rows and, where it asks for
+    H2 and is within its limits, its triangles and tetrahedra (as counted)."""
 
     def __init__(self, counts: list[int], edges: list[int]):
         super().__init__("split")
@@ -399,9 +400,11 @@ def _native_chunk(pts: list[Tensor], ts: list[float], dims: list[int], device, m
             tri = [max(0, int(lib.ph_batch_result_stat(res, c, 1))) for c in range(k)]
             tet = [max(0, int(lib.ph_batch_result_stat(res, c, 2))) for c in range(k)]
             edg = [max(0, int(lib.ph_batch_result_stat(res, c, 0))) for c in range(k)]
+            rows = [max(0, int(lib.ph_batch_result_stat(res, c, 3))) for c in range(k)]
+            live = [int(lib.ph_batch_result_status(res, c)) == L.PH_OK for c in range(k)]
         finally:
             lib.ph_batch_result_free(res)
-        raise _Split([a + b for a, b in zip(tri, tet)], edg)
+        raise _Split([r + (t + q if x == 2 and ok else 0) for r, t, q, x, ok in zip(rows, tri, tet, dims, live)], edg)
     if rc != L.PH_OK:
         raise L.PHError("ph_rips_persistence_batch", rc, lib.ph_last_error().decode(errors="replace"))
     try:

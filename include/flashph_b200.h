@@ -425,9 +425,10 @@ void ph_result_free(ph_result* result);
  * cloud's diagrams equal ph_rips_persistence on it alone, bit for bit.
  * Returns PH_ERR_CAPACITY, with *out set and the per-cloud counts filled,
  * when the union's simplices exceed the int32 rank range or, for more than
- * one cloud, max_batch_simplices (triangles, then triangles + tetrahedra;
- * 0: no budget): the caller splits the batch (ph_batch_result_stat gives each
- * cloud's edges and triangles) and frees *out. */
+ * one cloud, max_batch_simplices (the triangles that can be H1 pivots and
+ * those stored for H2, then the stored triangles and the tetrahedra; 0: no
+ * budget): the caller splits the batch (ph_batch_result_stat gives each cloud's
+ * counts) and frees *out. */
 typedef struct ph_batch_result ph_batch_result;
 int ph_rips_persistence_batch(const float* const* points, const int64_t* n, const int32_t* d,
                               const double* max_edge_length, const int32_t* max_dim, int32_t nclouds,
@@ -436,7 +437,8 @@ int ph_rips_persistence_batch(const float* const* points, const int64_t* n, cons
 /* PH_OK or PH_ERR_LIMIT for cloud c, and the limit's message ("" if none) */
 int32_t ph_batch_result_status(const ph_batch_result* result, int32_t cloud);
 const char* ph_batch_result_message(const ph_batch_result* result, int32_t cloud);
-/* per-cloud counts: k = 0 edges, 1 triangles, 2 tetrahedra (-1: not counted) */
+/* per-cloud counts: k = 0 edges, 1 triangles, 2 tetrahedra, 3 triangles that
+ * can be H1 pivots (-1: not counted) */
 int64_t ph_batch_result_stat(const ph_batch_result* result, int32_t cloud, int32_t k);
 /* nclouds + 1 row offsets of diagram dim in the batch's rows of that dim
  * (cloud c's rows are [out[c], out[c+1]); all zero when no cloud has dim) */
