@@ -490,6 +490,11 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
     if (keep2[c]) T2 += hper[c];
     span1 = std::max<i64>(span1, hrows[c]);
   }
+  if (std::find(keep1.begin(), keep1.end(), 1) == keep1.end()) {  // every cloud refused or done with H0
+    A.release_to(res->scratch);
+    *out = res;
+    return PH_OK;
+  }
   for (int c = 0; c < K; ++c) any_cleared = any_cleared || (any_h2 && !keep2[c] && hper[c] > 0);
   if (E + 3 * R1 >= (int64_t(1) << 31) || (K == 1 && E + 3 * T >= (int64_t(1) << 31)) ||
       E + 3 * T2 >= (int64_t(1) << 31) ||
