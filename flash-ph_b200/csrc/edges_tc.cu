@@ -55,13 +55,14 @@
 //                       columns (so that one accumulator is filled while the
 //                       other is read, and an item's thresholds are computed
 //                       once for its two row blocks); a warp reads its 32 TMEM
-//                       lanes x 64 columns in two loads (32 registers, no
-//                       spills at the 96 that 18 warps leave each), a tree of
+//                       lanes x 64 columns in two loads (32 registers of the
+//                       96 that 18 warps leave each), a tree of
 //                       three-input minima and one vote; only a chunk that
 //                       holds a candidate is read again, compared value by
 //                       value and compacted into a per-warp queue that spans
 //                       items and is recomputed with the exact chain 32 pairs
-//                       at a time, with warp-aggregated emission
+//                       at a time, with warp-aggregated emission, by all warps
+//                       between the same two items
 // What bounds it: an item (2 x 2 blocks) takes ~2,700 cycles at K = 16 and
 // ~3,100 at K = 64, in which a warp of the epilogue spends ~850 on loads and
 // minima, ~650 waiting for the accumulators, ~550 on the item's thresholds and
@@ -71,6 +72,15 @@
 // 50 at 6.0 4.67 ms; this form 3.08 and 4.05 ms. Accumulators of N = 128, four
 // in TMEM: 4.3 and 6.3 ms (the operand reads bound the MMA); 64 columns in one
 // go in 64 registers: 4.5 and 7.5 ms (spills).
+// Where candidates are many, their recomputation bounds it: each warp's queue
+// emptied when it was full, at a time of its own, made the others wait for it,
+// since an accumulator needs all sixteen. All queues emptied together, with
+// loads of 16 or 8 bytes where rows are aligned to them, for 90,000 Gaussian
+// points: 10 dimensions at 2, 20 and 80 neighbours a point 675, 1293 and 2381
+// us -> 652, 1048 and 1450; 50 dimensions 930, 1965, 4322 -> 759, 1251, 2060;
+// 150 dimensions (one row and one column block an item) 2912, 7330, 18,302 ->
+// 2293, 3414, 6220; 61 dimensions (loads of 4 bytes) 1053, 2782, 6099 -> 931,
+// 1873, 3840.
 // Each cloud's operand rows are padded to a multiple of 128 with rows whose
 // augmented columns carry 2^100, so padding never passes the screen. Every
 // wait is bounded (a few seconds of global time); a timeout sets
@@ -78,6 +88,7 @@
 // drained (again bounded) before TMEM is freed.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -482,6 +493,26 @@ __device__ __forceinline__ float exact_dsq(const float* __restrict__ x, const fl
   return acc;
 }
 
+// The same chain with loads of W floats (rows aligned to them). A warp's lanes
+// read a row each, so a load costs the L1 a line a lane whatever its width.
+template <int W>
+__device__ __forceinline__ float exact_dsq_wide(const float* __restrict__ x, const float* __restrict__ y, int d) {
+  using V = typename std::conditional<W == 4, float4, float2>::type;
+  float acc = 0.0f;
+#pragma unroll 4
+  for (int k = 0; k < d; k += W) {
+    const V a = __ldg(reinterpret_cast<const V*>(x + k)), b = __ldg(reinterpret_cast<const V*>(y + k));
+    const float* av = reinterpret_cast<const float*>(&a);
+    const float* bv = reinterpret_cast<const float*>(&b);
+#pragma unroll
+    for (int q = 0; q < W; ++q) {
+      const float df = __fsub_rn(av[q], bv[q]);
+      acc = __fmaf_rn(df, df, acc);
+    }
+  }
+  return acc;
+}
+
 // warp-aggregated append of the lanes with emit set
 __device__ __forceinline__ void emit_warp(bool emit, i64 gi, i64 gj, float acc, int lane, i32* __restrict__ oi,
                                           i32* __restrict__ oj, float* __restrict__ od, i64 cap,
@@ -504,7 +535,10 @@ __device__ __forceinline__ void emit_warp(bool emit, i64 gi, i64 gj, float acc, 
 
 // Exact chain for the first cnt queued cloud-local pairs of cloud qs, 32 at a
 // time with warp-aggregated emission. Kept out of line: the screening loop
-// around its call sites must stay small.
+// around its call sites must stay small. WIDE: loads of up to four floats, many
+// in flight, for the call between items; without, few registers, for the one in
+// the middle of a chunk (the caller's values stay in theirs).
+template <bool WIDE>
 __device__ __noinline__ void flush_queue(const uint2* __restrict__ queue, int cnt, const ph_cloud_seg qs,
                                          const float* __restrict__ pts_all, i32* __restrict__ oi,
                                          i32* __restrict__ oj, float* __restrict__ od, i64 cap,
@@ -512,6 +546,8 @@ __device__ __noinline__ void flush_queue(const uint2* __restrict__ queue, int cn
   const int lane = threadIdx.x & 31;
   __syncwarp();
   const float* P = pts_all + qs.pt_off;
+  const u32 odd = (u32)qs.d | (u32)((uintptr_t)P >> 2);  // in floats
+  const int width = (odd & 3) == 0 ? 4 : (odd & 1) == 0 ? 2 : 1;
   for (int e0 = 0; e0 < cnt; e0 += 32) {
     const int e = e0 + lane;
     bool emit = false;
@@ -522,7 +558,10 @@ __device__ __noinline__ void flush_queue(const uint2* __restrict__ queue, int cn
       qi = en.x;
       qj = en.y;
       if (qi < qj && qj < qs.n) {
-        acc = exact_dsq(P + qi * qs.d, P + qj * qs.d, qs.d);
+        const float *x = P + qi * qs.d, *y = P + qj * qs.d;
+        acc = WIDE && width == 4   ? exact_dsq_wide<4>(x, y, qs.d)
+              : WIDE && width == 2 ? exact_dsq_wide<2>(x, y, qs.d)
+                                   : exact_dsq(x, y, qs.d);
         emit = acc < qs.thr_sq;
       }
     }
@@ -543,8 +582,9 @@ struct Epilogue {
   unsigned long long* count;
   unsigned long long n_cand;
 
+  template <bool WIDE>
   __device__ void flush() {
-    flush_queue(queue, cnt, qs, pts, oi, oj, od, cap, count);
+    flush_queue<WIDE>(queue, cnt, qs, pts, oi, oj, od, cap, count);
     n_cand += (unsigned long long)cnt;
     cnt = 0;
   }
@@ -552,8 +592,8 @@ struct Epilogue {
 
 // The candidates among a warp's columns of the accumulator (read again: few
 // chunks hold one), queued: one compare per pair into a lane mask, the set bits one
-// per lane and round. Out of line, as flush_queue.
-__device__ __noinline__ void screen_chunk(Epilogue& e, u32 taddr, u32 i, u32 j0, int cols, float bound) {
+// per lane and round; returns how many are queued. Out of line, as flush_queue.
+__device__ __noinline__ int screen_chunk(Epilogue& e, u32 taddr, u32 i, u32 j0, int cols, float bound) {
   const u32 lt = lanemask_lt();
 #pragma unroll 1
   for (int half = 0; half < cols; half += 32) {
@@ -567,7 +607,7 @@ __device__ __noinline__ void screen_chunk(Epilogue& e, u32 taddr, u32 i, u32 j0,
     while (__any_sync(FULL, mask != 0)) {
       const bool has = mask != 0;
       const u32 m = __ballot_sync(FULL, has);
-      if (e.cnt + 32 > TC_QCAP) e.flush();
+      if (e.cnt + 32 > TC_QCAP) e.flush<false>();
       if (has) {
         e.queue[e.cnt + __popc(m & lt)] = make_uint2(i, j0 + half + (u32)__ffs(mask) - 1u);
         mask &= mask - 1;
@@ -575,6 +615,7 @@ __device__ __noinline__ void screen_chunk(Epilogue& e, u32 taddr, u32 i, u32 j0,
       e.cnt += __popc(m);
     }
   }
+  return e.cnt;
 }
 
 // ---- main kernel ------------------------------------------------------------------------
@@ -595,6 +636,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   __shared__ __align__(8) unsigned long long bars[BAR_N];
   __shared__ u32 tmem_sh;
   __shared__ int abort_sh;
+  __shared__ u32 flush_sh;  // joint flushes asked for so far
   __shared__ unsigned long long st_sh[2];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sA = smem;
@@ -627,6 +669,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       mbar_init(bar(BAR_TE + s), TC_EPI_WARPS);
     }
     abort_sh = 0;
+    flush_sh = 0;
     st_sh[0] = st_sh[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -771,9 +814,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   } else if (T > 0 && warp < TC_EPI_WARPS) {
     // Warpgroup g takes the g-th quarter of every accumulator's columns: half a
     // column block of an item, or a quarter of the only one. Candidates are
-    // queued as cloud-local pairs across items and recomputed 32 at a time (when
-    // the queue fills, the cloud changes, or the range ends), so the latency of
-    // the exact chain's loads is paid once per 32 candidates.
+    // queued as cloud-local pairs across items and recomputed 32 at a time, so the
+    // latency of the exact chain's loads is paid once per 32 candidates: between
+    // two items by all warps when one warp's queue is half full (the others wait
+    // for a warp that recomputes anyway, since every accumulator needs them all),
+    // when a queue fills within an item, when the cloud changes, at the end.
     const int q4 = warp & 3, g = warp >> 2;
     const int cols = 32 * sh.nb;            // columns of this warp
     const u32 col = (u32)(cols * g);        // the first of them
@@ -789,10 +834,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const u32 taddr = tmem + ((u32)(q4 * 32) << 16) + col;
     u32 unit = 0;  // row blocks met: accumulator unit & 1, phase (unit >> 1) & 1
     bool ok = true;
+    u32 epoch = 0;  // joint flushes done
     for (i64 t = 0; t < T; ++t) {
+      const u32 asked = *(volatile u32*)&flush_sh;
       if (it.c != cloud || it.I != group) {
         if (it.c != cloud) {
-          if (ep.cnt) ep.flush();
+          if (ep.cnt) ep.flush<true>();
           cloud = it.c;
           ep.qs = segs[cloud];
           sqthr = __double2float_ru(sqrt((double)ep.qs.thr_sq * thr_scale));
@@ -821,6 +868,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         it.next();
         rj = it.nh() > h ? blkrad[it.blk + it.J + h] : 0.0f;
       }
+      if (__any_sync(FULL, asked != epoch)) {
+        epoch = __shfl_sync(FULL, asked, 0);
+        if (ep.cnt) ep.flush<true>();
+      }
 #pragma unroll 1
       for (int r = 0; r < sh.nr; ++r, ++unit) {
         const int ts = (int)(unit & 1);
@@ -843,7 +894,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             least = fminf(least, least32(x));
           }
           if (__any_sync(FULL, least < b))
-            screen_chunk(ep, ta, i0 + (u32)(r * TC_T + q4 * 32 + lane), j0, cols, b);
+            if (screen_chunk(ep, ta, i0 + (u32)(r * TC_T + q4 * 32 + lane), j0, cols, b) > TC_QCAP / 2 && lane == 0)
+              atomicCAS(&flush_sh, epoch, epoch + 1);
         }
         asm volatile("tcgen05.fence::before_thread_sync;");
         __syncwarp();
@@ -871,7 +923,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         break;
       }
     }
-    if (ep.cnt) ep.flush();
+    if (ep.cnt) ep.flush<true>();
     if (stats && lane == 0) {
       atomicAdd(&st_sh[0], ep.n_cand);
       atomicAdd(&st_sh[1], n_forced);
