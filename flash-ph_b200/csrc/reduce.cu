@@ -58,6 +58,8 @@ struct RedCtl {
   int nres;
   int next;
   int abort;
+  int deferred;  // columns that k_reduce_short left
+  int next_deferred;
   int pad;
   unsigned long long pool_top;
   unsigned long long merges;
@@ -1316,9 +1318,11 @@ struct SharedCol {
   }
 };
 
+// `deferred` (null: all residual columns): the columns to reduce, ctl->deferred of them
 __global__ void __launch_bounds__(32 * RS_MAX_WARPS, 1)
     k_reduce_shared(i32 row_base, i64 K, const i32* __restrict__ state, const u64* __restrict__ rec, u64* owner,
-                    i32* pool, i64 pool_cap, int chunk, RedCtl* ctl, int* status, int max_steps, int nw) {
+                    i32* pool, i64 pool_cap, int chunk, RedCtl* ctl, int* status, int max_steps, int nw,
+                    const i32* __restrict__ deferred) {
   ph::pdl_wait();
   ph::pdl_trigger();
   extern __shared__ i32 rd_smem[];
@@ -1339,7 +1343,10 @@ __global__ void __launch_bounds__(32 * RS_MAX_WARPS, 1)
   // the counter and the states are a round trip each, as long as a round of
   // additions, so chunks are larger where few columns are residual.
   // (and the columns many, or one warp would get several of the last, longest)
-  const int fetch = (i64)ctl->nres * 16 < K && K >= RS_LONG_SWEEP ? 32 : RD_FETCH;
+  // (the columns deferred are long, so one at a time)
+  const i64 count = deferred ? (i64)ctl->deferred : K;
+  int* next = deferred ? &ctl->next_deferred : &ctl->next;
+  const int fetch = deferred ? 1 : ((i64)ctl->nres * 16 < K && K >= RS_LONG_SWEEP ? 32 : RD_FETCH);
 
   // reduces column c, whose record at wrec holds len0 entries, the first of them first0
   auto reduce_column = [&](i32 c, u64 wrec, int len0, i32 first0) {
@@ -1464,21 +1471,146 @@ __global__ void __launch_bounds__(32 * RS_MAX_WARPS, 1)
 
   for (;;) {
     int base = 0;
-    if (lane == 0) base = atomicAdd(&ctl->next, fetch);
+    if (lane == 0) base = atomicAdd(next, fetch);
     base = __shfl_sync(FULL, base, 0);
-    if (base < 0 || (i64)base >= K || *vabort) break;
-    const i64 mine = K - 1 - base - lane;
+    if (base < 0 || (i64)base >= count || *vabort) break;
+    i64 mine = deferred ? -1 : K - 1 - base - lane;
+    if (deferred && lane < fetch && (i64)base + lane < count) mine = deferred[base + lane];
     const bool res = lane < fetch && mine >= 0 && state[mine] == 2;
     // the records' places and heads of all of them at once
     const u64 at = res ? rec[mine] : 0ull;
     const int4 h = res ? __ldcg(reinterpret_cast<const int4*>(pool + at)) : make_int4(0, 0, 0, 0);
     for (u32 todo = __ballot_sync(FULL, res); todo && !*vabort; todo &= todo - 1) {
       const int l = __ffs(todo) - 1;
-      reduce_column((i32)(K - 1 - base - l), __shfl_sync(FULL, at, l), __shfl_sync(FULL, h.x, l),
+      reduce_column((i32)__shfl_sync(FULL, mine, l), __shfl_sync(FULL, at, l), __shfl_sync(FULL, h.x, l),
                     __shfl_sync(FULL, h.y, l));
     }
   }
   if (D.bad) set_status(status, PH_ERR_ARG);
+  if (lane == 0) {
+    if (n_merges) atomicAdd(&ctl->merges, n_merges);
+    if (n_takeovers) atomicAdd(&ctl->takeovers, n_takeovers);
+  }
+}
+
+// ---- short columns --------------------------------------------------------------------
+// Windows of many rows leave room for few warps an SM (four at 0.43M rows, two at
+// 0.87M, one up to 1.79M), and the columns of sparse complexes, most of them reduced in a few
+// additions, then wait for one another. Here they go first, 32 warps an SM: a
+// warp a column, a sorted list of up to SH_CAP entries in shared memory, one
+// addition a step. A column that grows past that, meets a record of more than
+// 31 entries or takes more than SH_STEPS steps is left to k_reduce_shared, from
+// its initial record on: a column may be reduced at any time, since claims are
+// ordered by column.
+// Both kernels, us: one addition a step in lists over all triangles, as before the
+// windows -> all columns in windows -> short ones first:
+//   1 window warp an SM: 300,000 points uniform in 2-D at 8 neighbours a point
+//     701 -> 3663 -> 235; 126,457 in 10-D clusters at 20 6154 -> 13,157 -> 1759;
+//     92,693 x 64 normal at 22 18,281 -> 29,268 -> 8019; 30,000 x 16 at 40
+//     24,169 -> 9892 -> 5004
+//   2: 100,000 on the sphere in 4-D at 16 1708 -> 2849 -> 857; 50,000 x 12 normal
+//     at 20 10,131 -> 4125 -> 2167; 60,000 on the sphere in 16-D at 30 153,942 ->
+//     29,679 -> 24,276
+//   3 and 4: 200,000 uniform in 4-D at 8 959 -> 1947 -> 295; 100,000 uniform in
+//     10-D at 12 5123 -> 2264 -> 1336
+//   5 to 8: 60,000 x 20 normal at 10 2736 -> 3004, 200,000 x 10 at 3 841 -> 1191
+//     (as many warps already, and two passes over the columns): not taken
+// Fewer steps leave larger columns to go last, whose claims displace the smaller
+// ones: on the sphere in 16-D 52,712 with 16, 26,445 with 32, 23,679 with 128.
+constexpr int SH_NT = 256;
+constexpr int SH_CAP = 256;
+constexpr int SH_STEPS = 64;
+constexpr int SH_MAX_WARPS = 4;  // window warps an SM up to which the short columns go first
+
+__global__ void __launch_bounds__(SH_NT, 4)
+    k_reduce_short(i32 row_base, i64 K, const i32* __restrict__ state, const u64* __restrict__ rec, u64* owner,
+                   i32* pool, i64 pool_cap, int chunk, RedCtl* ctl, int* status, int max_steps,
+                   i32* __restrict__ deferred) {
+  ph::pdl_wait();
+  ph::pdl_trigger();
+  __shared__ i32 lists[SH_NT / 32][2][SH_CAP];
+  const int lane = threadIdx.x & 31;
+  i32(*list)[SH_CAP] = lists[threadIdx.x >> 5];
+  volatile int* vabort = &ctl->abort;
+  PoolChunk chunk_state;
+  unsigned long long n_merges = 0, n_takeovers = 0;
+  // reduces column c, whose record at wrec holds k entries; the column that is left, -1: none
+  auto reduce_column = [&](i32 c, u64 wrec, int k) -> i32 {
+    if (k > SH_CAP) return c;
+    int cur = 0;
+    for (int i = lane; i < k; i += 32) list[0][i] = __ldcg(pool + wrec + 1 + i);
+    __syncwarp();
+    bool published = true;
+    for (int step = 0;; ++step) {
+      if (k == 0) return -1;  // the column vanished: it owns nothing
+      if (step >= max_steps) {
+        if (lane == 0) set_status(status, PH_ERR_ITER_LIMIT);
+        atomicExch(&ctl->abort, 1);
+        return -1;
+      }
+      const i32* W = list[cur];
+      const i32 p = W[0];
+      u64 ow = ld_acquire(owner + (p - row_base));
+      if (owner_col(ow) < c) {
+        if (!published) {
+          const unsigned long long at = pool_alloc(chunk_state, ctl, pool_cap, k + 1, chunk, status);
+          if (at == ~0ull) return -1;
+          if (lane == 0) pool[at] = k;
+          for (int i = lane; i < k; i += 32) pool[at + 1 + i] = W[i];
+          wrec = at;
+          published = true;
+        }
+        __syncwarp();
+        u64 old = 0;
+        if (lane == 0) old = atom_max_acq_rel(owner + (p - row_base), owner_word(c, wrec));
+        old = __shfl_sync(FULL, old, 0);
+        __syncwarp();
+        const i32 oc = owner_col(old);
+        if (oc < 0) return -1;  // claimed a free pivot
+        if (oc < c) {  // displaced a smaller column: it adds the claimer's content, which the list holds
+          ++n_takeovers;
+          c = oc;
+        }
+        ow = old;
+      }
+      if (owner_col(ow) == c && !published) {  // cannot happen: a column never owns a pivot it is still reducing
+        if (lane == 0) set_status(status, PH_ERR_ARG);
+        return -1;
+      }
+      if (step >= SH_STEPS) return c;
+      const u64 at = ow & OW_OFF;
+      const i32 head = (at + lane < (u64)pool_cap) ? __ldcg(pool + at + lane) : 0;
+      const int len = __shfl_sync(FULL, head, 0);
+      const i32 v = __shfl_down_sync(FULL, head, 1);
+      if (len > 31 || k + len > SH_CAP) return c;
+      k = warp_xor_small<false>(W, k, lane < len ? v : INT_MAX, len, list[cur ^ 1]);
+      __syncwarp();
+      cur ^= 1;
+      ++n_merges;
+      published = false;
+    }
+  };
+  for (;;) {
+    int base = 0;
+    if (lane == 0) base = atomicAdd(&ctl->next, 32);
+    base = __shfl_sync(FULL, base, 0);
+    if (base < 0 || (i64)base >= K || *vabort) break;
+    const i64 mine = K - 1 - base - lane;
+    const bool res = mine >= 0 && state[mine] == 2;
+    const u64 at = res ? rec[mine] : 0ull;
+    const int len = res ? __ldcg(pool + at) : 0;
+    i32 left = -1;  // lane l: what became of column l
+    for (u32 todo = __ballot_sync(FULL, res); todo && !*vabort; todo &= todo - 1) {
+      const int l = __ffs(todo) - 1;
+      const i32 x = reduce_column((i32)(K - 1 - base - l), __shfl_sync(FULL, at, l), __shfl_sync(FULL, len, l));
+      if (lane == l) left = x;
+    }
+    const u32 m = __ballot_sync(FULL, left >= 0);
+    int slot = 0;
+    if (lane == 0 && m) slot = atomicAdd(&ctl->deferred, __popc(m));
+    slot = __shfl_sync(FULL, slot, 0);
+    if (left >= 0) deferred[slot + __popc(m & lanemask_lt())] = left;
+  }
   if (lane == 0) {
     if (n_merges) atomicAdd(&ctl->merges, n_merges);
     if (n_takeovers) atomicAdd(&ctl->takeovers, n_takeovers);
@@ -1560,6 +1692,12 @@ int shared_warps(i64 span) {
   return (int)std::min<size_t>(RS_MAX_WARPS, RS_SMEM / 4 / rs_warp_words(words));
 }
 
+// whether the short columns go first (k_reduce_short)
+bool short_first(i64 span) {
+  const int w = shared_warps(span);
+  return w > 0 && w <= SH_MAX_WARPS;
+}
+
 // dense working-column slots in global memory (windows beyond shared memory):
 // one window per warp of the grid, when they fit in 1 GiB (else long columns
 // stay sorted lists in the pool)
@@ -1576,6 +1714,7 @@ extern "C" size_t ph_reduce_workspace_bytes(int64_t K, int64_t R, int64_t span) 
   span = span_or_all(R, span);
   const i64 dw = K > 0 ? dense_words(K, span) : 0;
   return Carve::need((size_t)R * 8) + Carve::need((size_t)K * 8) + Carve::need(sizeof(RedCtl)) +
+         (short_first(span) ? Carve::need((size_t)K * 4) : 0) +
          (dw ? Carve::need((size_t)dw * 4 * reduce_blocks(K) * RD_WARPS) : 0);
 }
 
@@ -1623,12 +1762,22 @@ int reduce_run(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32
   const int blocks = sw ? (int)std::max<i64>(1, std::min<i64>((K + sw - 1) / sw, ph::device_sms())) : reduce_blocks(K);
   // pool chunk per warp: small enough that the chunks of all warps fit a quarter of the pool
   const int chunk = (int)std::max<i64>(64, std::min<i64>(2048, pool_cap / (4 * (i64)blocks * warps)) & ~3);
+  i32* deferred = nullptr;
+  if (short_first(span)) {
+    if (!(deferred = c.take<i32>(K))) return PH_ERR_ARG;
+    const i64 short_warps = (i64)ph::device_sms() * 4 * (SH_NT / 32);
+    const int short_chunk = (int)(std::max<i64>(64, std::min<i64>(2048, pool_cap / (8 * short_warps))) & ~3);
+    ph::count_launch();
+    ph::launch_pdl(k_reduce_short, dim3((unsigned)std::min<i64>((K + SH_NT - 1) / SH_NT, (i64)ph::device_sms() * 4)),
+                   dim3(SH_NT), 0, s, row_base, K, (const i32*)col_state, (const u64*)rec, owner, pool, pool_cap,
+                   short_chunk, ctl, d_status, max_steps, deferred);
+  }
   ph::count_launch();
   if (sw) {
     const i64 words = window_words(span);
     ph::launch_pdl(k_reduce_shared, dim3(blocks), dim3(32 * sw), sw * rs_warp_words(words) * sizeof(u32), s, row_base,
                    K, (const i32*)col_state, (const u64*)rec, owner, pool, pool_cap, chunk, ctl, d_status, max_steps,
-                   (int)words);
+                   (int)words, (const i32*)deferred);
   } else {
     const i64 dw = dense_words(K, span);
     u32* dense = dw ? c.take<u32>(dw * (i64)blocks * RD_WARPS) : nullptr;
