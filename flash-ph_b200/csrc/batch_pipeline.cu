@@ -436,7 +436,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
     if (A.failed) return alloc_fail();
     if (!links.stash.rows) links.stash.cap = 0;
     if (E) {
-      const int rc = link_count(si, sj, E, graph, pre ? tkeep : nullptr, mask, links, lk_ws, lk_b, s);
+      const int rc = link_count(si, sj, E, graph, pre ? tkeep : nullptr, mask, INT64_MAX, links, lk_ws, lk_b, s);
       if (rc != PH_OK) return give_up(rc);
     } else {
       ph::zero_async(tri_off, sizeof(int64_t), s, links.row_off, sizeof(int64_t));

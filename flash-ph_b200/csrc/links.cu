@@ -216,9 +216,10 @@ __device__ __forceinline__ void list_at(const i32* list, int j, i32 (&x)[2]) {
 // fa, fb) by the whole group, where the lanes of the mask hold one each, the
 // one with link index i and other edges fa, fb. Returns the link's length
 // (uniform in the group). `list` is the group's LK_LIST G / 32 words of shared
-// memory.
+// memory. count_only: the length alone, no rows.
 template <int G, typename F>
-__device__ __forceinline__ int edge_rows(const Group<G>& gr, const Graph& g, const Ends& e, i32* list, F&& f) {
+__device__ __forceinline__ int edge_rows(const Group<G>& gr, const Graph& g, const Ends& e, i32* list, bool count_only,
+                                         F&& f) {
   constexpr int LIST = LK_LIST * G / 32;
   constexpr int U = G == 32 ? 4 : 2;  // row positions, or tests, a lane has in flight
   const int lane = gr.lane;
@@ -258,6 +259,7 @@ __device__ __forceinline__ int edge_rows(const Group<G>& gr, const Graph& g, con
     look(e.s0, w, rs, rl, in);
     const u32 vb = gr.ballot(in[0]);
     const int nl = __popc(vb), i = __popc(vb & lt);
+    if (count_only) return nl;
     if (in[0]) list[i] = w[0];
     gr.sync();
     bool open = in[0];
@@ -299,6 +301,7 @@ __device__ __forceinline__ int edge_rows(const Group<G>& gr, const Graph& g, con
     }
   }
   gr.sync();
+  if (count_only) return nl;
   for (int base = 0; base < held; base += G) {
     const int i = base + lane;
     const i32 w = i < held ? list[i] : 0;
@@ -451,7 +454,7 @@ __global__ void __launch_bounds__(LK_NT, LK_BLOCKS) k_links(const i32* __restric
                                                 LinkGraph lg, const uint8_t* __restrict__ keep,
                                                 const uint8_t* __restrict__ skip, i32* __restrict__ tri_cnt,
                                                 i32* __restrict__ row_cnt, i32* __restrict__ len_cnt,
-                                                LinkStash stash) {
+                                                LinkStash stash, i64 limit) {
   ph::pdl_wait();
   ph::pdl_trigger();
   constexpr int PER = 32 / G;  // edges a warp has in flight
@@ -467,10 +470,11 @@ __global__ void __launch_bounds__(LK_NT, LK_BLOCKS) k_links(const i32* __restric
   StashChunk<G> chunk;
   StashChunk<32> wchunk;  // of the edges the warp takes together
   i64 ntri = 0, nrow = 0;
+  bool over = false;
   auto walk = [&](const auto& grp, auto& ch, const Ends& e, i32* list) {
     const Graph g = graph_of(lg, e.a);
     int k = 0;
-    const int nl = edge_rows(grp, g, e, list, [&](bool mine, u32 lanes, int i, i32 fa, i32 fb) {
+    const int nl = edge_rows(grp, g, e, list, over, [&](bool mine, u32 lanes, int i, i32 fa, i32 fb) {
       const int z = __popc(lanes & grp.below()), n = __popc(lanes);
       ch.put(grp, stash, n, mine, z, LinkRow{e.m, k + z, i, fa, fb});
       if (mine) {
@@ -487,10 +491,23 @@ __global__ void __launch_bounds__(LK_NT, LK_BLOCKS) k_links(const i32* __restric
       nrow += k;
     }
   };
+  // Longest edges first (their links are the largest): once the triangles seen
+  // so far, brought together every 16 edges, are over the limit, no row is
+  // needed, and the rest is only counted. 70,166 points in 3-D with outliers,
+  // 1.5M edges, 14.7M triangles (limit 10M): 2510 -> 1895 us, the call 6.67 ->
+  // 6.05 ms (6.12 when all triangles were counted an edge without rows).
+  int turn = 0;
   for (i64 m0 = warp * PER; m0 < E; m0 += nwarps * PER) {
-    const i64 m = m0 + gr.base / G;
+    if (limit < LLONG_MAX && (++turn & 15) == 0 && !over) {
+      for (int o = 16; o > 0; o >>= 1) ntri += __shfl_xor_sync(FULL, ntri, o);
+      if (wp.lane == 0)
+        over = (i64)(atomicAdd(&stash.totals->triangles, (unsigned long long)ntri) + ntri) > limit;
+      over = __shfl_sync(FULL, over, 0);
+      ntri = 0;
+    }
+    const i64 m = E - 1 - (m0 + gr.base / G);
     Ends e{-1, 0, 0, 0, 0, 0, 0, false};
-    if (m < E) {
+    if (m >= 0) {
       const i32 a = ei[m], b = ej[m];
       if (keep && !keep[lg.vcloud[a]]) {  // a cloud already known to be over its limit counts nothing
         if (gr.lane == 0) {
@@ -801,13 +818,13 @@ int link_table_offsets(const ph_cloud_seg* segs, const i64* e_off, int nclouds, 
 size_t link_count_workspace_bytes(i64 E) { return scan_workspace_bytes(E); }
 
 int link_count(const i32* ei, const i32* ej, i64 E, const LinkGraph& g, const uint8_t* keep, const uint8_t* skip,
-               const LinkCounts& o, void* ws, size_t ws_bytes, cudaStream_t s) {
+               i64 limit, const LinkCounts& o, void* ws, size_t ws_bytes, cudaStream_t s) {
   if (E < 1) return PH_ERR_ARG;
   ph::zero_async(o.len_cnt, sizeof(i32) * E, s, o.cursor, sizeof(i32) * E);
   const int lanes = lanes_for(E, g.n);
   ph::count_launch();
   ph::launch_pdl(lanes == 8 ? k_links<8> : k_links<32>, dim3(links_grid(E, lanes)), dim3(LK_NT), 0, s, ei, ej, E, g,
-                 keep, skip, o.tri_cnt, o.row_cnt, o.len_cnt, o.stash);
+                 keep, skip, o.tri_cnt, o.row_cnt, o.len_cnt, o.stash, limit);
   if (o.tri_off) PH_TRY(scan_exclusive_i32_i64(o.tri_cnt, o.tri_off, E, ws, ws_bytes, s));
   PH_TRY(scan_exclusive_i32_i64(o.row_cnt, o.row_off, E, ws, ws_bytes, s));
   PH_TRY(scan_exclusive_i32_i32(o.len_cnt, o.off, E, ws, ws_bytes, s));

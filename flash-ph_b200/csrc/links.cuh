@@ -80,9 +80,11 @@ i64 link_stash_cap(i64 E, i64 n, i64 rows);
 int link_table(const LinkGraph& g, i32* table, cudaStream_t s);
 int link_table_offsets(const ph_cloud_seg* segs, const i64* e_off, int nclouds, i64 cap, i64* off, cudaStream_t s);
 size_t link_count_workspace_bytes(i64 E);
-// counts triangles and rows an edge; clouds with keep[cloud] == 0 count nothing (keep may be null)
+// counts triangles and rows an edge; clouds with keep[cloud] == 0 count nothing
+// (keep may be null); with more than `limit` triangles in all, the rows are not
+// complete
 int link_count(const i32* ei, const i32* ej, i64 E, const LinkGraph& g, const uint8_t* keep, const uint8_t* skip,
-               const LinkCounts& o, void* ws, size_t ws_bytes, cudaStream_t s);
+               i64 limit, const LinkCounts& o, void* ws, size_t ws_bytes, cudaStream_t s);
 // the nrows rows in order: largest edge, index among all triangles (row_tri
 // may be null), largest face not skipped; their entries in the lists of their
 // faces

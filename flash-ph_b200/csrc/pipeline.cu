@@ -505,7 +505,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
       links.stash.rows = attempt ? A.take<LinkRow>(links.stash.cap) : A.optional<LinkRow>(links.stash.cap);
       if (A.failed) return alloc_fail();
       if (!links.stash.rows) links.stash.cap = 0;
-      if (rc == PH_OK && E) rc = link_count(si, sj, E, graph, nullptr, mask, links, lk_ws, lk_b, s);
+      if (rc == PH_OK && E) rc = link_count(si, sj, E, graph, nullptr, mask, max_triangles, links, lk_ws, lk_b, s);
       if (rc != PH_OK) return give_up(rc);
       const int64_t* src[4] = {cnt + 8, cnt + 1, cnt + 9, cnt + 10};
       if (readback(src, 4, slots, s) != PH_OK) return give_up(PH_ERR_CUDA);
