@@ -449,7 +449,9 @@ struct StashChunk {
   }
 };
 
-template <int G>
+// LIMIT: counts only, once the triangles are over the limit (a variant of its
+// own: as an argument it cost the batches' pass 5%)
+template <int G, bool LIMIT>
 __global__ void __launch_bounds__(LK_NT, LK_BLOCKS) k_links(const i32* __restrict__ ei, const i32* __restrict__ ej, i64 E,
                                                 LinkGraph lg, const uint8_t* __restrict__ keep,
                                                 const uint8_t* __restrict__ skip, i32* __restrict__ tri_cnt,
@@ -474,7 +476,7 @@ __global__ void __launch_bounds__(LK_NT, LK_BLOCKS) k_links(const i32* __restric
   auto walk = [&](const auto& grp, auto& ch, const Ends& e, i32* list) {
     const Graph g = graph_of(lg, e.a);
     int k = 0;
-    const int nl = edge_rows(grp, g, e, list, over, [&](bool mine, u32 lanes, int i, i32 fa, i32 fb) {
+    const int nl = edge_rows(grp, g, e, list, LIMIT && over, [&](bool mine, u32 lanes, int i, i32 fa, i32 fb) {
       const int z = __popc(lanes & grp.below()), n = __popc(lanes);
       ch.put(grp, stash, n, mine, z, LinkRow{e.m, k + z, i, fa, fb});
       if (mine) {
@@ -491,23 +493,24 @@ __global__ void __launch_bounds__(LK_NT, LK_BLOCKS) k_links(const i32* __restric
       nrow += k;
     }
   };
-  // Longest edges first (their links are the largest): once the triangles seen
+  // With a limit, longest edges first (their links are the largest): once the triangles seen
   // so far, brought together every 16 edges, are over the limit, no row is
   // needed, and the rest is only counted. 70,166 points in 3-D with outliers,
   // 1.5M edges, 14.7M triangles (limit 10M): 2510 -> 1895 us, the call 6.67 ->
   // 6.05 ms (6.12 when all triangles were counted an edge without rows).
   int turn = 0;
   for (i64 m0 = warp * PER; m0 < E; m0 += nwarps * PER) {
-    if (limit < LLONG_MAX && (++turn & 15) == 0 && !over) {
+    if (LIMIT && (++turn & 15) == 0 && !over) {
       for (int o = 16; o > 0; o >>= 1) ntri += __shfl_xor_sync(FULL, ntri, o);
       if (wp.lane == 0)
         over = (i64)(atomicAdd(&stash.totals->triangles, (unsigned long long)ntri) + ntri) > limit;
       over = __shfl_sync(FULL, over, 0);
       ntri = 0;
     }
-    const i64 m = E - 1 - (m0 + gr.base / G);
+    i64 m = m0 + gr.base / G;
+    if (LIMIT) m = E - 1 - m;
     Ends e{-1, 0, 0, 0, 0, 0, 0, false};
-    if (m >= 0) {
+    if (m >= 0 && m < E) {
       const i32 a = ei[m], b = ej[m];
       if (keep && !keep[lg.vcloud[a]]) {  // a cloud already known to be over its limit counts nothing
         if (gr.lane == 0) {
@@ -822,8 +825,10 @@ int link_count(const i32* ei, const i32* ej, i64 E, const LinkGraph& g, const ui
   if (E < 1) return PH_ERR_ARG;
   ph::zero_async(o.len_cnt, sizeof(i32) * E, s, o.cursor, sizeof(i32) * E);
   const int lanes = lanes_for(E, g.n);
+  const auto kernel = limit < LLONG_MAX ? (lanes == 8 ? k_links<8, true> : k_links<32, true>)
+                                        : (lanes == 8 ? k_links<8, false> : k_links<32, false>);
   ph::count_launch();
-  ph::launch_pdl(lanes == 8 ? k_links<8> : k_links<32>, dim3(links_grid(E, lanes)), dim3(LK_NT), 0, s, ei, ej, E, g,
+  ph::launch_pdl(kernel, dim3(links_grid(E, lanes)), dim3(LK_NT), 0, s, ei, ej, E, g,
                  keep, skip, o.tri_cnt, o.row_cnt, o.len_cnt, o.stash, limit);
   if (o.tri_off) PH_TRY(scan_exclusive_i32_i64(o.tri_cnt, o.tri_off, E, ws, ws_bytes, s));
   PH_TRY(scan_exclusive_i32_i64(o.row_cnt, o.row_off, E, ws, ws_bytes, s));
