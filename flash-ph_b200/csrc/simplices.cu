@@ -291,13 +291,15 @@ __global__ void k_tri_words(const i32* __restrict__ ptr, i32* idx, i64 n, int nw
       continue;
     }
     const i32 first = g.vcloud ? (i32)g.segs[g.vcloud[a]].vbase : 0;
+    u32 twice = 0;
     for (int p = s + lane; p < e; p += 32) {
       const i32 b = idx[p] - first;
-      atomicOr(reinterpret_cast<u32*>(bits) + (b >> 5), 1u << (b & 31));
+      const u32 bit = 1u << (b & 31);
+      twice |= atomicOr(reinterpret_cast<u32*>(bits) + (b >> 5), bit) & bit;
       atomicOr(&used[b >> 11], 1u << ((b >> 6) & 31));
     }
-    __syncwarp();
-    int out = s, distinct = 0;
+    const bool repeats = __any_sync(FULL, twice != 0);
+    int out = s;
     for (int s0 = 0; s0 < nsum; s0 += 32) {
       const u32 mine = s0 + lane < nsum ? used[s0 + lane] : 0;
       for (u32 some = __ballot_sync(FULL, mine != 0); some; some &= some - 1) {
@@ -305,11 +307,9 @@ __global__ void k_tri_words(const i32* __restrict__ ptr, i32* idx, i64 n, int nw
         const u32 set = __shfl_sync(FULL, mine, l);
         if ((set >> lane) & 1u) {
           const int w = (s0 + l) * 32 + lane, o = out + __popc(set & lanemask_lt());
-          const u64 v = bits[w];
-          mask[o] = v;
+          mask[o] = bits[w];
           at[o] = (uint16_t)w;
           bits[w] = 0;
-          distinct += __popcll(v);
         }
         out += __popc(set);
       }
@@ -317,7 +317,7 @@ __global__ void k_tri_words(const i32* __restrict__ ptr, i32* idx, i64 n, int nw
     }
     if (lane == 0) len[a] = out - s;
     __syncwarp();
-    if (__reduce_add_sync(FULL, distinct) != e - s) {
+    if (repeats) {
       int p = s;
       for (int o = s; o < out; ++o)
         for (int half = 0; half < 2; ++half) {
