@@ -1318,11 +1318,12 @@ struct SharedCol {
   }
 };
 
-// `deferred` (null: all residual columns): the columns to reduce, ctl->deferred of them
+// `deferred`: the columns to reduce, ctl->deferred of them, where k_reduce_short
+// ran (null, or fewer residual columns than `few`: all of them)
 __global__ void __launch_bounds__(32 * RS_MAX_WARPS, 1)
     k_reduce_shared(i32 row_base, i64 K, const i32* __restrict__ state, const u64* __restrict__ rec, u64* owner,
                     i32* pool, i64 pool_cap, int chunk, RedCtl* ctl, int* status, int max_steps, int nw,
-                    const i32* __restrict__ deferred) {
+                    const i32* __restrict__ deferred, int few) {
   ph::pdl_wait();
   ph::pdl_trigger();
   extern __shared__ i32 rd_smem[];
@@ -1344,6 +1345,7 @@ __global__ void __launch_bounds__(32 * RS_MAX_WARPS, 1)
   // additions, so chunks are larger where few columns are residual.
   // (and the columns many, or one warp would get several of the last, longest)
   // (the columns deferred are long, so one at a time)
+  if (ctl->nres < few) deferred = nullptr;
   const i64 count = deferred ? (i64)ctl->deferred : K;
   int* next = deferred ? &ctl->next_deferred : &ctl->next;
   const int fetch = deferred ? 1 : ((i64)ctl->nres * 16 < K && K >= RS_LONG_SWEEP ? 32 : RD_FETCH);
@@ -1521,13 +1523,18 @@ constexpr int SH_NT = 256;
 constexpr int SH_CAP = 256;
 constexpr int SH_STEPS = 64;
 constexpr int SH_MAX_WARPS = 4;  // window warps an SM up to which the short columns go first
+// and residual columns a window warp from which they do (800 points on the
+// sphere, H2, 5.7 a warp: the call 1079 -> 1142 us with the short ones first; 331
+// x 50, H2, 15.7: 1450 -> 1340)
+constexpr int SH_FEW = 8;
 
 __global__ void __launch_bounds__(SH_NT, 4)
     k_reduce_short(i32 row_base, i64 K, const i32* __restrict__ state, const u64* __restrict__ rec, u64* owner,
                    i32* pool, i64 pool_cap, int chunk, RedCtl* ctl, int* status, int max_steps,
-                   i32* __restrict__ deferred) {
+                   i32* __restrict__ deferred, int few) {
   ph::pdl_wait();
   ph::pdl_trigger();
+  if (ctl->nres < few) return;
   __shared__ i32 lists[SH_NT / 32][2][SH_CAP];
   const int lane = threadIdx.x & 31;
   i32(*list)[SH_CAP] = lists[threadIdx.x >> 5];
@@ -1763,6 +1770,7 @@ int reduce_run(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32
   // pool chunk per warp: small enough that the chunks of all warps fit a quarter of the pool
   const int chunk = (int)std::max<i64>(64, std::min<i64>(2048, pool_cap / (4 * (i64)blocks * warps)) & ~3);
   i32* deferred = nullptr;
+  const int few = SH_FEW * sw * ph::device_sms();
   if (short_first(span)) {
     if (!(deferred = c.take<i32>(K))) return PH_ERR_ARG;
     const i64 short_warps = (i64)ph::device_sms() * 4 * (SH_NT / 32);
@@ -1770,14 +1778,14 @@ int reduce_run(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32
     ph::count_launch();
     ph::launch_pdl(k_reduce_short, dim3((unsigned)std::min<i64>((K + SH_NT - 1) / SH_NT, (i64)ph::device_sms() * 4)),
                    dim3(SH_NT), 0, s, row_base, K, (const i32*)col_state, (const u64*)rec, owner, pool, pool_cap,
-                   short_chunk, ctl, d_status, max_steps, deferred);
+                   short_chunk, ctl, d_status, max_steps, deferred, few);
   }
   ph::count_launch();
   if (sw) {
     const i64 words = window_words(span);
     ph::launch_pdl(k_reduce_shared, dim3(blocks), dim3(32 * sw), sw * rs_warp_words(words) * sizeof(u32), s, row_base,
                    K, (const i32*)col_state, (const u64*)rec, owner, pool, pool_cap, chunk, ctl, d_status, max_steps,
-                   (int)words, (const i32*)deferred);
+                   (int)words, (const i32*)deferred, few);
   } else {
     const i64 dw = dense_words(K, span);
     u32* dense = dw ? c.take<u32>(dw * (i64)blocks * RD_WARPS) : nullptr;
