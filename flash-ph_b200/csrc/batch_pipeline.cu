@@ -591,7 +591,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
     return (int)PH_OK;
   };
   for (int attempt = 0;; ++attempt) {
-    int rc = reduce_only(A, s, links.off, data1, E, 0, R1, (i32)E, span1, skip1, cmf1, pool1, st + 2, r1);
+    int rc = reduce_only(A, s, links.off, data1, E, 0, R1, (i32)E, span1, skip1, cmf1, pool1, attempt > 0, st + 2, r1);
     if (rc == PH_OK)
       rc = ph_batch_persistence_rows(r1.state, r1.piv, E, (i32)E, filt, nullptr, row_m, e_off, K, res->rows[1],
                                      row_off1, nrows1, r1_ws, r1_b, s);
@@ -701,7 +701,7 @@ extern "C" int ph_rips_persistence_batch(const float* const* points, const int64
   i64 pool2 = pool_capacity(4 * R2, T2);
   RedOut r2{};
   for (int attempt = 0;; ++attempt) {
-    int rc = reduce_only(A, s, off2, data2, T2, (i32)E, R2, (i32)(E + T2), span2, skip2, cmf2, pool2, st + 4, r2);
+    int rc = reduce_only(A, s, off2, data2, T2, (i32)E, R2, (i32)(E + T2), span2, skip2, cmf2, pool2, attempt > 0, st + 4, r2);
     if (rc == PH_OK)
       rc = ph_batch_persistence_rows(r2.state, r2.piv, T2, (i32)(E + T2), filt, tri_m, tet_m, t_off, K, res->rows[2],
                                      row_off2, nrows2, r2_ws, r2_b, s);

@@ -41,11 +41,12 @@ void count_launch();
 // The reducer's step cap per column (ph_set_reduce_limits; 2^24 by default)
 // and the cap on a native call's first reduction pool (0: none).
 long long reduce_max_steps();
-// ph_reduce of cofacet lists in any order (reduce.cu)
+// ph_reduce of cofacet lists in any order (reduce.cu); windows_only: all columns
+// by one pass (after an attempt that ran out of its pool)
 int reduce_lists(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32_t col_base, int64_t R,
                  int32_t row_base, int64_t span, const uint8_t* skip, const int32_t* row_cmf, int32_t* col_state,
                  int32_t* col_piv, int32_t* pool, int64_t pool_cap, int64_t* d_info, int* d_status, void* workspace,
-                 size_t workspace_bytes, cudaStream_t s);
+                 size_t workspace_bytes, bool windows_only, cudaStream_t s);
 // flag[row] = 1 for the pivots of the paired columns; map (may be null) takes
 // a reduction's row to the index flagged, negative for none (reduce.cu)
 int mark_pivots_mapped(const int32_t* col_state, const int32_t* col_piv, int64_t K, int32_t row_base,

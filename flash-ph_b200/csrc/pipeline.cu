@@ -223,7 +223,8 @@ i64 pool_capacity(i64 nnz, i64 K) {
 }
 
 int reduce_only(Arena& A, cudaStream_t s, const i32* off, const i32* data, i64 K, i32 col_base, i64 R,
-                i32 row_base, i64 span, const uint8_t* skip, const i32* cmf, i64 pool_cap, int* status, RedOut& o) {
+                i32 row_base, i64 span, const uint8_t* skip, const i32* cmf, i64 pool_cap, bool windows_only, int* status,
+                RedOut& o) {
   o.state = A.take<i32>(K);
   o.piv = A.take<i32>(K);
   o.info = A.take<int64_t>(4);
@@ -233,7 +234,7 @@ int reduce_only(Arena& A, cudaStream_t s, const i32* off, const i32* data, i64 K
   void* rws = A.bytes(rb);
   if (A.failed) return fail(PH_ERR_CUDA, "rips_persistence: device allocation failed");
   return reduce_lists(off, data, K, col_base, R, row_base, span, skip, cmf, o.state, o.piv, pool, pool_cap, o.info,
-                   status, rws, rb, s);
+                   status, rws, rb, windows_only, s);
 }
 
 }  // namespace pl
@@ -286,8 +287,8 @@ __global__ void k_single_seg(ph_cloud_seg* seg, int64_t* blk_off, int64_t n, int
 // one reduction (H1 or H2) and its persistence rows, enqueued
 int reduce_rows(Arena& A, cudaStream_t s, const i32* off, const i32* data, i64 K, i32 col_base, i64 R,
                 i32 row_base, const uint8_t* skip, const i32* cmf, const float* filt, const i32* col_m,
-                const i32* row_m, i64 pool_cap, int* status, float* rows, RedOut& o) {
-  PH_TRY(reduce_only(A, s, off, data, K, col_base, R, row_base, R, skip, cmf, pool_cap, status, o));
+                const i32* row_m, i64 pool_cap, bool windows_only, int* status, float* rows, RedOut& o) {
+  PH_TRY(reduce_only(A, s, off, data, K, col_base, R, row_base, R, skip, cmf, pool_cap, windows_only, status, o));
   const size_t pb = ph_persistence_rows_workspace_bytes(K);
   void* pws = A.bytes(pb);
   if (A.failed) return fail(PH_ERR_CUDA, "rips_persistence: device allocation failed");
@@ -624,7 +625,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   i64 pool1 = pool_capacity(3 * R1, E);
   RedOut r1{};
   for (int attempt = 0;; ++attempt) {
-    int rc = reduce_rows(A, s, links.off, data1, E, 0, R1, (i32)E, mask, cmf1, filt, nullptr, row_m, pool1, st + 2,
+    int rc = reduce_rows(A, s, links.off, data1, E, 0, R1, (i32)E, mask, cmf1, filt, nullptr, row_m, pool1, attempt > 0, st + 2,
                          res->rows[1], r1);
     if (rc != PH_OK) return give_up(rc);
     const int64_t* src[6] = {cnt + 2, r1.nrows, r1.info + 1, cnt + 11, cnt + 12, cnt + 13};
@@ -679,7 +680,7 @@ extern "C" int ph_rips_persistence(const float* d_points, int64_t n, int32_t d, 
   i64 pool2 = pool_capacity(4 * R2, T);
   RedOut r2{};
   for (int attempt = 0;; ++attempt) {
-    int rc = reduce_rows(A, s, off2, data2, T, (i32)E, R2, (i32)(E + T), skip2, cmf2, filt, tri_m, tet_m, pool2,
+    int rc = reduce_rows(A, s, off2, data2, T, (i32)E, R2, (i32)(E + T), skip2, cmf2, filt, tri_m, tet_m, pool2, attempt > 0,
                          st + 4, res->rows[2], r2);
     if (rc != PH_OK) return give_up(rc);
     const int64_t* src[4] = {cnt + 2, cnt + 3, r2.nrows, r2.info + 1};

@@ -179,7 +179,8 @@ struct RedOut {
 // One reduction (H1 or H2) of cofacet lists in any order, enqueued on s; span
 // as ph_reduce takes it.
 int reduce_only(Arena& A, cudaStream_t s, const i32* off, const i32* data, i64 K, i32 col_base, i64 R,
-                i32 row_base, i64 span, const uint8_t* skip, const i32* cmf, i64 pool_cap, int* status, RedOut& o);
+                i32 row_base, i64 span, const uint8_t* skip, const i32* cmf, i64 pool_cap, bool windows_only, int* status,
+                RedOut& o);
 
 // The forest of a batch's union graph: a block a cloud where every cloud fits
 // one (those that it turns out too slow for by the grid then), else

@@ -1517,6 +1517,11 @@ __global__ void __launch_bounds__(32 * RS_MAX_WARPS, 1)
 //     10-D at 12 5123 -> 2264 -> 1336
 //   5 to 8: 60,000 x 20 normal at 10 2736 -> 3004, 200,000 x 10 at 3 841 -> 1191
 //     (as many warps already, and two passes over the columns): not taken
+// Large columns that come last displace smaller ones, which are reduced again,
+// into new records: where that exhausts the pool, the next attempt goes without
+// this pass (72,252 points on the sphere in 16-D at 32 neighbours, a call: 158 ms
+// in windows alone, 212 with this pass in each of two attempts, 182
+// this way; 73,526 in 7-D, where the windows need two attempts too, 100, 134, 79).
 // Fewer steps leave larger columns to go last, whose claims displace the smaller
 // ones: on the sphere in 16-D 52,712 with 16, 26,445 with 32, 23,679 with 128.
 constexpr int SH_NT = 256;
@@ -1731,7 +1736,7 @@ template <bool SORTED>
 int reduce_run(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32_t col_base, int64_t R,
                int32_t row_base, int64_t span, const uint8_t* skip, const int32_t* row_cmf, int32_t* col_state,
                int32_t* col_piv, int32_t* pool, int64_t pool_cap, int64_t* d_info, int* d_status, void* workspace,
-               size_t workspace_bytes, cudaStream_t s) {
+               size_t workspace_bytes, bool windows_only, cudaStream_t s) {
   if (K < 0 || R < 0 || pool_cap < 0) return PH_ERR_ARG;
   if (K >= (int64_t(1) << 31) || R >= (int64_t(1) << 31) || pool_cap >= (int64_t(1) << OW_SHIFT))
     return PH_ERR_OVERFLOW;
@@ -1771,7 +1776,7 @@ int reduce_run(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32
   const int chunk = (int)std::max<i64>(64, std::min<i64>(2048, pool_cap / (4 * (i64)blocks * warps)) & ~3);
   i32* deferred = nullptr;
   const int few = SH_FEW * sw * ph::device_sms();
-  if (short_first(span)) {
+  if (short_first(span) && !windows_only) {
     if (!(deferred = c.take<i32>(K))) return PH_ERR_ARG;
     const i64 short_warps = (i64)ph::device_sms() * 4 * (SH_NT / 32);
     const int short_chunk = (int)(std::max<i64>(64, std::min<i64>(2048, pool_cap / (8 * short_warps))) & ~3);
@@ -1811,15 +1816,15 @@ extern "C" int ph_reduce(const int32_t* cof_off, const int32_t* cof_data, int64_
                          int64_t* d_info, int* d_status, void* workspace, size_t workspace_bytes,
                          void* stream) {
   return reduce_run<true>(cof_off, cof_data, K, col_base, R, row_base, span, skip, row_cmf, col_state, col_piv, pool,
-                          pool_cap, d_info, d_status, workspace, workspace_bytes, (cudaStream_t)stream);
+                          pool_cap, d_info, d_status, workspace, workspace_bytes, false, (cudaStream_t)stream);
 }
 
 int ph::reduce_lists(const int32_t* cof_off, const int32_t* cof_data, int64_t K, int32_t col_base, int64_t R,
                      int32_t row_base, int64_t span, const uint8_t* skip, const int32_t* row_cmf, int32_t* col_state,
                      int32_t* col_piv, int32_t* pool, int64_t pool_cap, int64_t* d_info, int* d_status,
-                     void* workspace, size_t workspace_bytes, cudaStream_t s) {
+                     void* workspace, size_t workspace_bytes, bool windows_only, cudaStream_t s) {
   return reduce_run<false>(cof_off, cof_data, K, col_base, R, row_base, span, skip, row_cmf, col_state, col_piv, pool,
-                           pool_cap, d_info, d_status, workspace, workspace_bytes, s);
+                           pool_cap, d_info, d_status, workspace, workspace_bytes, windows_only, s);
 }
 
 int ph::mark_pivots_mapped(const int32_t* col_state, const int32_t* col_piv, int64_t K, int32_t row_base,
