@@ -723,7 +723,11 @@ def run_precision(args, rank, local):
 def kernel_breakdown(pts, t, max_dim, flush, reps=3):
     """Per-stage device times of the staged pipeline (CUDA events around each
     stage's launches) and of the screened edge kernel alone, plus the sizes
-    the algorithmic byte and flop counts need. Runs outside the timed region."""
+    the algorithmic byte and flop counts need. Runs outside the timed region.
+    The staged pipeline runs the native call's sort, forest and reduction
+    kernels, but every triangle is a row of its reduction (the native call keeps
+    those that can be pivots), its cofacet rows are sorted beforehand, and gaps
+    between the launches of a stage count."""
     import torch
     from flashph_b200 import _timing, rips_persistence
     from flashph_b200.cohomology import enumerate_triangles
@@ -748,12 +752,9 @@ def kernel_breakdown(pts, t, max_dim, flush, reps=3):
     return stages, edge_ms, E, T
 
 
-# DRAM traffic per launch from ncu captures of this workload (profiles/*.md)
-NCU_TRAFFIC = {
-    "k_tc_edges": {"bytes": 2.288e6, "source": "profiles/k_tc_edges_20k_d10.md"},
-    "k_reduce": {"bytes": 0.8535e6, "source": "profiles/k_reduce_20k_d10_h1.md"},
-    "k_cluster_sort": {"bytes": 0.389e6, "source": "profiles/k_cluster_sort_20k_d10.md"},
-}
+# DRAM traffic per launch of this workload's native call, from ncu
+NCU_SOURCE = "profiles/native_call_kernels.md"
+NCU_TRAFFIC = {"k_tc_edges": 2.145e6, "k_reduce_shared": 1.232e6, "k_cluster_sort": 0.409e6}
 
 
 def rooflines(stages, edge_ms, n, d, E, T, pk, src):
@@ -765,8 +766,8 @@ def rooflines(stages, edge_ms, n, d, E, T, pk, src):
     out = {}
     out["edges"] = {"kernel": "k_tc_edges (tensor-core screened edge enumeration, with its 4 prep launches)",
                     "bound": "tensor", "achieved": round(tf, 2), "peak": bf16, "unit": "TFLOP/s",
-                    "frac": round(tf / bf16, 4), "traffic": NCU_TRAFFIC["k_tc_edges"]["bytes"],
-                    "traffic_source": NCU_TRAFFIC["k_tc_edges"]["source"],
+                    "frac": round(tf / bf16, 4), "traffic": NCU_TRAFFIC["k_tc_edges"],
+                    "traffic_source": NCU_SOURCE,
                     "algorithmic_flops_per_launch": mma_flops, "avg_launch_ms": round(edge_ms, 5),
                     "per_unit": "2 x 128 x 128 x 16*ceil((d+4)/16) MMA flops per 128x128 point tile, "
                                 "nt(nt+1)/2 tiles", "peak_source": f"bf16_tflops burst ({src} peaks file)"}
@@ -776,8 +777,8 @@ def rooflines(stages, edge_ms, n, d, E, T, pk, src):
         out["sort"] = {"kernel": "filtration sort (one fused k_cluster_sort launch: packed keys built on load, "
                                  "8 digit passes, edges rebuilt on store)", "bound": "hbm",
                        "achieved": round(gbs, 2), "peak": hbm, "unit": "GB/s", "frac": round(gbs / hbm, 5),
-                       "traffic": NCU_TRAFFIC["k_cluster_sort"]["bytes"],
-                       "traffic_source": NCU_TRAFFIC["k_cluster_sort"]["source"],
+                       "traffic": NCU_TRAFFIC["k_cluster_sort"],
+                       "traffic_source": NCU_SOURCE,
                        "traffic_note": "the fused filtration sort's launch: the 12 bytes per edge are read "
                                        "once, the passes stay in distributed shared memory",
                        "algorithmic_bytes_per_launch": byts,
@@ -787,15 +788,17 @@ def rooflines(stages, edge_ms, n, d, E, T, pk, src):
     if "h1.reduce" in stages:
         byts = 4.0 * (E + 1) + 4.0 * 3 * T + 4.0 * T + 1.0 * E + 8.0 * E + 8.0 * T
         gbs = byts / (stages["h1.reduce"] * 1e-3) / 1e9
-        out["h1.reduce"] = {"kernel": "k_reduce (H1, with classify/finish/rows)", "bound": "hbm",
+        out["h1.reduce"] = {"kernel": "k_reduce_shared (H1, staged: all triangles as rows, with classify/finish/rows)",
+                            "bound": "hbm",
                             "achieved": round(gbs, 3), "peak": hbm, "unit": "GB/s", "frac": round(gbs / hbm, 6),
-                            "traffic": NCU_TRAFFIC["k_reduce"]["bytes"],
-                            "traffic_source": NCU_TRAFFIC["k_reduce"]["source"],
+                            "traffic": NCU_TRAFFIC["k_reduce_shared"],
+                            "traffic_source": NCU_SOURCE,
                             "algorithmic_bytes_per_launch": byts, "avg_launch_ms": round(stages["h1.reduce"], 5),
                             "per_unit": "cofacet CSR (4 B per offset and entry), cmf 4 B and owner word 8 B per "
                                         "triangle, mask 1 B and state/pivot 8 B per edge",
-                            "note": "latency-bound: the reduction is a chain of dependent column additions "
-                                    "(the oracle's critical path), not a bandwidth problem",
+                            "note": "latency-bound: the reduction is a chain of dependent rounds of column "
+                                    "additions, not a bandwidth problem; the native call's H1 reduction has fewer "
+                                    "rows (the traffic is its launch's)",
                             "peak_source": f"hbm_gbs ({src} peaks file)"}
     return out
 
@@ -820,13 +823,17 @@ def l2_hop_ns(dev, mib=64, hops=200_000, seed=3):
 
 def latency_roofline(stage_ms, crit_path, hop_ns):
     """The H1 reduction against its latency bound: the oracle's critical path
-    (the longest chain of dependent column additions) times two dependent L2
-    loads per addition (the pivot's owner word, then the owning record)."""
-    min_ms = crit_path * 2 * hop_ns * 1e-6
-    return {"kernel": "k_reduce (H1, with classify/finish/rows)", "bound": "latency",
-            "crit_path": int(crit_path), "dependent_l2_loads_per_step": 2, "l2_hop_ns": round(hop_ns, 1),
+    (the longest chain of dependent column additions) in rounds of up to 32
+    additions, times two dependent L2 loads per round (the entries' owner words,
+    then the owning records)."""
+    rounds = -(-int(crit_path) // 32)
+    min_ms = rounds * 2 * hop_ns * 1e-6
+    return {"kernel": "k_reduce_shared (H1, staged, with classify/finish/rows)", "bound": "latency",
+            "crit_path": int(crit_path), "additions_per_round": 32, "min_rounds": rounds,
+            "dependent_l2_loads_per_round": 2, "l2_hop_ns": round(hop_ns, 1),
             "min_ms": round(min_ms, 4), "achieved_ms": round(stage_ms, 4), "frac": round(min_ms / stage_ms, 4),
-            "per_unit": "crit_path x 2 x measured dependent L2 load latency (one-thread pointer chase, 64 MiB)"}
+            "per_unit": "ceil(crit_path / 32) x 2 x measured dependent L2 load latency (one-thread pointer chase, "
+                        "64 MiB)"}
 
 
 def dist_setup():

@@ -79,8 +79,8 @@ struct Graph {
   i32 row;                       // bytes of a table row (n <= 16384)
 
   // The rank at (x, w), col the address of (0, w): one multiply-add and a load.
-  // The passes over links are bound by instruction issue (66% of the slots,
-  // 960 a dense edge, at 14% L1 and 97% L2 hits), not by the table's bytes.
+  // The passes over links are bound by instruction issue (64% of the slots,
+  // 770 a dense edge, at 15% L1 and 96% L2 hits), not by the table's bytes.
   // Index arithmetic in 64 bits and single list loads -> this: 1501 points in
   // 8 dimensions 217 -> 202 us, tetrahedra of 331 in 50 214 -> 193 us.
   __device__ __forceinline__ const char* col(i32 w) const { return tab + 4 * (i64)w; }

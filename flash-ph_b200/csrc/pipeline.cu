@@ -253,8 +253,14 @@ namespace {
 //    36-157; past n^2 (d + 8) = 5e8 the screen wins on sparse clouds (8000 x 10
 //    76 against 37 us) and the dense ones come to equal (20,000 x 10 507, 534);
 //  * blocks in grid order (edges_near) for larger clouds of up to four
-//    dimensions;
-//  * the tensor-core screen for the others.
+//    dimensions. The grid spans the finite points' box: a point far away leaves
+//    the others in few cells, and all pairs are looked at (50,000 x 3, H0, a
+//    call: direct 2482, 590 in grid order, with one point at 1000 times the
+//    spread 2001);
+//  * the tensor-core screen for the others, from five dimensions on. Calls with
+//    the direct kernel and this one, us: 20,000 x 5, 6 and 7 sparse 635, 624,
+//    633 -> 341, 321, 311, with 4M to 5M edges (H0) 1531, 1511, 1578 -> 584, 556,
+//    563; just past the line, 6500 points, 552 and 372 -> 368 and 287.
 enum class EdgeKernel { direct, screened, nearby };
 
 EdgeKernel edge_kernel(i64 n, int d, int edge_mode) {

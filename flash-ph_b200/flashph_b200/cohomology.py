@@ -136,8 +136,8 @@ _POOL_MAX = (1 << 33) - 1
 
 
 def pool_capacity(nnz: int, K: int) -> int:
-    """Initial reduction pool (int32 entries): the initial records (at most
-    2 nnz), per-warp chunks and the reduced columns; generous for small
+    """Initial reduction pool (int32 entries): the initial records (their
+    entries and up to four more a column), per-warp chunks and the reduced columns; generous for small
     problems, where a retry would cost more than the memory, and bounded by
     the record-offset range."""
     mult = 8 if nnz < (1 << 24) else 3

@@ -343,7 +343,9 @@ int ph_cof_max_face(const int32_t* faces_aos, const int32_t* f0, const int32_t* 
  * (cohomology_general.py:202-371).
  * col_state[c]: 0 skipped, 1 apparent, 2 reduced to a pivot, 3 essential.
  * col_piv[c]: pivot global rank (states 1 and 2) or -1.
- * pool: scratch for reduced columns, pool_cap int32 entries.
+ * pool: scratch for reduced columns, pool_cap int32 entries: the initial
+ * records, each a column's length and entries at a multiple of four, and
+ * room for the columns reduced.
  * span: the most rows one column's entries can span (its rows all lie in a
  * range of span consecutive ranks: in a batch, the largest row count of one
  * cloud); 0 or R for a single cloud. Working columns that become bitmaps
@@ -381,7 +383,7 @@ int ph_persistence_rows(const int32_t* col_state, const int32_t* col_piv, int64_
 /* rips_persistence for one cloud, every stage on `stream`: points (device,
  * n x d float32, n >= 2), max_edge_length (edges keep dist^2 <
  * fp32(max_edge_length^2)), max_dim 0..2, the reference's max_triangles /
- * max_tetrahedra limits, edge_mode 0 (tensor-core screen when 8 <= d <= 252),
+ * max_tetrahedra limits, edge_mode 0 (the fastest of three edge kernels by n and d),
  * 1 (screen), 2 (direct kernel). On success *out holds the diagrams on the
  * device; read them with ph_result_rows / ph_result_copy and release with
  * ph_result_free. A limit exceeded returns PH_ERR_LIMIT with the reference's
